@@ -35,6 +35,10 @@ extern "C" {
 #define INTFA_OUT_FP16 0             /* o as fp16: the Triton ops (flash_atten_full_int8.py:194-195) */
 #define INTFA_OUT_BF16 1             /* o as bf16: csrc/flash_fwd_hdim128_bf16_sm80_{full,half}_qi8.cu */
 
+#define INTFA_SCALE_F16_Q 1
+#define INTFA_SCALE_F16_K 2
+#define INTFA_SCALE_F16_V 4
+
 #define INTFA_VSCALE_PER_TENSOR  0   /* one V scale per (batch, head): benchmark.py:102-107 */
 #define INTFA_VSCALE_PER_CHANNEL 1   /* one V scale per (batch, head, channel)              */
 
@@ -53,19 +57,17 @@ int intfa_last_error(char* buf, size_t len);
  * Tensors are [B, H, N, D]; strides are in ELEMENTS for dims (B, H, N); the last
  * dim must be contiguous.  q,k: int8.  v: int8 (FULL) or fp16 (HALF).  o: fp16.
  * Byte strides of q/k/v and their base pointers must be multiples of 16 (TMA).
- * q_scale [B,H,Nq], k_scale [B,H,Nk]: fp32, contiguous over N, strides for (B,H).
- * v_scale (FULL only): fp32, element strides for (B,H,D); stride 0 over D
+ * q_scale [B,H,Nq], k_scale [B,H,Nk]: fp32 or fp16 (scale_f16), contiguous over N, strides for (B,H).
+ * v_scale (FULL only): fp32 or fp16, element strides for (B,H,D); stride 0 over D
  * broadcasts a per-(batch,head) scale.
  */
 typedef struct IntfaFwdParams {
   const void*  q;  const void* k;  const void* v;  void* o;
-  const float* q_scale;  const float* k_scale;  const float* v_scale;
+  const void* q_scale;  const void* k_scale;  const void* v_scale;
   int64_t q_stride[3];  int64_t k_stride[3];  int64_t v_stride[3];  int64_t o_stride[3];
   int64_t qs_stride[2]; int64_t ks_stride[2]; int64_t vs_stride[3];
   int32_t B, H, Nq, Nk, D;      /* D in {16,32,64,128,256} (flash_atten_full_int8.py:193).  Nq, Nk need not be multiples of the tile sizes (128 rows, G
-                                   columns): the last tiles are masked (csrc/mask.h:277-285); but every row of
-                                   k_scale must be ALLOCATED up to the next multiple of G floats (the values past
-                                   Nk are ignored) -- the scales of a KV step are fetched G at a time */
+                                   columns): the last tiles are masked (csrc/mask.h:277-285) */
   int32_t variant;              /* INTFA_VARIANT_* */
   int32_t causal;               /* 0/1; mask is (kv_offset + col) <= (q_offset + row) */
   float   sm_scale;             /* natural-log softmax scale; kernel multiplies by 1.44269504 */
@@ -106,6 +108,9 @@ typedef struct IntfaFwdParams {
      out the K tile of the n-th KV step the CTA runs, so the wait for it runs out, the CTA drains and `status`
      receives the wait's code -- the path a lost transfer would take. */
   int32_t debug_wait_limit_kcycles; int32_t debug_skip_k_load;
+  int32_t scale_f16;            /* bit set: that scale tensor is fp16 (as benchmark.py makes them), else fp32.
+                                   INTFA_SCALE_F16_Q / _K / _V; the kernel widens in place
+                                   (flash_atten_full_int8.py:37-38) */
 } IntfaFwdParams;
 
 /*

@@ -12,6 +12,7 @@ OK = 0
 ERR_INVALID_ARG, ERR_UNSUPPORTED, ERR_CUDA, ERR_DEVICE_WAIT, ERR_TOO_LARGE = -1, -2, -3, -4, -5
 VARIANT_FULL, VARIANT_HALF, VARIANT_HALF_FP8 = 0, 1, 2
 VSCALE_PER_TENSOR, VSCALE_PER_CHANNEL = 0, 1
+SCALE_F16_Q, SCALE_F16_K, SCALE_F16_V = 1, 2, 4
 
 EXPORTS = ("intfa_version", "intfa_last_error", "intfa_fwd", "intfa_quant_pertoken",
            "intfa_quant_v_workspace_bytes", "intfa_quant_v", "intfa_quant_qkv_workspace_bytes", "intfa_quant_qkv",
@@ -43,6 +44,7 @@ class IntfaFwdParams(ctypes.Structure):
         ("H_kv", ctypes.c_int32), ("o_dtype", ctypes.c_int32),
         ("kv_order", ctypes.c_int32), ("vs_stride_blk", ctypes.c_int64),
         ("debug_wait_limit_kcycles", ctypes.c_int32), ("debug_skip_k_load", ctypes.c_int32),
+        ("scale_f16", ctypes.c_int32),
     ]
 
 

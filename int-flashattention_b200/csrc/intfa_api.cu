@@ -90,15 +90,6 @@ int intfa_fwd(const IntfaFwdParams* p, void* stream) {
   if ((rc = check_tma_tensor("k", p->k, p->k_stride, 1))) return rc;
   if ((rc = check_tma_tensor("v", p->v, p->v_stride, p->variant == INTFA_VARIANT_HALF ? 2 : 1))) return rc;
   if (!p->q_scale || !p->k_scale) return set_error(INTFA_ERR_INVALID_ARG, "q_scale / k_scale is NULL");
-  if (!aligned16(p->k_scale) || p->ks_stride[0] % 4 != 0 || p->ks_stride[1] % 4 != 0)
-    return set_error(INTFA_ERR_INVALID_ARG, "k_scale must be 16-byte aligned with (B,H) strides that are multiples of 4");
-  {
-    // the K scales of a KV step are fetched G at a time: every row must have room up to the next multiple of G
-    const long long need = ((long long)p->Nk + p->G - 1) / p->G * p->G;
-    const int hk = p->H_kv > 0 ? p->H_kv : p->H;
-    if ((hk > 1 && p->ks_stride[1] < need) || (p->B > 1 && p->ks_stride[0] < need))
-      return set_error(INTFA_ERR_INVALID_ARG, "k_scale rows must be allocated up to the next multiple of G (%lld floats for Nk=%d)", need, p->Nk);
-  }
   if (full && !p->v_scale) return set_error(INTFA_ERR_INVALID_ARG, "v_scale is NULL (full-int8)");
   if (p->kv_order != 0 && p->kv_order != 1) return set_error(INTFA_ERR_INVALID_ARG, "kv_order must be 0 (ascending) or 1 (descending)");
   if (p->vs_stride_blk < 0) return set_error(INTFA_ERR_INVALID_ARG, "vs_stride_blk must not be negative");

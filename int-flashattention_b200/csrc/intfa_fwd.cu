@@ -53,6 +53,11 @@ __device__ __forceinline__ uint32_t pack_out(float x, float y, int bf16) {
   return *reinterpret_cast<const uint32_t*>(&h);
 }
 
+// element i of a scale tensor, widened to fp32 (flash_atten_full_int8.py:37-38 promotes in the kernel too)
+__device__ __forceinline__ float ld_scale(const void* s, long long i, int f16) {
+  return f16 ? __half2float(static_cast<const __half*>(s)[i]) : static_cast<const float*>(s)[i];
+}
+
 struct TileInfo {
   int bh, b, h, hk, mb, work, nsteps;   // hk: the K/V head this query head reads (grouped-query attention)
   int vh;                               // which D-wide slice of the V / output channels this pass covers (head dim 256: 0, 1)
@@ -119,15 +124,15 @@ static EncodeTiledFn get_encode_fn() {
   return fn;
 }
 
-// Work-item counters of the launches in flight: a ring of words inside the library image (no allocation at launch
-// time); each launch takes the next word and zeroes it on its stream.  A word comes round again after kTileCounters
-// launches of the process (all devices and streams share the cursor): a launch that is still queued or running
-// by then would have its counter zeroed under it, so at most kTileCounters launches may be in flight at a time.
+// Work-item counters of the launches in flight: a ring of word pairs inside the library image (no allocation at launch
+// time); each launch takes the next pair, which is zero and which its last CTA leaves zero again (a memset in front of
+// every launch cost 1 to 2 us of device time).  A pair comes round again after kTileCounters launches of the process
+// (all devices and streams share the cursor), so at most kTileCounters launches may be in flight at a time.
 // The per-device caches below are atomics: host threads may call into the library concurrently.
 constexpr int kTileCounters = 4096;
-__device__ static unsigned int g_tile_counters[kTileCounters];
+__device__ static unsigned int g_tile_counters[2 * kTileCounters];
 
-static int next_tile_counter(unsigned int** out, cudaStream_t stream) {
+static int next_tile_counter(unsigned int** out) {
   static std::atomic<unsigned int*> base[64];
   static std::atomic<unsigned int> next{0};
   int dev = 0;
@@ -140,10 +145,7 @@ static int next_tile_counter(unsigned int** out, cudaStream_t stream) {
     b = static_cast<unsigned int*>(sym);
     base[dev].store(b, std::memory_order_release);       // every thread computes the same address
   }
-  unsigned int* c = b + (next.fetch_add(1) % kTileCounters);
-  cudaError_t e = cudaMemsetAsync(c, 0, sizeof(unsigned int), stream);
-  if (e != cudaSuccess) return set_error(INTFA_ERR_CUDA, "cudaMemsetAsync(tile counter): %s", cudaGetErrorString(e));
-  *out = c;
+  *out = b + 2 * (next.fetch_add(1) % kTileCounters);
   return INTFA_OK;
 }
 
@@ -201,7 +203,8 @@ static int launch_pipe(const IntfaFwdParams* a, const KParams& kp, cudaStream_t 
   int grid = sms;
   if (grid > kp.num_tiles) grid = kp.num_tiles;
   KParams kpl = kp;
-  if ((rc = next_tile_counter(&kpl.tile_counter, stream))) return rc;
+  kpl.tile_counter = nullptr;
+  if (kp.num_tiles > grid && (rc = next_tile_counter(&kpl.tile_counter))) return rc;
   kern<<<grid, kPipeThreads, C::SMEM_BYTES, stream>>>(tmQ, tmK, tmV, kpl);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return set_error(INTFA_ERR_CUDA, "kernel launch: %s", cudaGetErrorString(e));
@@ -211,6 +214,7 @@ static int launch_pipe(const IntfaFwdParams* a, const KParams& kp, cudaStream_t 
 int fwd_dispatch(const IntfaFwdParams* a, cudaStream_t stream) {
   KParams kp;
   kp.qs = a->q_scale; kp.ks = a->k_scale; kp.vs = a->v_scale;
+  kp.scale_f16 = a->scale_f16;
   kp.o = reinterpret_cast<__half*>(a->o);
   kp.o_sb = a->o_stride[0]; kp.o_sh = a->o_stride[1]; kp.o_sn = a->o_stride[2];
   kp.qs_sb = a->qs_stride[0]; kp.qs_sh = a->qs_stride[1];

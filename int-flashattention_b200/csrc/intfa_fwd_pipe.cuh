@@ -2,11 +2,11 @@
 // (Included by intfa_fwd.cu inside namespace intfa, after the shared helpers.)
 //
 // 512 threads:
-//   warp 0        TMA producer (Q once per work item; K and V through rings of shared-memory stages, the K-scale
-//                 slices through a ring of their own); it also draws the work items from the global counter
+//   warp 0        TMA producer (Q once per work item; K and V through rings of shared-memory stages); it also draws
+//                 the work items: the CTA's own index first, then from a global counter
 //   warp 1        MMA issuer for S = Q K^T (whole warp runs the loop, one elected lane issues): up to three KV steps
 //                 ahead of the softmax groups, into S buffer (step mod 3)
-//   warp 2        TMEM allocator
+//   warp 2        TMEM allocator; then loads the K scales (fp32 or fp16, rows of any alignment) into a ring of their own
 //   warp 3        MMA issuer for O_j = P V
 //   warps 4-7     softmax group 0, warps 8-11 softmax group 1: one thread per query row.  The groups take
 //                 ALTERNATE KV steps (group g owns the steps whose running index is g mod 2), each with its own
@@ -69,9 +69,11 @@ struct PipeCfg {
   // for 128-column KV steps, where it measured +2..5 % on causal workloads; with 64-column steps its code costs the
   // non-causal case more (instruction cache) than it gives.
   static constexpr bool BAND_FAST = G == 128;
-  // instructions of never-executed filler between the softmax passes (see intfa_fwd_pipe_softmax.inc): 4 KB with the
-  // band path compiled in, else 2 KB, and none for full-int8 at head dim 64 -- each the best of a sweep
-  static constexpr int CODE_FILLER = BAND_FAST ? 256 : (FULL && D == 64) ? 0 : 128;
+  // instructions of never-executed filler between the softmax passes (see intfa_fwd_pipe_softmax.inc), the best of a sweep in
+  // steps of 1 KB for each kind of instantiation (`ragged`: the one that masks partial tiles).  With explicit shared-memory
+  // accesses it matters less than it did: +-1.5 % non-causal, +-4 % causal; the ragged one 294 us (256) to 343 us (0) at
+  // batch 2, 32/8 heads, 3001 tokens, causal.
+  static constexpr int code_filler_of(bool ragged) { return ragged ? 256 : BAND_FAST ? (FULL ? 448 : 384) : (FULL && D == 64) ? 0 : 128; }
   static constexpr bool MORE_SOFTMAX_REGS = !FULL || G == 128;
   static constexpr int SOFTMAX_REGS = MORE_SOFTMAX_REGS ? 152 : 136;
   static constexpr int CORR_REGS = MORE_SOFTMAX_REGS ? 168 : 184;
@@ -132,7 +134,8 @@ intfa_fwd_pipe_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
   using C = PipeCfg<D, G, FULL, DQ, F8V>;
   constexpr int NSK = C::NSK, NSV = C::NSV, NSB = C::NSB, NVH = C::NVH;
   extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  // (rounded up by an offset, not through an integer: the compiler then knows that all this is shared memory)
+  uint8_t* smem = smem_raw + ((0u - smem_u32(smem_raw)) & 1023u);
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
 
@@ -174,7 +177,7 @@ intfa_fwd_pipe_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
     mbar_init(BAR(B_OFULL), 1);
     mbar_init(BAR(B_OFREE), 4);
     for (int s = 0; s < NSK; ++s) {
-      mbar_init(BAR(B_KFULL + s), 1);
+      mbar_init(BAR(B_KFULL + s), 2);         // the producer's K tile and the scale loader's K scales
       mbar_init(BAR(B_KEMPTY + s), 1);
     }
     for (int s = 0; s < NSV; ++s) {
@@ -187,7 +190,7 @@ intfa_fwd_pipe_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
     }
     for (int i = 0; i < 4; ++i) {
       mbar_init(BAR(B_TILE + i), 1);
-      mbar_init(BAR(B_TDONE + i), 14);       // 2 MMA warps + 8 softmax warps + 4 accumulator warps
+      mbar_init(BAR(B_TDONE + i), 15);       // 2 MMA warps, the scale loader, 8 softmax warps, 4 accumulator warps
       mbar_init(BAR(B_AFULL + i), 4);
     }
     abort_flag[0] = 0;
@@ -211,7 +214,6 @@ intfa_fwd_pipe_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
   const uint32_t sK = smem_u32(smem + C::OFF_K);
   const uint32_t sV = smem_u32(smem + C::OFF_V);
   const uint32_t sP = smem_u32(smem + C::OFF_P);
-  const uint32_t sKS = smem_u32(smem + C::OFF_KS);
 
   // The int32 accumulator tiles start every KV step from the bit pattern of 1.5*2^23 (see kMagicI).  It is
   // written by the tensor core itself: an fp16 MMA (K = 16, no accumulate) of a constant operand with
@@ -260,7 +262,11 @@ intfa_fwd_pipe_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
           tile = drawn * NVH + (NVH - passes_left);      // the next pass over the same query tile, on this CTA
           --passes_left;
         } else {
-          tile = (int)atomicAdd(p.tile_counter, 1u);
+          if (tseq == 0) {
+            tile = (int)blockIdx.x;
+          } else {
+            tile = p.tile_counter ? (int)(gridDim.x + atomicAdd(p.tile_counter, 1u)) : p.num_tiles;
+          }
           if (tile >= p.num_tiles) {
             tile = -1;
           } else if (NVH > 1) {
@@ -281,18 +287,16 @@ intfa_fwd_pipe_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
 #pragma unroll
         for (int pn = 0; pn < C::QK_PANELS; ++pn)
           tma_load_4d(sQ + pn * (kBM * C::QK_ROWB), &tmQ, BAR(B_QFULL), pn * C::QK_ROWB, t.mb * kBM, t.h, t.b);
-        const float* ks_row = p.ks + (long long)t.b * p.ks_sb + (long long)t.hk * p.ks_sh;
         for (int j = 0; j < t.nsteps; ++j, ++kv_it) {
           const uint32_t s = kv_it % NSK, ph = (kv_it / NSK) & 1;
           ok = mbar_wait(BAR(B_KEMPTY + s), ph ^ 1, abort_flag, p.status, code_hi | PW_KE);
           if (!ok) break;
           const int jb = kv_tile_of_step(p, j, t.nsteps);
           if (p.skip_k_load == 0 || kv_it + 1 != (uint32_t)p.skip_k_load) {      // (test hook: a K tile that never arrives)
-            mbar_expect_tx(BAR(B_KFULL + s), C::K_BYTES + C::KS_BYTES);
+            mbar_expect_tx(BAR(B_KFULL + s), C::K_BYTES);
 #pragma unroll
             for (int pn = 0; pn < C::QK_PANELS; ++pn)
               tma_load_4d(sK + s * C::K_BYTES + pn * (G * C::QK_ROWB), &tmK, BAR(B_KFULL + s), pn * C::QK_ROWB, jb * G, t.hk, t.b);
-            bulk_load_1d(sKS + (kv_it % C::NKS) * C::KS_BYTES, ks_row + jb * G, C::KS_BYTES, BAR(B_KFULL + s));
           }
           const uint32_t sv = kv_it % NSV, phv = (kv_it / NSV) & 1;
           ok = mbar_wait(BAR(B_VEMPTY + sv), phv ^ 1, abort_flag, p.status, code_hi | PW_VE);
@@ -307,6 +311,47 @@ intfa_fwd_pipe_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
           }
         }
         ++tile_it;
+      }
+      // The last CTA to get here leaves the counter words zero for the next launch that is given them.
+      if (p.tile_counter && atomicAdd(p.tile_counter + 1, 1u) + 1u == gridDim.x) {
+        p.tile_counter[0] = 0u;
+        p.tile_counter[1] = 0u;
+      }
+    }
+    __syncwarp();
+  } else if (warp == 2) {
+    // -------------------------------------------------------------------- K scales
+    // The scales of KV step it go into slot it mod NKS together with the K tile (same K_EMPTY wait, second arrival on
+    // K_FULL).  Plain loads, one step ahead of the wait: rows may start anywhere (a cache of odd length) and hold fp16 or
+    // fp32; columns past Nk read as zero.
+    uint32_t kv_it = 0, tseq = 0;
+    bool ok = true;
+#pragma unroll 1
+    while (ok) {
+      const int tile = next_tile(tseq, lane == 0, true);
+      if (tile < 0) break;
+      const TileInfo t = decode_tile<RAGGED, NVH>(p, tile, G);
+      const long long row = (long long)t.b * p.ks_sb + (long long)t.hk * p.ks_sh;
+      float ks[G / 32];
+#pragma unroll 1
+      for (int j = -1; j < t.nsteps; ++j) {
+        if (j >= 0) {
+          const uint32_t s = kv_it % NSK, ph = (kv_it / NSK) & 1;
+          ok = mbar_wait_warp(BAR(B_KEMPTY + s), ph ^ 1, abort_flag, p.status, code_hi | PW_KE);
+          if (!ok) break;
+          float* slot = reinterpret_cast<float*>(smem + C::OFF_KS + (kv_it % C::NKS) * C::KS_BYTES) + lane;
+#pragma unroll
+          for (int i = 0; i < G / 32; ++i) slot[32 * i] = ks[i];
+          __syncwarp();
+          if (lane == 0) mbar_arrive(BAR(B_KFULL + s));
+          ++kv_it;
+        }
+        if (j + 1 < t.nsteps) {
+          const int col0 = kv_tile_of_step(p, j + 1, t.nsteps) * G + lane;
+#pragma unroll
+          for (int i = 0; i < G / 32; ++i)
+            ks[i] = !RAGGED || col0 + 32 * i < p.Nk ? ld_scale(p.ks, row + col0 + 32 * i, p.scale_f16 & INTFA_SCALE_F16_K) : 0.f;
+        }
       }
     }
     __syncwarp();

@@ -10,7 +10,8 @@ namespace intfa {
 
 // Arguments of the attention kernel (plain data, passed by value).
 struct KParams {
-  const float* qs; const float* ks; const float* vs;
+  const void* qs; const void* ks; const void* vs;   // fp32, or fp16 where scale_f16 says so
+  int scale_f16;                 // INTFA_SCALE_F16_* bits
   __half* o;
   long long o_sb, o_sh, o_sn;
   long long qs_sb, qs_sh, ks_sb, ks_sh, vs_sb, vs_sh, vs_sd;
@@ -31,7 +32,8 @@ struct KParams {
   int skip_k_load;               // test hook: 1-based KV step whose K tile the producer leaves out; 0: none
   int kv_desc;                   // 1: KV tiles visited last-to-first
   long long vs_sblk;             // element stride of the KV-tile axis of v_scale; 0: one scale row per (batch, head)
-  unsigned int* tile_counter;    // zeroed word the CTAs draw work-item indices from
+  unsigned int* tile_counter;    // {next work item beyond the first of every CTA, CTAs that are done}, both zero
+                                 // between launches; null when every CTA has one work item at most
 };
 
 // Records the calling thread's last error (printf-style) and returns `code`.

@@ -65,34 +65,20 @@ __device__ __forceinline__ uint32_t mbar_try_wait_parked(uint32_t bar, uint32_t 
 // drains and exits.
 constexpr uint32_t kParkNs = 20000;                 // longest single park; bounds how late an abort is seen
 
-// The abort flag and the clock are looked at every 64th poll only: the poll loop itself stays a
-// handful of instructions.
-// kSleepNs > 0: sleep that long between polls, so that a polling service warp leaves the issue
-// slots of its scheduler to the warps that compute.
-template <int kSleepNs>
-__device__ __forceinline__ bool mbar_wait_slow(uint32_t bar, uint32_t parity, volatile int* abort_flag, int* status, int code) {
-  long long t0 = 0;
-  uint32_t polls = 0;
-  while (true) {
-    if (kSleepNs > 0) __nanosleep(kSleepNs);
-    if (mbar_try_wait_parked(bar, parity, kParkNs)) return true;
-    if ((++polls & 63u) == 0u) {
-      if (*abort_flag) return false;
-      const long long now = clock64();
-      if (t0 == 0) t0 = now;
-      if (now - t0 > ((long long)abort_flag[1] << 10)) {
-        *abort_flag = 1;
-        if (status) atomicCAS(status, 0, code);
-        return false;
-      }
-    }
-  }
-}
-template <int kSleepNs = 0>
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag,
-                                          int* status, int code) {
+// (The slow path is small: there is one copy of it at every wait, and the instruction cache has to hold the loops of all
+// warp roles at once.)
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag, int* status, int code) {
   if (mbar_try_wait(bar, parity)) return true;
-  return mbar_wait_slow<kSleepNs>(bar, parity, abort_flag, status, code);
+  const uint32_t t0 = (uint32_t)(clock64() >> 10);
+#pragma unroll 1
+  while (!mbar_try_wait_parked(bar, parity, kParkNs)) {
+    if ((int)((uint32_t)(clock64() >> 10) - t0) > abort_flag[1]) {
+      *abort_flag = 1;
+      if (status) atomicCAS(status, 0, code);
+    }
+    if (*abort_flag) return false;
+  }
+  return true;
 }
 
 // The same wait made by a whole converged warp, with one verdict for all its lanes.
@@ -123,13 +109,6 @@ __device__ __forceinline__ void tma_load_4d(uint32_t dst, const void* tmap, uint
       "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes"
       " [%0], [%1, {%3, %4, %5, %6}], [%2];"
       ::"r"(dst), "l"(tmap), "r"(bar), "r"(c0), "r"(c1), "r"(c2), "r"(c3)
-      : "memory");
-}
-// plain 1-D bulk copy global -> shared; both addresses 16-byte aligned, bytes % 16 == 0
-__device__ __forceinline__ void bulk_load_1d(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
-  asm volatile(
-      "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-      ::"r"(dst), "l"(src), "r"(bytes), "r"(bar)
       : "memory");
 }
 __device__ __forceinline__ void prefetch_tmap(const void* tmap) {

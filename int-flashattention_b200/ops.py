@@ -72,19 +72,9 @@ def _prep_main(t):
     return t if _tma_ok(t) else t.contiguous()
 
 
-def _scales_f32(s):
-    """[B,H,N] scale -> fp32 contiguous (fp16 as benchmark.py makes it is widened by the library)."""
-    if s.dtype == torch.float32:
-        if s.is_contiguous():
-            return s if s.data_ptr() % 16 == 0 else s.clone()
-        return s.contiguous()
-    if s.dtype == torch.float16:
-        src = s.contiguous()
-        dst = torch.empty(src.shape, dtype=torch.float32, device=s.device)
-        with torch.cuda.device(s.device):      # the library launches on the current device
-            _lib.check(_lib.load().intfa_scales_f16_to_f32(src.data_ptr(), dst.data_ptr(), src.numel(), _stream(s)))
-        return dst
-    return s.to(torch.float32).contiguous()
+def _scales(s):
+    """Scales as the kernel reads them: fp32 or fp16 (what benchmark.py makes), contiguous over the last dim."""
+    return s.contiguous() if s.dtype in (torch.float32, torch.float16) else s.to(torch.float32).contiguous()
 
 
 def _fwd(variant, q, k, v, q_scale, k_scale, v_scale, causal, sm_scale, *, G=None, p_round="triton", kv_order="ascending",
@@ -114,12 +104,7 @@ def _fwd(variant, q, k, v, q_scale, k_scale, v_scale, causal, sm_scale, *, G=Non
     if G is None:
         G = default_G(D, variant)
     q, k, v = _prep_main(q), _prep_main(k), _prep_main(v)
-    qs, ks = _scales_f32(q_scale), _scales_f32(k_scale)
-    if Nk % G:
-        # the kernel fetches the K scales of a KV step G at a time: give every row room up to the next multiple of G
-        ks_pad = torch.zeros(ks.shape[:2] + ((Nk + G - 1) // G * G,), dtype=torch.float32, device=ks.device)
-        ks_pad[:, :, :Nk] = ks
-        ks = ks_pad
+    qs, ks = _scales(q_scale), _scales(k_scale)
     o = torch.empty((B, H, Nq, D) if write_o else (1, 1, 1, 8), dtype=out_dtype, device=q.device)  # :194-195
 
     P = _lib.IntfaFwdParams()
@@ -131,17 +116,16 @@ def _fwd(variant, q, k, v, q_scale, k_scale, v_scale, causal, sm_scale, *, G=Non
     P.o_stride = _lib._i64x3(*o.stride()[:3])
     P.qs_stride = _lib._i64x2(*qs.stride()[:2])
     P.ks_stride = _lib._i64x2(*ks.stride()[:2])
+    P.scale_f16 = (_lib.SCALE_F16_Q if qs.dtype == torch.float16 else 0) | (_lib.SCALE_F16_K if ks.dtype == torch.float16 else 0)
     keep = [q, k, v, qs, ks, o]
     if full:
-        vs = v_scale.to(torch.float32)
+        vs = _scales(v_scale)
+        P.scale_f16 |= _lib.SCALE_F16_V if vs.dtype == torch.float16 else 0
         if vs.dim() == 2:                      # (B,H): one scale per (batch, head), benchmark.py:102-107
-            vs = vs.contiguous()
             P.vs_stride = _lib._i64x3(vs.stride(0), vs.stride(1), 0)
         elif vs.dim() == 3:                    # (B,H,D): per channel
-            vs = vs.contiguous()
             P.vs_stride = _lib._i64x3(*vs.stride())
         elif vs.dim() == 4:                    # (B,H,ceil(Nk/G),D): one row per KV tile, the CUDA path's layout
-            vs = vs.contiguous()
             if vs.shape[2] != (Nk + G - 1) // G:
                 raise ValueError("per-tile v_scale needs ceil(Nk/G) = %d rows, got %d" % ((Nk + G - 1) // G, vs.shape[2]))
             P.vs_stride = _lib._i64x3(vs.stride(0), vs.stride(1), vs.stride(3))
