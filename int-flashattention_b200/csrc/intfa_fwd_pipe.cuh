@@ -73,7 +73,7 @@ struct PipeCfg {
   // steps of 1 KB for each kind of instantiation (`ragged`: the one that masks partial tiles).  With explicit shared-memory
   // accesses it matters less than it did: +-1.5 % non-causal, +-4 % causal; the ragged one 294 us (256) to 343 us (0) at
   // batch 2, 32/8 heads, 3001 tokens, causal.
-  static constexpr int code_filler_of(bool ragged) { return ragged ? 256 : BAND_FAST ? (FULL ? 448 : 384) : (FULL && D == 64) ? 0 : 128; }
+  __host__ __device__ static constexpr int code_filler_of(bool ragged) { return ragged ? 256 : BAND_FAST ? (FULL ? 448 : 384) : (FULL && D == 64) ? 0 : 128; }
   static constexpr bool MORE_SOFTMAX_REGS = !FULL || G == 128;
   static constexpr int SOFTMAX_REGS = MORE_SOFTMAX_REGS ? 152 : 136;
   static constexpr int CORR_REGS = MORE_SOFTMAX_REGS ? 168 : 184;
