@@ -152,6 +152,17 @@ int intfa_quant_v(const void* v, const int64_t v_stride[3],
                   void* workspace, size_t workspace_bytes, void* stream);
 
 /*
+ * intfa_quant_v in two launches and nothing to clear: the first takes the column absmax of v chunk by chunk into
+ * `workspace` (intfa_quant_v_partial_workspace_bytes() bytes, contents irrelevant), the second quantises.  Bit-identical
+ * to intfa_quant_v, which needs less scratch but clears it with a memset.
+ */
+size_t intfa_quant_v_partial_workspace_bytes(int32_t B, int32_t H, int32_t N, int32_t D);
+int intfa_quant_v_partial(const void* v, const int64_t v_stride[3],
+                          void* v8, float* scale, int32_t mode,
+                          int32_t B, int32_t H, int32_t N, int32_t D,
+                          void* workspace, size_t workspace_bytes, void* stream);
+
+/*
  * The two halves of intfa_quant_v, for a V tensor whose token axis is sharded over devices:
  * intfa_v_colmax accumulates (atomic max) the column absmax of the local shard into
  * `colmax` (B*H*D words holding fp32 bit patterns, which the CALLER zeroes first and may

@@ -15,7 +15,8 @@ VSCALE_PER_TENSOR, VSCALE_PER_CHANNEL = 0, 1
 SCALE_F16_Q, SCALE_F16_K, SCALE_F16_V = 1, 2, 4
 
 EXPORTS = ("intfa_version", "intfa_last_error", "intfa_fwd", "intfa_quant_pertoken",
-           "intfa_quant_v_workspace_bytes", "intfa_quant_v", "intfa_quant_qkv_workspace_bytes", "intfa_quant_qkv",
+           "intfa_quant_v_workspace_bytes", "intfa_quant_v", "intfa_quant_v_partial_workspace_bytes", "intfa_quant_v_partial",
+           "intfa_quant_qkv_workspace_bytes", "intfa_quant_qkv",
            "intfa_v_colmax", "intfa_v_quant_from_colmax", "intfa_quant_v_static",
            "intfa_quant_v_static_max_words", "intfa_scales_f16_to_f32", "intfa_sm_count")
 
@@ -80,6 +81,10 @@ def load():
     lib.intfa_quant_v_workspace_bytes.argtypes = [i32, i32, i32]
     lib.intfa_quant_v.restype = ctypes.c_int
     lib.intfa_quant_v.argtypes = [vp, ctypes.POINTER(i64), vp, vp, i32, i32, i32, i32, i32, vp, ctypes.c_size_t, vp]
+    lib.intfa_quant_v_partial_workspace_bytes.restype = ctypes.c_size_t
+    lib.intfa_quant_v_partial_workspace_bytes.argtypes = [i32, i32, i32, i32]
+    lib.intfa_quant_v_partial.restype = ctypes.c_int
+    lib.intfa_quant_v_partial.argtypes = lib.intfa_quant_v.argtypes
     lib.intfa_quant_qkv_workspace_bytes.restype = ctypes.c_size_t
     lib.intfa_quant_qkv_workspace_bytes.argtypes = [i32, i32, i32, i32]
     lib.intfa_quant_qkv.restype = ctypes.c_int

@@ -144,6 +144,22 @@ int intfa_quant_v(const void* v, const int64_t v_stride[3], void* v8, float* sca
   return quant_v(v, v_stride, v8, scale, mode, B, H, N, D, workspace, reinterpret_cast<cudaStream_t>(stream));
 }
 
+size_t intfa_quant_v_partial_workspace_bytes(int32_t B, int32_t H, int32_t N, int32_t D) {
+  return intfa_quant_qkv_workspace_bytes(B, H, N, D);
+}
+
+int intfa_quant_v_partial(const void* v, const int64_t v_stride[3], void* v8, float* scale, int32_t mode, int32_t B, int32_t H,
+                          int32_t N, int32_t D, void* workspace, size_t workspace_bytes, void* stream) {
+  int rc = check_quant_args(v, v_stride, v8, scale, B, H, N, D);
+  if (rc) return rc;
+  if (mode != INTFA_VSCALE_PER_TENSOR && mode != INTFA_VSCALE_PER_CHANNEL)
+    return set_error(INTFA_ERR_INVALID_ARG, "mode must be INTFA_VSCALE_PER_TENSOR or INTFA_VSCALE_PER_CHANNEL");
+  if (!workspace || workspace_bytes < intfa_quant_v_partial_workspace_bytes(B, H, N, D))
+    return set_error(INTFA_ERR_INVALID_ARG, "workspace missing or smaller than intfa_quant_v_partial_workspace_bytes()");
+  if ((long long)B * H > 65535) return set_error(INTFA_ERR_TOO_LARGE, "B*H=%lld exceeds 65535", (long long)B * H);
+  return quant_v_partial(v, v_stride, v8, scale, mode, B, H, N, D, workspace, reinterpret_cast<cudaStream_t>(stream));
+}
+
 size_t intfa_quant_qkv_workspace_bytes(int32_t B, int32_t H_kv, int32_t Nk, int32_t D) {
   if (B <= 0 || H_kv <= 0 || Nk <= 0 || D <= 0) return 0;
   return quant_qkv_workspace_bytes(B, H_kv, Nk, D);

@@ -211,11 +211,11 @@ __device__ __forceinline__ void colmax_chunk(const __half* __restrict__ x, long 
   }
 }
 
-template <int D>
+template <int D, bool ATOMIC>
 __global__ void __launch_bounds__(256) v_colmax_kernel(const __half* __restrict__ x, long long sB, long long sH,
                                                        long long sN, unsigned int* __restrict__ colmax, int H, int N,
                                                        int rows_per_cta) {
-  colmax_chunk<D, true>(x, sB, sH, sN, colmax, H, N, rows_per_cta, blockIdx.x, blockIdx.y, gridDim.y);
+  colmax_chunk<D, ATOMIC>(x, sB, sH, sN, colmax, H, N, rows_per_cta, blockIdx.x, blockIdx.y, gridDim.y);
 }
 
 // The first launch of the fused prologue: one grid over three jobs -- CTAs [0, gq) quantise the rows of Q,
@@ -353,7 +353,7 @@ int v_colmax(const void* v, const int64_t* st, void* colmax, int B, int H, int N
   if (sms <= 0) return set_error(INTFA_ERR_CUDA, "cannot query SM count");
   int rows_per_cta;
   dim3 grid(v_grid(B * H, N, sms, &rows_per_cta), B * H);
-  INTFA_D_SWITCH(D, (v_colmax_kernel<DD><<<grid, 256, 0, stream>>>((const __half*)v, st[0], st[1], st[2], (unsigned int*)colmax, H, N, rows_per_cta)))
+  INTFA_D_SWITCH(D, (v_colmax_kernel<DD, true><<<grid, 256, 0, stream>>>((const __half*)v, st[0], st[1], st[2], (unsigned int*)colmax, H, N, rows_per_cta)))
   return check_launch("v_colmax");
 }
 
@@ -413,6 +413,19 @@ int quant_qkv(const void* q, const void* k, const void* v, const int64_t* v_st, 
   int rc = check_launch("quant_qkv");
   if (rc || !v) return rc;
   return v_quant_launch(v, v_st, workspace, j.chunks, v8, vs, mode, B, Hkv, Nk, D, stream);
+}
+
+int quant_v_partial(const void* v, const int64_t* st, void* v8, float* scale, int mode, int B, int H, int N, int D, void* workspace,
+                    cudaStream_t stream) {
+  const int sms = sm_count_cached();
+  if (sms <= 0) return set_error(INTFA_ERR_CUDA, "cannot query SM count");
+  int rows_per_cta;
+  const int chunks = v_grid(B * H, N, sms, &rows_per_cta);
+  dim3 grid(chunks, B * H);
+  INTFA_D_SWITCH(D, (v_colmax_kernel<DD, false><<<grid, 256, 0, stream>>>((const __half*)v, st[0], st[1], st[2], (unsigned int*)workspace, H, N, rows_per_cta)))
+  int rc = check_launch("v_colmax");
+  if (rc) return rc;
+  return v_quant_launch(v, st, workspace, chunks, v8, scale, mode, B, H, N, D, stream);
 }
 
 int quant_v(const void* v, const int64_t* st, void* v8, float* scale, int mode, int B, int H, int N, int D,
