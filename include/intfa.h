@@ -111,6 +111,9 @@ typedef struct IntfaFwdParams {
   int32_t scale_f16;            /* bit set: that scale tensor is fp16 (as benchmark.py makes them), else fp32.
                                    INTFA_SCALE_F16_Q / _K / _V; the kernel widens in place
                                    (flash_atten_full_int8.py:37-38) */
+  /* Device scratch, contents irrelevant, 256-byte aligned: intfa_fwd_workspace_bytes() of them.  Calls of a few query rows
+     split the keys over the GPU and need it; without it (NULL, 0) they run the unsplit way. */
+  void* workspace; uint64_t workspace_bytes;
 } IntfaFwdParams;
 
 /*
@@ -121,6 +124,9 @@ typedef struct IntfaFwdParams {
  * csrc/flash_fwd_launch_template.h:116-191,469-523).
  */
 int intfa_fwd(const IntfaFwdParams* p, void* stream);
+
+/* Scratch that intfa_fwd() makes use of for these arguments (pointers are not looked at); 0: none. */
+size_t intfa_fwd_workspace_bytes(const IntfaFwdParams* p);
 
 /*
  * Fused quantisation prologue: fp16 -> int8 with absmax scales.

@@ -14,7 +14,7 @@ VARIANT_FULL, VARIANT_HALF, VARIANT_HALF_FP8 = 0, 1, 2
 VSCALE_PER_TENSOR, VSCALE_PER_CHANNEL = 0, 1
 SCALE_F16_Q, SCALE_F16_K, SCALE_F16_V = 1, 2, 4
 
-EXPORTS = ("intfa_version", "intfa_last_error", "intfa_fwd", "intfa_quant_pertoken",
+EXPORTS = ("intfa_version", "intfa_last_error", "intfa_fwd", "intfa_fwd_workspace_bytes", "intfa_quant_pertoken",
            "intfa_quant_v_workspace_bytes", "intfa_quant_v", "intfa_quant_v_partial_workspace_bytes", "intfa_quant_v_partial",
            "intfa_quant_qkv_workspace_bytes", "intfa_quant_qkv",
            "intfa_v_colmax", "intfa_v_quant_from_colmax", "intfa_quant_v_static",
@@ -46,6 +46,7 @@ class IntfaFwdParams(ctypes.Structure):
         ("kv_order", ctypes.c_int32), ("vs_stride_blk", ctypes.c_int64),
         ("debug_wait_limit_kcycles", ctypes.c_int32), ("debug_skip_k_load", ctypes.c_int32),
         ("scale_f16", ctypes.c_int32),
+        ("workspace", ctypes.c_void_p), ("workspace_bytes", ctypes.c_uint64),
     ]
 
 
@@ -75,6 +76,8 @@ def load():
     lib.intfa_last_error.argtypes = [ctypes.c_char_p, ctypes.c_size_t]
     lib.intfa_fwd.restype = ctypes.c_int
     lib.intfa_fwd.argtypes = [ctypes.POINTER(IntfaFwdParams), vp]
+    lib.intfa_fwd_workspace_bytes.restype = ctypes.c_size_t
+    lib.intfa_fwd_workspace_bytes.argtypes = [ctypes.POINTER(IntfaFwdParams)]
     lib.intfa_quant_pertoken.restype = ctypes.c_int
     lib.intfa_quant_pertoken.argtypes = [vp, ctypes.POINTER(i64), vp, vp, i32, i32, i32, i32, vp]
     lib.intfa_quant_v_workspace_bytes.restype = ctypes.c_size_t

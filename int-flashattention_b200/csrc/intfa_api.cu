@@ -106,7 +106,14 @@ int intfa_fwd(const IntfaFwdParams* p, void* stream) {
     return set_error(INTFA_ERR_INVALID_ARG, "state_acc must be 16-byte aligned");
   if (!p->write_o && !p->state_out) return set_error(INTFA_ERR_INVALID_ARG, "nothing to write: write_o and state_out are both 0");
   if (p->dbg_s && (p->dbg_tile < 0 || p->dbg_step < 0)) return set_error(INTFA_ERR_INVALID_ARG, "bad debug tap");
+  if (p->workspace && (reinterpret_cast<uintptr_t>(p->workspace) & 255u)) return set_error(INTFA_ERR_INVALID_ARG, "workspace must be 256-byte aligned");
+  if (decode_dispatch(p, reinterpret_cast<cudaStream_t>(stream), &rc)) return rc;
   return fwd_dispatch(p, reinterpret_cast<cudaStream_t>(stream));
+}
+
+size_t intfa_fwd_workspace_bytes(const IntfaFwdParams* p) {
+  if (!p || p->B <= 0 || p->H <= 0 || p->Nq <= 0 || p->Nk <= 0 || p->H_kv < 0 || (p->H_kv > 0 && p->H % p->H_kv != 0)) return 0;
+  return decode_workspace_bytes(p);
 }
 
 static int check_quant_args(const void* x, const int64_t* st, const void* x8, const float* scale, int B, int H, int N,

@@ -1,0 +1,796 @@
+// Attention of a few query rows against a long K/V cache (decode): the path that is bound by reading K and V once.
+//
+// The 128-row kernel gives such a call one CTA per (batch, query head) whose 128 rows are nearly all padding: it re-reads
+// K/V once per query head of a group and leaves most SMs without work (batch 1, 32/8 heads, 32768 keys, fp16 V: 369 us for
+// 102 MB, 0.28 TB/s).  Here
+//   * the query rows of all heads that share a K/V head are packed into one tile of 8 or 16 rows (R = (H/H_kv)*Nq rows,
+//     so K and V are read once for all of them; more than 16 rows take several tiles, which share K/V through L2);
+//   * the keys are split over as many CTAs as fill the GPU, and over the warps of a CTA;
+//   * the products run on m16n8 warp-level MMAs straight from registers: a warp-level tile is 8 or 16 rows tall where the
+//     smallest tcgen05 tile is 64, and operands go from global memory to the MMA without a shared-memory stage.  The
+//     order of the k index is free in a product, so every lane loads 16 contiguous bytes of a row and calls them its
+//     fragment; for P V the lane transposes the few keys it holds with byte permutes.
+//
+// full-int8: P is rounded to int8 against the RUNNING maximum of the row (keys taken G at a time, ascending), so the
+// maxima must be known before P: `scores_kernel` computes s = (fp32(S32)*s_q)*s_k, keeps it (fp32, in the order in which
+// the next kernel's lanes want it) and the maximum of each group of G keys; `pv_full_kernel` takes the prefix maximum at its
+// first group, and from there on does exactly what the one-pass kernel does: m' = max(m, groupmax*c), p = exp2(s*c - m'),
+// P8, O_j.  The final maximum is known too, so that every partial result is scaled to it at once
+// (acc += exp2(m_j - m_final) * O_j) and the splits add up without weights.
+// half-int8: P is fp16, whose rounding is relative: every warp keeps a running maximum of its own and the partial results
+// are combined with their weights (`pv_half_kernel`: scores and P V in one pass over K and V).
+#include <cuda_fp16.h>
+#include <cuda_bf16.h>
+#include <cuda_runtime.h>
+#include <stdint.h>
+
+#include "intfa_internal.h"
+#include "intfa_ptx.cuh"
+
+namespace intfa {
+
+namespace {
+
+constexpr int kThreads = 128, kWarps = 4;
+constexpr int kMaxLocalGroups = 64;       // groups of G keys per CTA of pv_full_kernel (their maxima sit in shared memory)
+constexpr float kMagicF = 12582912.0f;    // 1.5*2^23: added to an int32 below 2^22 as a bit pattern, it reads as fp32 1.5*2^23 + value
+constexpr int kMagicI = 0x4B400000;
+
+struct DParams {
+  const int8_t* q; const int8_t* k; const void* v; void* o;
+  long long qB, qH, qN, kB, kH, kN, vB, vH, vN, oB, oH, oN;
+  const void* qs; const void* ks; const void* vs;
+  long long qsB, qsH, ksB, ksH, vsB, vsH, vsD;
+  int scale_f16, o_bf16, causal;
+  int H, Hkv, ratio, Nq, R, tiles;        // R = ratio*Nq rows per K/V head, in `tiles` tiles of RT rows
+  int nvis;                               // keys that some row sees
+  long long limit0;                       // causal: row n sees the keys <= limit0 + n
+  float c;                                // sm_scale * log2(e)
+  int G, groups, splits, per_split;       // per_split: groups (full) or 64-key units (half) per split
+  float* lse;
+  float* scores; float* gmax;             // [unit][key tile of 8][NT][32 lanes][2]; [unit][groups][RT]
+  float* part; float* part_ml;            // [unit][splits][RT][D]; [unit][splits][RT][2]
+};
+
+__device__ __forceinline__ float scale_at(const void* s, long long i, int f16) {
+  return f16 ? __half2float(static_cast<const __half*>(s)[i]) : static_cast<const float*>(s)[i];
+}
+// streaming 16-byte load
+__device__ __forceinline__ uint4 ld16(const void* p) {
+  uint4 v;
+  asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ uint2 ld8(const void* p) {
+  uint2 v;
+  asm volatile("ld.global.nc.L1::no_allocate.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ void mma_s8(int (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+               : "+r"(d[0]), "+r"(d[1]), "+r"(d[2]), "+r"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ void mma_f16(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+               : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ float unmagic(int x) { return __int_as_float(x) - kMagicF; }
+// (programmatic launch: the next kernel of the chain may start; what the previous one wrote is there)
+__device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+// one (batch, K/V head, row tile)
+struct Unit {
+  int id, b, hk, tile;
+};
+__device__ __forceinline__ Unit unit_of(const DParams& p, int id) {
+  Unit u;
+  u.id = id;
+  u.tile = id % p.tiles;
+  const int bh = id / p.tiles;
+  u.b = bh / p.Hkv;
+  u.hk = bh - u.b * p.Hkv;
+  return u;
+}
+
+// Q fragments of a lane (g = lane/4, t = lane%4), its row scales and the last key its rows see.  Rows past R: zero.
+// Word i of chunk ch of row half hr sits at qf[ch][hr][i]: bytes ch*64 + t*16 + 4i of row g + 8*hr.
+template <int D, int NT>
+struct QRows {
+  static constexpr int CH = D / 64;
+  uint32_t w[CH][NT][4];
+  float s[NT];
+  int last[NT];
+  __device__ __forceinline__ void load(const DParams& p, const Unit& u, int g, int t) {
+#pragma unroll
+    for (int hr = 0; hr < NT; ++hr) {
+      const int r = u.tile * (8 * NT) + g + 8 * hr;
+      s[hr] = 0.f;
+      last[hr] = p.nvis - 1;
+#pragma unroll
+      for (int c = 0; c < CH; ++c) w[c][hr][0] = w[c][hr][1] = w[c][hr][2] = w[c][hr][3] = 0u;
+      if (r < p.R) {
+        const int h = u.hk * p.ratio + r / p.Nq, n = r % p.Nq;
+        const int8_t* q = p.q + u.b * p.qB + h * p.qH + n * p.qN + t * 16;
+#pragma unroll
+        for (int c = 0; c < CH; ++c) {
+          const uint4 x = *reinterpret_cast<const uint4*>(q + c * 64);
+          w[c][hr][0] = x.x; w[c][hr][1] = x.y; w[c][hr][2] = x.z; w[c][hr][3] = x.w;
+        }
+        s[hr] = scale_at(p.qs, u.b * p.qsB + h * p.qsH + n, p.scale_f16 & INTFA_SCALE_F16_Q);
+        if (p.causal && p.limit0 + n < last[hr]) last[hr] = (int)(p.limit0 + n);
+      }
+    }
+  }
+};
+
+// S^T for 8 keys: kw[c] = bytes c*64 + t*16 .. +15 of key g.  Result: rows g (d[0], d[1]) and g+8 (d[2], d[3]), keys 2t, 2t+1.
+template <int D, int NT>
+__device__ __forceinline__ void qk_tile(const QRows<D, NT>& q, const uint4 (&kw)[D / 64], int (&d)[4]) {
+  d[0] = d[1] = d[2] = d[3] = kMagicI;
+#pragma unroll
+  for (int c = 0; c < D / 64; ++c) {
+    const uint32_t z = 0u;
+    mma_s8(d, q.w[c][0][0], NT > 1 ? q.w[c][NT - 1][0] : z, q.w[c][0][1], NT > 1 ? q.w[c][NT - 1][1] : z, kw[c].x, kw[c].y);
+    mma_s8(d, q.w[c][0][2], NT > 1 ? q.w[c][NT - 1][2] : z, q.w[c][0][3], NT > 1 ? q.w[c][NT - 1][3] : z, kw[c].z, kw[c].w);
+  }
+}
+
+// ---------------------------------------------------------------------------------------------------------------
+// full-int8, first pass: scores and group maxima.  One warp takes one group of G keys at a time, 32 keys in flight.
+// Bound by reading K (67 MB at batch 16, 8 K/V heads, 4097 keys).
+// ---------------------------------------------------------------------------------------------------------------
+template <int D, int NT>
+__global__ void __launch_bounds__(kThreads) scores_kernel(const DParams p, int splits) {
+  constexpr int RT = 8 * NT, CH = D / 64;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
+  const Unit u = unit_of(p, blockIdx.x % (gridDim.x / splits));
+  const int split = blockIdx.x / (gridDim.x / splits);
+  pdl_launch();
+  QRows<D, NT> q;
+  q.load(p, u, g, t);
+  const int8_t* kb = p.k + u.b * p.kB + u.hk * p.kH + t * 16;
+  const long long ksb = u.b * p.ksB + u.hk * p.ksH;
+  const int kf16 = p.scale_f16 & INTFA_SCALE_F16_K;
+  const int ktiles = p.groups * (p.G / 8);
+  float2* sc = reinterpret_cast<float2*>(p.scores) + (long long)u.id * ktiles * NT * 32 + lane;
+  float* gm = p.gmax + (long long)u.id * p.groups * RT;
+  for (int grp = split * kWarps + warp; grp < p.groups; grp += splits * kWarps) {
+    float mx[NT];
+#pragma unroll
+    for (int i = 0; i < NT; ++i) mx[i] = -INFINITY;
+#pragma unroll 1
+    for (int kt = grp * (p.G / 8); kt < (grp + 1) * (p.G / 8); kt += 4) {
+      uint4 kw[4][CH];
+      float k0[4], k1[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int8_t* row = kb + (long long)min((kt + i) * 8 + g, p.nvis - 1) * p.kN;
+#pragma unroll
+        for (int c = 0; c < CH; ++c) kw[i][c] = ld16(row + c * 64);
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int key = (kt + i) * 8 + 2 * t;
+        k0[i] = scale_at(p.ks, ksb + min(key, p.nvis - 1), kf16);
+        k1[i] = scale_at(p.ks, ksb + min(key + 1, p.nvis - 1), kf16);
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        int d[4];
+        qk_tile<D, NT>(q, kw[i], d);
+        const int key = (kt + i) * 8 + 2 * t;
+#pragma unroll
+        for (int hr = 0; hr < NT; ++hr) {
+          float2 s;
+          s.x = key <= q.last[hr] ? unmagic(d[2 * hr]) * q.s[hr] * k0[i] : -1e30f;
+          s.y = key + 1 <= q.last[hr] ? unmagic(d[2 * hr + 1]) * q.s[hr] * k1[i] : -1e30f;
+          mx[hr] = max3(mx[hr], s.x, s.y);
+          sc[((kt + i) * NT + hr) * 32] = s;
+        }
+      }
+    }
+#pragma unroll
+    for (int hr = 0; hr < NT; ++hr) {
+      mx[hr] = fmaxf(mx[hr], __shfl_xor_sync(0xffffffffu, mx[hr], 1));
+      mx[hr] = fmaxf(mx[hr], __shfl_xor_sync(0xffffffffu, mx[hr], 2));
+      if (t == 0) gm[grp * RT + g + 8 * hr] = mx[hr];
+    }
+  }
+}
+
+// ---------------------------------------------------------------------------------------------------------------
+// output of one CTA: the 4 warps' results of RT rows x D channels are in red (weights applied), l and m in ml
+// ---------------------------------------------------------------------------------------------------------------
+__device__ __forceinline__ void store_row4(const DParams& p, const Unit& u, int r, int ch, const float (&x)[4]) {
+  const int h = u.hk * p.ratio + r / p.Nq, n = r % p.Nq;
+  __half* o = static_cast<__half*>(p.o) + u.b * p.oB + h * p.oH + n * p.oN + ch;
+  uint2 w;
+  if (p.o_bf16) {
+    const __nv_bfloat162 a = __floats2bfloat162_rn(x[0], x[1]), b = __floats2bfloat162_rn(x[2], x[3]);
+    w.x = *reinterpret_cast<const uint32_t*>(&a);
+    w.y = *reinterpret_cast<const uint32_t*>(&b);
+  } else {
+    const __half2 a = __floats2half2_rn(x[0], x[1]), b = __floats2half2_rn(x[2], x[3]);
+    w.x = *reinterpret_cast<const uint32_t*>(&a);
+    w.y = *reinterpret_cast<const uint32_t*>(&b);
+  }
+  *reinterpret_cast<uint2*>(o) = w;
+}
+// o = acc * (s_v/127) / l for 4 channels of row r
+template <bool FULL>
+__device__ __forceinline__ void finish_row4(const DParams& p, const Unit& u, int r, int ch, float4 a, float l) {
+  const float inv = 1.0f / l;
+  float x[4] = {a.x, a.y, a.z, a.w};
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    if constexpr (FULL) x[i] *= scale_at(p.vs, u.b * p.vsB + u.hk * p.vsH + (ch + i) * p.vsD, p.scale_f16 & INTFA_SCALE_F16_V) / 127.0f;
+    x[i] *= inv;
+  }
+  store_row4(p, u, r, ch, x);
+}
+__device__ __forceinline__ void store_lse(const DParams& p, const Unit& u, int r, float m, float l) {
+  const int h = u.hk * p.ratio + r / p.Nq, n = r % p.Nq;
+  if (p.lse) p.lse[((long long)u.b * p.H + h) * p.Nq + n] = m + log2f(l);
+}
+template <bool FULL, int D, int NT>
+__device__ __forceinline__ void cta_out(const DParams& p, const Unit& u, int split, const float* red, const float (*ml)[2]) {
+  constexpr int RT = 8 * NT;
+#pragma unroll
+  for (int e = threadIdx.x; e < RT * D / 4; e += kThreads) {
+    const int r = e / (D / 4), ch = e % (D / 4) * 4, row = u.tile * RT + r;
+    if (row >= p.R) continue;
+    float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int w = 0; w < kWarps; ++w) {
+      const float4 x = *reinterpret_cast<const float4*>(red + (w * RT + r) * (D + 4) + ch);
+      a.x += x.x; a.y += x.y; a.z += x.z; a.w += x.w;
+    }
+    if (p.splits == 1) {
+      finish_row4<FULL>(p, u, row, ch, a, ml[r][1]);
+      if (ch == 0) store_lse(p, u, row, ml[r][0], ml[r][1]);
+    } else {
+      const long long pr = ((long long)u.id * p.splits + split) * RT + r;
+      *reinterpret_cast<float4*>(p.part + pr * D + ch) = a;
+      if (ch == 0) *reinterpret_cast<float2*>(p.part_ml + pr * 2) = make_float2(ml[r][0], ml[r][1]);
+    }
+  }
+}
+
+// ---------------------------------------------------------------------------------------------------------------
+// full-int8, second pass: P from the kept scores, O = P V.  One warp takes 64 keys at a time (32 in flight ahead of the
+// arithmetic).  Bound by reading V.
+// ---------------------------------------------------------------------------------------------------------------
+template <int D, int NT>
+__global__ void __launch_bounds__(kThreads, NT == 1 ? 3 : 2) pv_full_kernel(const DParams p) {
+  constexpr int RT = 8 * NT, VB = D / 8, MT = D / 16;       // VB: bytes (channels) of a key that a lane holds; MT: 16-channel tiles
+  constexpr int W = VB / 4;                                 // ... in words
+  __shared__ __align__(16) float red[kWarps * RT * (D + 4)];
+  __shared__ __align__(16) float mg[kMaxLocalGroups * RT];  // running maximum (scaled) at each group of this CTA
+  __shared__ __align__(16) float ends[2][RT];               // prefix before the first group; final maximum
+  __shared__ float ml[RT][2];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
+  const int units = gridDim.x / p.splits;
+  const Unit u = unit_of(p, blockIdx.x % units);
+  const int split = blockIdx.x / units;
+  const int g0 = split * p.per_split, g1 = min(p.groups, g0 + p.per_split);
+  const int8_t* vb = static_cast<const int8_t*>(p.v) + u.b * p.vB + u.hk * p.vH + g * VB;
+  pdl_launch();
+
+  // this lane's 8 keys of a 32-key step: 2t, 2t+1 of each of the four 8-key tiles
+  uint32_t vn[8][W];
+  auto load_v = [&](int key0) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const int key = min(key0 + (i >> 1) * 8 + 2 * t + (i & 1), p.nvis - 1);
+      const int8_t* a = vb + (long long)key * p.vN;
+      if constexpr (W == 4) {
+        const uint4 x = ld16(a);
+        vn[i][0] = x.x; vn[i][1] = x.y; vn[i][2] = x.z; vn[i][3] = x.w;
+      } else {
+        const uint2 x = ld8(a);
+        vn[i][0] = x.x; vn[i][1] = x.y;
+      }
+    }
+  };
+  // (V does not depend on the first pass)
+  const int upg = p.G / 64, nun = (g1 - g0) * upg;          // 64-key units of this CTA
+  if (warp < nun) load_v((g0 * upg + warp) * 64);
+  pdl_wait();
+
+  // ---- running maxima of this CTA's groups and the final maximum
+  {
+    const float* gm = p.gmax + (long long)u.id * p.groups * RT;
+    constexpr int Q4 = RT / 4;                               // threads across a group's rows, 4 rows each
+    const int rq = tid % Q4 * 4;
+    float4 pre = make_float4(-INFINITY, -INFINITY, -INFINITY, -INFINITY), all = pre;
+#pragma unroll 4
+    for (int i = tid / Q4; i < p.groups; i += kThreads / Q4) {
+      const float4 x = *reinterpret_cast<const float4*>(gm + i * RT + rq);
+      all.x = fmaxf(all.x, x.x); all.y = fmaxf(all.y, x.y); all.z = fmaxf(all.z, x.z); all.w = fmaxf(all.w, x.w);
+      if (i < g0) {
+        pre.x = fmaxf(pre.x, x.x); pre.y = fmaxf(pre.y, x.y); pre.z = fmaxf(pre.z, x.z); pre.w = fmaxf(pre.w, x.w);
+      } else if (i < g1) {
+        *reinterpret_cast<float4*>(mg + (i - g0) * RT + rq) = x;
+      }
+    }
+    float4* sp = reinterpret_cast<float4*>(red);             // (red is free until the end)
+    sp[tid] = pre;
+    sp[kThreads + tid] = all;
+    __syncthreads();
+    if (tid < 2 * RT) {
+      const int which = tid / RT, r = tid % RT;
+      float m = -INFINITY;
+#pragma unroll 8
+      for (int i = 0; i < kThreads / Q4; ++i) m = fmaxf(m, red[(which * kThreads + i * Q4) * 4 + r]);
+      ends[which][r] = m * p.c;
+    }
+    __syncthreads();
+    if (tid < RT) {
+      float m = ends[0][tid];
+      for (int i = 0; i < g1 - g0; ++i) {
+        m = fmaxf(m, mg[i * RT + tid] * p.c);
+        mg[i * RT + tid] = m;
+      }
+    }
+    __syncthreads();
+  }
+
+  const float2* sc = reinterpret_cast<const float2*>(p.scores) + ((long long)u.id * p.groups * (p.G / 8) * NT) * 32 + lane;
+  float acc[NT][MT][4], lsum[NT];
+  float m_fin[NT][2], m_fin_g[NT];
+#pragma unroll
+  for (int n = 0; n < NT; ++n) {
+    lsum[n] = 0.f;
+    m_fin[n][0] = ends[1][n * 8 + 2 * t];
+    m_fin[n][1] = ends[1][n * 8 + 2 * t + 1];
+    m_fin_g[n] = ends[1][n * 8 + g];
+#pragma unroll
+    for (int i = 0; i < MT; ++i) acc[n][i][0] = acc[n][i][1] = acc[n][i][2] = acc[n][i][3] = 0.f;
+  }
+#pragma unroll 1
+  for (int un = warp; un < nun; un += kWarps) {
+    const int lg = un / upg;
+    float nm[NT], w_g[NT], rs[NT];
+    int o[NT][MT][4];
+#pragma unroll
+    for (int n = 0; n < NT; ++n) {
+      const float m = mg[lg * RT + n * 8 + g];
+      nm[n] = -m;
+      w_g[n] = ex2_approx(m - m_fin_g[n]);
+      rs[n] = 0.f;
+#pragma unroll
+      for (int i = 0; i < MT; ++i) o[n][i][0] = o[n][i][1] = o[n][i][2] = o[n][i][3] = kMagicI;
+    }
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+      const int key0 = (g0 * upg + un) * 64 + half * 32;
+      uint32_t vc[8][W];
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int j = 0; j < W; ++j) vc[i][j] = vn[i][j];
+      float2 s[NT][4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int n = 0; n < NT; ++n) s[n][i] = sc[((key0 / 8 + i) * NT + n) * 32];
+      if (half == 0) load_v(key0 + 32);
+      else if (un + kWarps < nun) load_v(key0 - 32 + kWarps * 64);
+      // P8 of this lane's keys: trunc(fp16(fp16(fp16(p)*127) + 0.5)), as in the 128-row kernel
+      uint32_t b[NT][2];
+#pragma unroll
+      for (int n = 0; n < NT; ++n)
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+          const float2 x = s[n][2 * q], y = s[n][2 * q + 1];
+          const float p0 = ex2_approx(fmaf(x.x, p.c, nm[n])), p1 = ex2_approx(fmaf(x.y, p.c, nm[n]));
+          const float p2 = ex2_approx(fmaf(y.x, p.c, nm[n])), p3 = ex2_approx(fmaf(y.y, p.c, nm[n]));
+          rs[n] += (p0 + p1) + (p2 + p3);
+          const __half2 h01 = __floats2half2_rn(p0, p1), h23 = __floats2half2_rn(p2, p3);
+          const uint32_t z01 = h2_fma(*reinterpret_cast<const uint32_t*>(&h01), 0x57F057F0u, 0x38003800u);
+          const uint32_t z23 = h2_fma(*reinterpret_cast<const uint32_t*>(&h23), 0x57F057F0u, 0x38003800u);
+          uint32_t u0, u1, u2, u3;
+          h2_floor_add(z01, kMagicF, u0, u1);
+          h2_floor_add(z23, kMagicF, u2, u3);
+          b[n][q] = __byte_perm(__byte_perm(u0, u1, 0x0040), __byte_perm(u2, u3, 0x0040), 0x5410);
+        }
+      // O^T (channels x rows): the 4 keys of a quad transposed, so that a word holds one channel's 4 keys
+#pragma unroll
+      for (int j = 0; j < W; ++j) {
+        uint32_t chn[4][2];
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+          const uint32_t x0 = vc[4 * q][j], x1 = vc[4 * q + 1][j], x2 = vc[4 * q + 2][j], x3 = vc[4 * q + 3][j];
+          const uint32_t a = __byte_perm(x0, x1, 0x5140), c = __byte_perm(x0, x1, 0x7362);
+          const uint32_t d = __byte_perm(x2, x3, 0x5140), e = __byte_perm(x2, x3, 0x7362);
+          chn[0][q] = __byte_perm(a, d, 0x5410);
+          chn[1][q] = __byte_perm(a, d, 0x7632);
+          chn[2][q] = __byte_perm(c, e, 0x5410);
+          chn[3][q] = __byte_perm(c, e, 0x7632);
+        }
+#pragma unroll
+        for (int n = 0; n < NT; ++n) {
+          mma_s8(o[n][2 * j], chn[0][0], chn[1][0], chn[0][1], chn[1][1], b[n][0], b[n][1]);
+          mma_s8(o[n][2 * j + 1], chn[2][0], chn[3][0], chn[2][1], chn[3][1], b[n][0], b[n][1]);
+        }
+      }
+    }
+#pragma unroll
+    for (int n = 0; n < NT; ++n) {
+      lsum[n] = fmaf(w_g[n], rs[n], lsum[n]);
+      const float w0 = ex2_approx(mg[lg * RT + n * 8 + 2 * t] - m_fin[n][0]), w1 = ex2_approx(mg[lg * RT + n * 8 + 2 * t + 1] - m_fin[n][1]);
+#pragma unroll
+      for (int i = 0; i < MT; ++i) {
+        acc[n][i][0] = fmaf(unmagic(o[n][i][0]), w0, acc[n][i][0]);
+        acc[n][i][1] = fmaf(unmagic(o[n][i][1]), w1, acc[n][i][1]);
+        acc[n][i][2] = fmaf(unmagic(o[n][i][2]), w0, acc[n][i][2]);
+        acc[n][i][3] = fmaf(unmagic(o[n][i][3]), w1, acc[n][i][3]);
+      }
+    }
+  }
+  // ---- the warps' results
+  if (tid < RT) {
+    ml[tid][0] = ends[1][tid];
+    ml[tid][1] = 0.f;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int n = 0; n < NT; ++n) {
+    // tile i of the lane: channel g*VB + 2i (entries 0, 1) and + 1 (2, 3) of rows 2t (0, 2) and 2t+1 (1, 3)
+#pragma unroll
+    for (int i = 0; i < MT; ++i) {
+      float* d = red + (warp * RT + n * 8 + 2 * t) * (D + 4) + g * VB + 2 * i;
+      *reinterpret_cast<float2*>(d) = make_float2(acc[n][i][0], acc[n][i][2]);
+      *reinterpret_cast<float2*>(d + D + 4) = make_float2(acc[n][i][1], acc[n][i][3]);
+    }
+    float l = lsum[n];
+    l += __shfl_xor_sync(0xffffffffu, l, 1);
+    l += __shfl_xor_sync(0xffffffffu, l, 2);
+    // (one warp after the other, so that the sum has one order)
+    for (int w = 0; w < kWarps; ++w) {
+      if (w == warp && t == 0) ml[n * 8 + g][1] += l;
+      __syncthreads();
+    }
+  }
+  cta_out<true, D, NT>(p, u, split, red, ml);
+}
+
+// ---------------------------------------------------------------------------------------------------------------
+// half-int8: scores, softmax and P V in one pass; one warp takes 32 keys at a time, with a running maximum of its own
+// ---------------------------------------------------------------------------------------------------------------
+template <int D, int NT>
+__global__ void __launch_bounds__(kThreads, 2) pv_half_kernel(const DParams p) {
+  constexpr int RT = 8 * NT, CH = D / 64, MT = D / 16;
+  __shared__ __align__(16) float red[kWarps * RT * (D + 4)];
+  __shared__ float wml[kWarps][RT][2];
+  __shared__ float ml[RT][2];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
+  const int units = gridDim.x / p.splits;
+  const Unit u = unit_of(p, blockIdx.x % units);
+  const int split = blockIdx.x / units;
+  const int k_begin = split * p.per_split * 64, k_end = min(p.nvis, k_begin + p.per_split * 64);
+  pdl_launch();
+  QRows<D, NT> q;
+  q.load(p, u, g, t);
+  const int8_t* kb = p.k + u.b * p.kB + u.hk * p.kH + t * 16;
+  const __half* vb = static_cast<const __half*>(p.v) + u.b * p.vB + u.hk * p.vH + g * 8;
+  const long long ksb = u.b * p.ksB + u.hk * p.ksH;
+  const int kf16 = p.scale_f16 & INTFA_SCALE_F16_K;
+  float acc[NT][MT][4], m[NT], l[NT];
+#pragma unroll
+  for (int n = 0; n < NT; ++n) {
+    m[n] = -INFINITY;
+    l[n] = 0.f;
+#pragma unroll
+    for (int i = 0; i < MT; ++i) acc[n][i][0] = acc[n][i][1] = acc[n][i][2] = acc[n][i][3] = 0.f;
+  }
+  uint4 kw[4][CH];
+  float k0[4], k1[4];
+  auto load_k = [&](int key0) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int8_t* row = kb + (long long)min(key0 + i * 8 + g, p.nvis - 1) * p.kN;
+#pragma unroll
+      for (int c = 0; c < CH; ++c) kw[i][c] = ld16(row + c * 64);
+      const int key = key0 + i * 8 + 2 * t;
+      k0[i] = scale_at(p.ks, ksb + min(key, p.nvis - 1), kf16);
+      k1[i] = scale_at(p.ks, ksb + min(key + 1, p.nvis - 1), kf16);
+    }
+  };
+  const int first = k_begin + warp * 32;
+  if (first < k_end) load_k(first);
+#pragma unroll 1
+  for (int key0 = first; key0 < k_end; key0 += kWarps * 32) {
+    // V of the first 16 keys is on its way while the scores are computed
+    uint4 v[4][CH];
+    auto load_v = [&](int h) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int key = min(key0 + h * 16 + (i >> 1) * 8 + 2 * t + (i & 1), p.nvis - 1);
+#pragma unroll
+        for (int c = 0; c < CH; ++c) v[i][c] = ld16(vb + (long long)key * p.vN + c * 64);
+      }
+    };
+    load_v(0);
+    float x[NT][4][2], mx[NT];
+#pragma unroll
+    for (int n = 0; n < NT; ++n) mx[n] = m[n];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      int d[4];
+      qk_tile<D, NT>(q, kw[i], d);
+      const int key = key0 + i * 8 + 2 * t;
+#pragma unroll
+      for (int n = 0; n < NT; ++n) {
+        x[n][i][0] = key <= q.last[n] ? unmagic(d[2 * n]) * q.s[n] * k0[i] * p.c : -1.0e30f;
+        x[n][i][1] = key + 1 <= q.last[n] ? unmagic(d[2 * n + 1]) * q.s[n] * k1[i] * p.c : -1.0e30f;
+        mx[n] = max3(mx[n], x[n][i][0], x[n][i][1]);
+      }
+    }
+    if (key0 + kWarps * 32 < k_end) load_k(key0 + kWarps * 32);
+    bool moved = false;
+    float al[NT];
+#pragma unroll
+    for (int n = 0; n < NT; ++n) {
+      mx[n] = fmaxf(mx[n], __shfl_xor_sync(0xffffffffu, mx[n], 1));
+      mx[n] = fmaxf(mx[n], __shfl_xor_sync(0xffffffffu, mx[n], 2));
+      mx[n] = fmaxf(mx[n], -1.0e29f);           // (a row that has seen no key yet: its p are 0)
+      al[n] = ex2_approx(m[n] - mx[n]);
+      moved |= mx[n] != m[n];
+      m[n] = mx[n];
+    }
+    if (__any_sync(0xffffffffu, moved)) {
+#pragma unroll
+      for (int n = 0; n < NT; ++n) {
+        l[n] *= al[n];
+        const float a0 = __shfl_sync(0xffffffffu, al[n], 8 * t), a1 = __shfl_sync(0xffffffffu, al[n], 8 * t + 4);   // rows 2t, 2t+1
+#pragma unroll
+        for (int i = 0; i < MT; ++i) {
+          acc[n][i][0] *= a0;
+          acc[n][i][1] *= a1;
+          acc[n][i][2] *= a0;
+          acc[n][i][3] *= a1;
+        }
+      }
+    }
+    uint32_t b[NT][4];
+#pragma unroll
+    for (int n = 0; n < NT; ++n)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const float p0 = ex2_approx(x[n][i][0] - m[n]), p1 = ex2_approx(x[n][i][1] - m[n]);
+        l[n] += p0 + p1;
+        const __half2 h = __floats2half2_rn(p0, p1);
+        b[n][i] = *reinterpret_cast<const uint32_t*>(&h);
+      }
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      // O^T (channels x rows): two keys of one channel in a word
+#pragma unroll
+      for (int c = 0; c < CH; ++c) {
+        const uint32_t* x0 = reinterpret_cast<const uint32_t*>(&v[0][c]);
+        const uint32_t* x1 = reinterpret_cast<const uint32_t*>(&v[1][c]);
+        const uint32_t* x2 = reinterpret_cast<const uint32_t*>(&v[2][c]);
+        const uint32_t* x3 = reinterpret_cast<const uint32_t*>(&v[3][c]);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const uint32_t a0 = __byte_perm(x0[j], x1[j], 0x5410), a1 = __byte_perm(x0[j], x1[j], 0x7632);
+          const uint32_t a2 = __byte_perm(x2[j], x3[j], 0x5410), a3 = __byte_perm(x2[j], x3[j], 0x7632);
+#pragma unroll
+          for (int n = 0; n < NT; ++n) mma_f16(acc[n][c * 4 + j], a0, a1, a2, a3, b[n][2 * h], b[n][2 * h + 1]);
+        }
+      }
+      if (h == 0) load_v(1);
+    }
+  }
+  // ---- the warps' results, scaled to the CTA's maximum
+#pragma unroll
+  for (int n = 0; n < NT; ++n) {
+    l[n] += __shfl_xor_sync(0xffffffffu, l[n], 1);
+    l[n] += __shfl_xor_sync(0xffffffffu, l[n], 2);
+    if (t == 0) {
+      wml[warp][n * 8 + g][0] = m[n];
+      wml[warp][n * 8 + g][1] = l[n];
+    }
+  }
+  __syncthreads();
+  auto cta_max = [&](int r) { return fmaxf(fmaxf(wml[0][r][0], wml[1][r][0]), fmaxf(wml[2][r][0], wml[3][r][0])); };
+  static_assert(kWarps == 4, "cta_max");
+  if (tid < RT) {
+    const float mm = cta_max(tid);
+    float ls = 0.f;
+    for (int w = 0; w < kWarps; ++w) ls += wml[w][tid][1] * (wml[w][tid][0] == -INFINITY ? 0.f : ex2_approx(wml[w][tid][0] - mm));
+    ml[tid][0] = mm;
+    ml[tid][1] = ls;
+  }
+#pragma unroll
+  for (int n = 0; n < NT; ++n) {
+    float w01[2];
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      const int r = n * 8 + 2 * t + e;
+      w01[e] = wml[warp][r][0] == -INFINITY ? 0.f : ex2_approx(wml[warp][r][0] - cta_max(r));
+    }
+#pragma unroll
+    for (int i = 0; i < MT; ++i) {
+      float* d = red + (warp * RT + n * 8 + 2 * t) * (D + 4) + (i / 4) * 64 + g * 8 + 2 * (i % 4);
+      *reinterpret_cast<float2*>(d) = make_float2(acc[n][i][0] * w01[0], acc[n][i][2] * w01[0]);
+      *reinterpret_cast<float2*>(d + D + 4) = make_float2(acc[n][i][1] * w01[1], acc[n][i][3] * w01[1]);
+    }
+  }
+  __syncthreads();
+  cta_out<false, D, NT>(p, u, split, red, ml);
+}
+
+// Sum of the splits' results, one CTA of D/4 threads per row.  (full: all on the final maximum already; half: weighted.)
+template <bool FULL, int D>
+__global__ void __launch_bounds__(D / 4) combine_kernel(const DParams p, int RT) {
+  const Unit u = unit_of(p, blockIdx.x / RT);
+  const int r = blockIdx.x % RT, row = u.tile * RT + r, ch = threadIdx.x * 4;
+  pdl_wait();
+  if (row >= p.R) return;
+  const long long base = (long long)u.id * p.splits * RT + r;
+  const float2* ml = reinterpret_cast<const float2*>(p.part_ml);
+  float m = -INFINITY;
+  if constexpr (FULL) {
+    m = ml[base].x;
+  } else {
+#pragma unroll 8
+    for (int s = 0; s < p.splits; ++s) m = fmaxf(m, ml[base + (long long)s * RT].x);
+  }
+  float l = 0.f;
+  float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 8
+  for (int s = 0; s < p.splits; ++s) {
+    const long long pr = base + (long long)s * RT;
+    const float2 x = ml[pr];
+    const float4 y = *reinterpret_cast<const float4*>(p.part + pr * D + ch);
+    const float w = FULL ? 1.f : (x.x == -INFINITY ? 0.f : ex2_approx(x.x - m));
+    l = fmaf(w, x.y, l);
+    a.x = fmaf(w, y.x, a.x); a.y = fmaf(w, y.y, a.y); a.z = fmaf(w, y.z, a.z); a.w = fmaf(w, y.w, a.w);
+  }
+  finish_row4<FULL>(p, u, row, ch, a, l);
+  if (ch == 0) store_lse(p, u, row, m, l);
+}
+
+// ---------------------------------------------------------------------------------------------------------------
+// host side
+// ---------------------------------------------------------------------------------------------------------------
+struct Plan {
+  bool use = false, full = false;
+  int NT = 1, tiles = 1, units = 0, nvis = 0, groups = 0, splits = 1, per_split = 1, score_splits = 1;
+  size_t off_gmax = 0, off_part = 0, off_ml = 0, bytes = 0;
+};
+
+Plan make_plan(const IntfaFwdParams* a, int sms) {
+  Plan pl;
+  const int Hkv = a->H_kv > 0 ? a->H_kv : a->H;
+  pl.full = a->variant == INTFA_VARIANT_FULL;
+  // The rule.  Rows: a 16-row tile costs this path about a ninth of what a 128-row tile costs the other one per key, and the
+  // other path takes a tile per query head, so the break-even lies above 128 rows a head; kDecodeRows keeps well clear of it.
+  // Options that the other path keeps: head dims 16, 32, 256, fp8 V (its rounding of P follows the running maximum, too),
+  // carried state, KV tiles last to first, per-tile V scales, RNE rounding, the debug tap, rows that see no key at all.
+  constexpr int kDecodeRows = 32;
+  if (a->Nq > kDecodeRows || (a->D != 64 && a->D != 128) || (!pl.full && a->variant != INTFA_VARIANT_HALF) || (a->G != 64 && a->G != 128)) return pl;
+  if (a->state_in || a->state_out || !a->write_o || a->kv_order || a->vs_stride_blk || (pl.full && a->p_round) || a->dbg_s || a->debug_skip_k_load) return pl;
+  if (!(a->sm_scale > 0.f) || (a->causal && a->q_offset < a->kv_offset)) return pl;
+  pl.nvis = a->Nk;
+  if (a->causal) {
+    const long long vis = a->q_offset + a->Nq - a->kv_offset;
+    if (vis < pl.nvis) pl.nvis = (int)vis;
+  }
+  const long long R = (long long)(a->H / Hkv) * a->Nq;
+  pl.NT = R > 8 ? 2 : 1;
+  const int RT = 8 * pl.NT;
+  pl.tiles = (int)((R + RT - 1) / RT);
+  const long long units = (long long)a->B * Hkv * pl.tiles;
+  if (units > (1 << 22)) return pl;
+  pl.units = (int)units;
+  // Splits: one wave of resident CTAs (3 per SM for full-int8 at 8 rows, 2 otherwise), at least one 64-key unit per warp
+  const int wave = sms * (pl.full && pl.NT == 1 ? 3 : 2);
+  const int key_units = (pl.nvis + 63) / 64;
+  pl.groups = (pl.nvis + a->G - 1) / a->G;
+  const int items = pl.full ? pl.groups : key_units;          // what a split is counted in
+  const int per_min = pl.full ? (a->G == 128 ? 2 : 4) : 2;    // at least 256 (half: 128) keys per CTA
+  int splits = wave / pl.units < 1 ? 1 : wave / pl.units;
+  int per = (items + splits - 1) / splits;
+  if (per < per_min) per = per_min;
+  if (pl.full && per > kMaxLocalGroups) per = kMaxLocalGroups;
+  pl.per_split = per;
+  pl.splits = (items + per - 1) / per;
+  pl.score_splits = sms * 8 / pl.units < 1 ? 1 : sms * 8 / pl.units;
+  if (pl.score_splits > (pl.groups + kWarps - 1) / kWarps) pl.score_splits = (pl.groups + kWarps - 1) / kWarps;
+  if ((long long)pl.units * pl.splits > 0x7fffffffLL || (long long)pl.units * pl.score_splits > 0x7fffffffLL) return pl;
+  size_t used = 0;
+  auto take = [&](size_t bytes) {
+    const size_t r = used;
+    used += (bytes + 255) / 256 * 256;
+    return r;
+  };
+  if (pl.full) {
+    take((size_t)pl.units * pl.groups * (a->G / 8) * pl.NT * 32 * 8);      // scores, at 0
+    pl.off_gmax = take((size_t)pl.units * pl.groups * RT * 4);
+  }
+  if (pl.splits > 1) {
+    pl.off_part = take((size_t)pl.units * pl.splits * RT * a->D * 4);
+    pl.off_ml = take((size_t)pl.units * pl.splits * RT * 8);
+  }
+  pl.bytes = used;
+  pl.use = true;
+  return pl;
+}
+
+// `chained`: the launch may begin while the one before it on the stream is still running (its kernel waits with pdl_wait)
+template <typename K, typename... A>
+int launch(K kernel, int grid, int threads, bool chained, cudaStream_t stream, A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(threads);
+  cfg.stream = stream;
+  cudaLaunchAttribute attr = {};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = chained ? 1 : 0;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, args...);
+  return e == cudaSuccess ? INTFA_OK : set_error(INTFA_ERR_CUDA, "decode launch: %s", cudaGetErrorString(e));
+}
+
+template <int D, int NT>
+int run(const Plan& pl, const DParams& p, cudaStream_t stream) {
+  int rc;
+  const int grid = pl.units * pl.splits;
+  if (pl.full) {
+    if ((rc = launch(scores_kernel<D, NT>, pl.units * pl.score_splits, kThreads, false, stream, p, pl.score_splits))) return rc;
+    if ((rc = launch(pv_full_kernel<D, NT>, grid, kThreads, true, stream, p))) return rc;
+  } else {
+    if ((rc = launch(pv_half_kernel<D, NT>, grid, kThreads, false, stream, p))) return rc;
+  }
+  if (pl.splits == 1) return INTFA_OK;
+  return pl.full ? launch(combine_kernel<true, D>, pl.units * 8 * NT, D / 4, true, stream, p, 8 * NT)
+                 : launch(combine_kernel<false, D>, pl.units * 8 * NT, D / 4, true, stream, p, 8 * NT);
+}
+
+}  // namespace
+
+size_t decode_workspace_bytes(const IntfaFwdParams* a) {
+  const int sms = sm_count_cached();
+  return make_plan(a, sms > 0 ? sms : 148).bytes;
+}
+
+bool decode_dispatch(const IntfaFwdParams* a, cudaStream_t stream, int* rc) {
+  const int sms = sm_count_cached();
+  if (sms <= 0) return false;
+  const Plan pl = make_plan(a, sms);
+  if (!pl.use || a->workspace_bytes < pl.bytes || (pl.bytes > 0 && !a->workspace)) return false;
+  DParams p;
+  p.q = static_cast<const int8_t*>(a->q); p.k = static_cast<const int8_t*>(a->k); p.v = a->v; p.o = a->o;
+  p.qB = a->q_stride[0]; p.qH = a->q_stride[1]; p.qN = a->q_stride[2];
+  p.kB = a->k_stride[0]; p.kH = a->k_stride[1]; p.kN = a->k_stride[2];
+  p.vB = a->v_stride[0]; p.vH = a->v_stride[1]; p.vN = a->v_stride[2];
+  p.oB = a->o_stride[0]; p.oH = a->o_stride[1]; p.oN = a->o_stride[2];
+  p.qs = a->q_scale; p.ks = a->k_scale; p.vs = a->v_scale;
+  p.qsB = a->qs_stride[0]; p.qsH = a->qs_stride[1]; p.ksB = a->ks_stride[0]; p.ksH = a->ks_stride[1];
+  p.vsB = a->vs_stride[0]; p.vsH = a->vs_stride[1]; p.vsD = a->vs_stride[2];
+  p.scale_f16 = a->scale_f16;
+  p.o_bf16 = a->o_dtype == INTFA_OUT_BF16;
+  p.causal = a->causal ? 1 : 0;
+  p.H = a->H; p.Hkv = a->H_kv > 0 ? a->H_kv : a->H; p.ratio = p.H / p.Hkv; p.Nq = a->Nq;
+  p.R = p.ratio * p.Nq; p.tiles = pl.tiles;
+  p.nvis = pl.nvis;
+  p.limit0 = a->q_offset - a->kv_offset;
+  p.c = a->sm_scale * 1.44269504f;
+  p.G = a->G; p.groups = pl.groups; p.splits = pl.splits; p.per_split = pl.per_split;
+  p.lse = a->lse_out;
+  char* ws = static_cast<char*>(a->workspace);
+  p.scores = reinterpret_cast<float*>(ws);
+  p.gmax = reinterpret_cast<float*>(ws + pl.off_gmax);
+  p.part = reinterpret_cast<float*>(ws + pl.off_part);
+  p.part_ml = reinterpret_cast<float*>(ws + pl.off_ml);
+  *rc = a->D == 128 ? (pl.NT == 2 ? run<128, 2>(pl, p, stream) : run<128, 1>(pl, p, stream))
+                    : (pl.NT == 2 ? run<64, 2>(pl, p, stream) : run<64, 1>(pl, p, stream));
+  return true;
+}
+
+}  // namespace intfa

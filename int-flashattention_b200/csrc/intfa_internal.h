@@ -41,6 +41,9 @@ int set_error(int code, const char* fmt, ...);
 // SM count of the current device, cached per device; <=0 on failure.
 int sm_count_cached();
 
+// Few query rows against many keys (intfa_decode.cu).  Returns false where the call is not one for that path.
+bool decode_dispatch(const IntfaFwdParams* a, cudaStream_t stream, int* rc);
+size_t decode_workspace_bytes(const IntfaFwdParams* a);
 int fwd_dispatch(const IntfaFwdParams* a, cudaStream_t stream);
 int quant_pertoken(const void* x, const int64_t* st, void* x8, float* scale, int B, int H, int N, int D,
                    cudaStream_t stream);

@@ -273,6 +273,12 @@ PyObject* forward(IntfaFwdParams& P, Options& o, c10::Device dev, bool causal, d
   }
   P.debug_wait_limit_kcycles = o.wait_kcycles;
   P.debug_skip_k_load = o.skip_k;
+  at::Tensor ws;
+  if (const size_t bytes = intfa_fwd_workspace_bytes(&P)) {
+    ws = empty({static_cast<int64_t>(bytes)}, at::kByte, dev);
+    P.workspace = ws.data_ptr();
+    P.workspace_bytes = bytes;
+  }
   const at::Tensor st = status_word(dev);
   P.status = st.data_ptr<int>();
   void* stream = stream_of(dev);

@@ -1,0 +1,59 @@
+"""GPU: a few query rows against a longer K/V cache (the path that packs the heads of a K/V head into one row tile and splits
+the keys over the GPU), against the CPU oracle.  Sizes sit at the edges of its tiles: 1 to 16 and more packed rows, key counts
+around the 8-, 32-, 64-key steps and the groups of G keys, one split and many, and the last row count the path takes."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+CASES = [
+    # variant, B, Hkv, ratio, Nq, Nk, D, G, causal, scales
+    ("full", 1, 1, 1, 1, 1, 128, 128, True, "fp32"),            # one key
+    ("full", 2, 2, 4, 1, 129, 128, 128, True, "fp16"),
+    ("full", 1, 2, 8, 1, 1000, 128, 64, True, "fp32"),          # exactly 8 rows
+    ("full", 1, 2, 4, 4, 4097, 128, 128, True, "fp16"),         # 16 rows, many splits, odd rows of the scales
+    ("full", 1, 1, 8, 5, 777, 128, 128, True, "fp32"),          # 40 rows: three row tiles
+    ("full", 1, 3, 1, 32, 65, 64, 64, True, "fp32"),            # the most rows a head
+    ("full", 1, 2, 1, 3, 2500, 64, 128, False, "fp16"),
+    ("full", 1, 1, 1, 2, 20000, 64, 64, True, "fp32"),          # more groups than one CTA may take
+    ("half", 1, 1, 1, 1, 1, 64, 128, True, "fp32"),
+    ("half", 2, 2, 4, 1, 31, 128, 128, True, "fp16"),
+    ("half", 1, 2, 8, 2, 1025, 128, 128, True, "fp32"),
+    ("half", 1, 1, 4, 9, 4100, 128, 64, True, "fp16"),          # 36 rows
+    ("half", 1, 3, 1, 32, 200, 64, 128, False, "fp32"),
+    ("half", 1, 2, 4, 1, 9000, 64, 128, True, "fp32"),
+]
+
+
+@pytest.mark.parametrize("variant,B,Hkv,ratio,Nq,Nk,D,G,causal,scales", CASES)
+def test_few_rows_against_a_cache(variant, B, Hkv, ratio, Nq, Nk, D, G, causal, scales, pkg, oracle):
+    dev = torch.device("cuda:0")
+    g = torch.Generator().manual_seed(Nk + 7 * Nq + D)
+    H = Hkv * ratio
+    q = torch.randn(B, H, Nq, D, generator=g).half()
+    k, v = (torch.randn(B, Hkv, Nk, D, generator=g).half() for _ in range(2))
+    k[:, :, Nk // 2:] *= 2                                       # the running maximum moves late as well
+    q8, qs = oracle.quant_pertoken(q)
+    k8, ks = oracle.quant_pertoken(k)
+    sm, off = D ** -0.5, (max(0, Nk - Nq) if causal else 0)
+    rep = lambda t: t.repeat_interleave(ratio, dim=1)
+    if scales == "fp32":
+        qs, ks = qs.float(), ks.float()
+    if variant == "full":
+        v8, vs = oracle.quant_perchannel(v)
+        ref, (m, l, _) = oracle.int8_attention(q8, rep(k8), rep(v8), qs, rep(ks), rep(vs), causal, sm, variant="full", G=G,
+                                               q_offset=off, return_state=True)
+        args = [t.to(dev) for t in (q8, k8, v8, qs, ks, vs)]
+        out, lse = pkg.attention_full_int8(*args, causal, sm, G=G, q_offset=off, return_lse=True)
+    else:
+        ref, (m, l, _) = oracle.int8_attention(q8, rep(k8), rep(v), qs, rep(ks), None, causal, sm, variant="half", G=G,
+                                               q_offset=off, return_state=True)
+        args = [t.to(dev) for t in (q8, k8, v, qs, ks)]
+        out, lse = pkg.attention_int8(*args, causal, sm, G=G, q_offset=off, return_lse=True)
+    pkg.check_status()
+    e = oracle.err_metrics(out.cpu(), ref)
+    assert e["max_abs"] <= 4e-3 and e["mean_rel"] <= 3e-4, e
+    assert (lse.cpu() - oracle.log2_lse(m, l)).abs().max() < 1e-3
+    fn = pkg.attention_full_int8 if variant == "full" else pkg.attention_int8
+    again = fn(*args, causal, sm, G=G, q_offset=off, out_dtype=torch.bfloat16)
+    assert ((again.float() - out.float()).abs() <= out.float().abs() * (2.0 ** -8 + 2.0 ** -11) + 1e-7).all()
