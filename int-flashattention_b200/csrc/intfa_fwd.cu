@@ -184,11 +184,7 @@ static int launch_pipe(const IntfaFwdParams* a, const KParams& kp, cudaStream_t 
   int rc;
   if ((rc = make_tmap(&tmQ, a->q, 1, a->q_stride, a->B, a->H, a->Nq, hd, C::QK_ROWB, kBM, swzQK))) return rc;
   if ((rc = make_tmap(&tmK, a->k, 1, a->k_stride, a->B, kv_heads(a), a->Nk, hd, C::QK_ROWB, G, swzQK))) return rc;
-  if constexpr (C::BYTE_PV) {
-    if ((rc = make_tmap(&tmV, a->v, 1, a->v_stride, a->B, kv_heads(a), a->Nk, hd, D, G, swzV))) return rc;
-  } else {
-    if ((rc = make_tmap(&tmV, a->v, 2, a->v_stride, a->B, kv_heads(a), a->Nk, hd, D >= 64 ? 64 : D, G, swzV))) return rc;
-  }
+  if ((rc = make_tmap(&tmV, a->v, C::BYTE_PV ? 1 : 2, a->v_stride, a->B, kv_heads(a), a->Nk, hd, C::V_BOXCH, G, swzV))) return rc;
   auto kern = intfa_fwd_pipe_kernel<D, G, FULL, PRNE, RAGGED, DQ, F8V>;
   static std::atomic<bool> attr_done[64];     // per instantiation and device (the attribute is per device)
   int dev = 0;
@@ -252,10 +248,11 @@ int fwd_dispatch(const IntfaFwdParams* a, cudaStream_t stream) {
     if (full) return rne ? launch_pipe<DD, GG, true, true, false, DQ>(a, kp, stream)                     \
                          : launch_pipe<DD, GG, true, false, false, DQ>(a, kp, stream);                   \
     if constexpr (HALF) {                                                                                \
-      if (f8v) return ragged ? launch_pipe<DD, GG, false, false, true, DQ, true>(a, kp, stream)          \
-                             : launch_pipe<DD, GG, false, false, false, DQ, true>(a, kp, stream);        \
-      return ragged ? launch_pipe<DD, GG, false, false, true, DQ>(a, kp, stream)                         \
-                    : launch_pipe<DD, GG, false, false, false, DQ>(a, kp, stream);                       \
+      constexpr int DH = DQ;       /* (half-int8 takes all channels in one pass) */                      \
+      if (f8v) return ragged ? launch_pipe<DH, GG, false, false, true, DH, true>(a, kp, stream)          \
+                             : launch_pipe<DH, GG, false, false, false, DH, true>(a, kp, stream);        \
+      return ragged ? launch_pipe<DH, GG, false, false, true, DH>(a, kp, stream)                         \
+                    : launch_pipe<DH, GG, false, false, false, DH>(a, kp, stream);                       \
     }                                                                                                    \
   }
   INTFA_CASE(128, 128, 128, 128, true)
@@ -268,7 +265,7 @@ int fwd_dispatch(const IntfaFwdParams* a, cudaStream_t stream) {
   INTFA_CASE(16, 32, 32, 32, false)      // head dim 16: the 32-wide kernel on zero-filled tiles
   INTFA_CASE(16, 32, 64, 32, true)
   INTFA_CASE(16, 32, 128, 32, true)
-  INTFA_CASE(256, 128, 128, 256, false)  // head dim 256: two passes of 128 V channels; fp16 V tiles at G = 128 do not fit
+  INTFA_CASE(256, 128, 128, 256, false)  // head dim 256: full-int8 in two passes of 128 V channels; fp16 V tiles at G = 128 do not fit
   INTFA_CASE(256, 128, 64, 256, true)
 #undef INTFA_CASE
   return set_error(INTFA_ERR_UNSUPPORTED, "unsupported (D=%d, G=%d, %s): G is 64 or 128 (32 too for full-int8 at head dims 16 and 32; half-int8 at head dim 256: 64 only)", D, G, full ? "full-int8" : "half-int8");
