@@ -6,9 +6,9 @@
 // reference's BLOCK_N, flash_atten_full_int8.py:30-70).
 //
 // One kernel family, intfa_fwd_pipe_kernel (intfa_fwd_pipe.cuh), serves full-int8 and half-int8 at head dims
-// 16 to 256: one CTA of 512 threads per SM -- TMA producer, two MMA-issuing warps (S = Q K^T with tcgen05.mma
-// kind::i8 into int32 TMEM accumulators; O_j = P V with kind::i8, or kind::f16 for half-int8), two softmax groups
-// on alternate KV steps, accumulator warps.
+// 16 to 256: one CTA per SM -- TMA producer, two MMA-issuing warps (S = Q K^T with tcgen05.mma
+// kind::i8 into int32 TMEM accumulators; O_j = P V with kind::i8, or kind::f16 for half-int8), softmax groups
+// that take the KV steps in turn, accumulator warps.
 //
 // Arithmetic contract (what the parity tests pin; reference lines in parentheses):
 //   s   = (fp32(S32) * s_q[row]) * s_k[col]                 (flash_atten_full_int8.py:36-38)
@@ -174,7 +174,7 @@ static constexpr CUtensorMapSwizzle swizzle_of_row_bytes(int bytes) {
 
 // One CTA per SM.  The tensor maps describe the tensors with their own head dim (a->D); the boxes are as wide as the
 // kernel's tiles, so at head dim 16 the upper half of every 32-wide box lies outside the tensor and arrives as zeros.
-template <int D, int G, bool FULL, bool PRNE, bool RAGGED, int DQ = D, bool F8V = false>
+template <int D, int G, bool FULL, bool PRNE, bool RAGGED, int DQ = D, bool F8V = false, bool POLITE = false>
 static int launch_pipe(const IntfaFwdParams* a, const KParams& kp, cudaStream_t stream) {
   using C = PipeCfg<D, G, FULL, DQ, F8V>;
   static_assert(C::SMEM_BYTES <= 227 * 1024, "shared memory");
@@ -185,7 +185,7 @@ static int launch_pipe(const IntfaFwdParams* a, const KParams& kp, cudaStream_t 
   if ((rc = make_tmap(&tmQ, a->q, 1, a->q_stride, a->B, a->H, a->Nq, hd, C::QK_ROWB, kBM, swzQK))) return rc;
   if ((rc = make_tmap(&tmK, a->k, 1, a->k_stride, a->B, kv_heads(a), a->Nk, hd, C::QK_ROWB, G, swzQK))) return rc;
   if ((rc = make_tmap(&tmV, a->v, C::BYTE_PV ? 1 : 2, a->v_stride, a->B, kv_heads(a), a->Nk, hd, C::V_BOXCH, G, swzV))) return rc;
-  auto kern = intfa_fwd_pipe_kernel<D, G, FULL, PRNE, RAGGED, DQ, F8V>;
+  auto kern = intfa_fwd_pipe_kernel<D, G, FULL, PRNE, RAGGED, DQ, F8V, POLITE>;
   static std::atomic<bool> attr_done[64];     // per instantiation and device (the attribute is per device)
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return set_error(INTFA_ERR_CUDA, "cannot query the current device");
@@ -201,7 +201,7 @@ static int launch_pipe(const IntfaFwdParams* a, const KParams& kp, cudaStream_t 
   KParams kpl = kp;
   kpl.tile_counter = nullptr;
   if (kp.num_tiles > grid && (rc = next_tile_counter(&kpl.tile_counter))) return rc;
-  kern<<<grid, kPipeThreads, C::SMEM_BYTES, stream>>>(tmQ, tmK, tmV, kpl);
+  kern<<<grid, C::THREADS, C::SMEM_BYTES, stream>>>(tmQ, tmK, tmV, kpl);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return set_error(INTFA_ERR_CUDA, "kernel launch: %s", cudaGetErrorString(e));
   return INTFA_OK;
@@ -241,6 +241,8 @@ int fwd_dispatch(const IntfaFwdParams* a, cudaStream_t stream) {
   // (so do calls with one v_scale row per KV tile: the code for them is compiled into that instantiation only)
   const bool ragged = (a->Nq % kBM) != 0 || (a->Nk % a->G) != 0 || a->vs_stride_blk != 0;
   // HD: head dim of the call; DD, DQ: the kernel's tile width and Q/K width for it; HALF: half-int8 built for this G
+  // (full-int8, head dim 128, non-causal: an instantiation whose service warps poll less, see the kernel)
+  if (D == 128 && G == 128 && full && !rne && !ragged && !kp.causal) return launch_pipe<128, 128, true, false, false, 128, false, true>(a, kp, stream);
 #define INTFA_CASE(HD, DD, GG, DQ, HALF)                                                                 \
   if (D == HD && G == GG) {                                                                              \
     if (full && ragged) return rne ? launch_pipe<DD, GG, true, true, true, DQ>(a, kp, stream)            \

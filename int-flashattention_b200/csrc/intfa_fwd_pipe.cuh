@@ -1,19 +1,19 @@
 // INT8 attention forward (full-int8 and half-int8): ONE CTA per SM, one 128-row query tile at a time.
 // (Included by intfa_fwd.cu inside namespace intfa, after the shared helpers.)
 //
-// 512 threads:
+// 512 threads with two softmax groups, 640 with three (PipeCfg::NGRP):
 //   warp 0        TMA producer (Q once per work item; K and V through rings of shared-memory stages); it also draws
 //                 the work items: the CTA's own index first, then from a global counter
 //   warp 1        MMA issuer for S = Q K^T (whole warp runs the loop, one elected lane issues): up to three KV steps
 //                 ahead of the softmax groups, into S buffer (step mod 3)
 //   warp 2        TMEM allocator; then loads the K scales (fp32 or fp16, rows of any alignment) into a ring of their own
 //   warp 3        MMA issuer for O_j = P V
-//   warps 4-7     softmax group 0, warps 8-11 softmax group 1: one thread per query row.  The groups take
-//                 ALTERNATE KV steps (group g owns the steps whose running index is g mod 2), each with its own
-//                 P buffer in shared memory, so that on every scheduler one warp is in pass A (dequantise, row
-//                 max: FMA pipe) while the other is in pass B (exp2, P: exp2 unit).  The running max m of a row
-//                 travels between the two threads that own it through shared memory, once per step.
-//   warps 12-15   accumulator update and epilogue, one thread per query row:
+//   warps 4-7, 8-11 (, 12-15)   softmax groups 0, 1 (, 2): one thread per query row.  The groups take the KV steps in
+//                 TURN (group g owns the steps whose running index is g mod NGRP), each with its own P buffer in shared
+//                 memory, so that on every scheduler one warp is in pass A (dequantise, row max: FMA pipe) while
+//                 another is in pass B (exp2, P: exp2 unit).  The running max m of a row travels between the threads
+//                 that own it through shared memory, once per step.
+//   the last 4 warps   accumulator update and epilogue, one thread per query row:
 //                 full-int8: A = A*alpha + fp32(O_j) with the fp32 row A in REGISTERS and O_j (int32) in TMEM;
 //                 half-int8: P V (fp16 MMA) accumulates straight into an fp32 accumulator in TMEM, these warps
 //                 multiply the row by alpha beforehand when some alpha of the warp's 32 rows is not 1.
@@ -24,12 +24,7 @@
 // The arithmetic contract is at the top of intfa_fwd.cu.
 #pragma once
 
-constexpr int kPipeThreads = 512;
-constexpr int kPipeSoftmaxThreads = 256;
 constexpr int kPipeCorrThreads = 128;
-// Registers: the CTA is launched with kPipeLaunchRegs per thread and setmaxnreg only moves registers around
-// INSIDE that allocation -- an increase beyond it would block for ever, hence the static_assert in PipeCfg.
-constexpr int kPipeLaunchRegs = (65536 / kPipeThreads) / 8 * 8;
 constexpr int kPipeServiceRegs = 40;
 
 // D: channels of V and of the accumulator that one pass covers (and the width the tensor-core tiles are built for);
@@ -44,6 +39,15 @@ template <int D, int G, bool FULL, int DQ = D, bool F8V = false>
 struct PipeCfg {
   static_assert(!(FULL && F8V), "fp8 V belongs to the half-int8 op");
   static constexpr bool BYTE_PV = FULL || F8V;                     // P and V elements are one byte
+  // Softmax groups of 128 threads.  Three (with 96 registers a thread, 16-column buffers) hide the hand-overs better than two
+  // (152 registers, 32 columns) where P is one byte and a step is 128 wide: batch 2, 32/8 heads, 3072 tokens, full-int8
+  // causal 267 -> 240 us, fp8 V causal 116 -> 105 us.  fp16 P (a third buffer leaves two K stages), 64-column steps and head
+  // dim 256 lose: 337 -> 351 us, 737 -> 767 us, 216 -> 237 us.
+  static constexpr int NGRP = (BYTE_PV && G == 128 && D == 128 && DQ == 128) ? 3 : 2;
+  static constexpr int THREADS = 256 + 128 * NGRP;
+  // Registers: the CTA is launched with LAUNCH_REGS per thread and setmaxnreg only moves registers around
+  // INSIDE that allocation -- an increase beyond it would block for ever, hence the static_assert below.
+  static constexpr int LAUNCH_REGS = (65536 / THREADS) / 8 * 8;
   static_assert(DQ == D || (DQ == 256 && D == 128), "head dims");
   static constexpr int NVH = DQ / D;                               // passes per query tile
   static constexpr int QK_ROWB = DQ < 128 ? DQ : 128;              // Q and K sit in shared memory as panels of [rows][QK_ROWB bytes]
@@ -72,30 +76,32 @@ struct PipeCfg {
   // non-causal case more (instruction cache) than it gives.
   static constexpr bool BAND_FAST = G == 128;
   // instructions of never-executed filler between the softmax passes (see intfa_fwd_pipe_softmax.inc), the best of a sweep in
-  // steps of 1 KB for each kind of instantiation (`ragged`: the one that masks partial tiles).  With explicit shared-memory
-  // accesses it matters less than it did: +-1.5 % non-causal, +-4 % causal; the ragged one 294 us (256) to 343 us (0) at
-  // batch 2, 32/8 heads, 3001 tokens, causal.
-  __host__ __device__ static constexpr int code_filler_of(bool ragged) { return ragged ? 256 : BAND_FAST ? (FULL ? 448 : 384) : (FULL && D == 64) ? 0 : 128; }
+  // steps of 1 KB for each kind of instantiation (`ragged`: masks partial tiles; `polite`: see the kernel).  Between the best
+  // and the worst of a sweep lie 1 to 2 % non-causal, 5 to 15 % causal.
+  __host__ __device__ static constexpr int code_filler_of(bool ragged, bool polite) {
+    return NGRP == 3 ? (!FULL ? 192 : ragged ? 64 : polite ? 128 : 256)
+         : ragged ? 256 : G == 128 ? (FULL ? 448 : 384) : D == 256 ? 256 : (FULL && D == 64) ? 0 : 128;
+  }
   static constexpr bool MORE_SOFTMAX_REGS = !FULL || G == 128;
-  static constexpr int SOFTMAX_REGS = MORE_SOFTMAX_REGS ? 152 : 136;
-  static constexpr int CORR_REGS = MORE_SOFTMAX_REGS ? 168 : 184;
-  static_assert(128 * kPipeServiceRegs + kPipeSoftmaxThreads * SOFTMAX_REGS + kPipeCorrThreads * CORR_REGS <=
-                    kPipeThreads * kPipeLaunchRegs, "setmaxnreg budget exceeds the registers the CTA is launched with");
+  static constexpr int SOFTMAX_REGS = NGRP == 3 ? (FULL ? 96 : 112) : MORE_SOFTMAX_REGS ? 152 : 136;
+  static constexpr int CORR_REGS = NGRP == 3 ? (FULL ? 152 : 96) : MORE_SOFTMAX_REGS ? 168 : 184;
+  static_assert(128 * kPipeServiceRegs + 128 * NGRP * SOFTMAX_REGS + kPipeCorrThreads * CORR_REGS <= THREADS * LAUNCH_REGS,
+                "setmaxnreg budget exceeds the registers the CTA is launched with");
   static constexpr int OFF_Q = 0;
   static constexpr int OFF_K = OFF_Q + Q_BYTES;
   static constexpr int OFF_V = OFF_K + NSK * K_BYTES;
-  static constexpr int OFF_P = OFF_V + NSV * V_BYTES;             // two P buffers
-  static constexpr int OFF_KS = OFF_P + 2 * P_BYTES;
+  static constexpr int OFF_P = OFF_V + NSV * V_BYTES;             // a P buffer per softmax group
+  static constexpr int OFF_KS = OFF_P + NGRP * P_BYTES;
   static constexpr int OFF_VSD = OFF_KS + NKS * KS_BYTES;         // s_v/127 per channel
   static constexpr int OFF_HM = OFF_VSD + D * 4;                  // [2 groups][128] float: running max after the group's latest step
-  static constexpr int OFF_RS = OFF_HM + 2 * 128 * 4;             // [4][128] float: row sum of P of step j, for the accumulator warps
+  static constexpr int OFF_RS = OFF_HM + NGRP * 128 * 4;             // [4][128] float: row sum of P of step j, for the accumulator warps
                                                                    //   (!L_IN_ACC: [2 groups][128] float, l after the group's latest step)
   static constexpr int OFF_ALPHA = OFF_RS + 4 * 128 * 4;          // [4][128] float: alpha of step j, for the accumulator warps
   static constexpr int OFF_FIN = OFF_ALPHA + 4 * 128 * 4;         // [2][128] float2: final running max of a work item (.x)
   static constexpr int OFF_MAGIC = OFF_FIN + 2 * 128 * 8;          // 4 KB constant fp16 operand of the "arm" MMA
   static constexpr int MAGIC_BYTES = 4096;
   static constexpr int OFF_BAR = OFF_MAGIC + MAGIC_BYTES;
-  static constexpr int NUM_BARS = 18 + 2 * NSK + 2 * NSV + 8 + 4 + 2 * NSB;
+  static constexpr int NUM_BARS = 20 + 2 * NSK + 2 * NSV + 8 + 4 + 2 * NSB;
   static constexpr int OFF_MISC = OFF_BAR + NUM_BARS * 8;
   static constexpr int SMEM_BYTES = OFF_MISC + 32 + 1024;
   // S buffer b at COL_S + b*G; then O_j (full-int8: the accumulator itself lives in registers) or the fp32
@@ -130,8 +136,11 @@ enum PipeWait { PW_TILE = 32, PW_QE, PW_KE, PW_VE, PW_QF, PW_KF, PW_VF, PW_SFREE
 
 // RAGGED: Nq / Nk are not multiples of 128 / G -- the last query tile and the last KV step are partial.  A separate
 // instantiation, so that the code of the common case stays as small as it was (instruction cache).
-template <int D, int G, bool FULL, bool PRNE, bool RAGGED, int DQ = D, bool F8V = false>
-__global__ void __launch_bounds__(kPipeThreads, 1)
+// POLITE: the service warps (0 to 3) sleep 20 ns between two looks at a barrier.  The dispatch ports are 88 % busy in steady
+// state (three groups, full-int8), so their polls cost: 341 -> 330 us non-causal.  Causal work items are short and wait for
+// the issue warps instead: 238 -> 245 us, so they keep polling.
+template <int D, int G, bool FULL, bool PRNE, bool RAGGED, int DQ = D, bool F8V = false, bool POLITE = false>
+__global__ void __launch_bounds__((PipeCfg<D, G, FULL, DQ, F8V>::THREADS), 1)
 intfa_fwd_pipe_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                       const __grid_constant__ CUtensorMap tmV, const KParams p) {
   using C = PipeCfg<D, G, FULL, DQ, F8V>;
@@ -145,20 +154,21 @@ intfa_fwd_pipe_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
   const uint32_t bar0 = smem_u32(smem + C::OFF_BAR);
   auto BAR = [&](int i) { return bar0 + 8u * i; };
   // mbarriers.  "commit" = arrived on by tcgen05.commit, i.e. when the MMAs issued so far are done.
+  constexpr int NGRP = C::NGRP;
   constexpr int B_QFULL = 0;      // TMA: Q tile landed
   constexpr int B_QEMPTY = 1;     // commit: last Q K^T of the work item done
-  constexpr int B_PFULL = 4;      // [2] softmax group b (4 warps): P in shared-memory buffer b, and S buffer b read out
-  constexpr int B_PFREE = 6;      // [2] commit: the P V that read P buffer b is done
+  constexpr int B_PFULL = 2;      // [NGRP] softmax group b (4 warps): P in shared-memory buffer b, and S buffer b read out
+  constexpr int B_PFREE = 5;      // [NGRP] commit: the P V that read P buffer b is done
   constexpr int B_OFULL = 8;      // commit: O_j = P V in TMEM
   constexpr int B_OFREE = 9;      // accumulator warps (4): O_j read out
-  constexpr int B_HL = 16;        // [2] !L_IN_ACC: softmax group g (4 warps): row sum after its step published
   constexpr int B_FIN = 10;       // [2] softmax (4 warps of one group): final (m, l) of the work item published; one
                                   //     barrier per slot, so that a short next work item cannot complete it twice
                                   //     before a slow accumulator warp has waited for the first completion
   constexpr int B_FINFREE = 12;   // [2] accumulator warps (4): they have read them
-  constexpr int B_HM = 14;        // [2] softmax group g (4 warps): running max after its step published
-  constexpr int B_KFULL = 18, B_KEMPTY = 18 + NSK, B_VFULL = 18 + 2 * NSK, B_VEMPTY = 18 + 2 * NSK + NSV;
-  constexpr int B_TILE = 18 + 2 * NSK + 2 * NSV, B_TDONE = B_TILE + 4;
+  constexpr int B_HM = 14;        // [NGRP] softmax group g (4 warps): running max after its step published
+  constexpr int B_HL = 17;        // [NGRP] !L_IN_ACC: softmax group g (4 warps): row sum after its step published
+  constexpr int B_KFULL = 20, B_KEMPTY = 20 + NSK, B_VFULL = 20 + 2 * NSK, B_VEMPTY = 20 + 2 * NSK + NSV;
+  constexpr int B_TILE = 20 + 2 * NSK + 2 * NSV, B_TDONE = B_TILE + 4;
   constexpr int B_AFULL = B_TDONE + 4;   // [4] half-int8: alpha of step j (slot j mod 4) published, for the accumulator warps
   constexpr int B_SFULL = B_AFULL + 4;   // [3] commit: S = Q K^T in TMEM buffer b
   constexpr int B_SFREE = B_SFULL + NSB; // [3] softmax group of the step (4 warps): S buffer b read out for good
@@ -169,12 +179,14 @@ intfa_fwd_pipe_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
   if (threadIdx.x == 0) {
     mbar_init(BAR(B_QFULL), 1);
     mbar_init(BAR(B_QEMPTY), 1);
-    for (int b = 0; b < 2; ++b) {
+    for (int b = 0; b < NGRP; ++b) {
       mbar_init(BAR(B_PFULL + b), 4);
       mbar_init(BAR(B_PFREE + b), 1);
-      mbar_init(BAR(B_FINFREE + b), 4);
       mbar_init(BAR(B_HM + b), 4);
       mbar_init(BAR(B_HL + b), 4);
+    }
+    for (int b = 0; b < 2; ++b) {
+      mbar_init(BAR(B_FINFREE + b), 4);
       mbar_init(BAR(B_FIN + b), 4);
     }
     mbar_init(BAR(B_OFULL), 1);
@@ -193,7 +205,7 @@ intfa_fwd_pipe_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
     }
     for (int i = 0; i < 4; ++i) {
       mbar_init(BAR(B_TILE + i), 1);
-      mbar_init(BAR(B_TDONE + i), 15);       // 2 MMA warps, the scale loader, 8 softmax warps, 4 accumulator warps
+      mbar_init(BAR(B_TDONE + i), 7 + 4 * NGRP);       // 2 MMA warps, the scale loader, accumulator and softmax warps
       mbar_init(BAR(B_AFULL + i), 4);
     }
     abort_flag[0] = 0;
@@ -234,7 +246,7 @@ intfa_fwd_pipe_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
   auto next_tile = [&](uint32_t& seq, bool ack, bool whole_warp) -> int {
     const uint32_t slot = seq & 3u, par = (seq >> 2) & 1u;
     ++seq;
-    bool got = mbar_wait(BAR(B_TILE + slot), par, abort_flag, p.status, code_hi | PW_TILE);
+    bool got = mbar_wait<POLITE>(BAR(B_TILE + slot), par, abort_flag, p.status, code_hi | PW_TILE);
     if (whole_warp) got = __all_sync(0xffffffffu, got);
     if (!got) return -1;
     const int t = tile_slot[slot];
@@ -257,7 +269,7 @@ intfa_fwd_pipe_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
       bool ok = true;
       while (ok) {
         if (tseq >= 4u) {
-          ok = mbar_wait(BAR(B_TDONE + (tseq & 3u)), ((tseq >> 2) - 1u) & 1u, abort_flag, p.status, code_hi | PW_TILE);
+          ok = mbar_wait<POLITE>(BAR(B_TDONE + (tseq & 3u)), ((tseq >> 2) - 1u) & 1u, abort_flag, p.status, code_hi | PW_TILE);
           if (!ok) break;
         }
         int tile;
@@ -284,7 +296,7 @@ intfa_fwd_pipe_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         if (tile < 0) break;
         const TileInfo t = decode_tile<RAGGED, NVH>(p, tile, G);
         if (t.nsteps == 0) continue;
-        ok = mbar_wait(BAR(B_QEMPTY), (tile_it & 1) ^ 1, abort_flag, p.status, code_hi | PW_QE);
+        ok = mbar_wait<POLITE>(BAR(B_QEMPTY), (tile_it & 1) ^ 1, abort_flag, p.status, code_hi | PW_QE);
         if (!ok) break;
         mbar_expect_tx(BAR(B_QFULL), C::Q_BYTES);
 #pragma unroll
@@ -292,7 +304,7 @@ intfa_fwd_pipe_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
           tma_load_4d(sQ + pn * (kBM * C::QK_ROWB), &tmQ, BAR(B_QFULL), pn * C::QK_ROWB, t.mb * kBM, t.h, t.b);
         for (int j = 0; j < t.nsteps; ++j, ++kv_it) {
           const uint32_t s = kv_it % NSK, ph = (kv_it / NSK) & 1;
-          ok = mbar_wait(BAR(B_KEMPTY + s), ph ^ 1, abort_flag, p.status, code_hi | PW_KE);
+          ok = mbar_wait<POLITE>(BAR(B_KEMPTY + s), ph ^ 1, abort_flag, p.status, code_hi | PW_KE);
           if (!ok) break;
           const int jb = kv_tile_of_step(p, j, t.nsteps);
           if (p.skip_k_load == 0 || kv_it + 1 != (uint32_t)p.skip_k_load) {      // (test hook: a K tile that never arrives)
@@ -302,7 +314,7 @@ intfa_fwd_pipe_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
               tma_load_4d(sK + s * C::K_BYTES + pn * (G * C::QK_ROWB), &tmK, BAR(B_KFULL + s), pn * C::QK_ROWB, jb * G, t.hk, t.b);
           }
           const uint32_t sv = kv_it % NSV, phv = (kv_it / NSV) & 1;
-          ok = mbar_wait(BAR(B_VEMPTY + sv), phv ^ 1, abort_flag, p.status, code_hi | PW_VE);
+          ok = mbar_wait<POLITE>(BAR(B_VEMPTY + sv), phv ^ 1, abort_flag, p.status, code_hi | PW_VE);
           if (!ok) break;
           mbar_expect_tx(BAR(B_VFULL + sv), C::V_BYTES);
 #pragma unroll
@@ -336,7 +348,7 @@ intfa_fwd_pipe_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
       for (int j = -1; j < t.nsteps; ++j) {
         if (j >= 0) {
           const uint32_t s = kv_it % NSK, ph = (kv_it / NSK) & 1;
-          ok = mbar_wait_warp(BAR(B_KEMPTY + s), ph ^ 1, abort_flag, p.status, code_hi | PW_KE);
+          ok = mbar_wait_warp<POLITE>(BAR(B_KEMPTY + s), ph ^ 1, abort_flag, p.status, code_hi | PW_KE);
           if (!ok) break;
           float* slot = reinterpret_cast<float*>(smem + C::OFF_KS + (kv_it % C::NKS) * C::KS_BYTES) + lane;
 #pragma unroll
@@ -372,18 +384,18 @@ intfa_fwd_pipe_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         if (tile < 0) break;
         const TileInfo t = decode_tile<RAGGED, NVH>(p, tile, G);
         if (t.nsteps == 0) continue;
-        ok = mbar_wait_warp(BAR(B_QFULL), tile_it & 1, abort_flag, p.status, code_hi | PW_QF);
+        ok = mbar_wait_warp<POLITE>(BAR(B_QFULL), tile_it & 1, abort_flag, p.status, code_hi | PW_QF);
         if (!ok) break;
         for (int j = 0; j < t.nsteps; ++j, ++kv_it) {
           const uint32_t s = kv_it % NSK, ph = (kv_it / NSK) & 1;
           const uint32_t sb = kv_it % NSB;
           // every S_FREE is waited for exactly once, in step order, so the phases of the barriers stay in step
           while (ok && sfree_seen + NSB <= kv_it) {
-            ok = mbar_wait_warp(BAR(B_SFREE + sfree_seen % NSB), (sfree_seen / NSB) & 1, abort_flag, p.status, code_hi | PW_SFREE);
+            ok = mbar_wait_warp<POLITE>(BAR(B_SFREE + sfree_seen % NSB), (sfree_seen / NSB) & 1, abort_flag, p.status, code_hi | PW_SFREE);
             ++sfree_seen;
           }
           if (!ok) break;
-          ok = mbar_wait_warp(BAR(B_KFULL + s), ph, abort_flag, p.status, code_hi | PW_KF);
+          ok = mbar_wait_warp<POLITE>(BAR(B_KFULL + s), ph, abort_flag, p.status, code_hi | PW_KF);
           if (!ok) break;
           tc_fence_after();
           const uint64_t bd0 = descK0 + (uint64_t)(s * (C::K_BYTES >> 4));
@@ -417,15 +429,15 @@ intfa_fwd_pipe_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         const TileInfo t = decode_tile<RAGGED, NVH>(p, tile, G);
         for (int j = 0; j < t.nsteps; ++j, ++kv_it) {
           const uint32_t s = kv_it % NSV, ph = (kv_it / NSV) & 1;
-          const uint32_t b = kv_it & 1;
+          const uint32_t b = kv_it % NGRP;
           // P(j) written; V(j) landed; full-int8: O_j of the previous step has been read out, half-int8: the
           // accumulator has been brought to this step's running max (and the previous P V has landed in it).
           // (One copy of the wait code for the three.)
 #pragma unroll 1
           for (int w = 0; w < 3; ++w) {
             const uint32_t wb = w == 0 ? BAR(B_PFULL + b) : w == 1 ? BAR(B_VFULL + s) : BAR(B_OFREE);
-            const uint32_t wp = w == 0 ? ((kv_it >> 1) & 1) : w == 1 ? ph : (FULL ? ((kv_it & 1) ^ 1) : (kv_it & 1));
-            ok = mbar_wait_warp(wb, wp, abort_flag, p.status, code_hi | (w == 0 ? PW_PFULL : w == 1 ? PW_VF : PW_OFREE));
+            const uint32_t wp = w == 0 ? ((kv_it / NGRP) & 1) : w == 1 ? ph : (FULL ? ((kv_it & 1) ^ 1) : (kv_it & 1));
+            ok = mbar_wait_warp<POLITE>(wb, wp, abort_flag, p.status, code_hi | (w == 0 ? PW_PFULL : w == 1 ? PW_VF : PW_OFREE));
             if (!ok) break;
           }
           if (!ok) break;
@@ -460,11 +472,11 @@ intfa_fwd_pipe_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
       }
     }
     __syncwarp();
-  } else if (warp >= 4 && warp < 12) {
+  } else if (warp >= 4 && warp < 4 + 4 * NGRP) {
     reg_alloc<C::SOFTMAX_REGS>();
 #include "intfa_fwd_pipe_softmax.inc"
-  } else if (warp >= 12) {
-    if constexpr (C::CORR_REGS > kPipeLaunchRegs) reg_alloc<C::CORR_REGS>(); else reg_dealloc<C::CORR_REGS>();
+  } else if (warp >= 4 + 4 * NGRP) {
+    if constexpr (C::CORR_REGS > C::LAUNCH_REGS) reg_alloc<C::CORR_REGS>(); else reg_dealloc<C::CORR_REGS>();
 #include "intfa_fwd_pipe_update.inc"
   }
 

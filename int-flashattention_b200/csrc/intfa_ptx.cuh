@@ -42,36 +42,22 @@ __device__ __forceinline__ uint32_t mbar_try_wait(uint32_t bar, uint32_t parity)
       : "memory");
   return done;
 }
-// try_wait that lets the hardware park the thread for up to `ns` nanoseconds (it is woken when the
-// phase completes), so a waiting warp does not burn issue slots in a poll loop
-__device__ __forceinline__ uint32_t mbar_try_wait_parked(uint32_t bar, uint32_t parity, uint32_t ns) {
-  uint32_t done;
-  asm volatile(
-      "{\n"
-      ".reg .pred p;\n"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n"
-      "selp.b32 %0, 1, 0, p;\n"
-      "}\n"
-      : "=r"(done)
-      : "r"(bar), "r"(parity), "r"(ns)
-      : "memory");
-  return done;
-}
-
 // Bounded wait.  Every spin in the kernels goes through here: after the limit (abort_flag[1], in units of 1024
 // SM cycles; 2^21 = about one second at B200 clocks unless a test shortens it) without completion the waiter
 // records `code` in *status (first writer wins), raises the CTA-wide abort flag (abort_flag[0]) and returns
 // false; every other waiter of the CTA sees the flag on its next look and returns false as well, so the CTA
 // drains and exits.
-constexpr uint32_t kParkNs = 20000;                 // longest single park; bounds how late an abort is seen
 
 // (The slow path is small: there is one copy of it at every wait, and the instruction cache has to hold the loops of all
 // warp roles at once.)
+// POLITE: the first four warps of the CTA sleep a little between two looks.
+template <bool POLITE>
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag, int* status, int code) {
   if (mbar_try_wait(bar, parity)) return true;
   const uint32_t t0 = (uint32_t)(clock64() >> 10);
 #pragma unroll 1
-  while (!mbar_try_wait_parked(bar, parity, kParkNs)) {
+  while (!mbar_try_wait(bar, parity)) {
+    if (POLITE && threadIdx.x < 128) __nanosleep(20);
     if ((int)((uint32_t)(clock64() >> 10) - t0) > abort_flag[1]) {
       *abort_flag = 1;
       if (status) atomicCAS(status, 0, code);
@@ -82,9 +68,10 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
 }
 
 // The same wait made by a whole converged warp, with one verdict for all its lanes.
+template <bool POLITE>
 __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile int* abort_flag,
                                                int* status, int code) {
-  return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, status, code));
+  return __all_sync(0xffffffffu, mbar_wait<POLITE>(bar, parity, abort_flag, status, code));
 }
 
 // N instructions (16 bytes each) that do nothing: filler to move the code behind it in the instruction cache.
