@@ -74,13 +74,13 @@ struct PipeCfg {
   // A vectorised pass A for the causal diagonal band (otherwise those steps take the general, scalar path): compiled in
   // for 128-column KV steps, where it measured +2..5 % on causal workloads; with 64-column steps its code costs the
   // non-causal case more (instruction cache) than it gives.
-  static constexpr bool BAND_FAST = G == 128;
+  static constexpr bool BAND_FAST = G == 128 || D == 256;
   // instructions of never-executed filler between the softmax passes (see intfa_fwd_pipe_softmax.inc), the best of a sweep in
   // steps of 1 KB for each kind of instantiation (`ragged`: masks partial tiles; `polite`: see the kernel).  Between the best
   // and the worst of a sweep lie 1 to 2 % non-causal, 5 to 15 % causal.
   __host__ __device__ static constexpr int code_filler_of(bool ragged, bool polite) {
     return NGRP == 3 ? (!FULL ? 192 : ragged ? 64 : polite ? 128 : 256)
-         : ragged ? 256 : G == 128 ? (FULL ? 448 : 384) : D == 256 ? 256 : (FULL && D == 64) ? 0 : 128;
+         : ragged ? 256 : G == 128 ? (FULL ? 448 : 384) : (D == 256 || (FULL && D == 64)) ? 0 : D == 32 ? 256 : 128;
   }
   static constexpr bool MORE_SOFTMAX_REGS = !FULL || G == 128;
   static constexpr int SOFTMAX_REGS = NGRP == 3 ? (FULL ? 96 : 112) : MORE_SOFTMAX_REGS ? 152 : 136;
@@ -101,13 +101,16 @@ struct PipeCfg {
   static constexpr int OFF_MAGIC = OFF_FIN + 2 * 128 * 8;          // 4 KB constant fp16 operand of the "arm" MMA
   static constexpr int MAGIC_BYTES = 4096;
   static constexpr int OFF_BAR = OFF_MAGIC + MAGIC_BYTES;
-  static constexpr int NUM_BARS = 20 + 2 * NSK + 2 * NSV + 8 + 4 + 2 * NSB;
+  static constexpr int NUM_BARS = 23 + 2 * NSK + 2 * NSV + 8 + 4 + 2 * NSB;
   static constexpr int OFF_MISC = OFF_BAR + NUM_BARS * 8;
   static constexpr int SMEM_BYTES = OFF_MISC + 32 + 1024;
   // S buffer b at COL_S + b*G; then O_j (full-int8: the accumulator itself lives in registers) or the fp32
   // accumulator the second MMA adds into (half-int8)
   static constexpr int COL_S = 0, COL_O = NSB * G, COL_ACC = NSB * G;
-  static_assert(NSB * G + D <= 512, "TMEM columns");
+  // full-int8: two O_j buffers where TMEM has the room (64-column steps), so that P V of the next step does not wait for
+  // the accumulator warps.  (Not with three groups: alpha and the row sums of a step would be overwritten too early.)
+  static constexpr int NO = FULL && NGRP == 2 && NSB * G + 2 * D <= 512 ? 2 : 1;
+  static_assert(NSB * G + NO * D <= 512, "TMEM columns");
   static constexpr int TMEM_COLS = 512;
   static_assert(FULL || G >= 64, "half-int8: fp16 P tiles are built from 64-column blocks");
   static constexpr uint64_t SWZ_QK = (QK_ROWB == 128) ? kSwz128 : (QK_ROWB == 64) ? kSwz64 : kSwz32;
@@ -144,7 +147,7 @@ __global__ void __launch_bounds__((PipeCfg<D, G, FULL, DQ, F8V>::THREADS), 1)
 intfa_fwd_pipe_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                       const __grid_constant__ CUtensorMap tmV, const KParams p) {
   using C = PipeCfg<D, G, FULL, DQ, F8V>;
-  constexpr int NSK = C::NSK, NSV = C::NSV, NSB = C::NSB, NVH = C::NVH;
+  constexpr int NSK = C::NSK, NSV = C::NSV, NSB = C::NSB, NVH = C::NVH, NO = C::NO;
   extern __shared__ uint8_t smem_raw[];
   // (rounded up by an offset, not through an integer: the compiler then knows that all this is shared memory)
   uint8_t* smem = smem_raw + ((0u - smem_u32(smem_raw)) & 1023u);
@@ -159,8 +162,8 @@ intfa_fwd_pipe_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
   constexpr int B_QEMPTY = 1;     // commit: last Q K^T of the work item done
   constexpr int B_PFULL = 2;      // [NGRP] softmax group b (4 warps): P in shared-memory buffer b, and S buffer b read out
   constexpr int B_PFREE = 5;      // [NGRP] commit: the P V that read P buffer b is done
-  constexpr int B_OFULL = 8;      // commit: O_j = P V in TMEM
-  constexpr int B_OFREE = 9;      // accumulator warps (4): O_j read out
+  constexpr int B_OFULL = 8;      // [NO] commit: O_j = P V in TMEM buffer (step mod NO)
+  constexpr int B_OFREE = C::NUM_BARS - 3;   // [NO] accumulator warps (4): O_j read out
   constexpr int B_FIN = 10;       // [2] softmax (4 warps of one group): final (m, l) of the work item published; one
                                   //     barrier per slot, so that a short next work item cannot complete it twice
                                   //     before a slow accumulator warp has waited for the first completion
@@ -189,8 +192,10 @@ intfa_fwd_pipe_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
       mbar_init(BAR(B_FINFREE + b), 4);
       mbar_init(BAR(B_FIN + b), 4);
     }
-    mbar_init(BAR(B_OFULL), 1);
-    mbar_init(BAR(B_OFREE), 4);
+    for (int b = 0; b < NO; ++b) {
+      mbar_init(BAR(B_OFULL + b), 1);
+      mbar_init(BAR(B_OFREE + b), 4);
+    }
     for (int s = 0; s < NSK; ++s) {
       mbar_init(BAR(B_KFULL + s), 2);         // the producer's K tile and the scale loader's K scales
       mbar_init(BAR(B_KEMPTY + s), 1);
@@ -435,8 +440,8 @@ intfa_fwd_pipe_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
           // (One copy of the wait code for the three.)
 #pragma unroll 1
           for (int w = 0; w < 3; ++w) {
-            const uint32_t wb = w == 0 ? BAR(B_PFULL + b) : w == 1 ? BAR(B_VFULL + s) : BAR(B_OFREE);
-            const uint32_t wp = w == 0 ? ((kv_it / NGRP) & 1) : w == 1 ? ph : (FULL ? ((kv_it & 1) ^ 1) : (kv_it & 1));
+            const uint32_t wb = w == 0 ? BAR(B_PFULL + b) : w == 1 ? BAR(B_VFULL + s) : BAR(B_OFREE + kv_it % NO);
+            const uint32_t wp = w == 0 ? ((kv_it / NGRP) & 1) : w == 1 ? ph : (FULL ? (((kv_it / NO) & 1) ^ 1) : (kv_it & 1));
             ok = mbar_wait_warp<POLITE>(wb, wp, abort_flag, p.status, code_hi | (w == 0 ? PW_PFULL : w == 1 ? PW_VF : PW_OFREE));
             if (!ok) break;
           }
@@ -446,9 +451,10 @@ intfa_fwd_pipe_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
           const uint64_t vd0 = descV0 + (uint64_t)(s * (C::V_BYTES >> 4));
           if (elect_one()) {
             if constexpr (FULL) {
-              umma_f16(tO, descArm, descArm, C::IDESC_ARM_O, 0);
+              const uint32_t tOj = tO + kv_it % NO * D;
+              umma_f16(tOj, descArm, descArm, C::IDESC_ARM_O, 0);
 #pragma unroll
-              for (int kk = 0; kk < G / 32; ++kk) umma_i8(tO, ad0 + 2 * kk, vd0 + kk * ((32 * C::V_ROWB) >> 4), C::IDESC_PV, 1);
+              for (int kk = 0; kk < G / 32; ++kk) umma_i8(tOj, ad0 + 2 * kk, vd0 + kk * ((32 * C::V_ROWB) >> 4), C::IDESC_PV, 1);
             } else if constexpr (F8V) {
               // e5m2 P x e5m2 V (both one byte, laid out like the int8 tiles), fp32 accumulate straight into the accumulator
               const uint32_t keep = (j > 0 || p.state_in) ? 1u : 0u;
@@ -463,7 +469,7 @@ intfa_fwd_pipe_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
                 umma_f16(tA, ad0 + (uint64_t)((kk >> 2) * ((kBM * 128) >> 4) + (kk & 3) * 2), vd0 + (uint64_t)(kk * ((16 * C::V_ROWB) >> 4)),
                          C::IDESC_PV, kk > 0 ? 1u : keep);
             }
-            umma_commit(BAR(B_OFULL));
+            umma_commit(BAR(B_OFULL + kv_it % NO));
             umma_commit(BAR(B_VEMPTY + s));
             umma_commit(BAR(B_PFREE + b));
           }
