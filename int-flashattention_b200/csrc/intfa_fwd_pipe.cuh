@@ -40,10 +40,10 @@ struct PipeCfg {
   static_assert(!(FULL && F8V), "fp8 V belongs to the half-int8 op");
   static constexpr bool BYTE_PV = FULL || F8V;                     // P and V elements are one byte
   // Softmax groups of 128 threads.  Three (with 96 registers a thread, 16-column buffers) hide the hand-overs better than two
-  // (152 registers, 32 columns) where P is one byte and a step is 128 wide: batch 2, 32/8 heads, 3072 tokens, full-int8
-  // causal 267 -> 240 us, fp8 V causal 116 -> 105 us.  fp16 P (a third buffer leaves two K stages), 64-column steps and head
-  // dim 256 lose: 337 -> 351 us, 737 -> 767 us, 216 -> 237 us.
-  static constexpr int NGRP = (BYTE_PV && G == 128 && D == 128 && DQ == 128) ? 3 : 2;
+  // (152 registers, 32 columns) where P is one byte and a step is 128 wide, and for full-int8 at head dim 64: batch 2, 32/8
+  // heads, 3072 tokens, full-int8 causal 267 -> 240 us, fp8 V causal 116 -> 105 us.  fp16 P (a third buffer leaves two K
+  // stages) and head dim 256 lose: 337 -> 351 us, 216 -> 237 us.
+  static constexpr int NGRP = ((BYTE_PV && G == 128 && D == 128 && DQ == 128) || (FULL && G == 64 && D == 64)) ? 3 : 2;
   static constexpr int THREADS = 256 + 128 * NGRP;
   // Registers: the CTA is launched with LAUNCH_REGS per thread and setmaxnreg only moves registers around
   // INSIDE that allocation -- an increase beyond it would block for ever, hence the static_assert below.
@@ -79,7 +79,7 @@ struct PipeCfg {
   // steps of 1 KB for each kind of instantiation (`ragged`: masks partial tiles; `polite`: see the kernel).  Between the best
   // and the worst of a sweep lie 1 to 2 % non-causal, 5 to 15 % causal.
   __host__ __device__ static constexpr int code_filler_of(bool ragged, bool polite) {
-    return NGRP == 3 ? (!FULL ? 192 : ragged ? 64 : polite ? 128 : 256)
+    return NGRP == 3 ? (!FULL ? 192 : (ragged && G == 128) ? 64 : polite ? 128 : 256)
          : ragged ? 256 : G == 128 ? (FULL ? 448 : 384) : (D == 256 || (FULL && D == 64)) ? 0 : D == 32 ? 256 : 128;
   }
   static constexpr bool MORE_SOFTMAX_REGS = !FULL || G == 128;
