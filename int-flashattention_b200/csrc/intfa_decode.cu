@@ -75,10 +75,6 @@ __device__ __forceinline__ void mma_f16(float (&d)[4], uint32_t a0, uint32_t a1,
                : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 __device__ __forceinline__ float unmagic(int x) { return __int_as_float(x) - kMagicF; }
-// (programmatic launch: the next kernel of the chain may start; what the previous one wrote is there)
-__device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-
 // one (batch, K/V head, row tile)
 struct Unit {
   int id, b, hk, tile;
@@ -146,6 +142,7 @@ __global__ void __launch_bounds__(kThreads) scores_kernel(const DParams p, int s
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
   const Unit u = unit_of(p, blockIdx.x % (gridDim.x / splits));
   const int split = blockIdx.x / (gridDim.x / splits);
+  pdl_wait();
   pdl_launch();
   QRows<D, NT> q;
   q.load(p, u, g, t);
@@ -275,7 +272,6 @@ __global__ void __launch_bounds__(kThreads, NT == 1 ? 3 : 2) pv_full_kernel(cons
   const int split = blockIdx.x / units;
   const int g0 = split * p.per_split, g1 = min(p.groups, g0 + p.per_split);
   const int8_t* vb = static_cast<const int8_t*>(p.v) + u.b * p.vB + u.hk * p.vH + g * VB;
-  pdl_launch();
 
   // this lane's 8 keys of a 32-key step: 2t, 2t+1 of each of the four 8-key tiles
   uint32_t vn[8][W];
@@ -293,10 +289,11 @@ __global__ void __launch_bounds__(kThreads, NT == 1 ? 3 : 2) pv_full_kernel(cons
       }
     }
   };
-  // (V does not depend on the first pass)
+  // (V is older than the first pass)
   const int upg = p.G / 64, nun = (g1 - g0) * upg;          // 64-key units of this CTA
   if (warp < nun) load_v((g0 * upg + warp) * 64);
   pdl_wait();
+  pdl_launch();
 
   // ---- running maxima of this CTA's groups and the final maximum
   {
@@ -470,6 +467,7 @@ __global__ void __launch_bounds__(kThreads, 2) pv_half_kernel(const DParams p) {
   const Unit u = unit_of(p, blockIdx.x % units);
   const int split = blockIdx.x / units;
   const int k_begin = split * p.per_split * 64, k_end = min(p.nvis, k_begin + p.per_split * 64);
+  pdl_wait();
   pdl_launch();
   QRows<D, NT> q;
   q.load(p, u, g, t);
@@ -629,6 +627,7 @@ __global__ void __launch_bounds__(D / 4) combine_kernel(const DParams p, int RT)
   const Unit u = unit_of(p, blockIdx.x / RT);
   const int r = blockIdx.x % RT, row = u.tile * RT + r, ch = threadIdx.x * 4;
   pdl_wait();
+  pdl_launch();
   if (row >= p.R) return;
   const long long base = (long long)u.id * p.splits * RT + r;
   const float2* ml = reinterpret_cast<const float2*>(p.part_ml);
@@ -721,35 +720,19 @@ Plan make_plan(const IntfaFwdParams* a, int sms) {
   return pl;
 }
 
-// `chained`: the launch may begin while the one before it on the stream is still running (its kernel waits with pdl_wait)
-template <typename K, typename... A>
-int launch(K kernel, int grid, int threads, bool chained, cudaStream_t stream, A... args) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(grid);
-  cfg.blockDim = dim3(threads);
-  cfg.stream = stream;
-  cudaLaunchAttribute attr = {};
-  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr.val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = &attr;
-  cfg.numAttrs = chained ? 1 : 0;
-  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, args...);
-  return e == cudaSuccess ? INTFA_OK : set_error(INTFA_ERR_CUDA, "decode launch: %s", cudaGetErrorString(e));
-}
-
 template <int D, int NT>
 int run(const Plan& pl, const DParams& p, cudaStream_t stream) {
   int rc;
   const int grid = pl.units * pl.splits;
   if (pl.full) {
-    if ((rc = launch(scores_kernel<D, NT>, pl.units * pl.score_splits, kThreads, false, stream, p, pl.score_splits))) return rc;
-    if ((rc = launch(pv_full_kernel<D, NT>, grid, kThreads, true, stream, p))) return rc;
+    if ((rc = launch_kernel("decode scores", scores_kernel<D, NT>, pl.units * pl.score_splits, kThreads, 0, stream, p, pl.score_splits))) return rc;
+    if ((rc = launch_kernel("decode P V", pv_full_kernel<D, NT>, grid, kThreads, 0, stream, p))) return rc;
   } else {
-    if ((rc = launch(pv_half_kernel<D, NT>, grid, kThreads, false, stream, p))) return rc;
+    if ((rc = launch_kernel("decode", pv_half_kernel<D, NT>, grid, kThreads, 0, stream, p))) return rc;
   }
   if (pl.splits == 1) return INTFA_OK;
-  return pl.full ? launch(combine_kernel<true, D>, pl.units * 8 * NT, D / 4, true, stream, p, 8 * NT)
-                 : launch(combine_kernel<false, D>, pl.units * 8 * NT, D / 4, true, stream, p, 8 * NT);
+  return pl.full ? launch_kernel("decode combine", combine_kernel<true, D>, pl.units * 8 * NT, D / 4, 0, stream, p, 8 * NT)
+                 : launch_kernel("decode combine", combine_kernel<false, D>, pl.units * 8 * NT, D / 4, 0, stream, p, 8 * NT);
 }
 
 }  // namespace

@@ -201,10 +201,7 @@ static int launch_pipe(const IntfaFwdParams* a, const KParams& kp, cudaStream_t 
   KParams kpl = kp;
   kpl.tile_counter = nullptr;
   if (kp.num_tiles > grid && (rc = next_tile_counter(&kpl.tile_counter))) return rc;
-  kern<<<grid, C::THREADS, C::SMEM_BYTES, stream>>>(tmQ, tmK, tmV, kpl);
-  cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) return set_error(INTFA_ERR_CUDA, "kernel launch: %s", cudaGetErrorString(e));
-  return INTFA_OK;
+  return launch_kernel("attention", kern, grid, C::THREADS, C::SMEM_BYTES, stream, tmQ, tmK, tmV, kpl);
 }
 
 int fwd_dispatch(const IntfaFwdParams* a, cudaStream_t stream) {

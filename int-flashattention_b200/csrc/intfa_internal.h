@@ -44,6 +44,26 @@ int sm_count_cached();
 // Few query rows against many keys (intfa_decode.cu).  Returns false where the call is not one for that path.
 bool decode_dispatch(const IntfaFwdParams* a, cudaStream_t stream, int* rc);
 size_t decode_workspace_bytes(const IntfaFwdParams* a);
+// Every kernel of this library is launched so that it may begin while the kernel before it on the stream is still running
+// (programmatic stream serialisation): its setup and the launch itself overlap the other's tail.  Each begins with
+// pdl_wait(), which returns when everything before it on the stream is done and visible, and only then may let the next one
+// begin (pdl_launch()): what a kernel reads ahead of its own wait is therefore older than the kernel before it.
+template <typename K, typename... A>
+inline int launch_kernel(const char* what, K kernel, dim3 grid, int threads, size_t smem, cudaStream_t stream, const A&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr = {};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, args...);
+  return e == cudaSuccess ? INTFA_OK : set_error(INTFA_ERR_CUDA, "%s launch: %s", what, cudaGetErrorString(e));
+}
+
 int fwd_dispatch(const IntfaFwdParams* a, cudaStream_t stream);
 int quant_pertoken(const void* x, const int64_t* st, void* x8, float* scale, int B, int H, int N, int D,
                    cudaStream_t stream);

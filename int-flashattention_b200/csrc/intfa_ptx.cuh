@@ -82,6 +82,10 @@ __device__ __forceinline__ void code_filler() {
   for (int i = 0; i < N; ++i) asm volatile("nanosleep.u32 0;");
 }
 
+// programmatic launch: wait for what is before this kernel on the stream; let the kernel behind it begin (see launch_kernel)
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // generic-proxy writes (st.shared) -> visible to the async proxy (TMA / tcgen05.mma operand reads)
 __device__ __forceinline__ void fence_proxy_async_smem() {
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");

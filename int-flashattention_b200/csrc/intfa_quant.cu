@@ -152,6 +152,8 @@ __global__ void __launch_bounds__(256) quant_pertoken_kernel(const __half* __res
                                                              long long sN, int8_t* __restrict__ x8,
                                                              float* __restrict__ scale, int H, int N,
                                                              long long total_rows) {
+  pdl_wait();
+  pdl_launch();
   pertoken_rows<D, CONTIG>(x, sB, sH, sN, x8, scale, H, N, total_rows, blockIdx.x, gridDim.x);
 }
 
@@ -215,6 +217,8 @@ template <int D, bool ATOMIC>
 __global__ void __launch_bounds__(256) v_colmax_kernel(const __half* __restrict__ x, long long sB, long long sH,
                                                        long long sN, unsigned int* __restrict__ colmax, int H, int N,
                                                        int rows_per_cta) {
+  pdl_wait();
+  pdl_launch();
   colmax_chunk<D, ATOMIC>(x, sB, sH, sN, colmax, H, N, rows_per_cta, blockIdx.x, blockIdx.y, gridDim.y);
 }
 
@@ -229,6 +233,8 @@ struct QkvJob {
 template <int D>
 __global__ void __launch_bounds__(256) quant_qkv_kernel(const QkvJob j) {
   const int cta = blockIdx.x;
+  pdl_wait();
+  pdl_launch();
   if (cta < j.gq) {
     pertoken_rows<D, true>(j.q, 0, 0, 0, j.q8, j.qs, 1, 1, j.q_rows, cta, j.gq);
   } else if (cta < j.gq + j.gk) {
@@ -252,6 +258,8 @@ __global__ void __launch_bounds__(256) v_quant_kernel(const __half* __restrict__
   const int bh = gridDim.y - 1 - blockIdx.y;     // last slab first: the column-absmax pass read it last
   const int b = bh / H, h = bh - b * H;
   const uint64_t once = l2_policy_evict_first();
+  pdl_wait();
+  pdl_launch();
   if (threadIdx.x < 32) {
     // every channel's absmax; for the per-(batch,head) mode reduce them to one
     constexpr int CPL = (D + 31) / 32;     // channels per lane
@@ -301,6 +309,8 @@ __global__ void __launch_bounds__(256) v_quant_kernel(const __half* __restrict__
 }
 
 __global__ void scales_f16_to_f32_kernel(const __half* __restrict__ src, float* __restrict__ dst, long long n) {
+  pdl_wait();
+  pdl_launch();
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
     dst[i] = __half2float(src[i]);
 }
@@ -315,12 +325,6 @@ __global__ void scales_f16_to_f32_kernel(const __half* __restrict__ src, float* 
     default: { constexpr int DD = 256; CALL; } break;  \
   }
 
-static int check_launch(const char* what) {
-  cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) return set_error(INTFA_ERR_CUDA, "%s launch: %s", what, cudaGetErrorString(e));
-  return INTFA_OK;
-}
-
 int quant_pertoken(const void* x, const int64_t* st, void* x8, float* scale, int B, int H, int N, int D,
                    cudaStream_t stream) {
   const long long rows = (long long)B * H * N;
@@ -331,11 +335,13 @@ int quant_pertoken(const void* x, const int64_t* st, void* x8, float* scale, int
   const int grid = (int)(want < (long long)sms * 8 ? (want < 1 ? 1 : want) : (long long)sms * 8);
   if (rows >= (1LL << 31)) return set_error(INTFA_ERR_TOO_LARGE, "quant_pertoken: B*H*N must be below 2^31");
   const bool contig = st[2] == D && st[1] == (int64_t)N * D && st[0] == (int64_t)H * N * D;
+  int rc = INTFA_OK;
 #define INTFA_QPT(CC) \
-  quant_pertoken_kernel<DD, CC><<<grid, 256, 0, stream>>>((const __half*)x, st[0], st[1], st[2], (int8_t*)x8, scale, H, N, rows)
+  rc = launch_kernel("quant_pertoken", quant_pertoken_kernel<DD, CC>, dim3(grid), 256, 0, stream, (const __half*)x, (long long)st[0], \
+                     (long long)st[1], (long long)st[2], (int8_t*)x8, scale, H, N, rows)
   INTFA_D_SWITCH(D, if (contig) INTFA_QPT(true); else INTFA_QPT(false))
 #undef INTFA_QPT
-  return check_launch("quant_pertoken");
+  return rc;
 }
 
 static int v_grid(int BH, int N, int sms, int* rows_per_cta) {
@@ -353,8 +359,10 @@ int v_colmax(const void* v, const int64_t* st, void* colmax, int B, int H, int N
   if (sms <= 0) return set_error(INTFA_ERR_CUDA, "cannot query SM count");
   int rows_per_cta;
   dim3 grid(v_grid(B * H, N, sms, &rows_per_cta), B * H);
-  INTFA_D_SWITCH(D, (v_colmax_kernel<DD, true><<<grid, 256, 0, stream>>>((const __half*)v, st[0], st[1], st[2], (unsigned int*)colmax, H, N, rows_per_cta)))
-  return check_launch("v_colmax");
+  int rc = INTFA_OK;
+  INTFA_D_SWITCH(D, (rc = launch_kernel("v_colmax", v_colmax_kernel<DD, true>, grid, 256, 0, stream, (const __half*)v, (long long)st[0],
+                                        (long long)st[1], (long long)st[2], (unsigned int*)colmax, H, N, rows_per_cta)))
+  return rc;
 }
 
 static int v_quant_launch(const void* v, const int64_t* st, const void* colmax, int nparts, void* v8, float* scale, int mode,
@@ -364,8 +372,10 @@ static int v_quant_launch(const void* v, const int64_t* st, const void* colmax, 
   int rows_per_cta;
   dim3 grid(v_grid(B * H, N, sms, &rows_per_cta), B * H);
   const int pc = mode == INTFA_VSCALE_PER_CHANNEL;
-  INTFA_D_SWITCH(D, (v_quant_kernel<DD><<<grid, 256, 0, stream>>>((const __half*)v, st[0], st[1], st[2], (const unsigned int*)colmax, (int8_t*)v8, scale, pc, H, N, rows_per_cta, nparts)))
-  return check_launch("v_quant");
+  int rc = INTFA_OK;
+  INTFA_D_SWITCH(D, (rc = launch_kernel("v_quant", v_quant_kernel<DD>, grid, 256, 0, stream, (const __half*)v, (long long)st[0], (long long)st[1],
+                                        (long long)st[2], (const unsigned int*)colmax, (int8_t*)v8, scale, pc, H, N, rows_per_cta, nparts)))
+  return rc;
 }
 
 int v_quant_from_colmax(const void* v, const int64_t* st, const void* colmax, void* v8, float* scale, int mode, int B,
@@ -409,8 +419,8 @@ int quant_qkv(const void* q, const void* k, const void* v, const int64_t* v_st, 
     gv = j.chunks * B * Hkv;
   }
   const int grid = j.gq + j.gk + gv;
-  INTFA_D_SWITCH(D, (quant_qkv_kernel<DD><<<grid, 256, 0, stream>>>(j)))
-  int rc = check_launch("quant_qkv");
+  int rc = INTFA_OK;
+  INTFA_D_SWITCH(D, (rc = launch_kernel("quant_qkv", quant_qkv_kernel<DD>, dim3(grid), 256, 0, stream, j)))
   if (rc || !v) return rc;
   return v_quant_launch(v, v_st, workspace, j.chunks, v8, vs, mode, B, Hkv, Nk, D, stream);
 }
@@ -422,8 +432,9 @@ int quant_v_partial(const void* v, const int64_t* st, void* v8, float* scale, in
   int rows_per_cta;
   const int chunks = v_grid(B * H, N, sms, &rows_per_cta);
   dim3 grid(chunks, B * H);
-  INTFA_D_SWITCH(D, (v_colmax_kernel<DD, false><<<grid, 256, 0, stream>>>((const __half*)v, st[0], st[1], st[2], (unsigned int*)workspace, H, N, rows_per_cta)))
-  int rc = check_launch("v_colmax");
+  int rc = INTFA_OK;
+  INTFA_D_SWITCH(D, (rc = launch_kernel("v_colmax", v_colmax_kernel<DD, false>, grid, 256, 0, stream, (const __half*)v, (long long)st[0],
+                                        (long long)st[1], (long long)st[2], (unsigned int*)workspace, H, N, rows_per_cta)))
   if (rc) return rc;
   return v_quant_launch(v, st, workspace, chunks, v8, scale, mode, B, H, N, D, stream);
 }
@@ -490,8 +501,7 @@ int scales_f16_to_f32(const void* src, float* dst, long long n, cudaStream_t str
   if (n <= 0) return INTFA_OK;
   long long blocks = (n + 255) / 256;
   if (blocks > 4096) blocks = 4096;
-  scales_f16_to_f32_kernel<<<(int)blocks, 256, 0, stream>>>((const __half*)src, dst, n);
-  return check_launch("scales_f16_to_f32");
+  return launch_kernel("scales_f16_to_f32", scales_f16_to_f32_kernel, dim3((int)blocks), 256, 0, stream, (const __half*)src, dst, n);
 }
 
 }  // namespace intfa
