@@ -1,4 +1,5 @@
-// Attention of a few query rows against a long K/V cache (decode): the path that is bound by reading K and V once.
+// Attention of a few query rows against a long K/V cache (decode), and of short prompts: where 128-row tiles are mostly
+// padding or too few to fill the GPU.  With one row a head this path is bound by reading K and V once.
 //
 // The 128-row kernel gives such a call one CTA per (batch, query head) whose 128 rows are nearly all padding: it re-reads
 // K/V once per query head of a group and leaves most SMs without work (batch 1, 32/8 heads, 32768 keys, fp16 V: 369 us for
@@ -662,15 +663,34 @@ struct Plan {
   size_t off_gmax = 0, off_part = 0, off_ml = 0, bytes = 0;
 };
 
+// Which path?  Times in microseconds, fitted to measurements of both paths at 1 to 2048 rows and 77 to 16384 keys (B200):
+//   here       launches, then `u` per 64 keys of a 16-row tile and SM.  Per row and key that is 2 to 3.5 times what the other
+//              path costs with all its rows alive, but rows are padded to 8 or 16 instead of 128 and keys are split.
+//   128 rows   `c0` (pipeline fill), then `s` per KV step of G keys: the longest work item, or what an SM gets of all steps.
+// The margin of 10 % keeps the 128-row kernel where the two are alike.
+bool faster_than_tiles(const IntfaFwdParams* a, const Plan& pl, int sms) {
+  const bool d128 = a->D == 128;
+  const double u = pl.full ? (d128 ? 0.59 : 0.45) : (d128 ? 0.50 : 0.27);
+  const double here = (pl.full ? 7.0 : 4.5) + (pl.splits > 1 ? 3.0 : 0.0) +
+                      u * (pl.NT == 1 ? 0.6 : 1.0) * (double)pl.units * ((pl.nvis + 63) / 64) / sms;
+  const double c0 = pl.full ? 8.0 : 6.5, s = pl.full ? (a->G == 64 ? 0.80 : 1.35) : 1.30;
+  const long long mb = (a->Nq + 127) / 128, items = (long long)a->B * a->H * mb;
+  const double steps = (double)((pl.nvis + a->G - 1) / a->G);
+  const double mean = a->causal ? steps - 0.5 * a->Nq / a->G : steps;      // steps of an average work item
+  const double per_sm = items * (mean < 1 ? 1 : mean) / sms + 0.4 * steps;
+  const double tiles = c0 + s * (items <= sms || per_sm < steps ? steps : per_sm);
+  return here < 0.9 * tiles;
+}
+
 Plan make_plan(const IntfaFwdParams* a, int sms) {
   Plan pl;
   const int Hkv = a->H_kv > 0 ? a->H_kv : a->H;
   pl.full = a->variant == INTFA_VARIANT_FULL;
-  // The rule.  Rows: a 16-row tile costs this path about a ninth of what a 128-row tile costs the other one per key, and the
-  // other path takes a tile per query head, so the break-even lies above 128 rows a head; kDecodeRows keeps well clear of it.
-  // Options that the other path keeps: head dims 16, 32, 256, fp8 V (its rounding of P follows the running maximum, too),
+  // Options that the 128-row kernel keeps: head dims 16, 32, 256, fp8 V (its rounding of P follows the running maximum, too),
   // carried state, KV tiles last to first, per-tile V scales, RNE rounding, the debug tap, rows that see no key at all.
-  constexpr int kDecodeRows = 32;
+  // Calls of more than kDecodeRows rows a head stay there too: a pass continued through carried state is the same as one pass
+  // bit for bit only where both run the same kernel, and that is what long sequences are cut up for.
+  constexpr int kDecodeRows = 256;
   if (a->Nq > kDecodeRows || (a->D != 64 && a->D != 128) || (!pl.full && a->variant != INTFA_VARIANT_HALF) || (a->G != 64 && a->G != 128)) return pl;
   if (a->state_in || a->state_out || !a->write_o || a->kv_order || a->vs_stride_blk || (pl.full && a->p_round) || a->dbg_s || a->debug_skip_k_load) return pl;
   if (!(a->sm_scale > 0.f) || (a->causal && a->q_offset < a->kv_offset)) return pl;
@@ -691,7 +711,7 @@ Plan make_plan(const IntfaFwdParams* a, int sms) {
   const int key_units = (pl.nvis + 63) / 64;
   pl.groups = (pl.nvis + a->G - 1) / a->G;
   const int items = pl.full ? pl.groups : key_units;          // what a split is counted in
-  const int per_min = pl.full ? (a->G == 128 ? 2 : 4) : 2;    // at least 256 (half: 128) keys per CTA
+  const int per_min = pl.full ? 512 / a->G : 8;               // at least 512 keys per CTA: fewer are not worth the combine launch
   int splits = wave / pl.units < 1 ? 1 : wave / pl.units;
   int per = (items + splits - 1) / splits;
   if (per < per_min) per = per_min;
@@ -701,6 +721,7 @@ Plan make_plan(const IntfaFwdParams* a, int sms) {
   pl.score_splits = sms * 8 / pl.units < 1 ? 1 : sms * 8 / pl.units;
   if (pl.score_splits > (pl.groups + kWarps - 1) / kWarps) pl.score_splits = (pl.groups + kWarps - 1) / kWarps;
   if ((long long)pl.units * pl.splits > 0x7fffffffLL || (long long)pl.units * pl.score_splits > 0x7fffffffLL) return pl;
+  if (!faster_than_tiles(a, pl, sms)) return pl;
   size_t used = 0;
   auto take = [&](size_t bytes) {
     const size_t r = used;

@@ -16,6 +16,10 @@ CASES = [
     ("full", 1, 3, 1, 32, 65, 64, 64, True, "fp32"),            # the most rows a head
     ("full", 1, 2, 1, 3, 2500, 64, 128, False, "fp16"),
     ("full", 1, 1, 1, 2, 20000, 64, 64, True, "fp32"),          # more groups than one CTA may take
+    ("full", 1, 2, 1, 256, 256, 64, 64, True, "fp32"),          # short prompts: the most rows a head, causal over the whole tile
+    ("full", 1, 2, 2, 131, 700, 128, 128, True, "fp16"),
+    ("half", 1, 2, 1, 77, 77, 64, 128, True, "fp32"),
+    ("half", 1, 1, 2, 200, 1100, 128, 128, False, "fp16"),
     ("half", 1, 1, 1, 1, 1, 64, 128, True, "fp32"),
     ("half", 2, 2, 4, 1, 31, 128, 128, True, "fp16"),
     ("half", 1, 2, 8, 2, 1025, 128, 128, True, "fp32"),
