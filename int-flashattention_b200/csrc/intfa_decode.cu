@@ -14,7 +14,7 @@
 //
 // full-int8: P is rounded to int8 against the RUNNING maximum of the row (keys taken G at a time, ascending), so the
 // maxima must be known before P: `scores_kernel` computes s = (fp32(S32)*s_q)*s_k, keeps it (fp32, in the order in which
-// the next kernel's lanes want it) and the maximum of each group of G keys; `pv_full_kernel` takes the prefix maximum at its
+// the next kernel's lanes want it) and the maximum of each 64 keys; `pv_full_kernel` takes the prefix maximum at its
 // first group, and from there on does exactly what the one-pass kernel does: m' = max(m, groupmax*c), p = exp2(s*c - m'),
 // P8, O_j.  The final maximum is known too, so that every partial result is scaled to it at once
 // (acc += exp2(m_j - m_final) * O_j) and the splits add up without weights.
@@ -33,7 +33,7 @@ namespace intfa {
 namespace {
 
 constexpr int kThreads = 128, kWarps = 4;
-constexpr int kMaxLocalGroups = 64;       // groups of G keys per CTA of pv_full_kernel (their maxima sit in shared memory)
+constexpr int kMaxLocalUnits = 128;       // 64-key units per CTA of pv_full_kernel (their maxima sit in shared memory)
 constexpr float kMagicF = 12582912.0f;    // 1.5*2^23: added to an int32 below 2^22 as a bit pattern, it reads as fp32 1.5*2^23 + value
 constexpr int kMagicI = 0x4B400000;
 
@@ -49,7 +49,7 @@ struct DParams {
   float c;                                // sm_scale * log2(e)
   int G, groups, splits, per_split;       // per_split: groups (full) or 64-key units (half) per split
   float* lse;
-  float* scores; float* gmax;             // [unit][key tile of 8][NT][32 lanes][2]; [unit][groups][RT]
+  float* scores; float* gmax;             // [unit][key tile of 8][NT][32 lanes][2]; [unit][64-key units][RT]
   float* part; float* part_ml;            // [unit][splits][RT][D]; [unit][splits][RT][2]
 };
 
@@ -134,7 +134,7 @@ __device__ __forceinline__ void qk_tile(const QRows<D, NT>& q, const uint4 (&kw)
 }
 
 // ---------------------------------------------------------------------------------------------------------------
-// full-int8, first pass: scores and group maxima.  One warp takes one group of G keys at a time, 32 keys in flight.
+// full-int8, first pass: scores and maxima.  One warp takes 64 keys at a time, 32 in flight; CTAs fill one wave.
 // Bound by reading K (67 MB at batch 16, 8 K/V heads, 4097 keys).
 // ---------------------------------------------------------------------------------------------------------------
 template <int D, int NT>
@@ -150,15 +150,15 @@ __global__ void __launch_bounds__(kThreads) scores_kernel(const DParams p, int s
   const int8_t* kb = p.k + u.b * p.kB + u.hk * p.kH + t * 16;
   const long long ksb = u.b * p.ksB + u.hk * p.ksH;
   const int kf16 = p.scale_f16 & INTFA_SCALE_F16_K;
-  const int ktiles = p.groups * (p.G / 8);
+  const int units64 = p.groups * (p.G / 64), ktiles = units64 * 8;
   float2* sc = reinterpret_cast<float2*>(p.scores) + (long long)u.id * ktiles * NT * 32 + lane;
-  float* gm = p.gmax + (long long)u.id * p.groups * RT;
-  for (int grp = split * kWarps + warp; grp < p.groups; grp += splits * kWarps) {
+  float* gm = p.gmax + (long long)u.id * units64 * RT;
+  for (int un = split * kWarps + warp; un < units64; un += splits * kWarps) {
     float mx[NT];
 #pragma unroll
     for (int i = 0; i < NT; ++i) mx[i] = -INFINITY;
 #pragma unroll 1
-    for (int kt = grp * (p.G / 8); kt < (grp + 1) * (p.G / 8); kt += 4) {
+    for (int kt = un * 8; kt < un * 8 + 8; kt += 4) {
       uint4 kw[4][CH];
       float k0[4], k1[4];
 #pragma unroll
@@ -192,7 +192,7 @@ __global__ void __launch_bounds__(kThreads) scores_kernel(const DParams p, int s
     for (int hr = 0; hr < NT; ++hr) {
       mx[hr] = fmaxf(mx[hr], __shfl_xor_sync(0xffffffffu, mx[hr], 1));
       mx[hr] = fmaxf(mx[hr], __shfl_xor_sync(0xffffffffu, mx[hr], 2));
-      if (t == 0) gm[grp * RT + g + 8 * hr] = mx[hr];
+      if (t == 0) gm[un * RT + g + 8 * hr] = mx[hr];
     }
   }
 }
@@ -264,7 +264,7 @@ __global__ void __launch_bounds__(kThreads, NT == 1 ? 3 : 2) pv_full_kernel(cons
   constexpr int RT = 8 * NT, VB = D / 8, MT = D / 16;       // VB: bytes (channels) of a key that a lane holds; MT: 16-channel tiles
   constexpr int W = VB / 4;                                 // ... in words
   __shared__ __align__(16) float red[kWarps * RT * (D + 4)];
-  __shared__ __align__(16) float mg[kMaxLocalGroups * RT];  // running maximum (scaled) at each group of this CTA
+  __shared__ __align__(16) float mg[kMaxLocalUnits * RT];   // running maximum (scaled) at the group of each 64-key unit of this CTA
   __shared__ __align__(16) float ends[2][RT];               // prefix before the first group; final maximum
   __shared__ float ml[RT][2];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
@@ -298,18 +298,19 @@ __global__ void __launch_bounds__(kThreads, NT == 1 ? 3 : 2) pv_full_kernel(cons
 
   // ---- running maxima of this CTA's groups and the final maximum
   {
-    const float* gm = p.gmax + (long long)u.id * p.groups * RT;
+    const int units64 = p.groups * upg, u0 = g0 * upg;
+    const float* gm = p.gmax + (long long)u.id * units64 * RT;
     constexpr int Q4 = RT / 4;                               // threads across a group's rows, 4 rows each
     const int rq = tid % Q4 * 4;
     float4 pre = make_float4(-INFINITY, -INFINITY, -INFINITY, -INFINITY), all = pre;
 #pragma unroll 4
-    for (int i = tid / Q4; i < p.groups; i += kThreads / Q4) {
+    for (int i = tid / Q4; i < units64; i += kThreads / Q4) {
       const float4 x = *reinterpret_cast<const float4*>(gm + i * RT + rq);
       all.x = fmaxf(all.x, x.x); all.y = fmaxf(all.y, x.y); all.z = fmaxf(all.z, x.z); all.w = fmaxf(all.w, x.w);
-      if (i < g0) {
+      if (i < u0) {
         pre.x = fmaxf(pre.x, x.x); pre.y = fmaxf(pre.y, x.y); pre.z = fmaxf(pre.z, x.z); pre.w = fmaxf(pre.w, x.w);
-      } else if (i < g1) {
-        *reinterpret_cast<float4*>(mg + (i - g0) * RT + rq) = x;
+      } else if (i < u0 + nun) {
+        *reinterpret_cast<float4*>(mg + (i - u0) * RT + rq) = x;
       }
     }
     float4* sp = reinterpret_cast<float4*>(red);             // (red is free until the end)
@@ -326,9 +327,12 @@ __global__ void __launch_bounds__(kThreads, NT == 1 ? 3 : 2) pv_full_kernel(cons
     __syncthreads();
     if (tid < RT) {
       float m = ends[0][tid];
-      for (int i = 0; i < g1 - g0; ++i) {
-        m = fmaxf(m, mg[i * RT + tid] * p.c);
+      for (int i = 0; i < nun; i += upg) {
+        float x = mg[i * RT + tid];
+        if (upg == 2) x = fmaxf(x, mg[(i + 1) * RT + tid]);
+        m = fmaxf(m, x * p.c);
         mg[i * RT + tid] = m;
+        if (upg == 2) mg[(i + 1) * RT + tid] = m;
       }
     }
     __syncthreads();
@@ -348,12 +352,11 @@ __global__ void __launch_bounds__(kThreads, NT == 1 ? 3 : 2) pv_full_kernel(cons
   }
 #pragma unroll 1
   for (int un = warp; un < nun; un += kWarps) {
-    const int lg = un / upg;
     float nm[NT], w_g[NT], rs[NT];
     int o[NT][MT][4];
 #pragma unroll
     for (int n = 0; n < NT; ++n) {
-      const float m = mg[lg * RT + n * 8 + g];
+      const float m = mg[un * RT + n * 8 + g];
       nm[n] = -m;
       w_g[n] = ex2_approx(m - m_fin_g[n]);
       rs[n] = 0.f;
@@ -417,7 +420,7 @@ __global__ void __launch_bounds__(kThreads, NT == 1 ? 3 : 2) pv_full_kernel(cons
 #pragma unroll
     for (int n = 0; n < NT; ++n) {
       lsum[n] = fmaf(w_g[n], rs[n], lsum[n]);
-      const float w0 = ex2_approx(mg[lg * RT + n * 8 + 2 * t] - m_fin[n][0]), w1 = ex2_approx(mg[lg * RT + n * 8 + 2 * t + 1] - m_fin[n][1]);
+      const float w0 = ex2_approx(mg[un * RT + n * 8 + 2 * t] - m_fin[n][0]), w1 = ex2_approx(mg[un * RT + n * 8 + 2 * t + 1] - m_fin[n][1]);
 #pragma unroll
       for (int i = 0; i < MT; ++i) {
         acc[n][i][0] = fmaf(unmagic(o[n][i][0]), w0, acc[n][i][0]);
@@ -458,7 +461,7 @@ __global__ void __launch_bounds__(kThreads, NT == 1 ? 3 : 2) pv_full_kernel(cons
 // half-int8: scores, softmax and P V in one pass; one warp takes 32 keys at a time, with a running maximum of its own
 // ---------------------------------------------------------------------------------------------------------------
 template <int D, int NT>
-__global__ void __launch_bounds__(kThreads, 2) pv_half_kernel(const DParams p) {
+__global__ void __launch_bounds__(kThreads, D == 64 && NT == 1 ? 3 : 2) pv_half_kernel(const DParams p) {
   constexpr int RT = 8 * NT, CH = D / 64, MT = D / 16;
   __shared__ __align__(16) float red[kWarps * RT * (D + 4)];
   __shared__ float wml[kWarps][RT][2];
@@ -706,8 +709,9 @@ Plan make_plan(const IntfaFwdParams* a, int sms) {
   const long long units = (long long)a->B * Hkv * pl.tiles;
   if (units > (1 << 22)) return pl;
   pl.units = (int)units;
-  // Splits: one wave of resident CTAs (3 per SM for full-int8 at 8 rows, 2 otherwise), at least one 64-key unit per warp
-  const int wave = sms * (pl.full && pl.NT == 1 ? 3 : 2);
+  // Splits: one wave of resident CTAs, as the kernels' launch bounds have it (two CTAs an SM or four for full-int8 at 8 rows:
+  // 35 -> 44 us at batch 16, 4097 keys; three for half-int8 at 128 channels: 26.5 -> 30 us at 32768 keys)
+  const int wave = sms * (pl.NT == 1 && (pl.full || a->D == 64) ? 3 : 2);
   const int key_units = (pl.nvis + 63) / 64;
   pl.groups = (pl.nvis + a->G - 1) / a->G;
   const int items = pl.full ? pl.groups : key_units;          // what a split is counted in
@@ -715,11 +719,13 @@ Plan make_plan(const IntfaFwdParams* a, int sms) {
   int splits = wave / pl.units < 1 ? 1 : wave / pl.units;
   int per = (items + splits - 1) / splits;
   if (per < per_min) per = per_min;
-  if (pl.full && per > kMaxLocalGroups) per = kMaxLocalGroups;
+  if (pl.full && per > kMaxLocalUnits * 64 / a->G) per = kMaxLocalUnits * 64 / a->G;
   pl.per_split = per;
   pl.splits = (items + per - 1) / per;
-  pl.score_splits = sms * 8 / pl.units < 1 ? 1 : sms * 8 / pl.units;
-  if (pl.score_splits > (pl.groups + kWarps - 1) / kWarps) pl.score_splits = (pl.groups + kWarps - 1) / kWarps;
+  const int score_ctas = sms * (a->D == 128 ? 5 : 6);                      // resident at their register counts
+  pl.score_splits = score_ctas / pl.units < 1 ? 1 : score_ctas / pl.units;
+  const int score_cap = (pl.groups * (a->G / 64) + kWarps - 1) / kWarps;
+  if (pl.score_splits > score_cap) pl.score_splits = score_cap;
   if ((long long)pl.units * pl.splits > 0x7fffffffLL || (long long)pl.units * pl.score_splits > 0x7fffffffLL) return pl;
   if (!faster_than_tiles(a, pl, sms)) return pl;
   size_t used = 0;
@@ -730,7 +736,7 @@ Plan make_plan(const IntfaFwdParams* a, int sms) {
   };
   if (pl.full) {
     take((size_t)pl.units * pl.groups * (a->G / 8) * pl.NT * 32 * 8);      // scores, at 0
-    pl.off_gmax = take((size_t)pl.units * pl.groups * RT * 4);
+    pl.off_gmax = take((size_t)pl.units * pl.groups * (a->G / 64) * RT * 4);
   }
   if (pl.splits > 1) {
     pl.off_part = take((size_t)pl.units * pl.splits * RT * a->D * 4);
