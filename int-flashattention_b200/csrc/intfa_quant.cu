@@ -245,31 +245,61 @@ __global__ void __launch_bounds__(256) quant_qkv_kernel(const QkvJob j) {
   }
 }
 
+// The V quantising pass.  Its start is a serial chain (maxima -> scales -> reciprocals), so every thread takes part in
+// reducing the partial maxima (one warp doing it cost 5 us of latency at 8 chunks), and `early` (the kernel before this one
+// on the stream is the column-absmax pass, so V is older) has the first rows on their way meanwhile.
 template <int D>
 __global__ void __launch_bounds__(256) v_quant_kernel(const __half* __restrict__ x, long long sB, long long sH,
                                                       long long sN, const unsigned int* __restrict__ colmax,
                                                       int8_t* __restrict__ x8, float* __restrict__ scale,
-                                                      int per_channel, int H, int N, int rows_per_cta, int nparts) {
+                                                      int per_channel, int H, int N, int rows_per_cta, int nparts, int early) {
   constexpr int LPR = D / 8;
   constexpr int RPW = 32 / LPR;
+  constexpr int PG = 256 / D;            // partial maxima in parallel
+  __shared__ float s_max[PG][D];
   __shared__ float s_scale[D];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
   const int sub = lane % LPR;
   const int bh = gridDim.y - 1 - blockIdx.y;     // last slab first: the column-absmax pass read it last
   const int b = bh / H, h = bh - b * H;
   const uint64_t once = l2_policy_evict_first();
+  const __half* base = x + b * sB + h * sH + sub * 8;
+  int8_t* obase = x8 + (long long)bh * N * D + sub * 8;
+  const int r_begin = blockIdx.x * rows_per_cta;
+  const int r_end = min(N, r_begin + rows_per_cta);
+  int r0 = r_begin + warp * RPW + lane / LPR;
+  uint4 v[kQuantUnroll];
+  auto load = [&]() {
+#pragma unroll
+    for (int u = 0; u < kQuantUnroll; ++u) {
+      const int r = r0 + u * nw * RPW;
+      v[u] = r < r_end ? ld_hint(base + r * sN, once) : make_uint4(0, 0, 0, 0);
+    }
+  };
+  if (early) load();
   pdl_wait();
   pdl_launch();
+  if (!early) load();
+  {
+    // every channel's absmax (colmax is [nparts][B*H][D]: one row, or the partial maxima of the pass before)
+    const int ch = threadIdx.x % D;
+    float a = 0.f;
+#pragma unroll 4
+    for (int c = threadIdx.x / D; c < nparts; c += PG) a = fmaxf(a, __uint_as_float(__ldcg(colmax + ((long long)c * gridDim.y + bh) * D + ch)));
+    s_max[threadIdx.x / D][ch] = a;
+  }
+  __syncthreads();
   if (threadIdx.x < 32) {
-    // every channel's absmax; for the per-(batch,head) mode reduce them to one
+    // ... and for the per-(batch,head) mode their maximum
     constexpr int CPL = (D + 31) / 32;     // channels per lane
     float a[CPL];
     float all = 0.f;
 #pragma unroll
     for (int i = 0; i < CPL; ++i) {
-      a[i] = 0.f;      // colmax is [nparts][B*H][D]: one row, or the partial maxima of the fused first launch
+      a[i] = 0.f;
       if (lane + 32 * i < D)
-        for (int c = 0; c < nparts; ++c) a[i] = fmaxf(a[i], __uint_as_float(colmax[((long long)c * gridDim.y + bh) * D + lane + 32 * i]));
+#pragma unroll
+        for (int c = 0; c < PG; ++c) a[i] = fmaxf(a[i], s_max[c][lane + 32 * i]);
       all = fmaxf(all, a[i]);
     }
 #pragma unroll
@@ -289,21 +319,17 @@ __global__ void __launch_bounds__(256) v_quant_kernel(const __half* __restrict__
   Scale2 k[4];
 #pragma unroll
   for (int i = 0; i < 4; ++i) k[i] = make_scale2(s_scale[sub * 8 + 2 * i], s_scale[sub * 8 + 2 * i + 1]);
-  const __half* base = x + b * sB + h * sH + sub * 8;
-  int8_t* obase = x8 + (long long)bh * N * D + sub * 8;
-  const int r_begin = blockIdx.x * rows_per_cta;
-  const int r_end = min(N, r_begin + rows_per_cta);
-  for (int r0 = r_begin + warp * RPW + lane / LPR; r0 < r_end; r0 += nw * RPW * kQuantUnroll) {
-    uint4 v[kQuantUnroll];
+  while (r0 < r_end) {
+    uint4 w[kQuantUnroll];
+#pragma unroll
+    for (int u = 0; u < kQuantUnroll; ++u) w[u] = v[u];
+    const int r1 = r0;
+    r0 += nw * RPW * kQuantUnroll;
+    if (r0 < r_end) load();
 #pragma unroll
     for (int u = 0; u < kQuantUnroll; ++u) {
-      const int r = r0 + u * nw * RPW;
-      v[u] = r < r_end ? ld_hint(base + r * sN, once) : make_uint4(0, 0, 0, 0);
-    }
-#pragma unroll
-    for (int u = 0; u < kQuantUnroll; ++u) {
-      const int r = r0 + u * nw * RPW;
-      if (r < r_end) st_hint(obase + (long long)r * D, quant8(v[u], k), once);
+      const int r = r1 + u * nw * RPW;
+      if (r < r_end) st_hint(obase + (long long)r * D, quant8(w[u], k), once);
     }
   }
 }
@@ -365,7 +391,7 @@ int v_colmax(const void* v, const int64_t* st, void* colmax, int B, int H, int N
   return rc;
 }
 
-static int v_quant_launch(const void* v, const int64_t* st, const void* colmax, int nparts, void* v8, float* scale, int mode,
+static int v_quant_launch(const void* v, const int64_t* st, const void* colmax, int nparts, bool early, void* v8, float* scale, int mode,
                           int B, int H, int N, int D, cudaStream_t stream) {
   const int sms = sm_count_cached();
   if (sms <= 0) return set_error(INTFA_ERR_CUDA, "cannot query SM count");
@@ -374,13 +400,13 @@ static int v_quant_launch(const void* v, const int64_t* st, const void* colmax, 
   const int pc = mode == INTFA_VSCALE_PER_CHANNEL;
   int rc = INTFA_OK;
   INTFA_D_SWITCH(D, (rc = launch_kernel("v_quant", v_quant_kernel<DD>, grid, 256, 0, stream, (const __half*)v, (long long)st[0], (long long)st[1],
-                                        (long long)st[2], (const unsigned int*)colmax, (int8_t*)v8, scale, pc, H, N, rows_per_cta, nparts)))
+                                        (long long)st[2], (const unsigned int*)colmax, (int8_t*)v8, scale, pc, H, N, rows_per_cta, nparts, early ? 1 : 0)))
   return rc;
 }
 
 int v_quant_from_colmax(const void* v, const int64_t* st, const void* colmax, void* v8, float* scale, int mode, int B,
                         int H, int N, int D, cudaStream_t stream) {
-  return v_quant_launch(v, st, colmax, 1, v8, scale, mode, B, H, N, D, stream);
+  return v_quant_launch(v, st, colmax, 1, false, v8, scale, mode, B, H, N, D, stream);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -422,7 +448,7 @@ int quant_qkv(const void* q, const void* k, const void* v, const int64_t* v_st, 
   int rc = INTFA_OK;
   INTFA_D_SWITCH(D, (rc = launch_kernel("quant_qkv", quant_qkv_kernel<DD>, dim3(grid), 256, 0, stream, j)))
   if (rc || !v) return rc;
-  return v_quant_launch(v, v_st, workspace, j.chunks, v8, vs, mode, B, Hkv, Nk, D, stream);
+  return v_quant_launch(v, v_st, workspace, j.chunks, true, v8, vs, mode, B, Hkv, Nk, D, stream);
 }
 
 int quant_v_partial(const void* v, const int64_t* st, void* v8, float* scale, int mode, int B, int H, int N, int D, void* workspace,
@@ -436,7 +462,7 @@ int quant_v_partial(const void* v, const int64_t* st, void* v8, float* scale, in
   INTFA_D_SWITCH(D, (rc = launch_kernel("v_colmax", v_colmax_kernel<DD, false>, grid, 256, 0, stream, (const __half*)v, (long long)st[0],
                                         (long long)st[1], (long long)st[2], (unsigned int*)workspace, H, N, rows_per_cta)))
   if (rc) return rc;
-  return v_quant_launch(v, st, workspace, chunks, v8, scale, mode, B, H, N, D, stream);
+  return v_quant_launch(v, st, workspace, chunks, true, v8, scale, mode, B, H, N, D, stream);
 }
 
 int quant_v(const void* v, const int64_t* st, void* v8, float* scale, int mode, int B, int H, int N, int D,
