@@ -5,8 +5,8 @@
 //   amax  = max |x|                       (exact in fp16)
 //   scale = fp16( fp32(amax) / 127 )      (IEEE fp32 division, then round-to-nearest fp16)
 //   q     = int8( rint( fp16( fp32(x) / fp32(scale) ) ) )   (rint = half-to-even, as torch.round)
-// The per-element division is evaluated as a correctly rounded quotient from one reciprocal per
-// row/channel and two fmas (see quant_pair), so it costs no division instruction per element.
+// The per-element division is one product with the reciprocal of the row's or channel's scale, which gives the same
+// bytes (see quant_pair).
 // Scales are written as fp32 holding the fp16-representable value.  amax == 0 gives
 // scale 0 and q 0 (the reference computes 0/0 there).
 //
@@ -29,42 +29,36 @@ namespace intfa {
 __device__ __forceinline__ float scale_from_amax(float amax) {
   return __half2float(__float2half_rn(__fdiv_rn(amax, 127.0f)));
 }
-// Correctly rounded x / s without a division per element (Markstein): with r = RN(1/s),
-// q0 = RN(x*r), e = x - q0*s (exact in one fma), q = RN(q0 + e*r) equals RN(x/s) unless the
-// significand of s is all ones -- impossible here because s is an fp16 value held in fp32.
-// Then the reference's rounding chain: fp16(q), and rint() done IN fp16 by adding 1536 = 1.5*2^10 (the sum has
-// an ulp of 1, so its round-to-nearest-even is rint, and its bit pattern is 0x6600 + n: the two's-complement
-// integer is the low byte).  Everything runs two elements per instruction (packed fp32, fp16x2): these kernels
-// are as much bound by instruction issue as by HBM.
+// fp16(RN32(x / s)) without a division per element: with r = RN32(1/s), fp16(RN32(x*r)) is the same number.  x and s are
+// fp16 values, so x/s = (X/S) * 2^k with X, S < 2^11.  Where rounding to fp16 can turn -- at a midpoint m of two fp16
+// numbers, whose significand M is odd and below 2^12 -- x/s is never equal to m (M would have to divide X) and at least
+// 1/(M*S) > 1.0007 * 2^-23 away from it, relative to m; RN32(x*r) is at most 2^-23 + 2^-48 away from x/s, hence on the same
+// side of m, and so is RN32(x/s).  (Below the fp16 normal range the result is rounded to 0 in any case.)
+// Then rint() done IN fp16 by adding 1536 = 1.5*2^10 (the sum has an ulp of 1, so its round-to-nearest-even is rint, and
+// its bit pattern is 0x6600 + n: the two's-complement integer is the low byte).  Everything runs two elements per
+// instruction (packed fp32, fp16x2): these kernels are as much bound by instruction issue as by HBM.
 // A zero scale (an all-zero row or channel; the reference computes 0/0 there) is given the reciprocal 0, which makes
 // every quotient 0.
-struct Scale2 { uint64_t neg_s, r; };      // (-s, -s') and (1/s, 1/s') of two neighbouring elements
 __device__ __forceinline__ float safe_rcp(float s) { return s == 0.f ? 0.f : __frcp_rn(s); }
-__device__ __forceinline__ Scale2 make_scale2(float s0, float s1) {
-  Scale2 k;
-  k.neg_s = f2_pack(-s0, -s1);
-  k.r = f2_pack(safe_rcp(s0), safe_rcp(s1));
-  return k;
-}
-// two fp16 inputs -> two int8 in bytes 0 and 2 of the result
-__device__ __forceinline__ uint32_t quant_pair(__half2 x, const Scale2& k) {
+// two fp16 inputs -> two int8 in bytes 0 and 2 of the result; r: the reciprocals of their scales
+__device__ __forceinline__ uint32_t quant_pair(__half2 x, uint64_t r) {
   const float2 f = __half22float2(x);
-  const uint64_t X = f2_pack(f.x, f.y);
-  const uint64_t q0 = f2_mul(X, k.r);
-  const uint64_t e = f2_fma(q0, k.neg_s, X);
   float qa, qb;
-  f2_unpack(f2_fma(e, k.r, q0), qa, qb);
-  const __half2 t = __floats2half2_rn(qa, qb);
-  const __half2 u = __hadd2(t, __half2(__ushort_as_half(0x6600), __ushort_as_half(0x6600)));
+  f2_unpack(f2_mul(f2_pack(f.x, f.y), r), qa, qb);
+  const __half2 u = __hadd2(__floats2half2_rn(qa, qb), __half2(__ushort_as_half(0x6600), __ushort_as_half(0x6600)));
   return *reinterpret_cast<const uint32_t*>(&u);
 }
-__device__ __forceinline__ float amax8(const uint4& v) {
+// the absmax of the even and of the odd elements
+__device__ __forceinline__ __half2 amax8(const uint4& v) {
   const __half2* h = reinterpret_cast<const __half2*>(&v);
-  __half2 m = __hmax2(__hmax2(__habs2(h[0]), __habs2(h[1])), __hmax2(__habs2(h[2]), __habs2(h[3])));
-  return fmaxf(__low2float(m), __high2float(m));
+  return __hmax2(__hmax2(__habs2(h[0]), __habs2(h[1])), __hmax2(__habs2(h[2]), __habs2(h[3])));
 }
-// k[i]: the scales of elements 2i, 2i+1 of the 8
-__device__ __forceinline__ uint2 quant8(const uint4& v, const Scale2 (&k)[4]) {
+__device__ __forceinline__ __half2 shfl_xor_h2(__half2 x, int o) {
+  const uint32_t y = __shfl_xor_sync(0xffffffffu, *reinterpret_cast<const uint32_t*>(&x), o);
+  return *reinterpret_cast<const __half2*>(&y);
+}
+// k[i]: the reciprocals of the scales of elements 2i, 2i+1 of the 8
+__device__ __forceinline__ uint2 quant8(const uint4& v, const uint64_t (&k)[4]) {
   const __half2* h2 = reinterpret_cast<const __half2*>(&v);
   const uint32_t u0 = quant_pair(h2[0], k[0]), u1 = quant_pair(h2[1], k[1]);
   const uint32_t u2 = quant_pair(h2[2], k[2]), u3 = quant_pair(h2[3], k[3]);
@@ -97,6 +91,27 @@ __device__ __forceinline__ void st_hint(void* p, uint2 v, uint64_t policy) {
 }
 
 constexpr int kQuantUnroll = 4;    // independent 128-bit loads in flight per lane
+
+// Scales of the four rows that the LPR lanes of a row group hold 8 elements of each (m: absmax of each lane's part): s[u] and
+// its reciprocal k[u].  The division, the rounding and the reciprocal cost more instructions than the quantisation of a
+// load itself, so no lane does them for all four rows: the rows' maxima are reduced as two fp16 pairs, the first step
+// of the butterfly leaves each lane one pair, and lane `sub` ends with the scale of row 2*(sub & 1) + (sub >> 1 & 1)
+// (returned), whose reciprocal the others fetch from it.
+template <int LPR>
+__device__ __forceinline__ float row_scales(const __half2 (&m)[4], int lane, float (&k)[4]) {
+  static_assert(kQuantUnroll == 4 && LPR >= 4, "one lane per row");
+  const __half2 p01 = __hmax2(__lows2half2(m[0], m[1]), __highs2half2(m[0], m[1]));
+  const __half2 p23 = __hmax2(__lows2half2(m[2], m[3]), __highs2half2(m[2], m[3]));
+  const bool odd = lane & 1;
+  __half2 p = __hmax2(odd ? p23 : p01, shfl_xor_h2(odd ? p01 : p23, 1));
+#pragma unroll
+  for (int o = 2; o < LPR; o <<= 1) p = __hmax2(p, shfl_xor_h2(p, o));
+  const float s = scale_from_amax((lane & 2) ? __high2float(p) : __low2float(p));
+  const float r = safe_rcp(s);
+#pragma unroll
+  for (int u = 0; u < 4; ++u) k[u] = __shfl_sync(0xffffffffu, r, (u >> 1) | ((u & 1) << 1), LPR);
+  return s;
+}
 
 // Per-token quantisation of the rows that CTA `cta` of `ncta` owns (a grid-stride loop over groups of rows).
 template <int D, bool CONTIG>
@@ -131,17 +146,28 @@ __device__ __forceinline__ void pertoken_rows(const __half* __restrict__ x, long
         }
       }
     }
+    float k[kQuantUnroll];
+    if constexpr (LPR >= 4) {
+      const __half2 m[4] = {amax8(v[0]), amax8(v[1]), amax8(v[2]), amax8(v[3])};
+      const float s = row_scales<LPR>(m, lane, k);
+      const long long row = row0 + (2 * (sub & 1) + (sub >> 1 & 1)) * RPW + lane / LPR;
+      if (sub < 4 && row < total_rows) scale[row] = s;
+    } else {
+#pragma unroll
+      for (int u = 0; u < kQuantUnroll; ++u) {
+        __half2 m = amax8(v[u]);
+        m = __hmax2(m, shfl_xor_h2(m, 1));
+        const float s = scale_from_amax(fmaxf(__low2float(m), __high2float(m)));
+        k[u] = safe_rcp(s);
+        if (sub == 0 && rows[u] < total_rows) scale[rows[u]] = s;
+      }
+    }
 #pragma unroll
     for (int u = 0; u < kQuantUnroll; ++u) {
-      float a = amax8(v[u]);
-#pragma unroll
-      for (int o = LPR / 2; o > 0; o >>= 1) a = fmaxf(a, __shfl_xor_sync(0xffffffffu, a, o));
-      const float s = scale_from_amax(a);
       if (rows[u] < total_rows) {
-        const Scale2 k1 = make_scale2(s, s);
-        const Scale2 k[4] = {k1, k1, k1, k1};
-        st_hint(x8 + rows[u] * D + sub * 8, quant8(v[u], k), once);
-        if (sub == 0) scale[rows[u]] = s;
+        const uint64_t k1 = f2_pack(k[u], k[u]);
+        const uint64_t kk[4] = {k1, k1, k1, k1};
+        st_hint(x8 + rows[u] * D + sub * 8, quant8(v[u], kk), once);
       }
     }
   }
@@ -316,9 +342,9 @@ __global__ void __launch_bounds__(256) v_quant_kernel(const __half* __restrict__
       scale[bh] = s_scale[0];
     }
   }
-  Scale2 k[4];
+  uint64_t k[4];
 #pragma unroll
-  for (int i = 0; i < 4; ++i) k[i] = make_scale2(s_scale[sub * 8 + 2 * i], s_scale[sub * 8 + 2 * i + 1]);
+  for (int i = 0; i < 4; ++i) k[i] = f2_pack(safe_rcp(s_scale[sub * 8 + 2 * i]), safe_rcp(s_scale[sub * 8 + 2 * i + 1]));
   while (r0 < r_end) {
     uint4 w[kQuantUnroll];
 #pragma unroll
