@@ -380,12 +380,11 @@ __global__ void scales_f16_to_f32_kernel(const __half* __restrict__ src, float* 
 int quant_pertoken(const void* x, const int64_t* st, void* x8, float* scale, int B, int H, int N, int D,
                    cudaStream_t stream) {
   const long long rows = (long long)B * H * N;
-  const int sms = sm_count_cached();
-  if (sms <= 0) return set_error(INTFA_ERR_CUDA, "cannot query SM count");
   const int rpw = 32 / (D / 8) * kQuantUnroll;
-  long long want = (rows + 8LL * rpw - 1) / (8LL * rpw);          // CTAs of 8 warps, one row group each
-  const int grid = (int)(want < (long long)sms * 8 ? (want < 1 ? 1 : want) : (long long)sms * 8);
   if (rows >= (1LL << 31)) return set_error(INTFA_ERR_TOO_LARGE, "quant_pertoken: B*H*N must be below 2^31");
+  // CTAs of 8 warps, one row group a warp: no loop, so a CTA's stores never hold back its own next loads (with a grid of 8
+  // CTAs an SM in a loop 18.6 us at 262144 rows of 128, now 16.7; at 1048576 rows 80 -> 67 us)
+  const int grid = (int)((rows + 8LL * rpw - 1) / (8LL * rpw));
   const bool contig = st[2] == D && st[1] == (int64_t)N * D && st[0] == (int64_t)H * N * D;
   int rc = INTFA_OK;
 #define INTFA_QPT(CC) \
