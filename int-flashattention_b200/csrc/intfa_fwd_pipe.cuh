@@ -39,11 +39,15 @@ template <int D, int G, bool FULL, int DQ = D, bool F8V = false>
 struct PipeCfg {
   static_assert(!(FULL && F8V), "fp8 V belongs to the half-int8 op");
   static constexpr bool BYTE_PV = FULL || F8V;                     // P and V elements are one byte
+  // fp16 P goes back into TMEM, over the first half of its own S buffer, and P V takes it from there (A operand in TMEM): no
+  // P buffers in shared memory (32 KB each), which makes room for a third softmax group and four V stages, no swizzled
+  // stores and no proxy fence.  Two groups with P in shared memory before: batch 4, 32 heads, 4096 tokens causal 732 -> 639 us,
+  // batch 2 non-causal 668 -> 565 us.  The S buffer goes back when the P V is done.
+  static constexpr bool P_TMEM = !BYTE_PV && D == 128 && DQ == 128 && G == 128;
   // Softmax groups of 128 threads.  Three (with 96 registers a thread, 16-column buffers) hide the hand-overs better than two
   // (152 registers, 32 columns) where P is one byte and a step is 128 wide, and for full-int8 at head dim 64: batch 2, 32/8
-  // heads, 3072 tokens, full-int8 causal 267 -> 240 us, fp8 V causal 116 -> 105 us.  fp16 P (a third buffer leaves two K
-  // stages) and head dim 256 lose: 337 -> 351 us, 216 -> 237 us.
-  static constexpr int NGRP = ((BYTE_PV && G == 128 && D == 128 && DQ == 128) || (FULL && G == 64 && D == 64)) ? 3 : 2;
+  // heads, 3072 tokens, full-int8 causal 267 -> 240 us, fp8 V causal 116 -> 105 us.  Head dim 256 loses: 216 -> 237 us.
+  static constexpr int NGRP = P_TMEM || (BYTE_PV && G == 128 && D == 128 && DQ == 128) || (FULL && G == 64 && D == 64) ? 3 : 2;
   static constexpr int THREADS = 256 + 128 * NGRP;
   // Registers: the CTA is launched with LAUNCH_REGS per thread and setmaxnreg only moves registers around
   // INSIDE that allocation -- an increase beyond it would block for ever, hence the static_assert below.
@@ -55,11 +59,11 @@ struct PipeCfg {
   static constexpr int Q_BYTES = kBM * DQ;
   static constexpr int K_BYTES = G * DQ;
   static constexpr int V_BYTES = BYTE_PV ? G * D : G * D * 2;         // int8, or fp16 as D/64 boxes of [G keys][64 channels]
-  static constexpr int P_BYTES = BYTE_PV ? kBM * G : kBM * G * 2;     // int8, or fp16 as G/64 blocks of [128 rows][64 columns]
+  static constexpr int P_BYTES = P_TMEM ? 0 : BYTE_PV ? kBM * G : kBM * G * 2;     // int8, or fp16 as G/64 blocks of [128 rows][64 columns]
   static constexpr int KS_BYTES = G * 4;
   static constexpr bool BIG = DQ > 128 && (G == 128 || D == 256);   // 32 KB K tiles, or 32 KB V tiles: three stages are what fits
   static constexpr int NSK = BIG ? 3 : 4;                          // K stages
-  static constexpr int NSV = BIG ? 3 : (BYTE_PV || G == 64) ? 4 : 2;  // V stages (fp16 V tiles are twice the size)
+  static constexpr int NSV = BIG ? 3 : (BYTE_PV || G == 64 || P_TMEM) ? 4 : 2;  // V stages (fp16 V tiles are twice the size)
   static constexpr int NKS = 8;                                    // K-scale slots: a slot is rewritten 8 steps later, when
                                                                    // the three S buffers have long forced its step out
   static constexpr int NSB = 3;                                    // S buffers in TMEM
@@ -111,6 +115,7 @@ struct PipeCfg {
   // the accumulator warps.  (Not with three groups: alpha and the row sums of a step would be overwritten too early.)
   static constexpr int NO = FULL && NGRP == 2 && NSB * G + 2 * D <= 512 ? 2 : 1;
   static_assert(NSB * G + NO * D <= 512, "TMEM columns");
+  static_assert(!P_TMEM || NGRP == NSB, "P of a group stays in the S buffer of its step");
   static constexpr int TMEM_COLS = 512;
   static_assert(FULL || G >= 64, "half-int8: fp16 P tiles are built from 64-column blocks");
   static constexpr uint64_t SWZ_QK = (QK_ROWB == 128) ? kSwz128 : (QK_ROWB == 64) ? kSwz64 : kSwz32;
@@ -175,6 +180,7 @@ intfa_fwd_pipe_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
   constexpr int B_AFULL = B_TDONE + 4;   // [4] half-int8: alpha of step j (slot j mod 4) published, for the accumulator warps
   constexpr int B_SFULL = B_AFULL + 4;   // [3] commit: S = Q K^T in TMEM buffer b
   constexpr int B_SFREE = B_SFULL + NSB; // [3] softmax group of the step (4 warps): S buffer b read out for good
+                                         //     (P_TMEM: commit: the P V that read P from it is done)
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + C::OFF_MISC);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + C::OFF_MISC + 4);
   volatile int* tile_slot = reinterpret_cast<volatile int*>(smem + C::OFF_MISC + 16);
@@ -206,7 +212,7 @@ intfa_fwd_pipe_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
     }
     for (int b = 0; b < NSB; ++b) {
       mbar_init(BAR(B_SFULL + b), 1);
-      mbar_init(BAR(B_SFREE + b), 4);
+      mbar_init(BAR(B_SFREE + b), C::P_TMEM ? 1 : 4);
     }
     for (int i = 0; i < 4; ++i) {
       mbar_init(BAR(B_TILE + i), 1);
@@ -469,12 +475,15 @@ intfa_fwd_pipe_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
               const uint32_t keep = (j > 0 || p.state_in) ? 1u : 0u;
 #pragma unroll
               for (int kk = 0; kk < G / 16; ++kk)
-                umma_f16(tA, ad0 + (uint64_t)((kk >> 2) * ((kBM * 128) >> 4) + (kk & 3) * 2), vd0 + (uint64_t)(kk * ((16 * C::V_ROWB) >> 4)),
+                if constexpr (C::P_TMEM)
+                  umma_f16_ts(tA, tS + b * G + kk * 8, vd0 + (uint64_t)(kk * ((16 * C::V_ROWB) >> 4)), C::IDESC_PV, kk > 0 ? 1u : keep);
+                else
+                  umma_f16(tA, ad0 + (uint64_t)((kk >> 2) * ((kBM * 128) >> 4) + (kk & 3) * 2), vd0 + (uint64_t)(kk * ((16 * C::V_ROWB) >> 4)),
                          C::IDESC_PV, kk > 0 ? 1u : keep);
             }
             umma_commit(BAR(B_OFULL + kv_it % NO));
             umma_commit(BAR(B_VEMPTY + s));
-            umma_commit(BAR(B_PFREE + b));
+            umma_commit(C::P_TMEM ? BAR(B_SFREE + b) : BAR(B_PFREE + b));
           }
           __syncwarp();
         }
