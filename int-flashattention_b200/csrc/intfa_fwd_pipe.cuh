@@ -41,13 +41,14 @@ struct PipeCfg {
   static constexpr bool BYTE_PV = FULL || F8V;                     // P and V elements are one byte
   // fp16 P goes back into TMEM, over the first half of its own S buffer, and P V takes it from there (A operand in TMEM): no
   // P buffers in shared memory (32 KB each), which makes room for a third softmax group and four V stages, no swizzled
-  // stores and no proxy fence.  Two groups with P in shared memory before: batch 4, 32 heads, 4096 tokens causal 732 -> 639 us,
-  // batch 2 non-causal 668 -> 565 us.  The S buffer goes back when the P V is done.
-  static constexpr bool P_TMEM = !BYTE_PV && D == 128 && DQ == 128 && G == 128;
+  // stores and no proxy fence.  Two groups with P in shared memory before: batch 4, 32 heads, 4096 tokens causal 733 -> 640 us,
+  // batch 2 non-causal 659 -> 565 us, batch 2 causal at d=64 347 -> 308 us.  The S buffer goes back when the P V is done.  With
+  // 64-column steps two groups stay the better (422 -> 398 us at d=64, three 401; 431 -> 421, 438 at d=128; 302 -> 288, 291 at d=256).
+  static constexpr bool P_TMEM = !BYTE_PV;
   // Softmax groups of 128 threads.  Three (with 96 registers a thread, 16-column buffers) hide the hand-overs better than two
   // (152 registers, 32 columns) where P is one byte and a step is 128 wide, and for full-int8 at head dim 64: batch 2, 32/8
   // heads, 3072 tokens, full-int8 causal 267 -> 240 us, fp8 V causal 116 -> 105 us.  Head dim 256 loses: 216 -> 237 us.
-  static constexpr int NGRP = P_TMEM || (BYTE_PV && G == 128 && D == 128 && DQ == 128) || (FULL && G == 64 && D == 64) ? 3 : 2;
+  static constexpr int NGRP = (P_TMEM && G == 128) || (BYTE_PV && G == 128 && D == 128 && DQ == 128) || (FULL && G == 64 && D == 64) ? 3 : 2;
   static constexpr int THREADS = 256 + 128 * NGRP;
   // Registers: the CTA is launched with LAUNCH_REGS per thread and setmaxnreg only moves registers around
   // INSIDE that allocation -- an increase beyond it would block for ever, hence the static_assert below.
@@ -59,14 +60,15 @@ struct PipeCfg {
   static constexpr int Q_BYTES = kBM * DQ;
   static constexpr int K_BYTES = G * DQ;
   static constexpr int V_BYTES = BYTE_PV ? G * D : G * D * 2;         // int8, or fp16 as D/64 boxes of [G keys][64 channels]
-  static constexpr int P_BYTES = P_TMEM ? 0 : BYTE_PV ? kBM * G : kBM * G * 2;     // int8, or fp16 as G/64 blocks of [128 rows][64 columns]
+  static constexpr int P_BYTES = P_TMEM ? 0 : kBM * G;              // int8 or e5m2
   static constexpr int KS_BYTES = G * 4;
   static constexpr bool BIG = DQ > 128 && (G == 128 || D == 256);   // 32 KB K tiles, or 32 KB V tiles: three stages are what fits
   static constexpr int NSK = BIG ? 3 : 4;                          // K stages
-  static constexpr int NSV = BIG ? 3 : (BYTE_PV || G == 64 || P_TMEM) ? 4 : 2;  // V stages (fp16 V tiles are twice the size)
+  static constexpr int NSV = BIG ? 3 : 4;                          // V stages
   static constexpr int NKS = 8;                                    // K-scale slots: a slot is rewritten 8 steps later, when
                                                                    // the three S buffers have long forced its step out
   static constexpr int NSB = 3;                                    // S buffers in TMEM
+  static constexpr int NPB = P_TMEM ? NSB : NGRP;                  // P buffers
   // Who carries the row sum l = l*alpha + rowsum(P)?  Where a KV step is as wide as the head (G >= D) the accumulator
   // warps do, next to the accumulator row: the softmax groups then meet once per step (running max) instead of
   // twice.  Where the head is wider than the step (head_dim 128 at G = 64) the accumulator warps are the busier
@@ -115,15 +117,14 @@ struct PipeCfg {
   // the accumulator warps.  (Not with three groups: alpha and the row sums of a step would be overwritten too early.)
   static constexpr int NO = FULL && NGRP == 2 && NSB * G + 2 * D <= 512 ? 2 : 1;
   static_assert(NSB * G + NO * D <= 512, "TMEM columns");
-  static_assert(!P_TMEM || NGRP == NSB, "P of a group stays in the S buffer of its step");
   static constexpr int TMEM_COLS = 512;
-  static_assert(FULL || G >= 64, "half-int8: fp16 P tiles are built from 64-column blocks");
+  static_assert(FULL || G >= 64, "half-int8");
   static constexpr uint64_t SWZ_QK = (QK_ROWB == 128) ? kSwz128 : (QK_ROWB == 64) ? kSwz64 : kSwz32;
   static constexpr uint32_t SBO_QK = 8 * QK_ROWB;
   // start-address offset (16-byte units) of the kk-th 32-byte K slice of a [ROWS][DQ] operand
   __host__ __device__ static constexpr uint32_t qk_slice(int kk, int rows) { return (uint32_t)((kk / 4) * ((rows * QK_ROWB) >> 4) + 2 * (kk % 4)); }
-  static constexpr uint64_t SWZ_P = BYTE_PV ? ((G == 128) ? kSwz128 : (G == 64) ? kSwz64 : kSwz32) : kSwz128;
-  static constexpr uint32_t SBO_P = BYTE_PV ? 8 * G : 1024;
+  static constexpr uint64_t SWZ_P = (G == 128) ? kSwz128 : (G == 64) ? kSwz64 : kSwz32;
+  static constexpr uint32_t SBO_P = 8 * G;
   // V rows: boxes of at most 128 bytes of channels
   static constexpr int V_ROWB = D * (BYTE_PV ? 1 : 2) < 128 ? D * (BYTE_PV ? 1 : 2) : 128;
   static constexpr int V_BOXES = D * (BYTE_PV ? 1 : 2) / V_ROWB;
@@ -165,7 +166,9 @@ intfa_fwd_pipe_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
   constexpr int NGRP = C::NGRP;
   constexpr int B_QFULL = 0;      // TMA: Q tile landed
   constexpr int B_QEMPTY = 1;     // commit: last Q K^T of the work item done
-  constexpr int B_PFULL = 2;      // [NGRP] softmax group b (4 warps): P in shared-memory buffer b, and S buffer b read out
+  constexpr int B_PFULL = 2;      // [NGRP] softmax group b (4 warps): P in shared-memory buffer b
+                                  //     (P_TMEM: [NSB], P in S buffer b: a group may be done with its next step before the
+                                  //     P V of this one is issued)
   constexpr int B_PFREE = 5;      // [NGRP] commit: the P V that read P buffer b is done
   constexpr int B_OFULL = 8;      // [NO] commit: O_j = P V in TMEM buffer (step mod NO)
   constexpr int B_OFREE = C::NUM_BARS - 3;   // [NO] accumulator warps (4): O_j read out
@@ -188,8 +191,8 @@ intfa_fwd_pipe_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
   if (threadIdx.x == 0) {
     mbar_init(BAR(B_QFULL), 1);
     mbar_init(BAR(B_QEMPTY), 1);
+    for (int b = 0; b < C::NPB; ++b) mbar_init(BAR(B_PFULL + b), 4);
     for (int b = 0; b < NGRP; ++b) {
-      mbar_init(BAR(B_PFULL + b), 4);
       mbar_init(BAR(B_PFREE + b), 1);
       mbar_init(BAR(B_HM + b), 4);
       mbar_init(BAR(B_HL + b), 4);
@@ -443,14 +446,14 @@ intfa_fwd_pipe_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         const TileInfo t = decode_tile<RAGGED, NVH>(p, tile, G);
         for (int j = 0; j < t.nsteps; ++j, ++kv_it) {
           const uint32_t s = kv_it % NSV, ph = (kv_it / NSV) & 1;
-          const uint32_t b = kv_it % NGRP;
+          const uint32_t b = kv_it % C::NPB;
           // P(j) written; V(j) landed; full-int8: O_j of the previous step has been read out, half-int8: the
           // accumulator has been brought to this step's running max (and the previous P V has landed in it).
           // (One copy of the wait code for the three.)
 #pragma unroll 1
           for (int w = 0; w < 3; ++w) {
             const uint32_t wb = w == 0 ? BAR(B_PFULL + b) : w == 1 ? BAR(B_VFULL + s) : BAR(B_OFREE + kv_it % NO);
-            const uint32_t wp = w == 0 ? ((kv_it / NGRP) & 1) : w == 1 ? ph : (FULL ? (((kv_it / NO) & 1) ^ 1) : (kv_it & 1));
+            const uint32_t wp = w == 0 ? ((kv_it / C::NPB) & 1) : w == 1 ? ph : (FULL ? (((kv_it / NO) & 1) ^ 1) : (kv_it & 1));
             ok = mbar_wait_warp<POLITE>(wb, wp, abort_flag, p.status, code_hi | (w == 0 ? PW_PFULL : w == 1 ? PW_VF : PW_OFREE));
             if (!ok) break;
           }
@@ -470,16 +473,12 @@ intfa_fwd_pipe_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
 #pragma unroll
               for (int kk = 0; kk < G / 32; ++kk) umma_f8(tA, ad0 + 2 * kk, vd0 + kk * ((32 * C::V_ROWB) >> 4), C::IDESC_PV, kk > 0 ? 1u : keep);
             } else {
-              // fp16 P (K-major, 64-column blocks of 128-byte rows) x fp16 V (MN-major), fp32 accumulate straight
+              // fp16 P (TMEM) x fp16 V (MN-major), fp32 accumulate straight
               // into the accumulator; the first P V of a fresh work item overwrites it
               const uint32_t keep = (j > 0 || p.state_in) ? 1u : 0u;
 #pragma unroll
               for (int kk = 0; kk < G / 16; ++kk)
-                if constexpr (C::P_TMEM)
-                  umma_f16_ts(tA, tS + b * G + kk * 8, vd0 + (uint64_t)(kk * ((16 * C::V_ROWB) >> 4)), C::IDESC_PV, kk > 0 ? 1u : keep);
-                else
-                  umma_f16(tA, ad0 + (uint64_t)((kk >> 2) * ((kBM * 128) >> 4) + (kk & 3) * 2), vd0 + (uint64_t)(kk * ((16 * C::V_ROWB) >> 4)),
-                         C::IDESC_PV, kk > 0 ? 1u : keep);
+                umma_f16_ts(tA, tS + b * G + kk * 8, vd0 + (uint64_t)(kk * ((16 * C::V_ROWB) >> 4)), C::IDESC_PV, kk > 0 ? 1u : keep);
             }
             umma_commit(BAR(B_OFULL + kv_it % NO));
             umma_commit(BAR(B_VEMPTY + s));

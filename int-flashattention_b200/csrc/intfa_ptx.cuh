@@ -347,6 +347,7 @@ __device__ __forceinline__ void tmem_ldw(uint32_t a, uint32_t (&r)[16]) { tmem_l
 __device__ __forceinline__ void tmem_ldw(uint32_t a, uint32_t (&r)[32]) { tmem_ld32(a, r); }
 __device__ __forceinline__ void tmem_ldw_wait(uint32_t (&r)[16]) { tmem_ld_wait16(r); }
 __device__ __forceinline__ void tmem_ldw_wait(uint32_t (&r)[32]) { tmem_ld_wait(r); }
+__device__ __forceinline__ void tmem_stw(uint32_t a, const uint32_t (&r)[8]) { tmem_st8(a, r); }
 __device__ __forceinline__ void tmem_stw(uint32_t a, const uint32_t (&r)[16]) { tmem_st16(a, r); }
 __device__ __forceinline__ void tmem_stw(uint32_t a, const uint32_t (&r)[32]) { tmem_st32(a, r); }
 

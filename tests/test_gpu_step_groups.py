@@ -7,7 +7,7 @@ import torch
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("variant,D,G", [("full", 128, 128), ("full", 64, 64), ("full", 32, 32), ("f8", 128, 128), ("half", 128, 128),
+@pytest.mark.parametrize("variant,D,G", [("full", 128, 128), ("full", 64, 64), ("full", 32, 32), ("f8", 128, 128), ("half", 128, 128), ("half", 64, 64), ("half", 32, 64), ("half", 128, 64),
                                          ("half", 256, 64), ("f8", 256, 64)])
 @pytest.mark.parametrize("N,causal", [(128, False), (257, True), (384, False), (500, False), (640, True)])
 def test_step_counts_that_are_no_multiple_of_the_groups(variant, D, G, N, causal, pkg, oracle):
