@@ -39,16 +39,18 @@ template <int D, int G, bool FULL, int DQ = D, bool F8V = false>
 struct PipeCfg {
   static_assert(!(FULL && F8V), "fp8 V belongs to the half-int8 op");
   static constexpr bool BYTE_PV = FULL || F8V;                     // P and V elements are one byte
-  // fp16 P goes back into TMEM, over the first half of its own S buffer, and P V takes it from there (A operand in TMEM): no
-  // P buffers in shared memory (32 KB each), which makes room for a third softmax group and four V stages, no swizzled
+  // P goes back into TMEM, over the first half of its own S buffer, and P V takes it from there (A operand in TMEM): no
+  // P buffers in shared memory (32 KB each for fp16), which makes room for a third softmax group and four V stages, no swizzled
   // stores and no proxy fence.  Two groups with P in shared memory before: batch 4, 32 heads, 4096 tokens causal 733 -> 640 us,
   // batch 2 non-causal 659 -> 565 us, batch 2 causal at d=64 347 -> 308 us.  The S buffer goes back when the P V is done.  With
   // 64-column steps two groups stay the better (422 -> 398 us at d=64, three 401; 431 -> 421, 438 at d=128; 302 -> 288, 291 at d=256).
-  static constexpr bool P_TMEM = !BYTE_PV;
+  // One-byte P: the same for fp8 V with 64-column steps (d=64 401 -> 380 us).  Three groups with small P buffers lose more from
+  // the S buffer's later return than they gain: fp8 V 301 -> 322 us, full-int8 383 -> 388, 64-column steps 714 -> 737.
+  static constexpr bool P_TMEM = !BYTE_PV || (F8V && G == 64);
   // Softmax groups of 128 threads.  Three (with 96 registers a thread, 16-column buffers) hide the hand-overs better than two
   // (152 registers, 32 columns) where P is one byte and a step is 128 wide, and for full-int8 at head dim 64: batch 2, 32/8
   // heads, 3072 tokens, full-int8 causal 267 -> 240 us, fp8 V causal 116 -> 105 us.  Head dim 256 loses: 216 -> 237 us.
-  static constexpr int NGRP = (P_TMEM && G == 128) || (BYTE_PV && G == 128 && D == 128 && DQ == 128) || (FULL && G == 64 && D == 64) ? 3 : 2;
+  static constexpr int NGRP = (!BYTE_PV && G == 128) || (BYTE_PV && G == 128 && D == 128 && DQ == 128) || (FULL && G == 64 && D == 64) ? 3 : 2;
   static constexpr int THREADS = 256 + 128 * NGRP;
   // Registers: the CTA is launched with LAUNCH_REGS per thread and setmaxnreg only moves registers around
   // INSIDE that allocation -- an increase beyond it would block for ever, hence the static_assert below.
@@ -68,6 +70,7 @@ struct PipeCfg {
   static constexpr int NKS = 8;                                    // K-scale slots: a slot is rewritten 8 steps later, when
                                                                    // the three S buffers have long forced its step out
   static constexpr int NSB = 3;                                    // S buffers in TMEM
+  static constexpr int P_PER_COL = BYTE_PV ? 4 : 2;                // P_TMEM: elements of P in a TMEM column
   static constexpr int NPB = P_TMEM ? NSB : NGRP;                  // P buffers
   // Who carries the row sum l = l*alpha + rowsum(P)?  Where a KV step is as wide as the head (G >= D) the accumulator
   // warps do, next to the accumulator row: the softmax groups then meet once per step (running max) instead of
@@ -85,6 +88,7 @@ struct PipeCfg {
   // steps of 1 KB for each kind of instantiation (`ragged`: masks partial tiles; `polite`: see the kernel).  Between the best
   // and the worst of a sweep lie 1 to 2 % non-causal, 5 to 15 % causal.
   __host__ __device__ static constexpr int code_filler_of(bool ragged, bool polite) {
+    if (P_TMEM) return G == 128 ? (ragged ? 0 : 192) : D == 256 ? (ragged ? 384 : 0) : D == 128 ? (ragged ? 256 : 128) : ragged ? 128 : 256;
     return NGRP == 3 ? (!FULL ? 192 : (ragged && G == 128) ? 64 : polite ? 128 : 256)
          : ragged ? 256 : G == 128 ? (FULL ? 448 : 384) : (D == 256 || (FULL && D == 64)) ? 0 : D == 32 ? 256 : 128;
   }
@@ -471,7 +475,10 @@ intfa_fwd_pipe_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
               // e5m2 P x e5m2 V (both one byte, laid out like the int8 tiles), fp32 accumulate straight into the accumulator
               const uint32_t keep = (j > 0 || p.state_in) ? 1u : 0u;
 #pragma unroll
-              for (int kk = 0; kk < G / 32; ++kk) umma_f8(tA, ad0 + 2 * kk, vd0 + kk * ((32 * C::V_ROWB) >> 4), C::IDESC_PV, kk > 0 ? 1u : keep);
+              for (int kk = 0; kk < G / 32; ++kk) {
+                if constexpr (C::P_TMEM) umma_f8_ts(tA, tS + b * G + kk * 8, vd0 + kk * ((32 * C::V_ROWB) >> 4), C::IDESC_PV, kk > 0 ? 1u : keep);
+                else umma_f8(tA, ad0 + 2 * kk, vd0 + kk * ((32 * C::V_ROWB) >> 4), C::IDESC_PV, kk > 0 ? 1u : keep);
+              }
             } else {
               // fp16 P (TMEM) x fp16 V (MN-major), fp32 accumulate straight
               // into the accumulator; the first P V of a fresh work item overwrites it
