@@ -69,7 +69,10 @@ struct PipeCfg {
   static constexpr int NSV = BIG ? 3 : 4;                          // V stages
   static constexpr int NKS = 8;                                    // K-scale slots: a slot is rewritten 8 steps later, when
                                                                    // the three S buffers have long forced its step out
-  static constexpr int NSB = 3;                                    // S buffers in TMEM
+  // S buffers in TMEM.  Four where a step's buffer waits for its P V and there is room (d=64: 385 -> 371 us, d=128 at G=64 421 ->
+  // 414; no gain at d=256).
+  static constexpr int NSB = P_TMEM && G == 64 && D <= 128 ? 4 : 3;
+  static constexpr int NRS = NSB == 4 ? 8 : 4;                     // row-sum slots: step j's is read at step j+1, when P V j+1 may be out
   static constexpr int P_PER_COL = BYTE_PV ? 4 : 2;                // P_TMEM: elements of P in a TMEM column
   static constexpr int NPB = P_TMEM ? NSB : NGRP;                  // P buffers
   // Who carries the row sum l = l*alpha + rowsum(P)?  Where a KV step is as wide as the head (G >= D) the accumulator
@@ -106,7 +109,7 @@ struct PipeCfg {
   static constexpr int OFF_HM = OFF_VSD + D * 4;                  // [2 groups][128] float: running max after the group's latest step
   static constexpr int OFF_RS = OFF_HM + NGRP * 128 * 4;             // [4][128] float: row sum of P of step j, for the accumulator warps
                                                                    //   (!L_IN_ACC: [2 groups][128] float, l after the group's latest step)
-  static constexpr int OFF_ALPHA = OFF_RS + 4 * 128 * 4;          // [4][128] float: alpha of step j, for the accumulator warps
+  static constexpr int OFF_ALPHA = OFF_RS + NRS * 128 * 4;          // [4][128] float: alpha of step j, for the accumulator warps
   static constexpr int OFF_FIN = OFF_ALPHA + 4 * 128 * 4;         // [2][128] float2: final running max of a work item (.x)
   static constexpr int OFF_MAGIC = OFF_FIN + 2 * 128 * 8;          // 4 KB constant fp16 operand of the "arm" MMA
   static constexpr int MAGIC_BYTES = 4096;
@@ -197,7 +200,7 @@ intfa_fwd_pipe_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
     mbar_init(BAR(B_QEMPTY), 1);
     for (int b = 0; b < C::NPB; ++b) mbar_init(BAR(B_PFULL + b), 4);
     for (int b = 0; b < NGRP; ++b) {
-      mbar_init(BAR(B_PFREE + b), 1);
+      if (!C::P_TMEM) mbar_init(BAR(B_PFREE + b), 1);      // (the fourth P-full barrier otherwise)
       mbar_init(BAR(B_HM + b), 4);
       mbar_init(BAR(B_HL + b), 4);
     }
