@@ -61,3 +61,21 @@ def test_few_rows_against_a_cache(variant, B, Hkv, ratio, Nq, Nk, D, G, causal, 
     fn = pkg.attention_full_int8 if variant == "full" else pkg.attention_int8
     again = fn(*args, causal, sm, G=G, q_offset=off, out_dtype=torch.bfloat16)
     assert ((again.float() - out.float()).abs() <= out.float().abs() * (2.0 ** -8 + 2.0 ** -11) + 1e-7).all()
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("Nq,Nk", [(1, 77), (77, 77), (2, 4097), (3, 8)])
+def test_an_infinity_in_the_last_key_of_v(Nq, Nk, D, pkg, oracle):
+    """It reaches its own channel only, as an infinity: the keys that fill up the last step weigh nothing."""
+    g = torch.Generator().manual_seed(Nk + D)
+    q, k, v = (torch.randn(1, 2, n, D, generator=g).half() for n in (Nq, Nk, Nk))
+    v[:, :, -1, 3] = float("inf")
+    v[:, :, -1, D - 1] = -float("inf")
+    (q8, qs), (k8, ks) = oracle.quant_pertoken(q), oracle.quant_pertoken(k)
+    out = pkg.attention_int8(*(t.cuda() for t in (q8, k8, v, qs.float(), ks.float())), False, D ** -0.5).cpu()
+    v[:, :, -1, 3] = v[:, :, -1, D - 1] = 0
+    ref = oracle.attention_int8(q8, k8, v, qs, ks, False, D ** -0.5, G=128)
+    assert (out[..., 3] == float("inf")).all() and (out[..., D - 1] == -float("inf")).all()
+    out[..., 3], out[..., D - 1] = ref[..., 3], ref[..., D - 1]
+    e = oracle.err_metrics(out, ref)
+    assert e["max_abs"] <= 4e-3 and e["mean_rel"] <= 3e-4, e
