@@ -185,8 +185,9 @@ __global__ void __launch_bounds__(kThreads) scores_kernel(const DParams p, int s
 #pragma unroll
         for (int hr = 0; hr < NT; ++hr) {
           float2 s;
-          s.x = key <= q.last[hr] ? unmagic(d[2 * hr]) * q.s[hr] * k0[i] : -1e30f;
-          s.y = key + 1 <= q.last[hr] ? unmagic(d[2 * hr + 1]) * q.s[hr] * k1[i] : -1e30f;
+          // (what a row does not see: the next pass scales it by sm_scale, so no finite number would do)
+          s.x = key <= q.last[hr] ? unmagic(d[2 * hr]) * q.s[hr] * k0[i] : -INFINITY;
+          s.y = key + 1 <= q.last[hr] ? unmagic(d[2 * hr + 1]) * q.s[hr] * k1[i] : -INFINITY;
           mx[hr] = max3(mx[hr], s.x, s.y);
           sc[((kt + i) * NT + hr) * 32] = s;
         }

@@ -79,3 +79,16 @@ def test_an_infinity_in_the_last_key_of_v(Nq, Nk, D, pkg, oracle):
     out[..., 3], out[..., D - 1] = ref[..., 3], ref[..., D - 1]
     e = oracle.err_metrics(out, ref)
     assert e["max_abs"] <= 4e-3 and e["mean_rel"] <= 3e-4, e
+
+
+@pytest.mark.parametrize("sm", [1e-27, 1e-30, 1e-37])
+@pytest.mark.parametrize("Nq,Nk,G", [(1, 300, 128), (5, 70, 64), (77, 77, 64)])
+def test_masked_keys_weigh_nothing_at_any_softmax_scale(Nq, Nk, G, sm, pkg, oracle):
+    g = torch.Generator().manual_seed(Nk)
+    q, k, v = (torch.randn(1, 2, n, 64, generator=g).half() for n in (Nq, Nk, Nk))
+    (q8, qs), (k8, ks), (v8, vs) = oracle.quant_pertoken(q), oracle.quant_pertoken(k), oracle.quant_perchannel(v)
+    off = (Nk - Nq) // 3
+    ref = oracle.attention_full_int8(q8, k8, v8, qs, ks, vs, True, sm, G=G, q_offset=off)
+    out = pkg.attention_full_int8(*(t.cuda() for t in (q8, k8, v8, qs, ks, vs)), True, sm, G=G, q_offset=off)
+    e = oracle.err_metrics(out.cpu(), ref)
+    assert e["max_abs"] <= 4e-3 and e["mean_rel"] <= 3e-4, e
