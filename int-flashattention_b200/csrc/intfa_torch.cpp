@@ -206,6 +206,9 @@ void set_sizes(IntfaFwdParams& P, const at::Tensor& q, const at::Tensor& k, cons
   P.H_kv = k.size(1);                       // grouped-query attention: fewer K/V heads than query heads
   if (P.H_kv <= 0 || v.size(1) != P.H_kv || P.H % P.H_kv != 0)
     raise(PyExc_ValueError, "k and v must have the same number of heads, dividing the " + std::to_string(P.H) + " query heads");
+  // (longer ones are read in part)
+  if (k.size(0) < P.B || v.size(0) < P.B) raise(PyExc_ValueError, "k and v must have the batch size of q, " + std::to_string(P.B));
+  if (v.size(2) < P.Nk) raise(PyExc_ValueError, "v must have the " + std::to_string(P.Nk) + " keys of k, got " + std::to_string(v.size(2)));
   P.variant = full ? INTFA_VARIANT_FULL : is(v, at::kFloat8_e5m2) ? INTFA_VARIANT_HALF_FP8 : INTFA_VARIANT_HALF;
   P.G = G != kAutoG ? G : default_G(P.D, full);
 }
@@ -216,6 +219,11 @@ void check_v_type(const at::Tensor& v, bool full) {
   if (full && !is(v, at::kChar)) raise(PyExc_TypeError, "full-int8: v must be int8");
   // V (and with it P) in fp8: flash_atten_int8.py:55-56
   if (!full && !is(v, at::kHalf) && !is(v, at::kFloat8_e5m2)) raise(PyExc_TypeError, "half-int8: v must be float16 or float8_e5m2");
+}
+// The kernels read a scale tensor by its strides: `last` is the index of the last element they touch.
+void need_scales(const at::Tensor& s, const char* what, int64_t last) {
+  if (last >= s.numel())
+    raise(PyExc_ValueError, std::string(what) + " is too short: element " + std::to_string(last) + " is read, it holds " + std::to_string(s.numel()));
 }
 void check_head_dims(const at::Tensor& q, const at::Tensor& k, const at::Tensor& v) {
   // shape constraints, as flash_atten_full_int8.py:189-193
@@ -250,7 +258,12 @@ PyObject* forward(IntfaFwdParams& P, Options& o, c10::Device dev, bool causal, d
     P.lse_out = lse.data_ptr<float>();
   }
   if (o.have_state || o.return_state) {
-    if (!o.have_state) {
+    if (o.have_state) {
+      const int64_t rows = B * H * Nq;
+      for (const at::Tensor* x : {&o.m, &o.l, &o.acc})
+        if (x->device() != dev || x->numel() < (x == &o.acc ? rows * D : rows))
+          raise(PyExc_ValueError, "state is (m, l [B,H,Nq], acc [B,H,Nq,D]) on the device of q");
+    } else {
       o.m = empty({B, H, Nq}, at::kFloat, dev);
       o.l = empty({B, H, Nq}, at::kFloat, dev);
       o.acc = empty({B, H, Nq, D}, at::kFloat, dev);
@@ -310,6 +323,8 @@ PyObject* fwd(PyObject*, PyObject* const* a, Py_ssize_t n, PyObject* kwnames) {
     const at::Tensor &qs0 = tensor(a[4], "q_scale"), &ks0 = tensor(a[5], "k_scale");
     for (const at::Tensor* t : {&q0, &k0, &v0, &qs0, &ks0}) need_cuda(*t);
     if (a[6] != Py_None) need_cuda(tensor(a[6], "v_scale"));
+    for (const at::Tensor* t : {&k0, &v0, &qs0, &ks0})
+      if (t->device() != q0.device()) raise(PyExc_ValueError, "all tensors must be on the device of q");
     if (!is(q0, at::kChar) || !is(k0, at::kChar)) raise(PyExc_TypeError, "q and k must be int8");
     check_v_type(v0, full);
     need_4d(q0, "q");
@@ -338,6 +353,11 @@ PyObject* fwd(PyObject*, PyObject* const* a, Py_ssize_t n, PyObject* kwnames) {
       P.qs_stride[i] = qs.stride(i);
       P.ks_stride[i] = ks.stride(i);
     }
+    need_scales(qs, "q_scale", (P.B - 1) * P.qs_stride[0] + (P.H - 1) * P.qs_stride[1] + P.Nq - 1);
+    need_scales(ks, "k_scale", (P.B - 1) * P.ks_stride[0] + (P.H_kv - 1) * P.ks_stride[1] + P.Nk - 1);
+    // (where the last KV step is partial, rows of another length have always been an error)
+    if (P.G > 0 && P.Nk % P.G != 0 && (ks.dim() != 3 || ks.size(2) != P.Nk))
+      raise(PyExc_ValueError, "k_scale must have shape (B,H," + std::to_string(P.Nk) + ")");
     P.scale_f16 = (is(qs, at::kHalf) ? INTFA_SCALE_F16_Q : 0) | (is(ks, at::kHalf) ? INTFA_SCALE_F16_K : 0);
     if (full) {
       vs = scales(tensor(a[6], "v_scale"));
@@ -356,6 +376,9 @@ PyObject* fwd(PyObject*, PyObject* const* a, Py_ssize_t n, PyObject* kwnames) {
           raise(PyExc_ValueError, "per-tile v_scale needs ceil(Nk/G) = " + std::to_string(want) + " rows, got " + std::to_string(vs.size(2)));
         P.vs_stride_blk = vs.stride(2);
       }
+      if (vs.device() != dev) raise(PyExc_ValueError, "all tensors must be on the device of q");
+      need_scales(vs, "v_scale", (P.B - 1) * P.vs_stride[0] + (P.H_kv - 1) * P.vs_stride[1] + (P.D - 1) * P.vs_stride[2] +
+                                     (d == 4 ? (vs.size(2) - 1) * P.vs_stride_blk : 0));
     }
     return forward(P, o, dev, truth(a[7]), as_double(a[8]));
   } catch (const PySet&) {
@@ -432,6 +455,7 @@ struct Qkv {
 };
 Qkv qkv_in(const at::Tensor& q0, const at::Tensor& k0, const at::Tensor* v0) {
   Qkv x;
+  if (k0.device() != q0.device() || (v0 && v0->device() != q0.device())) raise(PyExc_ValueError, "q, k and v must be on the same device");
   x.q = quant_in(q0).contiguous();
   x.k = quant_in(k0).contiguous();
   if (v0) {
@@ -444,6 +468,7 @@ Qkv qkv_in(const at::Tensor& q0, const at::Tensor& k0, const at::Tensor* v0) {
   x.D = x.q.size(3);
   x.Hkv = x.k.size(1);
   x.Nk = x.k.size(2);
+  if (x.k.size(0) < x.B) raise(PyExc_ValueError, "k must have the batch size of q, " + std::to_string(x.B));
   return x;
 }
 void run_quant_qkv(const Qkv& x, void* q8, void* k8, void* v8, float* qs, float* ks, float* vs, int mode, void* ws, size_t ws_bytes) {
@@ -470,6 +495,7 @@ PyObject* quant_qkv(PyObject*, PyObject* const* a, Py_ssize_t n) {
     const c10::Device dev = q0.device();
     c10::cuda::CUDAGuard guard(dev);
     const Qkv x = qkv_in(q0, k0, have_v ? &tensor(a[2], "v") : nullptr);
+    if (x.k.size(3) != x.D) raise(PyExc_ValueError, "q and k must have the same head dim");
     at::Tensor q8 = empty({x.B, x.H, x.Nq, x.D}, at::kChar, dev), k8 = empty({x.B, x.Hkv, x.Nk, x.D}, at::kChar, dev);
     at::Tensor qs = empty({x.B, x.H, x.Nq}, at::kFloat, dev), ks = empty({x.B, x.Hkv, x.Nk}, at::kFloat, dev);
     if (!have_v) {
@@ -507,6 +533,7 @@ PyObject* flash(PyObject*, PyObject* const* a, Py_ssize_t n, PyObject* kwnames) 
     at::Tensor v = x.v;
     if (!full) {
       need_cuda(v0);
+      if (v0.device() != dev) raise(PyExc_ValueError, "q, k and v must be on the same device");
       check_v_type(v0, false);
       need_4d(v0, "v");
       v = tma_ready(v0);
