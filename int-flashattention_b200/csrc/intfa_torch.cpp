@@ -337,7 +337,11 @@ PyObject* fwd(PyObject*, PyObject* const* a, Py_ssize_t n, PyObject* kwnames) {
     set_sizes(P, q0, k0, v0, full, o.G);
     const c10::Device dev = q0.device();
     c10::cuda::CUDAGuard guard(dev);
-    const at::Tensor q = tma_ready(q0), k = tma_ready(k0), v = tma_ready(v0), qs = scales(qs0), ks = scales(ks0);
+    const at::Tensor q = tma_ready(q0), k = tma_ready(k0), v = tma_ready(v0), qs = scales(qs0);
+    at::Tensor ks = scales(ks0);
+    // (where the last KV step is partial, one scale per (batch, head) has always stood for all its keys)
+    const bool ragged = P.G > 0 && P.Nk % P.G != 0;
+    if (ragged && ks.dim() == 3 && ks.size(2) == 1) ks = ks.expand({ks.size(0), ks.size(1), P.Nk}).contiguous();
     at::Tensor vs;
     P.q = q.data_ptr();
     P.k = k.data_ptr();
@@ -355,8 +359,8 @@ PyObject* fwd(PyObject*, PyObject* const* a, Py_ssize_t n, PyObject* kwnames) {
     }
     need_scales(qs, "q_scale", (P.B - 1) * P.qs_stride[0] + (P.H - 1) * P.qs_stride[1] + P.Nq - 1);
     need_scales(ks, "k_scale", (P.B - 1) * P.ks_stride[0] + (P.H_kv - 1) * P.ks_stride[1] + P.Nk - 1);
-    // (where the last KV step is partial, rows of another length have always been an error)
-    if (P.G > 0 && P.Nk % P.G != 0 && (ks.dim() != 3 || ks.size(2) != P.Nk))
+    // (... and rows of another length an error)
+    if (ragged && (ks.dim() != 3 || ks.size(2) != P.Nk))
       raise(PyExc_ValueError, "k_scale must have shape (B,H," + std::to_string(P.Nk) + ")");
     P.scale_f16 = (is(qs, at::kHalf) ? INTFA_SCALE_F16_Q : 0) | (is(ks, at::kHalf) ? INTFA_SCALE_F16_K : 0);
     if (full) {

@@ -55,6 +55,19 @@ def test_a_k_scale_of_another_length_on_a_ragged_call_is_refused(pkg):
             _call(pkg, dict(t, ks=torch.ones(B, HKV, n, device="cuda:0")), G=64)
 
 
+@pytest.mark.parametrize("variant", ["full", "half"])
+@pytest.mark.parametrize("Nq,Nk", [(1, 77), (130, 200)])
+def test_one_k_scale_for_all_keys_of_a_ragged_call(variant, Nq, Nk, pkg):
+    g = torch.Generator().manual_seed(2)
+    t = _tensors(Nq, Nk, variant)
+    for n in ("q", "k", "v"):
+        t[n] = torch.randint(-127, 128, t[n].shape, generator=g).to(t[n].dtype).cuda()
+    one = torch.tensor([[1.0, 2.0], [0.5, 3.0]], device="cuda:0").view(B, HKV, 1) / 500
+    for dtype in (torch.float32, torch.float16):
+        got = _call(pkg, dict(t, ks=one.to(dtype)), True, q_offset=Nk - Nq)
+        assert torch.equal(got, _call(pkg, dict(t, ks=one.to(dtype).expand(B, HKV, Nk).contiguous()), True, q_offset=Nk - Nq))
+
+
 def test_longer_tensors_are_read_in_part(pkg):
     g = torch.Generator().manual_seed(1)
     t = _tensors(128, 256, "full")
