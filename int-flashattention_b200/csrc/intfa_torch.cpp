@@ -96,8 +96,12 @@ const char* const kNames[N_COUNT] = {"G", "p_round", "kv_order", "state", "q_off
                                      "write_o", "debug_tap", "out_dtype", "debug_wait"};
 PyObject* g_names[N_COUNT];             // interned
 
+// int(o) and float(o): any number, a tensor of one element, a string
 int64_t as_long(PyObject* o) {
-  const long long v = PyLong_AsLongLong(o);
+  PyObject* i = PyNumber_Long(o);
+  if (!i) throw PySet();
+  const long long v = PyLong_AsLongLong(i);
+  Py_DECREF(i);
   if (v == -1 && PyErr_Occurred()) throw PySet();
   return v;
 }
@@ -107,8 +111,10 @@ bool truth(PyObject* o) {
   return v != 0;
 }
 double as_double(PyObject* o) {
-  const double v = PyFloat_AsDouble(o);
-  if (v == -1.0 && PyErr_Occurred()) throw PySet();
+  PyObject* f = PyNumber_Float(o);
+  if (!f) throw PySet();
+  const double v = PyFloat_AS_DOUBLE(f);
+  Py_DECREF(f);
   return v;
 }
 bool equals(PyObject* s, const char* w) { return PyUnicode_Check(s) && PyUnicode_CompareWithASCIIString(s, w) == 0; }
@@ -129,12 +135,12 @@ int name_index(PyObject* name) {
 void pair_of_ints(PyObject* v, int* a, int* b) {
   PyObject* t = PySequence_Tuple(v);
   if (!t) throw PySet();
+  PyObject* i[2] = {nullptr, nullptr};
   const bool ok = PyTuple_GET_SIZE(t) == 2;
-  long x = 0, y = 0;
-  if (ok) {
-    x = PyLong_AsLong(PyTuple_GET_ITEM(t, 0));
-    y = PyLong_AsLong(PyTuple_GET_ITEM(t, 1));
-  }
+  for (int n = 0; ok && n < 2 && (n == 0 || i[0]); ++n) i[n] = PyNumber_Long(PyTuple_GET_ITEM(t, n));
+  const long x = i[0] ? PyLong_AsLong(i[0]) : 0, y = i[1] ? PyLong_AsLong(i[1]) : 0;
+  Py_XDECREF(i[0]);
+  Py_XDECREF(i[1]);
   Py_DECREF(t);
   if (PyErr_Occurred()) throw PySet();
   if (!ok) raise(PyExc_ValueError, "expected a pair");

@@ -101,3 +101,22 @@ def test_the_prologue_refuses_short_tensors(variant, pkg):
         with pytest.raises(ValueError):
             pkg.quant_qkv(*bad)
     pkg.check_status()
+
+
+def test_options_take_any_number(pkg):
+    g = torch.Generator().manual_seed(3)
+    t = _tensors(130, 200, "full")
+    for n in ("q", "k", "v"):
+        t[n] = torch.randint(-127, 128, t[n].shape, generator=g).to(torch.int8).cuda()
+    t["qs"] *= 0.01
+    t["ks"] *= 0.01
+    args = [t[n] for n in ("q", "k", "v", "qs", "ks", "vs")]
+    want = pkg.attention_full_int8(*args, True, 0.125, G=64, q_offset=70, kv_offset=0, debug_tap=(1, 0))
+    got = pkg.attention_full_int8(*args, True, "0.125", G=64.0, q_offset=torch.tensor(70.0), kv_offset=0.0, debug_tap=[1.0, torch.tensor(0)])
+    assert torch.equal(got[0], want[0]) and torch.equal(got[1][0], want[1][0])
+    for kw in ({"G": "wide"}, {"q_offset": float("nan")}, {"debug_tap": (1, "x")}, {"debug_tap": (1, 2, 3)}):
+        with pytest.raises(ValueError):
+            pkg.attention_full_int8(*args, True, 0.125, **kw)
+    for kw in ({"q_offset": None}, {"debug_tap": 1}, {"debug_tap": ([], 0)}):
+        with pytest.raises(TypeError):
+            pkg.attention_full_int8(*args, True, 0.125, **kw)
