@@ -57,7 +57,8 @@ int intfa_last_error(char* buf, size_t len);
  * Tensors are [B, H, N, D]; strides are in ELEMENTS for dims (B, H, N); the last
  * dim must be contiguous.  q,k: int8.  v: int8 (FULL) or fp16 (HALF).  o: fp16.
  * Byte strides of q/k/v and their base pointers must be multiples of 16 (TMA).
- * q_scale [B,H,Nq], k_scale [B,H,Nk]: fp32 or fp16 (scale_f16), contiguous over N, strides for (B,H).
+ * q_scale [B,H,Nq], k_scale [B,H,Nk]: fp32 or fp16 (scale_f16), contiguous over N, strides for (B,H); rows of k_scale
+ * are at least Nk elements apart.
  * v_scale (FULL only): fp32 or fp16, element strides for (B,H,D); stride 0 over D
  * broadcasts a per-(batch,head) scale.
  */

@@ -90,6 +90,9 @@ int intfa_fwd(const IntfaFwdParams* p, void* stream) {
   if ((rc = check_tma_tensor("k", p->k, p->k_stride, 1))) return rc;
   if ((rc = check_tma_tensor("v", p->v, p->v_stride, p->variant == INTFA_VARIANT_HALF ? 2 : 1))) return rc;
   if (!p->q_scale || !p->k_scale) return set_error(INTFA_ERR_INVALID_ARG, "q_scale / k_scale is NULL");
+  if (((p->H_kv > 0 ? p->H_kv : p->H) > 1 && p->ks_stride[1] < p->Nk) || (p->B > 1 && p->ks_stride[0] < p->Nk))
+    return set_error(INTFA_ERR_INVALID_ARG, "k_scale rows must hold Nk = %d elements each: strides %lld, %lld", p->Nk, (long long)p->ks_stride[0],
+                     (long long)p->ks_stride[1]);
   if (full && !p->v_scale) return set_error(INTFA_ERR_INVALID_ARG, "v_scale is NULL (full-int8)");
   if (p->kv_order != 0 && p->kv_order != 1) return set_error(INTFA_ERR_INVALID_ARG, "kv_order must be 0 (ascending) or 1 (descending)");
   if (p->vs_stride_blk < 0) return set_error(INTFA_ERR_INVALID_ARG, "vs_stride_blk must not be negative");

@@ -93,6 +93,24 @@ def test_validation_rejects_before_launch(lib):
     assert h.intfa_quant_v_workspace_bytes(2, 3, 128) == 2 * 3 * 128 * 4
 
 
+@pytest.mark.parametrize("Nk", [128, 200])
+def test_k_scale_rows_shorter_than_nk_are_refused(lib, Nk):
+    """(No pointer is followed before the strides have been looked at.)"""
+    h = lib.load()
+    P = lib.IntfaFwdParams()
+    P.q = P.k = P.v = P.o = P.q_scale = P.k_scale = P.v_scale = 1 << 20
+    for n in ("q_stride", "k_stride", "v_stride", "o_stride"):
+        setattr(P, n, lib._i64x3(2 * 256 * 128, 256 * 128, 128))
+    P.B, P.H, P.Nq, P.Nk, P.D, P.G, P.sm_scale, P.write_o, P.o_dtype = 2, 2, 256, Nk, 128, 128, 0.1, 1, 0
+    for strides in ((2 * Nk, Nk - 1), (Nk - 1, Nk), (0, Nk), (2 * Nk, 0)):
+        P.ks_stride = lib._i64x2(*strides)
+        assert h.intfa_fwd(ctypes.byref(P), None) == lib.ERR_INVALID_ARG
+        assert "k_scale rows" in lib.last_error()
+    P.ks_stride, P.o = lib._i64x2(2 * Nk, Nk), None                       # the next thing to be refused
+    assert h.intfa_fwd(ctypes.byref(P), None) == lib.ERR_INVALID_ARG
+    assert "o is NULL" in lib.last_error()
+
+
 def test_python_surface_refuses_cpu_tensors(pkg):
     import torch
     q = torch.zeros(1, 1, 128, 64, dtype=torch.int8)
