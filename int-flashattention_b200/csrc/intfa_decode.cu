@@ -44,6 +44,7 @@ struct DParams {
   long long qsB, qsH, ksB, ksH, vsB, vsH, vsD;
   int scale_f16, o_bf16, causal;
   int H, Hkv, ratio, Nq, R, tiles;        // R = ratio*Nq rows per K/V head, in `tiles` tiles of RT rows
+  int unit0;                              // the launch's first unit (its scratch begins with this one)
   int nvis;                               // keys that some row sees
   long long limit0;                       // causal: row n sees the keys <= limit0 + n
   float c;                                // sm_scale * log2(e)
@@ -82,11 +83,12 @@ struct Const {
 };
 // one (batch, K/V head, row tile)
 struct Unit {
-  int id, b, hk, tile;
+  int id, b, hk, tile;                    // id: counted from the launch's first, as scratch is
 };
 __device__ __forceinline__ Unit unit_of(const DParams& p, int id) {
   Unit u;
   u.id = id;
+  id += p.unit0;
   u.tile = id % p.tiles;
   const int bh = id / p.tiles;
   u.b = bh / p.Hkv;
@@ -752,7 +754,7 @@ __global__ void __launch_bounds__(kCombineThreads) combine_many_kernel(const DPa
 // ---------------------------------------------------------------------------------------------------------------
 struct Plan {
   bool use = false, full = false;
-  int NT = 1, tiles = 1, units = 0, nvis = 0, groups = 0, splits = 1, per_split = 1, score_splits = 1;
+  int NT = 1, tiles = 1, units = 0, slice = 0, nvis = 0, groups = 0, splits = 1, per_split = 1, score_splits = 1;
   size_t off_gmax = 0, off_part = 0, off_ml = 0, bytes = 0;
 };
 
@@ -761,10 +763,15 @@ struct Plan {
 //              path costs with all its rows alive, but rows are padded to 8 or 16 instead of 128 and keys are split.
 //   128 rows   `c0` (pipeline fill), then `s` per KV step of G keys: the longest work item, or what an SM gets of all steps.
 // The margin of 10 % keeps the 128-row kernel where the two are alike.
+// Scratch of one call, unless one unit needs more.  The scores of full-int8 are fp32 and padded to 8 or 16 rows, up to as much
+// again as K and V, so a call that needs more takes its units in slices that share it, one after the other.
+constexpr size_t kMaxScratch = (size_t)128 << 20;
+
 bool faster_than_tiles(const IntfaFwdParams* a, const Plan& pl, int sms) {
   const bool d128 = a->D == 128;
   const double u = pl.full ? (d128 ? 0.59 : 0.45) : (d128 ? 0.50 : 0.27);
-  const double here = (pl.full ? 7.0 : 4.5) + (pl.splits > 1 ? 3.0 : 0.0) +
+  const int slices = (pl.units + pl.slice - 1) / pl.slice;
+  const double here = ((pl.full ? 7.0 : 4.5) + (pl.splits > 1 ? 3.0 : 0.0)) * slices +
                       u * (pl.NT == 1 ? 0.6 : 1.0) * (double)pl.units * ((pl.nvis + 63) / 64) / sms;
   const double c0 = pl.full ? 8.0 : 6.5, s = pl.full ? (a->G == 64 ? 0.80 : 1.35) : 1.30;
   const long long mb = (a->Nq + 127) / 128, items = (long long)a->B * a->H * mb;
@@ -798,25 +805,44 @@ Plan make_plan(const IntfaFwdParams* a, int sms) {
   pl.tiles = (int)((R + RT - 1) / RT);
   const long long units = (long long)a->B * Hkv * pl.tiles;
   if (units > (1 << 22)) return pl;
-  pl.units = (int)units;
+  pl.units = pl.slice = (int)units;
+  pl.groups = (pl.nvis + a->G - 1) / a->G;
   // Splits: one wave of resident CTAs, as the kernels' launch bounds have it (two CTAs an SM or four for full-int8 at 8 rows:
   // 35 -> 44 us at batch 16, 4097 keys; three for half-int8 at 128 channels: 26.5 -> 30 us at 32768 keys)
   const int wave = sms * (pl.NT == 1 && (pl.full || a->D == 64) ? 3 : 2);
   const int key_units = (pl.nvis + 63) / 64;
-  pl.groups = (pl.nvis + a->G - 1) / a->G;
+  size_t per_unit_scores = 0, per_unit_max = 0;
+  if (pl.full) {
+    if (pl.nvis > (1 << 27)) return pl;                                    // (the kernels count a unit's scores in 32 bits)
+    per_unit_scores = (size_t)pl.groups * (a->G / 8) * pl.NT * 32 * 8;
+    per_unit_max = (size_t)pl.groups * (a->G / 64) * RT * 4;
+    const size_t most = (kMaxScratch - (8u << 20)) / (per_unit_scores + per_unit_max);       // (the rest: the splits' results)
+    const int fit = most < 1 ? 1 : most > (1u << 22) ? 1 << 22 : (int)most, least = (pl.units + fit - 1) / fit;
+    // As few slices as fit, or up to three more where their CTAs fill the waves better (16 rows, 512 units of 8192 keys, one
+    // slice 301 us: 3 slices 380, 4 308, 5 328, 6 305; 8 rows, 512 units of 16384 keys, one slice 470: 448, 440, 419, 414)
+    double best = 0;
+    for (int n = least; n <= least + 3 && (n == 1 || least > 1); ++n) {
+      const int slice = (pl.units + n - 1) / n, ctas = slice < wave ? wave / slice * slice : slice;
+      const double fill = (double)ctas / ((ctas + wave - 1) / wave * wave);
+      if (fill > best * 1.02) {
+        best = fill;
+        pl.slice = slice;
+      }
+    }
+  }
   const int items = pl.full ? pl.groups : key_units;          // what a split is counted in
   const int per_min = pl.full ? 512 / a->G : 8;               // at least 512 keys per CTA: fewer are not worth the combine launch
-  int splits = wave / pl.units < 1 ? 1 : wave / pl.units;
+  int splits = wave / pl.slice < 1 ? 1 : wave / pl.slice;
   int per = (items + splits - 1) / splits;
   if (per < per_min) per = per_min;
   if (pl.full && per > kMaxLocalUnits * 64 / a->G) per = kMaxLocalUnits * 64 / a->G;
   pl.per_split = per;
   pl.splits = (items + per - 1) / per;
   const int score_ctas = sms * (a->D == 128 ? 5 : 6);                      // resident at their register counts
-  pl.score_splits = score_ctas / pl.units < 1 ? 1 : score_ctas / pl.units;
+  pl.score_splits = score_ctas / pl.slice < 1 ? 1 : score_ctas / pl.slice;
   const int score_cap = (pl.groups * (a->G / 64) + kWarps - 1) / kWarps;
   if (pl.score_splits > score_cap) pl.score_splits = score_cap;
-  if ((long long)pl.units * pl.splits > 0x7fffffffLL || (long long)pl.units * pl.score_splits > 0x7fffffffLL) return pl;
+  if ((long long)pl.slice * pl.splits > 0x7fffffffLL || (long long)pl.slice * pl.score_splits > 0x7fffffffLL) return pl;
   if (!faster_than_tiles(a, pl, sms)) return pl;
   size_t used = 0;
   auto take = [&](size_t bytes) {
@@ -825,12 +851,12 @@ Plan make_plan(const IntfaFwdParams* a, int sms) {
     return r;
   };
   if (pl.full) {
-    take((size_t)pl.units * pl.groups * (a->G / 8) * pl.NT * 32 * 8);      // scores, at 0
-    pl.off_gmax = take((size_t)pl.units * pl.groups * (a->G / 64) * RT * 4);
+    take(pl.slice * per_unit_scores);                                      // scores, at 0
+    pl.off_gmax = take(pl.slice * per_unit_max);
   }
   if (pl.splits > 1) {
-    pl.off_part = take((size_t)pl.units * pl.splits * RT * a->D * 4);
-    pl.off_ml = take((size_t)pl.units * pl.splits * RT * 8);
+    pl.off_part = take((size_t)pl.slice * pl.splits * RT * a->D * 4);
+    pl.off_ml = take((size_t)pl.slice * pl.splits * RT * 8);
   }
   pl.bytes = used;
   pl.use = true;
@@ -838,22 +864,29 @@ Plan make_plan(const IntfaFwdParams* a, int sms) {
 }
 
 template <int D, int NT>
-int run(const Plan& pl, const DParams& p, cudaStream_t stream) {
+int run_slice(const Plan& pl, int units, const DParams& p, cudaStream_t stream) {
   int rc;
-  const int grid = pl.units * pl.splits;
+  const int grid = units * pl.splits;
   if (pl.full) {
-    if ((rc = launch_kernel("decode scores", scores_kernel<D, NT>, pl.units * pl.score_splits, kThreads, 0, stream, p, pl.score_splits))) return rc;
+    if ((rc = launch_kernel("decode scores", scores_kernel<D, NT>, units * pl.score_splits, kThreads, 0, stream, p, pl.score_splits))) return rc;
     if ((rc = launch_kernel("decode P V", pv_full_kernel<D, NT>, grid, kThreads, 0, stream, p))) return rc;
   } else {
     if ((rc = launch_kernel("decode", pv_half_kernel<D, NT>, grid, kThreads, 0, stream, p))) return rc;
   }
   if (pl.splits == 1) return INTFA_OK;
-  const int rows = pl.units * 8 * NT;
+  const int rows = units * 8 * NT;
   auto combine = [&](auto few, auto many) {
     return pl.splits <= few_splits(pl.full) ? launch_kernel("decode combine", few, rows, D / 4, 0, stream, p, 8 * NT)
                                    : launch_kernel("decode combine", many, rows, combine_threads(D, pl.splits), 0, stream, p, 8 * NT);
   };
   return pl.full ? combine(combine_kernel<true, D>, combine_many_kernel<true, D>) : combine(combine_kernel<false, D>, combine_many_kernel<false, D>);
+}
+// (Slices share scratch: each kernel waits for the one before it on the stream before it writes any.)
+template <int D, int NT>
+int run(const Plan& pl, DParams p, cudaStream_t stream) {
+  for (p.unit0 = 0; p.unit0 < pl.units; p.unit0 += pl.slice)
+    if (const int rc = run_slice<D, NT>(pl, pl.units - p.unit0 < pl.slice ? pl.units - p.unit0 : pl.slice, p, stream)) return rc;
+  return INTFA_OK;
 }
 
 }  // namespace

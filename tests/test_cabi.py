@@ -111,6 +111,27 @@ def test_k_scale_rows_shorter_than_nk_are_refused(lib, Nk):
     assert "o is NULL" in lib.last_error()
 
 
+def test_scratch_has_a_bound(lib):
+    """Batches, heads and lengths of a cache that fills the GPU: 128 MiB are enough, or what one K/V head needs."""
+    h = lib.load()
+    P = lib.IntfaFwdParams()
+    P.causal, P.sm_scale, P.write_o = 1, 0.1, 1
+    seen = 0
+    for variant in (lib.VARIANT_FULL, lib.VARIANT_HALF):
+        for D, G in ((64, 64), (64, 128), (128, 64), (128, 128)):
+            for B in (1, 7, 64, 1000):
+                for Hkv, ratio in ((1, 1), (8, 4), (32, 1), (8, 8), (1, 64)):
+                    for Nq in (1, 4, 16, 256):
+                        for Nk in (300, 4097, 65536, 1000003, 5000000):
+                            P.variant, P.D, P.G, P.B, P.H, P.H_kv, P.Nq, P.Nk, P.q_offset = variant, D, G, B, Hkv * ratio, Hkv, Nq, Nk, Nk - Nq
+                            n = h.intfa_fwd_workspace_bytes(ctypes.byref(P))
+                            assert n <= max(128 << 20, 72 * (Nk + 128)), (n, variant, D, G, B, Hkv, ratio, Nq, Nk)
+                            seen += n > 64 << 20
+    assert seen > 100
+    P.variant, P.D, P.G, P.B, P.H, P.H_kv, P.Nq, P.Nk, P.q_offset = lib.VARIANT_FULL, 128, 128, 4, 64, 8, 8, 65536, 65528
+    assert 0 < h.intfa_fwd_workspace_bytes(ctypes.byref(P)) <= 128 << 20          # 0.55 GB of scores for 0.54 GB of K and V
+
+
 def test_python_surface_refuses_cpu_tensors(pkg):
     import torch
     q = torch.zeros(1, 1, 128, 64, dtype=torch.int8)

@@ -13,9 +13,9 @@ CASES = [
     ("full", 1, 2, 8, 1, 1000, 128, 64, True, "fp32"),          # exactly 8 rows
     ("full", 1, 2, 4, 4, 4097, 128, 128, True, "fp16"),         # 16 rows, many splits, odd rows of the scales
     ("full", 1, 1, 8, 5, 777, 128, 128, True, "fp32"),          # 40 rows: three row tiles
-    ("full", 1, 3, 1, 32, 65, 64, 64, True, "fp32"),            # the most rows a head
+    ("full", 1, 3, 1, 32, 65, 64, 64, True, "fp32"),            # one group and one key
     ("full", 1, 2, 1, 3, 2500, 64, 128, False, "fp16"),
-    ("full", 1, 1, 1, 2, 20000, 64, 64, True, "fp32"),          # more groups than one CTA may take
+    ("full", 1, 1, 1, 2, 20000, 64, 64, True, "fp32"),          # 40 splits of the fewest keys
     ("full", 1, 2, 1, 256, 256, 64, 64, True, "fp32"),          # short prompts: the most rows a head, causal over the whole tile
     ("full", 1, 2, 2, 131, 700, 128, 128, True, "fp16"),
     ("half", 1, 2, 1, 77, 77, 64, 128, True, "fp32"),
@@ -92,3 +92,39 @@ def test_masked_keys_weigh_nothing_at_any_softmax_scale(Nq, Nk, G, sm, pkg, orac
     out = pkg.attention_full_int8(*(t.cuda() for t in (q8, k8, v8, qs, ks, vs)), True, sm, G=G, q_offset=off)
     e = oracle.err_metrics(out.cpu(), ref)
     assert e["max_abs"] <= 4e-3 and e["mean_rel"] <= 3e-4, e
+
+
+@pytest.mark.parametrize("variant,B,Hkv,ratio,Nk,D,G", [
+    ("full", 115, 2, 1, 8700, 64, 64),        # one split but for the limit of 8192 keys a CTA: a full one and a short one
+    ("full", 115, 2, 1, 8700, 64, 128),
+    ("full", 15, 10, 1, 6000, 128, 128),      # 2 to 3 splits of many units a warp
+    ("full", 10, 10, 9, 5000, 64, 64),        # ... with 16 rows
+    ("half", 20, 5, 1, 6000, 64, 128),
+    ("half", 15, 10, 12, 4100, 128, 128),
+    ("full", 16, 8, 1, 33000, 64, 64),        # more scores than the scratch holds: two slices of the heads and more
+    ("full", 33, 5, 9, 13000, 64, 128),
+])
+def test_long_caches_of_many_heads(variant, B, Hkv, ratio, Nk, D, G, pkg, oracle):
+    dev = torch.device("cuda:0")
+    g = torch.Generator(device=dev).manual_seed(Nk)
+    H = Hkv * ratio
+    rand = lambda h, n: torch.randn(B, h, n, D, device=dev, dtype=torch.float16, generator=g)
+    (q8, qs), k, v = pkg.quant_pertoken(rand(H, 1)), rand(Hkv, Nk), rand(Hkv, Nk)
+    k[:, :, Nk // 2:] *= 2
+    k8, ks = pkg.quant_pertoken(k)
+    vs = None
+    if variant == "full":
+        v, vs = pkg.quant_perchannel(v)
+        out, lse = pkg.attention_full_int8(q8, k8, v, qs, ks, vs, True, D ** -0.5, G=G, q_offset=Nk - 1, return_lse=True)
+    else:
+        out, lse = pkg.attention_int8(q8, k8, v, qs, ks, True, D ** -0.5, G=G, q_offset=Nk - 1, return_lse=True)
+    pkg.check_status()
+    for b, hk in {(0, 0), (B // 2, Hkv - 1), (B // 2, 0), (B - 1, Hkv - 1)}:
+        one = lambda t: t[b:b + 1, hk:hk + 1].cpu()
+        of = lambda t: t[b:b + 1, hk * ratio:(hk + 1) * ratio].cpu()
+        rep = lambda t: one(t).repeat_interleave(ratio, dim=1)
+        ref, (m, l, _) = oracle.int8_attention(of(q8), rep(k8), rep(v), of(qs), rep(ks), rep(vs) if vs is not None else None, True, D ** -0.5,
+                                               variant=variant, G=G, q_offset=Nk - 1, return_state=True)
+        e = oracle.err_metrics(of(out), ref)
+        assert e["max_abs"] <= 4e-3 and e["mean_rel"] <= 3e-4, (b, hk, e)
+        assert (of(lse) - oracle.log2_lse(m, l)).abs().max() < 1e-3
