@@ -42,7 +42,10 @@ extern "C" {
 #define INTFA_VSCALE_PER_TENSOR  0   /* one V scale per (batch, head): benchmark.py:102-107 */
 #define INTFA_VSCALE_PER_CHANNEL 1   /* one V scale per (batch, head, channel)              */
 
-/* Library version (major*10000 + minor*100 + patch). */
+/* Library version (major*10000 + minor*100 + patch).  IntfaFwdParams has no size field and has grown between versions (200:
+   scale_f16, workspace, workspace_bytes): a caller whose header has another INTFA_VERSION than intfa_version() returns
+   must not call intfa_fwd(), which would read past the caller's struct. */
+#define INTFA_VERSION 200
 int intfa_version(void);
 
 /* Copies the calling thread's last error message (NUL terminated) into buf. */

@@ -8,6 +8,7 @@ import os
 _PKG_DIR = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_PKG_DIR, "libintfa.so")
 
+VERSION = 200           # INTFA_VERSION of the header that IntfaFwdParams below mirrors
 OK = 0
 ERR_INVALID_ARG, ERR_UNSUPPORTED, ERR_CUDA, ERR_DEVICE_WAIT, ERR_TOO_LARGE = -1, -2, -3, -4, -5
 VARIANT_FULL, VARIANT_HALF, VARIANT_HALF_FP8 = 0, 1, 2
@@ -72,6 +73,9 @@ def load():
     vp, i32, i64 = ctypes.c_void_p, ctypes.c_int32, ctypes.c_int64
     lib.intfa_version.restype = ctypes.c_int
     lib.intfa_version.argtypes = []
+    if lib.intfa_version() != VERSION:       # (its IntfaFwdParams may be longer than the one here)
+        raise RuntimeError("%s has version %d, this binding is for %d: build it again with `python "
+                           "int-flashattention_b200/build.py`" % (LIB_PATH, lib.intfa_version(), VERSION))
     lib.intfa_last_error.restype = ctypes.c_int
     lib.intfa_last_error.argtypes = [ctypes.c_char_p, ctypes.c_size_t]
     lib.intfa_fwd.restype = ctypes.c_int

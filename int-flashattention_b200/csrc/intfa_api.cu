@@ -55,7 +55,7 @@ static bool head_dim_ok(int D) { return D == 16 || D == 32 || D == 64 || D == 12
 
 extern "C" {
 
-int intfa_version(void) { return 100; }
+int intfa_version(void) { return INTFA_VERSION; }
 
 int intfa_last_error(char* buf, size_t len) {
   if (!buf || len == 0) return INTFA_ERR_INVALID_ARG;

@@ -58,8 +58,30 @@ def test_struct_layout_matches_header(lib, tmp_path):
 def test_version_and_error_text(lib):
     h = lib.load()
     assert h.intfa_version() >= 100
+    assert h.intfa_version() == lib.VERSION == int(re.search(r"#define INTFA_VERSION (\d+)", open(HEADER).read()).group(1))
     assert h.intfa_fwd(None, None) == lib.ERR_INVALID_ARG
     assert "NULL" in lib.last_error()
+
+
+# what the struct ends with in each version: no version has two layouts
+LAST_FIELD = {200: ("workspace_bytes", 400)}
+
+
+def test_every_struct_layout_has_its_own_version(lib):
+    last = lib.IntfaFwdParams._fields_[-1][0]
+    assert (last, ctypes.sizeof(lib.IntfaFwdParams)) == LAST_FIELD[lib.VERSION]
+
+
+def test_a_library_of_another_version_is_refused(lib, monkeypatch):
+    class Other:
+        def __getattr__(self, name):
+            f = lambda *a: lib.VERSION - 100
+            setattr(self, name, f)
+            return f
+    monkeypatch.setattr(lib, "_lib", None)
+    monkeypatch.setattr(lib.ctypes, "CDLL", lambda path: Other())
+    with pytest.raises(RuntimeError, match="version"):
+        lib.load()
 
 
 def test_validation_rejects_before_launch(lib):
