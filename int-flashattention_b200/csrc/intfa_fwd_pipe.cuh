@@ -67,8 +67,7 @@ struct PipeCfg {
   static constexpr bool BIG = DQ > 128 && (G == 128 || D == 256);   // 32 KB K tiles, or 32 KB V tiles: three stages are what fits
   static constexpr int NSK = BIG ? 3 : 4;                          // K stages
   static constexpr int NSV = BIG ? 3 : 4;                          // V stages
-  static constexpr int NKS = 8;                                    // K-scale slots: a slot is rewritten 8 steps later, when
-                                                                   // the three S buffers have long forced its step out
+  static constexpr int NKS = 8;                                    // K-scale slots (see the warp that fills them)
   // S buffers in TMEM.  Four where a step's buffer waits for its P V and there is room (d=64: 385 -> 371 us, d=128 at G=64 421 ->
   // 414; no gain at d=256).
   static constexpr int NSB = P_TMEM && G == 64 && D <= 128 ? 4 : 3;
@@ -188,8 +187,10 @@ intfa_fwd_pipe_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
   constexpr int B_KFULL = 20, B_KEMPTY = 20 + NSK, B_VFULL = 20 + 2 * NSK, B_VEMPTY = 20 + 2 * NSK + NSV;
   constexpr int B_TILE = 20 + 2 * NSK + 2 * NSV, B_TDONE = B_TILE + 4;
   constexpr int B_AFULL = B_TDONE + 4;   // [4] half-int8: alpha of step j (slot j mod 4) published, for the accumulator warps
-  constexpr int B_SFULL = B_AFULL + 4;   // [3] commit: S = Q K^T in TMEM buffer b
-  constexpr int B_SFREE = B_SFULL + NSB; // [3] softmax group of the step (4 warps): S buffer b read out for good
+  constexpr int B_SFULL = B_AFULL + 4;   // [NSB] commit: S = Q K^T in TMEM buffer b; scale loader: the step's K scales in
+                                         //     shared memory (the arrival of the warp that wrote them is what lets the
+                                         //     softmax warps see them)
+  constexpr int B_SFREE = B_SFULL + NSB; // [NSB] softmax group of the step (4 warps): S buffer b read out for good
                                          //     (P_TMEM: commit: the P V that read P from it is done)
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + C::OFF_MISC);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + C::OFF_MISC + 4);
@@ -213,7 +214,7 @@ intfa_fwd_pipe_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
       mbar_init(BAR(B_OFREE + b), 4);
     }
     for (int s = 0; s < NSK; ++s) {
-      mbar_init(BAR(B_KFULL + s), 2);         // the producer's K tile and the scale loader's K scales
+      mbar_init(BAR(B_KFULL + s), 1);
       mbar_init(BAR(B_KEMPTY + s), 1);
     }
     for (int s = 0; s < NSV; ++s) {
@@ -221,7 +222,7 @@ intfa_fwd_pipe_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
       mbar_init(BAR(B_VEMPTY + s), 1);
     }
     for (int b = 0; b < NSB; ++b) {
-      mbar_init(BAR(B_SFULL + b), 1);
+      mbar_init(BAR(B_SFULL + b), 2);         // Q K^T done; the K scales of the step are written
       mbar_init(BAR(B_SFREE + b), C::P_TMEM ? 1 : 4);
     }
     for (int i = 0; i < 4; ++i) {
@@ -356,9 +357,12 @@ intfa_fwd_pipe_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
     __syncwarp();
   } else if (warp == 2) {
     // -------------------------------------------------------------------- K scales
-    // The scales of KV step it go into slot it mod NKS together with the K tile (same K_EMPTY wait, second arrival on
-    // K_FULL).  Plain loads, one step ahead of the wait: rows may start anywhere (a cache of odd length) and hold fp16 or
-    // fp32; columns past Nk read as zero.
+    // The scales of KV step it go into slot it mod NKS, and the softmax warps see them through S_FULL of the step, which they
+    // wait for anyway.  This warp waits for S_FULL of the step NSB back first: so that its arrival counts for its own step, and
+    // because the softmax groups are done with the step another NSB back by then, whose slot this is at the latest.
+    // Plain loads, one step ahead of the wait: rows may start anywhere (a cache of odd length) and hold fp16 or fp32; columns
+    // past Nk read as zero.
+    static_assert(C::NKS >= 2 * NSB, "K-scale slots");
     uint32_t kv_it = 0, tseq = 0;
     bool ok = true;
 #pragma unroll 1
@@ -371,14 +375,14 @@ intfa_fwd_pipe_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
 #pragma unroll 1
       for (int j = -1; j < t.nsteps; ++j) {
         if (j >= 0) {
-          const uint32_t s = kv_it % NSK, ph = (kv_it / NSK) & 1;
-          ok = mbar_wait_warp<POLITE>(BAR(B_KEMPTY + s), ph ^ 1, abort_flag, p.status, code_hi | PW_KE);
+          const uint32_t s = kv_it % NSB, ph = (kv_it / NSB) & 1;
+          ok = mbar_wait_warp<POLITE>(BAR(B_SFULL + s), ph ^ 1, abort_flag, p.status, code_hi | PW_SFULL);
           if (!ok) break;
           float* slot = reinterpret_cast<float*>(smem + C::OFF_KS + (kv_it % C::NKS) * C::KS_BYTES) + lane;
 #pragma unroll
           for (int i = 0; i < G / 32; ++i) slot[32 * i] = ks[i];
           __syncwarp();
-          if (lane == 0) mbar_arrive(BAR(B_KFULL + s));
+          if (lane == 0) mbar_arrive(BAR(B_SFULL + s));
           ++kv_it;
         }
         if (j + 1 < t.nsteps) {
