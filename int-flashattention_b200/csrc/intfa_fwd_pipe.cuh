@@ -82,17 +82,18 @@ struct PipeCfg {
   // setmaxnreg split between the softmax and the accumulator warps.  The accumulator row of 128 channels fits either
   // way; with 128-column KV steps, and for half-int8 (no accumulator row in registers), the softmax passes gain more
   // from 16 further registers than the update loses (measured +2..3 %); full-int8 at G = 64 is the other way round.
-  // A vectorised pass A for the causal diagonal band (otherwise those steps take the general, scalar path): compiled in
-  // for 128-column KV steps, where it measured +2..5 % on causal workloads; with 64-column steps its code costs the
-  // non-causal case more (instruction cache) than it gives.
-  static constexpr bool BAND_FAST = G == 128 || D == 256;
+  // A vectorised pass A for the causal diagonal band and the last, partial step (otherwise those take the general, scalar
+  // path): compiled in for 128-column KV steps, where it measured +2..5 % on causal workloads, and for 32-column steps of
+  // ragged lengths (batch 8, 32 heads, 1000 tokens causal at d=32: 273 -> 212 us, 64 x 32 x 250: 327 -> 224).  Elsewhere its
+  // code costs the steps that need no mask more (instruction cache) than it gives (2 x 16 x 4096 at d=32: 573 -> 631).
+  __host__ __device__ static constexpr bool band_fast(bool ragged) { return G == 128 || D == 256 || (G == 32 && ragged); }
   // instructions of never-executed filler between the softmax passes (see intfa_fwd_pipe_softmax.inc), the best of a sweep in
   // steps of 1 KB for each kind of instantiation (`ragged`: masks partial tiles; `polite`: see the kernel).  Between the best
   // and the worst of a sweep lie 1 to 2 % non-causal, 5 to 15 % causal.
   __host__ __device__ static constexpr int code_filler_of(bool ragged, bool polite) {
     if (P_TMEM) return G == 128 ? (ragged ? 0 : 192) : D == 256 ? (ragged ? 384 : 0) : D == 128 ? (ragged ? 256 : 128) : ragged ? 128 : 256;
     return NGRP == 3 ? (!FULL ? 192 : (ragged && G == 128) ? 64 : polite ? 128 : 256)
-         : ragged ? 256 : G == 128 ? (FULL ? 448 : 384) : (D == 256 || (FULL && D == 64)) ? 0 : D == 32 ? 256 : 128;
+         : ragged ? (G == 32 ? 128 : FULL && G == 128 && D <= 64 ? 384 : 256) : G == 128 ? (!FULL ? 320 : DQ == 256 ? 448 : 64) : D == 32 ? 256 : 320;
   }
   static constexpr bool MORE_SOFTMAX_REGS = !FULL || G == 128;
   static constexpr int SOFTMAX_REGS = NGRP == 3 ? (FULL ? 96 : 112) : MORE_SOFTMAX_REGS ? 152 : 136;
