@@ -468,7 +468,7 @@ __global__ void __launch_bounds__(kThreads, NT == 1 ? 3 : 2) pv_full_kernel(cons
 // half-int8: scores, softmax and P V in one pass; one warp takes 32 keys at a time, with a running maximum of its own
 // ---------------------------------------------------------------------------------------------------------------
 template <int D, int NT>
-__global__ void __launch_bounds__(kThreads, D == 64 && NT == 1 ? 3 : 2) pv_half_kernel(const DParams p) {
+__global__ void __launch_bounds__(kThreads, D == 64 ? 3 : 2) pv_half_kernel(const DParams p) {
   constexpr int RT = 8 * NT, CH = D / 64, MT = D / 16;
   __shared__ __align__(16) float red[kWarps * RT * (D + 4)];
   __shared__ float wml[kWarps][RT][2];
