@@ -129,7 +129,7 @@ typedef struct IntfaFwdParams {
  */
 int intfa_fwd(const IntfaFwdParams* p, void* stream);
 
-/* Scratch that intfa_fwd() makes use of for these arguments (pointers are not looked at); 0: none.  At most 128 MiB, or
+/* Scratch that intfa_fwd() makes use of for these arguments (pointers are not looked at); 0: none.  At most 256 MiB, or
    72 bytes a key where a single K/V head has so many that it needs more. */
 size_t intfa_fwd_workspace_bytes(const IntfaFwdParams* p);
 

@@ -764,8 +764,9 @@ struct Plan {
 //   128 rows   `c0` (pipeline fill), then `s` per KV step of G keys: the longest work item, or what an SM gets of all steps.
 // The margin of 10 % keeps the 128-row kernel where the two are alike.
 // Scratch of one call, unless one unit needs more.  The scores of full-int8 are fp32 and padded to 8 or 16 rows, up to as much
-// again as K and V, so a call that needs more takes its units in slices that share it, one after the other.
-constexpr size_t kMaxScratch = (size_t)128 << 20;
+// again as K and V, so a call that needs more takes its units in slices that share it, one after the other.  (Half of this
+// bound cuts up calls of few units, which then leave SMs idle: 128 units of 16384 keys 91 -> 104 to 110 us.)
+constexpr size_t kMaxScratch = (size_t)256 << 20;
 
 bool faster_than_tiles(const IntfaFwdParams* a, const Plan& pl, int sms) {
   const bool d128 = a->D == 128;

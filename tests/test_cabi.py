@@ -134,7 +134,7 @@ def test_k_scale_rows_shorter_than_nk_are_refused(lib, Nk):
 
 
 def test_scratch_has_a_bound(lib):
-    """Batches, heads and lengths of a cache that fills the GPU: 128 MiB are enough, or what one K/V head needs."""
+    """Batches, heads and lengths of a cache that fills the GPU: 256 MiB are enough, or what one K/V head needs."""
     h = lib.load()
     P = lib.IntfaFwdParams()
     P.causal, P.sm_scale, P.write_o = 1, 0.1, 1
@@ -147,11 +147,11 @@ def test_scratch_has_a_bound(lib):
                         for Nk in (300, 4097, 65536, 1000003, 5000000):
                             P.variant, P.D, P.G, P.B, P.H, P.H_kv, P.Nq, P.Nk, P.q_offset = variant, D, G, B, Hkv * ratio, Hkv, Nq, Nk, Nk - Nq
                             n = h.intfa_fwd_workspace_bytes(ctypes.byref(P))
-                            assert n <= max(128 << 20, 72 * (Nk + 128)), (n, variant, D, G, B, Hkv, ratio, Nq, Nk)
+                            assert n <= max(256 << 20, 72 * (Nk + 128)), (n, variant, D, G, B, Hkv, ratio, Nq, Nk)
                             seen += n > 64 << 20
     assert seen > 100
     P.variant, P.D, P.G, P.B, P.H, P.H_kv, P.Nq, P.Nk, P.q_offset = lib.VARIANT_FULL, 128, 128, 4, 64, 8, 8, 65536, 65528
-    assert 0 < h.intfa_fwd_workspace_bytes(ctypes.byref(P)) <= 128 << 20          # 0.55 GB of scores for 0.54 GB of K and V
+    assert 0 < h.intfa_fwd_workspace_bytes(ctypes.byref(P)) <= 256 << 20          # 0.55 GB of scores for 0.54 GB of K and V
 
 
 def test_python_surface_refuses_cpu_tensors(pkg):

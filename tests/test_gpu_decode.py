@@ -101,8 +101,8 @@ def test_masked_keys_weigh_nothing_at_any_softmax_scale(Nq, Nk, G, sm, pkg, orac
     ("full", 10, 10, 9, 5000, 64, 64),        # ... with 16 rows
     ("half", 20, 5, 1, 6000, 64, 128),
     ("half", 15, 10, 12, 4100, 128, 128),
-    ("full", 16, 8, 1, 33000, 64, 64),        # more scores than the scratch holds: two slices of the heads and more
-    ("full", 33, 5, 9, 13000, 64, 128),
+    ("full", 32, 8, 1, 33000, 64, 64),        # more scores than the scratch holds: two slices of the heads and more
+    ("full", 66, 5, 9, 13000, 64, 128),
 ])
 def test_long_caches_of_many_heads(variant, B, Hkv, ratio, Nk, D, G, pkg, oracle):
     dev = torch.device("cuda:0")
