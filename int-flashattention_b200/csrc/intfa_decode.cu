@@ -15,8 +15,8 @@
 // full-int8: P is rounded to int8 against the RUNNING maximum of the row (keys taken G at a time, ascending), so the
 // maxima must be known before P: `scores_kernel` computes s = (fp32(S32)*s_q)*s_k, keeps it (fp32, in the order in which
 // the next kernel's lanes want it) and the maximum of each 64 keys; `pv_full_kernel` takes the prefix maximum at its
-// first group, and from there on does exactly what the one-pass kernel does: m' = max(m, groupmax*c), p = exp2(s*c - m'),
-// P8, O_j.  The final maximum is known too, so that every partial result is scaled to it at once
+// first group, and from there on does what the one-pass kernel does: m' = max(m, groupmax*c), p = exp2(s*c - m'), P8, O_j
+// (with s*c - m' as one fma on masked groups too, where that kernel rounds s*c first).  The final maximum is known too, so that every partial result is scaled to it at once
 // (acc += exp2(m_j - m_final) * O_j) and the splits add up without weights.
 // half-int8: P is fp16, whose rounding is relative: every warp keeps a running maximum of its own and the partial results
 // are combined with their weights (`pv_half_kernel`: scores and P V in one pass over K and V).
@@ -758,29 +758,44 @@ struct Plan {
   size_t off_gmax = 0, off_part = 0, off_ml = 0, bytes = 0;
 };
 
-// Which path?  Times in microseconds, fitted to measurements of both paths at 1 to 2048 rows and 77 to 16384 keys (B200):
-//   here       launches, then `u` per 64 keys of a 16-row tile and SM.  Per row and key that is 2 to 3.5 times what the other
-//              path costs with all its rows alive, but rows are padded to 8 or 16 instead of 128 and keys are split.
-//   128 rows   `c0` (pipeline fill), then `s` per KV step of G keys: the longest work item, or what an SM gets of all steps.
-// The margin of 10 % keeps the 128-row kernel where the two are alike.
 // Scratch of one call, unless one unit needs more.  The scores of full-int8 are fp32 and padded to 8 or 16 rows, up to as much
 // again as K and V, so a call that needs more takes its units in slices that share it, one after the other.  (Half of this
 // bound cuts up calls of few units, which then leave SMs idle: 128 units of 16384 keys 91 -> 104 to 110 us.)
 constexpr size_t kMaxScratch = (size_t)256 << 20;
 
-bool faster_than_tiles(const IntfaFwdParams* a, const Plan& pl, int sms) {
-  const bool d128 = a->D == 128;
-  const double u = pl.full ? (d128 ? 0.59 : 0.45) : (d128 ? 0.50 : 0.27);
+// Which path?  Times in microseconds, fitted to 3 781 calls that were timed on both (1 to 256 rows a head, 50 to 16384 keys, 1 to
+// 512 heads in all; B200):
+//   here       `fixed` and `combine` for the launches; `unit` per 64 keys of a row tile and SM (times `one_half` for tiles of 8
+//              rows); `wave` for each further wave of CTAs
+//   128 rows   `fill`, then `step` per KV step of G keys and `next` for each further work item of an SM.  The work items of
+//              these calls are of one length, so an SM has a whole number of them.
+// Typical error 5 to 15 %.  Over those calls the choice costs 0.3 % against the better path each time, and 48 of them more
+// than 10 %.  (One step time for any G and head dim, and no term for waves, before: 0.5 %, 72 of 1 610 calls more than 10 %, up
+// to twice the time for half-int8 with 64-column steps.)
+struct FewTimes {
+  double fixed, combine, unit, one_half, wave;
+};
+struct TileTimes {
+  double fill, step, next;
+};
+constexpr FewTimes kFew[2][2] = {{{5.41, 3.22, 0.267, 1.04, 1.40}, {6.14, 3.35, 0.490, 1.02, 3.27}},        // half-int8: d = 64, 128
+                                 {{7.52, 1.93, 0.386, 0.73, 3.01}, {8.70, 1.80, 0.540, 0.81, 4.46}}};       // full-int8
+constexpr TileTimes kTiles[2][2][2] = {{{{8.99, 0.694, 6.59}, {6.92, 1.179, 2.21}},                         // half-int8, d = 64: G = 64, 128
+                                        {{9.23, 0.765, 6.47}, {7.49, 1.235, 2.46}}},
+                                       {{{8.71, 0.838, 4.72}, {7.01, 1.432, 2.71}}, {{10.43, 0.962, 7.97}, {8.72, 1.359, 3.80}}}};
+bool faster_than_tiles(const IntfaFwdParams* a, const Plan& pl, int wave, int sms) {
+  const FewTimes& f = kFew[pl.full][a->D == 128];
+  const TileTimes& t = kTiles[pl.full][a->D == 128][a->G == 128];
   const int slices = (pl.units + pl.slice - 1) / pl.slice;
-  const double here = ((pl.full ? 7.0 : 4.5) + (pl.splits > 1 ? 3.0 : 0.0)) * slices +
-                      u * (pl.NT == 1 ? 0.6 : 1.0) * (double)pl.units * ((pl.nvis + 63) / 64) / sms;
-  const double c0 = pl.full ? 8.0 : 6.5, s = pl.full ? (a->G == 64 ? 0.80 : 1.35) : 1.30;
-  const long long mb = (a->Nq + 127) / 128, items = (long long)a->B * a->H * mb;
+  const double waves = (double)pl.slice * pl.splits / wave;
+  const double here = (f.fixed + (pl.splits > 1 ? f.combine : 0.0) + (waves > 1 ? f.wave * (waves - 1) : 0.0)) * slices +
+                      f.unit * (pl.NT == 1 ? f.one_half : 1.0) * (double)pl.units * ((pl.nvis + 63) / 64) / sms;
+  const long long items = (long long)a->B * a->H * ((a->Nq + 127) / 128);
+  const double rounds = (double)((items + sms - 1) / sms);
   const double steps = (double)((pl.nvis + a->G - 1) / a->G);
-  const double mean = a->causal ? steps - 0.5 * a->Nq / a->G : steps;      // steps of an average work item
-  const double per_sm = items * (mean < 1 ? 1 : mean) / sms + 0.4 * steps;
-  const double tiles = c0 + s * (items <= sms || per_sm < steps ? steps : per_sm);
-  return here < 0.9 * tiles;
+  double mean = a->causal ? steps - 0.5 * a->Nq / a->G : steps;             // steps of an average work item
+  if (mean < 1) mean = 1;
+  return here < t.fill + t.step * (rounds > 1 ? rounds * mean : steps) + t.next * (rounds - 1);
 }
 
 Plan make_plan(const IntfaFwdParams* a, int sms) {
@@ -844,7 +859,7 @@ Plan make_plan(const IntfaFwdParams* a, int sms) {
   const int score_cap = (pl.groups * (a->G / 64) + kWarps - 1) / kWarps;
   if (pl.score_splits > score_cap) pl.score_splits = score_cap;
   if ((long long)pl.slice * pl.splits > 0x7fffffffLL || (long long)pl.slice * pl.score_splits > 0x7fffffffLL) return pl;
-  if (!faster_than_tiles(a, pl, sms)) return pl;
+  if (!faster_than_tiles(a, pl, wave, sms)) return pl;
   size_t used = 0;
   auto take = [&](size_t bytes) {
     const size_t r = used;

@@ -133,6 +133,21 @@ def test_k_scale_rows_shorter_than_nk_are_refused(lib, Nk):
     assert "o is NULL" in lib.last_error()
 
 
+@pytest.mark.parametrize("D,G,B,H,Hkv,Nq,Nk,few", [
+    (128, 64, 64, 8, 1, 24, 200, True),           # 26 us on the few-rows path, 51 on 128-row tiles
+    (64, 64, 2, 16, 16, 129, 500, True),          # 12 us, 16
+    (64, 128, 16, 32, 8, 1, 4097, True),          # decode
+    (128, 128, 4, 32, 8, 256, 1024, False),       # 147 us against 35
+    (128, 128, 2, 16, 16, 160, 6000, False),      # 153 against 73
+])
+def test_full_int8_takes_the_faster_path(lib, D, G, B, H, Hkv, Nq, Nk, few):
+    """(Scratch tells which: the few-rows path of full-int8 always needs some, 128-row tiles never.)"""
+    P = lib.IntfaFwdParams()
+    P.causal, P.sm_scale, P.write_o, P.variant = 1, 0.1, 1, lib.VARIANT_FULL
+    P.D, P.G, P.B, P.H, P.H_kv, P.Nq, P.Nk, P.q_offset = D, G, B, H, Hkv, Nq, Nk, Nk - Nq
+    assert (lib.load().intfa_fwd_workspace_bytes(ctypes.byref(P)) > 0) == few
+
+
 def test_scratch_has_a_bound(lib):
     """Batches, heads and lengths of a cache that fills the GPU: 256 MiB are enough, or what one K/V head needs."""
     h = lib.load()
