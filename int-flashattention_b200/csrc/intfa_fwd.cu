@@ -258,7 +258,7 @@ int fwd_dispatch(const IntfaFwdParams* a, cudaStream_t stream) {
   INTFA_CASE(128, 128, 64, 128, true)
   INTFA_CASE(64, 64, 64, 64, true)
   INTFA_CASE(64, 64, 128, 64, true)
-  INTFA_CASE(32, 32, 32, 32, false)      // G = 32: full-int8 only (fp16 P tiles need 64 columns)
+  INTFA_CASE(32, 32, 32, 32, false)      // G = 32: full-int8 only (half-int8 is built for 64 columns and more)
   INTFA_CASE(32, 32, 64, 32, true)
   INTFA_CASE(32, 32, 128, 32, true)
   INTFA_CASE(16, 32, 32, 32, false)      // head dim 16: the 32-wide kernel on zero-filled tiles

@@ -4,13 +4,13 @@
 // 512 threads with two softmax groups, 640 with three (PipeCfg::NGRP):
 //   warp 0        TMA producer (Q once per work item; K and V through rings of shared-memory stages); it also draws
 //                 the work items: the CTA's own index first, then from a global counter
-//   warp 1        MMA issuer for S = Q K^T (whole warp runs the loop, one elected lane issues): up to three KV steps
-//                 ahead of the softmax groups, into S buffer (step mod 3)
+//   warp 1        MMA issuer for S = Q K^T (whole warp runs the loop, one elected lane issues): up to NSB (three or four) KV
+//                 steps ahead of the softmax groups, into S buffer (step mod NSB)
 //   warp 2        TMEM allocator; then loads the K scales (fp32 or fp16, rows of any alignment) into a ring of their own
 //   warp 3        MMA issuer for O_j = P V
 //   warps 4-7, 8-11 (, 12-15)   softmax groups 0, 1 (, 2): one thread per query row.  The groups take the KV steps in
 //                 TURN (group g owns the steps whose running index is g mod NGRP), each with its own P buffer in shared
-//                 memory, so that on every scheduler one warp is in pass A (dequantise, row max: FMA pipe) while
+//                 memory (or with P over its scores in TMEM: PipeCfg::P_TMEM), so that on every scheduler one warp is in pass A (dequantise, row max: FMA pipe) while
 //                 another is in pass B (exp2, P: exp2 unit).  The running max m of a row travels between the threads
 //                 that own it through shared memory, once per step.
 //   the last 4 warps   accumulator update and epilogue, one thread per query row:
@@ -18,7 +18,7 @@
 //                 half-int8: P V (fp16 MMA) accumulates straight into an fp32 accumulator in TMEM, these warps
 //                 multiply the row by alpha beforehand when some alpha of the warp's 32 rows is not 1.
 //                 They also carry the row sum l = l*alpha + rowsum(P) (see PipeCfg::L_IN_ACC).
-// TMEM columns: S0 [0,G) | S1 [G,2G) | S2 [2G,3G) | O_j, or the half-int8 accumulator [3G, 3G+D)  (<= 512).
+// TMEM columns: NSB S buffers of G | NO O_j buffers of D, or the half-int8 accumulator of D  (<= 512).
 // S and O_j are int32 accumulators that start each KV step from the bit pattern of 1.5*2^23, written by a
 // small fp16 MMA ahead of the int8 MMAs, so that the threads read fp32(S32) + 1.5*2^23 without a conversion.
 // The arithmetic contract is at the top of intfa_fwd.cu.
@@ -106,9 +106,9 @@ struct PipeCfg {
   static constexpr int OFF_P = OFF_V + NSV * V_BYTES;             // a P buffer per softmax group
   static constexpr int OFF_KS = OFF_P + NGRP * P_BYTES;
   static constexpr int OFF_VSD = OFF_KS + NKS * KS_BYTES;         // s_v/127 per channel
-  static constexpr int OFF_HM = OFF_VSD + D * 4;                  // [2 groups][128] float: running max after the group's latest step
-  static constexpr int OFF_RS = OFF_HM + NGRP * 128 * 4;             // [4][128] float: row sum of P of step j, for the accumulator warps
-                                                                   //   (!L_IN_ACC: [2 groups][128] float, l after the group's latest step)
+  static constexpr int OFF_HM = OFF_VSD + D * 4;                  // [NGRP][128] float: running max after the group's latest step
+  static constexpr int OFF_RS = OFF_HM + NGRP * 128 * 4;             // [NRS][128] float: row sum of P of step j, for the accumulator warps
+                                                                   //   (!L_IN_ACC: [NGRP][128] float, l after the group's latest step)
   static constexpr int OFF_ALPHA = OFF_RS + NRS * 128 * 4;          // [4][128] float: alpha of step j, for the accumulator warps
   static constexpr int OFF_FIN = OFF_ALPHA + 4 * 128 * 4;         // [2][128] float2: final running max of a work item (.x)
   static constexpr int OFF_MAGIC = OFF_FIN + 2 * 128 * 8;          // 4 KB constant fp16 operand of the "arm" MMA
@@ -152,9 +152,10 @@ enum PipeWait { PW_TILE = 32, PW_QE, PW_KE, PW_VE, PW_QF, PW_KF, PW_VF, PW_SFREE
 
 // RAGGED: Nq / Nk are not multiples of 128 / G -- the last query tile and the last KV step are partial.  A separate
 // instantiation, so that the code of the common case stays as small as it was (instruction cache).
-// POLITE: the service warps (0 to 3) sleep 20 ns between two looks at a barrier.  The dispatch ports are 88 % busy in steady
-// state (three groups, full-int8), so their polls cost: 341 -> 330 us non-causal.  Causal work items are short and wait for
-// the issue warps instead: 238 -> 245 us, so they keep polling.
+// POLITE: the service warps (0 to 3) sleep 20 ns between two looks at a barrier, and the softmax groups take the running max
+// before pass A (HM_LATE).  With three groups of full-int8 and every step of a work item alike, 341 -> 330 us; causal work
+// items, whose steps are fewer and partly masked, lose by it (238 -> 245 us) and keep polling.  Chosen by causality and not by
+// the length of a work item, which has not been measured for itself.
 template <int D, int G, bool FULL, bool PRNE, bool RAGGED, int DQ = D, bool F8V = false, bool POLITE = false>
 __global__ void __launch_bounds__((PipeCfg<D, G, FULL, DQ, F8V>::THREADS), 1)
 intfa_fwd_pipe_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
@@ -281,7 +282,7 @@ intfa_fwd_pipe_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
     return t;
   };
 
-  // registers: 512 x 128 at launch; the service warps and the accumulator warps give theirs to the softmax warps
+  // registers (THREADS x LAUNCH_REGS at launch): the service warps give most of theirs to the others
   if (warp < 4) reg_dealloc<kPipeServiceRegs>();
 
   if (warp == 0) {
@@ -400,8 +401,7 @@ intfa_fwd_pipe_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
       // ------------------------------------------------------------------ MMA issuer for S = Q K^T
       // The whole warp runs the loop and the waits (warp-uniform control flow keeps the descriptor arithmetic
       // off the per-thread path); one elected lane issues the tensor-core instructions.
-      // Step it goes into S buffer it mod 3 as soon as the step three back has been read out of it and K has landed --
-      // up to three steps ahead of the softmax groups.  The K stage is handed back by the tensor core itself (the
+      // Step it goes into S buffer it mod NSB as soon as the step NSB back has been read out of it and K has landed.  The K stage is handed back by the tensor core itself (the
       // K scales sit in a ring of their own).
       uint32_t kv_it = 0, tile_it = 0, tseq = 0, sfree_seen = 0;
       bool ok = true;

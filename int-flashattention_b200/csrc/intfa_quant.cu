@@ -14,7 +14,8 @@
 // maxima are reduced with warp shuffles.  Per-token: one pass.  V (per-channel or
 // per-(batch,head)): a column-absmax pass, then the quantising pass.  The fused entry (quant_qkv) runs the Q rows,
 // the K rows and the V column-absmax pass as ONE launch (partial maxima per chunk, plain stores) and the V
-// quantising pass as a second; the stand-alone V entries use atomicMax into a small scratch array instead.
+// quantising pass as a second.  The stand-alone V entries: partial maxima as well (intfa_quant_v_partial, which the Python
+// operators call), or atomicMax into a small array (intfa_quant_v, intfa_v_colmax, intfa_quant_v_static).
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
