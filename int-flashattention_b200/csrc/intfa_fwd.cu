@@ -58,8 +58,11 @@ __device__ __forceinline__ float ld_scale(const void* s, long long i, int f16) {
   return f16 ? __half2float(static_cast<const __half*>(s)[i]) : static_cast<const float*>(s)[i];
 }
 
-struct TileInfo {
-  int bh, b, h, hk, mb, work, nsteps;   // hk: the K/V head this query head reads (grouped-query attention)
+// A work item, as the producer warp publishes it in shared memory (the divisions are made once, not by every warp role: they are
+// most of what lies between two work items, and code that the instruction cache does not have to hold six times).
+struct __align__(16) TileInfo {
+  int bh, b, h, hk, mb, work;           // hk: the K/V head this query head reads (grouped-query attention)
+  int nsteps;                           // KV steps (below zero: no more work items)
   int vh;                               // which D-wide slice of the V / output channels this pass covers (head dim 256: 0, 1)
 };
 
@@ -224,7 +227,7 @@ int fwd_dispatch(const IntfaFwdParams* a, cudaStream_t stream) {
   kp.state_in = a->state_in; kp.state_out = a->state_out; kp.write_o = a->write_o;
   kp.dbg_s = a->dbg_s; kp.dbg_p = a->dbg_p; kp.dbg_tile = a->dbg_tile; kp.dbg_step = a->dbg_step;
   kp.status = a->status;
-  kp.wait_limit_kcycles = a->debug_wait_limit_kcycles > 0 ? a->debug_wait_limit_kcycles : (1 << 21);   // default: 2^31 cycles, about a second
+  kp.wait_limit_kcycles = a->debug_wait_limit_kcycles > 0 && a->debug_wait_limit_kcycles < (1 << 21) ? a->debug_wait_limit_kcycles : (1 << 21);   // at most 2^31 cycles, about a second
   kp.skip_k_load = a->debug_skip_k_load;
   kp.kv_desc = a->kv_order ? 1 : 0;
   kp.vs_sblk = a->vs_stride_blk;

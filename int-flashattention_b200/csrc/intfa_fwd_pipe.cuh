@@ -74,6 +74,7 @@ struct PipeCfg {
   static constexpr int NRS = NSB == 4 ? 8 : 4;                     // row-sum slots: step j's is read at step j+1, when P V j+1 may be out
   static constexpr int P_PER_COL = BYTE_PV ? 4 : 2;                // P_TMEM: elements of P in a TMEM column
   static constexpr int NPB = P_TMEM ? NSB : NGRP;                  // P buffers
+  static constexpr int NPBAR = P_TMEM ? 0 : NGRP;                  // ... and their barriers, where they are in shared memory
   // Who carries the row sum l = l*alpha + rowsum(P)?  Where a KV step is as wide as the head (G >= D) the accumulator
   // warps do, next to the accumulator row: the softmax groups then meet once per step (running max) instead of
   // twice.  Where the head is wider than the step (head_dim 128 at G = 64) the accumulator warps are the busier
@@ -113,8 +114,9 @@ struct PipeCfg {
   static constexpr int OFF_FIN = OFF_ALPHA + 4 * 128 * 4;         // [2][128] float2: final running max of a work item (.x)
   static constexpr int OFF_MAGIC = OFF_FIN + 2 * 128 * 8;          // 4 KB constant fp16 operand of the "arm" MMA
   static constexpr int MAGIC_BYTES = 4096;
-  static constexpr int OFF_BAR = OFF_MAGIC + MAGIC_BYTES;
-  static constexpr int NUM_BARS = 23 + 2 * NSK + 2 * NSV + 8 + 4 + 2 * NSB;
+  static constexpr int OFF_TILE = OFF_MAGIC + MAGIC_BYTES;         // [4] TileInfo: the work-item ring
+  static constexpr int OFF_BAR = OFF_TILE + 4 * (int)sizeof(TileInfo);
+  static constexpr int NUM_BARS = 14 + NPBAR + 2 * NSK + 2 * NSV + 12 + NSB;
   static constexpr int OFF_MISC = OFF_BAR + NUM_BARS * 8;
   static constexpr int SMEM_BYTES = OFF_MISC + 32 + 1024;
   // S buffer b at COL_S + b*G; then O_j (full-int8: the accumulator itself lives in registers) or the fp32
@@ -124,6 +126,10 @@ struct PipeCfg {
   // the accumulator warps.  (Not with three groups: alpha and the row sums of a step would be overwritten too early.)
   static constexpr int NO = FULL && NGRP == 2 && NSB * G + 2 * D <= 512 ? 2 : 1;
   static_assert(NSB * G + NO * D <= 512, "TMEM columns");
+  // The barrier on which an MMA warp waits for a step is a K or V stage's (see the kernel).  No arrival for step j may come before
+  // the wait for the step that had the barrier before it: what arrives follows from that step's S, P or O_j buffer being free
+  // again, so there must not be more of these than stages.
+  static_assert(NSB <= NSK && NPB <= NSV && NO <= NSV, "ready barriers");
   static constexpr int TMEM_COLS = 512;
   static_assert(FULL || G >= 64, "half-int8");
   static constexpr uint64_t SWZ_QK = (QK_ROWB == 128) ? kSwz128 : (QK_ROWB == 64) ? kSwz64 : kSwz32;
@@ -147,7 +153,7 @@ struct PipeCfg {
   static constexpr uint32_t IDESC_ARM_O = make_idesc(1, 0, 0, 0, 0, kBM, D);
 };
 
-enum PipeWait { PW_TILE = 32, PW_QE, PW_KE, PW_VE, PW_QF, PW_KF, PW_VF, PW_SFREE, PW_PFULL, PW_OFREE, PW_SFULL,
+enum PipeWait { PW_TILE = 32, PW_QE, PW_KE, PW_VE, PW_QF, PW_QKRDY, PW_PVRDY, PW_SFULL,
                 PW_PFREE, PW_HM, PW_OFULL, PW_FIN, PW_FINFREE, PW_HL, PW_AFULL };
 
 // RAGGED: Nq / Nk are not multiples of 128 / G -- the last query tile and the last KV step are partial.  A separate
@@ -174,36 +180,39 @@ intfa_fwd_pipe_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
   constexpr int NGRP = C::NGRP;
   constexpr int B_QFULL = 0;      // TMA: Q tile landed
   constexpr int B_QEMPTY = 1;     // commit: last Q K^T of the work item done
-  constexpr int B_PFULL = 2;      // [NGRP] softmax group b (4 warps): P in shared-memory buffer b
-                                  //     (P_TMEM: [NSB], P in S buffer b: a group may be done with its next step before the
-                                  //     P V of this one is issued)
-  constexpr int B_PFREE = 5;      // [NGRP] commit: the P V that read P buffer b is done
-  constexpr int B_OFULL = 8;      // [NO] commit: O_j = P V in TMEM buffer (step mod NO)
-  constexpr int B_OFREE = C::NUM_BARS - 3;   // [NO] accumulator warps (4): O_j read out
-  constexpr int B_FIN = 10;       // [2] softmax (4 warps of one group): final (m, l) of the work item published; one
+  constexpr int B_OFULL = 2;      // [NO] commit: O_j = P V in TMEM buffer (step mod NO)
+  constexpr int B_FIN = 4;        // [2] softmax (4 warps of one group): final (m, l) of the work item published; one
                                   //     barrier per slot, so that a short next work item cannot complete it twice
                                   //     before a slow accumulator warp has waited for the first completion
-  constexpr int B_FINFREE = 12;   // [2] accumulator warps (4): they have read them
-  constexpr int B_HM = 14;        // [NGRP] softmax group g (4 warps): running max after its step published
-  constexpr int B_HL = 17;        // [NGRP] !L_IN_ACC: softmax group g (4 warps): row sum after its step published
-  constexpr int B_KFULL = 20, B_KEMPTY = 20 + NSK, B_VFULL = 20 + 2 * NSK, B_VEMPTY = 20 + 2 * NSK + NSV;
-  constexpr int B_TILE = 20 + 2 * NSK + 2 * NSV, B_TDONE = B_TILE + 4;
+  constexpr int B_FINFREE = 6;    // [2] accumulator warps (4): they have read them
+  constexpr int B_HM = 8;         // [NGRP] softmax group g (4 warps): running max after its step published
+  constexpr int B_HL = 11;        // [NGRP] !L_IN_ACC: softmax group g (4 warps): row sum after its step published
+  // What an MMA warp needs for step j arrives on ONE barrier, which belongs to the step's K or V stage: a wait that finds
+  // everything there costs these warps 200 to 350 cycles, and three of them in a row were the longest part of the way from P to
+  // the next S (half-int8, batch 2, 32 heads, 4096 tokens: 567 -> 518 us; full-int8 at head dim 32: 1131 -> 887 us).
+  constexpr int B_QKRDY = 14;               // [NSK] TMA: K tile landed; softmax group of step j - NSB (4 warps): S buffer read out
+                                            //     for good (P_TMEM: commit: the P V that read P from it is done)
+  constexpr int B_KEMPTY = B_QKRDY + NSK;   // [NSK] commit: the Q K^T that read the stage is done
+  constexpr int B_PVRDY = B_KEMPTY + NSK;   // [NSV] TMA: V tile landed; softmax group of step j (4 warps): P written; accumulator
+                                            //     warps (4): O_j of step j - NO read out (half-int8: the accumulator row is at
+                                            //     step j's running max)
+  constexpr int B_VEMPTY = B_PVRDY + NSV;   // [NSV] commit: the P V that read the stage is done
+  constexpr int B_PFREE = B_VEMPTY + NSV;   // [NPBAR] commit: the P V that read shared-memory P buffer b is done
+  constexpr int B_TILE = B_PFREE + C::NPBAR, B_TDONE = B_TILE + 4;
   constexpr int B_AFULL = B_TDONE + 4;   // [4] half-int8: alpha of step j (slot j mod 4) published, for the accumulator warps
+  constexpr int SFREE_ARRIVALS = C::P_TMEM ? 1 : 4;
   constexpr int B_SFULL = B_AFULL + 4;   // [NSB] commit: S = Q K^T in TMEM buffer b; scale loader: the step's K scales in
                                          //     shared memory (the arrival of the warp that wrote them is what lets the
                                          //     softmax warps see them)
-  constexpr int B_SFREE = B_SFULL + NSB; // [NSB] softmax group of the step (4 warps): S buffer b read out for good
-                                         //     (P_TMEM: commit: the P V that read P from it is done)
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + C::OFF_MISC);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + C::OFF_MISC + 4);
-  volatile int* tile_slot = reinterpret_cast<volatile int*>(smem + C::OFF_MISC + 16);
+  TileInfo* tile_slot = reinterpret_cast<TileInfo*>(smem + C::OFF_TILE);
 
   if (threadIdx.x == 0) {
     mbar_init(BAR(B_QFULL), 1);
     mbar_init(BAR(B_QEMPTY), 1);
-    for (int b = 0; b < C::NPB; ++b) mbar_init(BAR(B_PFULL + b), 4);
+    for (int b = 0; b < C::NPBAR; ++b) mbar_init(BAR(B_PFREE + b), 1);
     for (int b = 0; b < NGRP; ++b) {
-      if (!C::P_TMEM) mbar_init(BAR(B_PFREE + b), 1);      // (the fourth P-full barrier otherwise)
       mbar_init(BAR(B_HM + b), 4);
       mbar_init(BAR(B_HL + b), 4);
     }
@@ -211,29 +220,27 @@ intfa_fwd_pipe_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
       mbar_init(BAR(B_FINFREE + b), 4);
       mbar_init(BAR(B_FIN + b), 4);
     }
-    for (int b = 0; b < NO; ++b) {
-      mbar_init(BAR(B_OFULL + b), 1);
-      mbar_init(BAR(B_OFREE + b), 4);
-    }
+    for (int b = 0; b < NO; ++b) mbar_init(BAR(B_OFULL + b), 1);
     for (int s = 0; s < NSK; ++s) {
-      mbar_init(BAR(B_KFULL + s), 1);
+      mbar_init(BAR(B_QKRDY + s), 1 + SFREE_ARRIVALS);
       mbar_init(BAR(B_KEMPTY + s), 1);
     }
     for (int s = 0; s < NSV; ++s) {
-      mbar_init(BAR(B_VFULL + s), 1);
+      mbar_init(BAR(B_PVRDY + s), 1 + 4 + 4);
       mbar_init(BAR(B_VEMPTY + s), 1);
     }
-    for (int b = 0; b < NSB; ++b) {
-      mbar_init(BAR(B_SFULL + b), 2);         // Q K^T done; the K scales of the step are written
-      mbar_init(BAR(B_SFREE + b), C::P_TMEM ? 1 : 4);
-    }
+    for (int b = 0; b < NSB; ++b) mbar_init(BAR(B_SFULL + b), 2);         // Q K^T done; the K scales of the step are written
+    // the first steps find their S and O_j buffers free
+    for (int j = 0; j < NSB; ++j) mbar_arrive_n(BAR(B_QKRDY + j), SFREE_ARRIVALS);
+    if (FULL)
+      for (int j = 0; j < NO; ++j) mbar_arrive_n(BAR(B_PVRDY + j), 4);
     for (int i = 0; i < 4; ++i) {
       mbar_init(BAR(B_TILE + i), 1);
       mbar_init(BAR(B_TDONE + i), 7 + 4 * NGRP);       // 2 MMA warps, the scale loader, accumulator and softmax warps
       mbar_init(BAR(B_AFULL + i), 4);
     }
     abort_flag[0] = 0;
-    abort_flag[1] = p.wait_limit_kcycles;
+    abort_flag[1] = (int)((uint32_t)p.wait_limit_kcycles << 10);
     mbar_init_fence();
     fence_proxy_async_smem();
   }
@@ -270,15 +277,16 @@ intfa_fwd_pipe_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
   const uint64_t descArm = make_smem_desc(smem_u32(smem + C::OFF_MAGIC), 128, 256, 0);
 
   // work items: drawn from a global counter by the producer, published in a 4-slot ring
-  auto next_tile = [&](uint32_t& seq, bool ack, bool whole_warp) -> int {
-    const uint32_t slot = seq & 3u, par = (seq >> 2) & 1u;
+  auto wait_tile = [&](uint32_t seq) { return mbar_wait_warp<POLITE>(BAR(B_TILE + (seq & 3u)), (seq >> 2) & 1u, abort_flag, p.status, code_hi | PW_TILE); };
+  auto next_tile = [&](uint32_t& seq) -> TileInfo {
+    const uint32_t slot = seq & 3u;
+    TileInfo t;
+    t.nsteps = -1;
+    if (!wait_tile(seq)) return t;
     ++seq;
-    bool got = mbar_wait<POLITE>(BAR(B_TILE + slot), par, abort_flag, p.status, code_hi | PW_TILE);
-    if (whole_warp) got = __all_sync(0xffffffffu, got);
-    if (!got) return -1;
-    const int t = tile_slot[slot];
-    if (whole_warp) __syncwarp();
-    if (ack) mbar_arrive(BAR(B_TDONE + slot));
+    t = tile_slot[slot];
+    __syncwarp();
+    if (lane == 0) mbar_arrive(BAR(B_TDONE + slot));
     return t;
   };
 
@@ -317,11 +325,13 @@ intfa_fwd_pipe_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
             passes_left = NVH - 1;
           }
         }
-        tile_slot[tseq & 3u] = tile;
+        TileInfo t;
+        t.nsteps = -1;
+        if (tile >= 0) t = decode_tile<RAGGED, NVH>(p, tile, G);
+        tile_slot[tseq & 3u] = t;
         mbar_arrive(BAR(B_TILE + (tseq & 3u)));
         ++tseq;
         if (tile < 0) break;
-        const TileInfo t = decode_tile<RAGGED, NVH>(p, tile, G);
         if (t.nsteps == 0) continue;
         ok = mbar_wait<POLITE>(BAR(B_QEMPTY), (tile_it & 1) ^ 1, abort_flag, p.status, code_hi | PW_QE);
         if (!ok) break;
@@ -335,18 +345,18 @@ intfa_fwd_pipe_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
           if (!ok) break;
           const int jb = kv_tile_of_step(p, j, t.nsteps);
           if (p.skip_k_load == 0 || kv_it + 1 != (uint32_t)p.skip_k_load) {      // (test hook: a K tile that never arrives)
-            mbar_expect_tx(BAR(B_KFULL + s), C::K_BYTES);
+            mbar_expect_tx(BAR(B_QKRDY + s), C::K_BYTES);
 #pragma unroll
             for (int pn = 0; pn < C::QK_PANELS; ++pn)
-              tma_load_4d(sK + s * C::K_BYTES + pn * (G * C::QK_ROWB), &tmK, BAR(B_KFULL + s), pn * C::QK_ROWB, jb * G, t.hk, t.b);
+              tma_load_4d(sK + s * C::K_BYTES + pn * (G * C::QK_ROWB), &tmK, BAR(B_QKRDY + s), pn * C::QK_ROWB, jb * G, t.hk, t.b);
           }
           const uint32_t sv = kv_it % NSV, phv = (kv_it / NSV) & 1;
           ok = mbar_wait<POLITE>(BAR(B_VEMPTY + sv), phv ^ 1, abort_flag, p.status, code_hi | PW_VE);
           if (!ok) break;
-          mbar_expect_tx(BAR(B_VFULL + sv), C::V_BYTES);
+          mbar_expect_tx(BAR(B_PVRDY + sv), C::V_BYTES);
 #pragma unroll
           for (int c = 0; c < C::V_BOXES; ++c)
-            tma_load_4d(sV + sv * C::V_BYTES + c * (G * C::V_ROWB), &tmV, BAR(B_VFULL + sv), t.vh * D + c * C::V_BOXCH, jb * G, t.hk, t.b);
+            tma_load_4d(sV + sv * C::V_BYTES + c * (G * C::V_ROWB), &tmV, BAR(B_PVRDY + sv), t.vh * D + c * C::V_BOXCH, jb * G, t.hk, t.b);
         }
         ++tile_it;
       }
@@ -369,9 +379,8 @@ intfa_fwd_pipe_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
     bool ok = true;
 #pragma unroll 1
     while (ok) {
-      const int tile = next_tile(tseq, lane == 0, true);
-      if (tile < 0) break;
-      const TileInfo t = decode_tile<RAGGED, NVH>(p, tile, G);
+      const TileInfo t = next_tile(tseq);
+      if (t.nsteps < 0) break;
       const long long row = (long long)t.b * p.ks_sb + (long long)t.hk * p.ks_sh;
       float ks[G / 32];
 #pragma unroll 1
@@ -403,28 +412,21 @@ intfa_fwd_pipe_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
       // off the per-thread path); one elected lane issues the tensor-core instructions.
       // Step it goes into S buffer it mod NSB as soon as the step NSB back has been read out of it and K has landed.  The K stage is handed back by the tensor core itself (the
       // K scales sit in a ring of their own).
-      uint32_t kv_it = 0, tile_it = 0, tseq = 0, sfree_seen = 0;
+      uint32_t kv_it = 0, tile_it = 0, tseq = 0;
       bool ok = true;
       // operand descriptors of stage 0 / K step 0; the start-address field (16-byte units) takes the offsets
       const uint64_t descQ0 = make_smem_desc(sQ, 16, C::SBO_QK, C::SWZ_QK);
       const uint64_t descK0 = make_smem_desc(sK, 16, C::SBO_QK, C::SWZ_QK);
       while (ok) {
-        const int tile = next_tile(tseq, lane == 0, true);
-        if (tile < 0) break;
-        const TileInfo t = decode_tile<RAGGED, NVH>(p, tile, G);
+        const TileInfo t = next_tile(tseq);
+        if (t.nsteps < 0) break;
         if (t.nsteps == 0) continue;
         ok = mbar_wait_warp<POLITE>(BAR(B_QFULL), tile_it & 1, abort_flag, p.status, code_hi | PW_QF);
         if (!ok) break;
         for (int j = 0; j < t.nsteps; ++j, ++kv_it) {
           const uint32_t s = kv_it % NSK, ph = (kv_it / NSK) & 1;
           const uint32_t sb = kv_it % NSB;
-          // every S_FREE is waited for exactly once, in step order, so the phases of the barriers stay in step
-          while (ok && sfree_seen + NSB <= kv_it) {
-            ok = mbar_wait_warp<POLITE>(BAR(B_SFREE + sfree_seen % NSB), (sfree_seen / NSB) & 1, abort_flag, p.status, code_hi | PW_SFREE);
-            ++sfree_seen;
-          }
-          if (!ok) break;
-          ok = mbar_wait_warp<POLITE>(BAR(B_KFULL + s), ph, abort_flag, p.status, code_hi | PW_KF);
+          ok = mbar_wait_warp<POLITE>(BAR(B_QKRDY + s), ph, abort_flag, p.status, code_hi | PW_QKRDY);
           if (!ok) break;
           tc_fence_after();
           const uint64_t bd0 = descK0 + (uint64_t)(s * (C::K_BYTES >> 4));
@@ -447,28 +449,17 @@ intfa_fwd_pipe_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
     {
       // ------------------------------------------------------------------ MMA issuer for O_j = P V
       // A warp of its own, so that a Q K^T whose S buffer is free never queues behind the wait for a P tile.
-      // Per step j: [P(j) written] [V(j) landed] [O_j of step j-1 read out] PV(j).
       uint32_t kv_it = 0, tseq = 0;
       bool ok = true;
       const uint64_t descP0 = make_smem_desc(sP, 16, C::SBO_P, C::SWZ_P);
       const uint64_t descV0 = make_smem_desc(sV, C::V_BOXES > 1 ? G * C::V_ROWB : 16, C::SBO_V, C::SWZ_V);
       while (ok) {
-        const int tile = next_tile(tseq, lane == 0, true);
-        if (tile < 0) break;
-        const TileInfo t = decode_tile<RAGGED, NVH>(p, tile, G);
+        const TileInfo t = next_tile(tseq);
+        if (t.nsteps < 0) break;
         for (int j = 0; j < t.nsteps; ++j, ++kv_it) {
           const uint32_t s = kv_it % NSV, ph = (kv_it / NSV) & 1;
           const uint32_t b = kv_it % C::NPB;
-          // P(j) written; V(j) landed; full-int8: O_j of the previous step has been read out, half-int8: the
-          // accumulator has been brought to this step's running max (and the previous P V has landed in it).
-          // (One copy of the wait code for the three.)
-#pragma unroll 1
-          for (int w = 0; w < 3; ++w) {
-            const uint32_t wb = w == 0 ? BAR(B_PFULL + b) : w == 1 ? BAR(B_VFULL + s) : BAR(B_OFREE + kv_it % NO);
-            const uint32_t wp = w == 0 ? ((kv_it / C::NPB) & 1) : w == 1 ? ph : (FULL ? (((kv_it / NO) & 1) ^ 1) : (kv_it & 1));
-            ok = mbar_wait_warp<POLITE>(wb, wp, abort_flag, p.status, code_hi | (w == 0 ? PW_PFULL : w == 1 ? PW_VF : PW_OFREE));
-            if (!ok) break;
-          }
+          ok = mbar_wait_warp<POLITE>(BAR(B_PVRDY + s), ph, abort_flag, p.status, code_hi | PW_PVRDY);
           if (!ok) break;
           tc_fence_after();
           const uint64_t ad0 = descP0 + (uint64_t)(b * (C::P_BYTES >> 4));
@@ -497,7 +488,7 @@ intfa_fwd_pipe_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
             }
             umma_commit(BAR(B_OFULL + kv_it % NO));
             umma_commit(BAR(B_VEMPTY + s));
-            umma_commit(C::P_TMEM ? BAR(B_SFREE + b) : BAR(B_PFREE + b));
+            umma_commit(C::P_TMEM ? BAR(B_QKRDY + (kv_it + NSB) % NSK) : BAR(B_PFREE + b));
           }
           __syncwarp();
         }

@@ -26,6 +26,9 @@ __device__ __forceinline__ void mbar_init_fence() {
 __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
+__device__ __forceinline__ void mbar_arrive_n(uint32_t bar, uint32_t n) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(n) : "memory");
+}
 __device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
 }
@@ -42,8 +45,8 @@ __device__ __forceinline__ uint32_t mbar_try_wait(uint32_t bar, uint32_t parity)
       : "memory");
   return done;
 }
-// Bounded wait.  Every spin in the kernels goes through here: after the limit (abort_flag[1], in units of 1024
-// SM cycles; 2^21 = about one second at B200 clocks unless a test shortens it) without completion the waiter
+// Bounded wait.  Every spin in the kernels goes through here: after the limit (abort_flag[1], in SM
+// cycles; 2^31 = about one second at B200 clocks unless a test shortens it) without completion the waiter
 // records `code` in *status (first writer wins), raises the CTA-wide abort flag (abort_flag[0]) and returns
 // false; every other waiter of the CTA sees the flag on its next look and returns false as well, so the CTA
 // drains and exits.
@@ -54,11 +57,11 @@ __device__ __forceinline__ uint32_t mbar_try_wait(uint32_t bar, uint32_t parity)
 template <bool POLITE>
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag, int* status, int code) {
   if (mbar_try_wait(bar, parity)) return true;
-  const uint32_t t0 = (uint32_t)(clock64() >> 10);
+  const uint32_t t0 = (uint32_t)clock();
 #pragma unroll 1
   while (!mbar_try_wait(bar, parity)) {
     if (POLITE && threadIdx.x < 128) __nanosleep(20);
-    if ((int)((uint32_t)(clock64() >> 10) - t0) > abort_flag[1]) {
+    if ((uint32_t)clock() - t0 > (uint32_t)abort_flag[1]) {
       *abort_flag = 1;
       if (status) atomicCAS(status, 0, code);
     }
@@ -72,6 +75,18 @@ template <bool POLITE>
 __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile int* abort_flag,
                                                int* status, int code) {
   return __all_sync(0xffffffffu, mbar_wait<POLITE>(bar, parity, abort_flag, status, code));
+}
+
+// Two barriers at once: where both phases are complete already, the two looks cost one latency.
+template <bool POLITE>
+__device__ __forceinline__ bool mbar_wait2_warp(uint32_t bar0, uint32_t parity0, int code0, uint32_t bar1, uint32_t parity1, int code1,
+                                                volatile int* abort_flag, int* status) {
+  const uint32_t a = mbar_try_wait(bar0, parity0), b = mbar_try_wait(bar1, parity1);
+  if (__all_sync(0xffffffffu, a & b)) return true;
+#pragma unroll 1
+  for (int w = 0; w < 2; ++w)
+    if (!mbar_wait_warp<POLITE>(w ? bar1 : bar0, w ? parity1 : parity0, abort_flag, status, w ? code1 : code0)) return false;
+  return true;
 }
 
 // N instructions (16 bytes each) that do nothing: filler to move the code behind it in the instruction cache.
