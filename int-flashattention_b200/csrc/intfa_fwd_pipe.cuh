@@ -171,7 +171,9 @@ intfa_fwd_pipe_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
   extern __shared__ uint8_t smem_raw[];
   // (rounded up by an offset, not through an integer: the compiler then knows that all this is shared memory)
   uint8_t* smem = smem_raw + ((0u - smem_u32(smem_raw)) & 1023u);
-  const int warp = threadIdx.x >> 5;
+  // (Uniform for the compiler: with the plain quotient every role's code is in a branch that it must take for divergent, and
+  // all descriptors, barrier addresses and counters sit in vector registers.)
+  const int warp = warp_uniform(threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
 
   const uint32_t bar0 = smem_u32(smem + C::OFF_BAR);
@@ -251,7 +253,7 @@ intfa_fwd_pipe_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
   }
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = warp_uniform(*tmem_slot);
   const uint32_t tS = tmem_base + C::COL_S;
   const uint32_t tO = tmem_base + C::COL_O;
   const uint32_t tA = tmem_base + C::COL_ACC;
@@ -284,8 +286,15 @@ intfa_fwd_pipe_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
     t.nsteps = -1;
     if (!wait_tile(seq)) return t;
     ++seq;
-    t = tile_slot[slot];
-    __syncwarp();
+    const TileInfo& s = tile_slot[slot];
+    t.b = warp_uniform(s.b);
+    t.h = warp_uniform(s.h);
+    t.hk = warp_uniform(s.hk);
+    t.mb = warp_uniform(s.mb);
+    t.bh = warp_uniform(s.bh);
+    t.work = warp_uniform(s.work);
+    t.vh = 0;
+    t.nsteps = warp_uniform(s.nsteps);
     if (lane == 0) mbar_arrive(BAR(B_TDONE + slot));
     return t;
   };
@@ -294,17 +303,21 @@ intfa_fwd_pipe_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
   if (warp < 4) reg_dealloc<kPipeServiceRegs>();
 
   if (warp == 0) {
-    if (lane == 0) {
+    {
       // ------------------------------------------------------------------ TMA producer
-      prefetch_tmap(&tmQ);
-      prefetch_tmap(&tmK);
-      prefetch_tmap(&tmV);
+      // (the whole warp runs the loop, one lane issues: as in the MMA warps)
+      if (lane == 0) {
+        prefetch_tmap(&tmQ);
+        prefetch_tmap(&tmK);
+        prefetch_tmap(&tmV);
+      }
       uint32_t kv_it = 0, tile_it = 0, tseq = 0;
       int drawn = 0, passes_left = 0;      // NVH > 1: the query tile in hand and how many of its passes are still to publish
       bool ok = true;
+#pragma unroll 1
       while (ok) {
         if (tseq >= 4u) {
-          ok = mbar_wait<POLITE>(BAR(B_TDONE + (tseq & 3u)), ((tseq >> 2) - 1u) & 1u, abort_flag, p.status, code_hi | PW_TILE);
+          ok = mbar_wait_warp<POLITE>(BAR(B_TDONE + (tseq & 3u)), ((tseq >> 2) - 1u) & 1u, abort_flag, p.status, code_hi | PW_TILE);
           if (!ok) break;
         }
         int tile;
@@ -315,7 +328,11 @@ intfa_fwd_pipe_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
           if (tseq == 0) {
             tile = (int)blockIdx.x;
           } else {
-            tile = p.tile_counter ? (int)(gridDim.x + atomicAdd(p.tile_counter, 1u)) : p.num_tiles;
+            tile = p.num_tiles;
+            if (p.tile_counter) {
+              if (lane == 0) tile = (int)(gridDim.x + atomicAdd(p.tile_counter, 1u));
+              tile = warp_uniform(tile);
+            }
           }
           if (tile >= p.num_tiles) {
             tile = -1;
@@ -328,40 +345,50 @@ intfa_fwd_pipe_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         TileInfo t;
         t.nsteps = -1;
         if (tile >= 0) t = decode_tile<RAGGED, NVH>(p, tile, G);
-        tile_slot[tseq & 3u] = t;
-        mbar_arrive(BAR(B_TILE + (tseq & 3u)));
+        if (lane == 0) {
+          tile_slot[tseq & 3u] = t;
+          mbar_arrive(BAR(B_TILE + (tseq & 3u)));
+        }
         ++tseq;
         if (tile < 0) break;
         if (t.nsteps == 0) continue;
-        ok = mbar_wait<POLITE>(BAR(B_QEMPTY), (tile_it & 1) ^ 1, abort_flag, p.status, code_hi | PW_QE);
+        ok = mbar_wait_warp<POLITE>(BAR(B_QEMPTY), (tile_it & 1) ^ 1, abort_flag, p.status, code_hi | PW_QE);
         if (!ok) break;
-        mbar_expect_tx(BAR(B_QFULL), C::Q_BYTES);
+        if (elect_one()) {
+          mbar_expect_tx(BAR(B_QFULL), C::Q_BYTES);
 #pragma unroll
-        for (int pn = 0; pn < C::QK_PANELS; ++pn)
-          tma_load_4d(sQ + pn * (kBM * C::QK_ROWB), &tmQ, BAR(B_QFULL), pn * C::QK_ROWB, t.mb * kBM, t.h, t.b);
+          for (int pn = 0; pn < C::QK_PANELS; ++pn)
+            tma_load_4d(sQ + pn * (kBM * C::QK_ROWB), &tmQ, BAR(B_QFULL), pn * C::QK_ROWB, t.mb * kBM, t.h, t.b);
+        }
+        __syncwarp();
+#pragma unroll 1
         for (int j = 0; j < t.nsteps; ++j, ++kv_it) {
           const uint32_t s = kv_it % NSK, ph = (kv_it / NSK) & 1;
-          ok = mbar_wait<POLITE>(BAR(B_KEMPTY + s), ph ^ 1, abort_flag, p.status, code_hi | PW_KE);
+          ok = mbar_wait_warp<POLITE>(BAR(B_KEMPTY + s), ph ^ 1, abort_flag, p.status, code_hi | PW_KE);
           if (!ok) break;
           const int jb = kv_tile_of_step(p, j, t.nsteps);
-          if (p.skip_k_load == 0 || kv_it + 1 != (uint32_t)p.skip_k_load) {      // (test hook: a K tile that never arrives)
+          if ((p.skip_k_load == 0 || kv_it + 1 != (uint32_t)p.skip_k_load) && elect_one()) {      // (test hook: a K tile that never arrives)
             mbar_expect_tx(BAR(B_QKRDY + s), C::K_BYTES);
 #pragma unroll
             for (int pn = 0; pn < C::QK_PANELS; ++pn)
               tma_load_4d(sK + s * C::K_BYTES + pn * (G * C::QK_ROWB), &tmK, BAR(B_QKRDY + s), pn * C::QK_ROWB, jb * G, t.hk, t.b);
           }
           const uint32_t sv = kv_it % NSV, phv = (kv_it / NSV) & 1;
-          ok = mbar_wait<POLITE>(BAR(B_VEMPTY + sv), phv ^ 1, abort_flag, p.status, code_hi | PW_VE);
+          __syncwarp();
+          ok = mbar_wait_warp<POLITE>(BAR(B_VEMPTY + sv), phv ^ 1, abort_flag, p.status, code_hi | PW_VE);
           if (!ok) break;
-          mbar_expect_tx(BAR(B_PVRDY + sv), C::V_BYTES);
+          if (elect_one()) {
+            mbar_expect_tx(BAR(B_PVRDY + sv), C::V_BYTES);
 #pragma unroll
-          for (int c = 0; c < C::V_BOXES; ++c)
-            tma_load_4d(sV + sv * C::V_BYTES + c * (G * C::V_ROWB), &tmV, BAR(B_PVRDY + sv), t.vh * D + c * C::V_BOXCH, jb * G, t.hk, t.b);
+            for (int c = 0; c < C::V_BOXES; ++c)
+              tma_load_4d(sV + sv * C::V_BYTES + c * (G * C::V_ROWB), &tmV, BAR(B_PVRDY + sv), t.vh * D + c * C::V_BOXCH, jb * G, t.hk, t.b);
+          }
+          __syncwarp();
         }
         ++tile_it;
       }
       // The last CTA to get here leaves the counter words zero for the next launch that is given them.
-      if (p.tile_counter && atomicAdd(p.tile_counter + 1, 1u) + 1u == gridDim.x) {
+      if (lane == 0 && p.tile_counter && atomicAdd(p.tile_counter + 1, 1u) + 1u == gridDim.x) {
         p.tile_counter[0] = 0u;
         p.tile_counter[1] = 0u;
       }
@@ -417,12 +444,14 @@ intfa_fwd_pipe_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
       // operand descriptors of stage 0 / K step 0; the start-address field (16-byte units) takes the offsets
       const uint64_t descQ0 = make_smem_desc(sQ, 16, C::SBO_QK, C::SWZ_QK);
       const uint64_t descK0 = make_smem_desc(sK, 16, C::SBO_QK, C::SWZ_QK);
+#pragma unroll 1
       while (ok) {
         const TileInfo t = next_tile(tseq);
         if (t.nsteps < 0) break;
         if (t.nsteps == 0) continue;
         ok = mbar_wait_warp<POLITE>(BAR(B_QFULL), tile_it & 1, abort_flag, p.status, code_hi | PW_QF);
         if (!ok) break;
+#pragma unroll 1
         for (int j = 0; j < t.nsteps; ++j, ++kv_it) {
           const uint32_t s = kv_it % NSK, ph = (kv_it / NSK) & 1;
           const uint32_t sb = kv_it % NSB;
@@ -453,9 +482,11 @@ intfa_fwd_pipe_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
       bool ok = true;
       const uint64_t descP0 = make_smem_desc(sP, 16, C::SBO_P, C::SWZ_P);
       const uint64_t descV0 = make_smem_desc(sV, C::V_BOXES > 1 ? G * C::V_ROWB : 16, C::SBO_V, C::SWZ_V);
+#pragma unroll 1
       while (ok) {
         const TileInfo t = next_tile(tseq);
         if (t.nsteps < 0) break;
+#pragma unroll 1
         for (int j = 0; j < t.nsteps; ++j, ++kv_it) {
           const uint32_t s = kv_it % NSV, ph = (kv_it / NSV) & 1;
           const uint32_t b = kv_it % C::NPB;

@@ -14,6 +14,10 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
 
+// A value that all lanes of a converged warp have in common, in the form in which the compiler knows it: what follows from it
+// (addresses, descriptors, loop counters, branches) then lives in uniform registers instead of one register per lane.
+__device__ __forceinline__ int warp_uniform(int x) { return __shfl_sync(0xffffffffu, x, 0); }
+
 // ---------------------------------------------------------------------------
 // mbarrier
 // ---------------------------------------------------------------------------
