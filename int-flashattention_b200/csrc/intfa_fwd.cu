@@ -97,6 +97,11 @@ __device__ __forceinline__ TileInfo decode_tile(const KParams& p, int tile, int 
 // KV tile visited at step j of a work item with n steps: ascending, or last tile first
 __device__ __forceinline__ int kv_tile_of_step(const KParams& p, int j, int n) { return p.kv_desc ? n - 1 - j : j; }
 
+template <bool B>
+struct Const {
+  static constexpr bool value = B;
+};
+
 // byte offset of 16-byte chunk `chunk` of row `row` inside a swizzled [rows][ROWB bytes] tile
 template <int ROWB>
 __device__ __forceinline__ uint32_t swz_off(int row, int chunk) {
@@ -177,7 +182,7 @@ static constexpr CUtensorMapSwizzle swizzle_of_row_bytes(int bytes) {
 
 // One CTA per SM.  The tensor maps describe the tensors with their own head dim (a->D); the boxes are as wide as the
 // kernel's tiles, so at head dim 16 the upper half of every 32-wide box lies outside the tensor and arrives as zeros.
-template <int D, int G, bool FULL, bool PRNE, bool RAGGED, int DQ = D, bool F8V = false, bool POLITE = false>
+template <int D, int G, bool FULL, bool PRNE, bool RAGGED, int DQ = D, bool F8V = false, bool STEADY = false>
 static int launch_pipe(const IntfaFwdParams* a, const KParams& kp, cudaStream_t stream) {
   using C = PipeCfg<D, G, FULL, DQ, F8V>;
   static_assert(C::SMEM_BYTES <= 227 * 1024, "shared memory");
@@ -188,7 +193,7 @@ static int launch_pipe(const IntfaFwdParams* a, const KParams& kp, cudaStream_t 
   if ((rc = make_tmap(&tmQ, a->q, 1, a->q_stride, a->B, a->H, a->Nq, hd, C::QK_ROWB, kBM, swzQK))) return rc;
   if ((rc = make_tmap(&tmK, a->k, 1, a->k_stride, a->B, kv_heads(a), a->Nk, hd, C::QK_ROWB, G, swzQK))) return rc;
   if ((rc = make_tmap(&tmV, a->v, C::BYTE_PV ? 1 : 2, a->v_stride, a->B, kv_heads(a), a->Nk, hd, C::V_BOXCH, G, swzV))) return rc;
-  auto kern = intfa_fwd_pipe_kernel<D, G, FULL, PRNE, RAGGED, DQ, F8V, POLITE>;
+  auto kern = intfa_fwd_pipe_kernel<D, G, FULL, PRNE, RAGGED, DQ, F8V, STEADY>;
   static std::atomic<bool> attr_done[64];     // per instantiation and device (the attribute is per device)
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return set_error(INTFA_ERR_CUDA, "cannot query the current device");

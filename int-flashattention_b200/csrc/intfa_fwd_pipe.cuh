@@ -89,11 +89,11 @@ struct PipeCfg {
   // code costs the steps that need no mask more (instruction cache) than it gives (2 x 16 x 4096 at d=32: 573 -> 631).
   __host__ __device__ static constexpr bool band_fast(bool ragged) { return G == 128 || D == 256 || (G == 32 && ragged); }
   // instructions of never-executed filler between the softmax passes (see intfa_fwd_pipe_softmax.inc), the best of a sweep in
-  // steps of 1 KB for each kind of instantiation (`ragged`: masks partial tiles; `polite`: see the kernel).  Between the best
+  // steps of 1 KB for each kind of instantiation (`ragged`: masks partial tiles; `steady`: see the kernel).  Between the best
   // and the worst of a sweep lie 1 to 2 % non-causal, 5 to 15 % causal.
-  __host__ __device__ static constexpr int code_filler_of(bool ragged, bool polite) {
+  __host__ __device__ static constexpr int code_filler_of(bool ragged, bool steady) {
     if (P_TMEM) return G == 128 ? (ragged ? 0 : 192) : D == 256 ? (ragged ? 384 : 0) : D == 128 ? (ragged ? 256 : 128) : ragged ? 128 : 256;
-    return NGRP == 3 ? (!FULL ? 192 : (ragged && G == 128) ? 64 : polite ? 128 : 256)
+    return NGRP == 3 ? (!FULL ? 192 : (ragged && G == 128) ? 64 : steady ? 128 : 256)
          : ragged ? (G == 32 ? 128 : FULL && G == 128 && D <= 64 ? 384 : 256) : G == 128 ? (!FULL ? 320 : DQ == 256 ? 448 : 64) : D == 32 ? 256 : 320;
   }
   static constexpr bool MORE_SOFTMAX_REGS = !FULL || G == 128;
@@ -158,11 +158,8 @@ enum PipeWait { PW_TILE = 32, PW_QE, PW_KE, PW_VE, PW_QF, PW_QKRDY, PW_PVRDY, PW
 
 // RAGGED: Nq / Nk are not multiples of 128 / G -- the last query tile and the last KV step are partial.  A separate
 // instantiation, so that the code of the common case stays as small as it was (instruction cache).
-// POLITE: the service warps (0 to 3) sleep 20 ns between two looks at a barrier, and the softmax groups take the running max
-// before pass A (HM_LATE).  With three groups of full-int8 and every step of a work item alike, 341 -> 330 us; causal work
-// items, whose steps are fewer and partly masked, lose by it (238 -> 245 us) and keep polling.  Chosen by causality and not by
-// the length of a work item, which has not been measured for itself.
-template <int D, int G, bool FULL, bool PRNE, bool RAGGED, int DQ = D, bool F8V = false, bool POLITE = false>
+// STEADY: non-causal full-int8 with three groups, whose groups take the running max over before pass A (see the softmax warps).
+template <int D, int G, bool FULL, bool PRNE, bool RAGGED, int DQ = D, bool F8V = false, bool STEADY = false>
 __global__ void __launch_bounds__((PipeCfg<D, G, FULL, DQ, F8V>::THREADS), 1)
 intfa_fwd_pipe_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                       const __grid_constant__ CUtensorMap tmV, const KParams p) {
@@ -279,7 +276,7 @@ intfa_fwd_pipe_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
   const uint64_t descArm = make_smem_desc(smem_u32(smem + C::OFF_MAGIC), 128, 256, 0);
 
   // work items: drawn from a global counter by the producer, published in a 4-slot ring
-  auto wait_tile = [&](uint32_t seq) { return mbar_wait_warp<POLITE>(BAR(B_TILE + (seq & 3u)), (seq >> 2) & 1u, abort_flag, p.status, code_hi | PW_TILE); };
+  auto wait_tile = [&](uint32_t seq) { return mbar_wait_warp(BAR(B_TILE + (seq & 3u)), (seq >> 2) & 1u, abort_flag, p.status, code_hi | PW_TILE); };
   auto next_tile = [&](uint32_t& seq) -> TileInfo {
     const uint32_t slot = seq & 3u;
     TileInfo t;
@@ -317,7 +314,7 @@ intfa_fwd_pipe_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
 #pragma unroll 1
       while (ok) {
         if (tseq >= 4u) {
-          ok = mbar_wait_warp<POLITE>(BAR(B_TDONE + (tseq & 3u)), ((tseq >> 2) - 1u) & 1u, abort_flag, p.status, code_hi | PW_TILE);
+          ok = mbar_wait_warp(BAR(B_TDONE + (tseq & 3u)), ((tseq >> 2) - 1u) & 1u, abort_flag, p.status, code_hi | PW_TILE);
           if (!ok) break;
         }
         int tile;
@@ -352,7 +349,7 @@ intfa_fwd_pipe_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         ++tseq;
         if (tile < 0) break;
         if (t.nsteps == 0) continue;
-        ok = mbar_wait_warp<POLITE>(BAR(B_QEMPTY), (tile_it & 1) ^ 1, abort_flag, p.status, code_hi | PW_QE);
+        ok = mbar_wait_warp(BAR(B_QEMPTY), (tile_it & 1) ^ 1, abort_flag, p.status, code_hi | PW_QE);
         if (!ok) break;
         if (elect_one()) {
           mbar_expect_tx(BAR(B_QFULL), C::Q_BYTES);
@@ -364,7 +361,7 @@ intfa_fwd_pipe_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
 #pragma unroll 1
         for (int j = 0; j < t.nsteps; ++j, ++kv_it) {
           const uint32_t s = kv_it % NSK, ph = (kv_it / NSK) & 1;
-          ok = mbar_wait_warp<POLITE>(BAR(B_KEMPTY + s), ph ^ 1, abort_flag, p.status, code_hi | PW_KE);
+          ok = mbar_wait_warp(BAR(B_KEMPTY + s), ph ^ 1, abort_flag, p.status, code_hi | PW_KE);
           if (!ok) break;
           const int jb = kv_tile_of_step(p, j, t.nsteps);
           if ((p.skip_k_load == 0 || kv_it + 1 != (uint32_t)p.skip_k_load) && elect_one()) {      // (test hook: a K tile that never arrives)
@@ -375,7 +372,7 @@ intfa_fwd_pipe_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
           }
           const uint32_t sv = kv_it % NSV, phv = (kv_it / NSV) & 1;
           __syncwarp();
-          ok = mbar_wait_warp<POLITE>(BAR(B_VEMPTY + sv), phv ^ 1, abort_flag, p.status, code_hi | PW_VE);
+          ok = mbar_wait_warp(BAR(B_VEMPTY + sv), phv ^ 1, abort_flag, p.status, code_hi | PW_VE);
           if (!ok) break;
           if (elect_one()) {
             mbar_expect_tx(BAR(B_PVRDY + sv), C::V_BYTES);
@@ -414,7 +411,7 @@ intfa_fwd_pipe_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
       for (int j = -1; j < t.nsteps; ++j) {
         if (j >= 0) {
           const uint32_t s = kv_it % NSB, ph = (kv_it / NSB) & 1;
-          ok = mbar_wait_warp<POLITE>(BAR(B_SFULL + s), ph ^ 1, abort_flag, p.status, code_hi | PW_SFULL);
+          ok = mbar_wait_warp(BAR(B_SFULL + s), ph ^ 1, abort_flag, p.status, code_hi | PW_SFULL);
           if (!ok) break;
           float* slot = reinterpret_cast<float*>(smem + C::OFF_KS + (kv_it % C::NKS) * C::KS_BYTES) + lane;
 #pragma unroll
@@ -449,13 +446,13 @@ intfa_fwd_pipe_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         const TileInfo t = next_tile(tseq);
         if (t.nsteps < 0) break;
         if (t.nsteps == 0) continue;
-        ok = mbar_wait_warp<POLITE>(BAR(B_QFULL), tile_it & 1, abort_flag, p.status, code_hi | PW_QF);
+        ok = mbar_wait_warp(BAR(B_QFULL), tile_it & 1, abort_flag, p.status, code_hi | PW_QF);
         if (!ok) break;
 #pragma unroll 1
         for (int j = 0; j < t.nsteps; ++j, ++kv_it) {
           const uint32_t s = kv_it % NSK, ph = (kv_it / NSK) & 1;
           const uint32_t sb = kv_it % NSB;
-          ok = mbar_wait_warp<POLITE>(BAR(B_QKRDY + s), ph, abort_flag, p.status, code_hi | PW_QKRDY);
+          ok = mbar_wait_warp(BAR(B_QKRDY + s), ph, abort_flag, p.status, code_hi | PW_QKRDY);
           if (!ok) break;
           tc_fence_after();
           const uint64_t bd0 = descK0 + (uint64_t)(s * (C::K_BYTES >> 4));
@@ -490,7 +487,7 @@ intfa_fwd_pipe_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         for (int j = 0; j < t.nsteps; ++j, ++kv_it) {
           const uint32_t s = kv_it % NSV, ph = (kv_it / NSV) & 1;
           const uint32_t b = kv_it % C::NPB;
-          ok = mbar_wait_warp<POLITE>(BAR(B_PVRDY + s), ph, abort_flag, p.status, code_hi | PW_PVRDY);
+          ok = mbar_wait_warp(BAR(B_PVRDY + s), ph, abort_flag, p.status, code_hi | PW_PVRDY);
           if (!ok) break;
           tc_fence_after();
           const uint64_t ad0 = descP0 + (uint64_t)(b * (C::P_BYTES >> 4));
