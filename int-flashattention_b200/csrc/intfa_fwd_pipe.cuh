@@ -229,7 +229,9 @@ intfa_fwd_pipe_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
       mbar_init(BAR(B_VEMPTY + s), 1);
     }
     for (int b = 0; b < NSB; ++b) mbar_init(BAR(B_SFULL + b), 2);         // Q K^T done; the K scales of the step are written
-    // the first steps find their S and O_j buffers free
+    // the very first step finds the running max (and l) handed over, the first steps their S and O_j buffers free
+    mbar_arrive_n(BAR(B_HM + NGRP - 1), 4);
+    mbar_arrive_n(BAR(B_HL + NGRP - 1), 4);
     for (int j = 0; j < NSB; ++j) mbar_arrive_n(BAR(B_QKRDY + j), SFREE_ARRIVALS);
     if (FULL)
       for (int j = 0; j < NO; ++j) mbar_arrive_n(BAR(B_PVRDY + j), 4);
@@ -436,7 +438,7 @@ intfa_fwd_pipe_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
       // off the per-thread path); one elected lane issues the tensor-core instructions.
       // Step it goes into S buffer it mod NSB as soon as the step NSB back has been read out of it and K has landed.  The K stage is handed back by the tensor core itself (the
       // K scales sit in a ring of their own).
-      uint32_t kv_it = 0, tile_it = 0, tseq = 0;
+      uint32_t kv_it = 0, tile_it = 0, tseq = 0, sb = 0;    // sb: kv_it mod NSB
       bool ok = true;
       // operand descriptors of stage 0 / K step 0; the start-address field (16-byte units) takes the offsets
       const uint64_t descQ0 = make_smem_desc(sQ, 16, C::SBO_QK, C::SWZ_QK);
@@ -451,7 +453,6 @@ intfa_fwd_pipe_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
 #pragma unroll 1
         for (int j = 0; j < t.nsteps; ++j, ++kv_it) {
           const uint32_t s = kv_it % NSK, ph = (kv_it / NSK) & 1;
-          const uint32_t sb = kv_it % NSB;
           ok = mbar_wait_warp(BAR(B_QKRDY + s), ph, abort_flag, p.status, code_hi | PW_QKRDY);
           if (!ok) break;
           tc_fence_after();
@@ -466,6 +467,7 @@ intfa_fwd_pipe_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
             if (j + 1 == t.nsteps) umma_commit(BAR(B_QEMPTY));
           }
           __syncwarp();
+          sb = sb + 1 == NSB ? 0 : sb + 1;
         }
         ++tile_it;
       }
@@ -475,7 +477,7 @@ intfa_fwd_pipe_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
     {
       // ------------------------------------------------------------------ MMA issuer for O_j = P V
       // A warp of its own, so that a Q K^T whose S buffer is free never queues behind the wait for a P tile.
-      uint32_t kv_it = 0, tseq = 0;
+      uint32_t kv_it = 0, tseq = 0, b = 0;                   // b: kv_it mod NPB
       bool ok = true;
       const uint64_t descP0 = make_smem_desc(sP, 16, C::SBO_P, C::SWZ_P);
       const uint64_t descV0 = make_smem_desc(sV, C::V_BOXES > 1 ? G * C::V_ROWB : 16, C::SBO_V, C::SWZ_V);
@@ -486,7 +488,6 @@ intfa_fwd_pipe_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
 #pragma unroll 1
         for (int j = 0; j < t.nsteps; ++j, ++kv_it) {
           const uint32_t s = kv_it % NSV, ph = (kv_it / NSV) & 1;
-          const uint32_t b = kv_it % C::NPB;
           ok = mbar_wait_warp(BAR(B_PVRDY + s), ph, abort_flag, p.status, code_hi | PW_PVRDY);
           if (!ok) break;
           tc_fence_after();
@@ -519,6 +520,7 @@ intfa_fwd_pipe_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
             umma_commit(C::P_TMEM ? BAR(B_QKRDY + (kv_it + NSB) % NSK) : BAR(B_PFREE + b));
           }
           __syncwarp();
+          b = b + 1 == C::NPB ? 0 : b + 1;
         }
       }
     }

@@ -407,6 +407,32 @@ __device__ __forceinline__ void h2_floor_add(uint32_t h2, float addend, uint32_t
       : "r"(h2), "f"(addend));
 }
 
+// The same of the high half alone, as a multiple of 256: 256 * (1.5*2^23 + floor(h)); and of the low half alone.
+__device__ __forceinline__ float h2_floor_hi(uint32_t h2) {
+  float r;
+  asm("{\n"
+      ".reg .b16 lo, hi, k;\n"
+      "mov.b32 {lo, hi}, %1;\n"
+      "mov.b16 k, 0x5C00;\n"
+      "fma.rm.f32.f16 %0, hi, k, %2;\n"
+      "}\n"
+      : "=f"(r)
+      : "r"(h2), "f"(256.f * 12582912.0f));
+  return r;
+}
+__device__ __forceinline__ uint32_t h2_floor_add_lo(uint32_t h2, float addend) {
+  uint32_t r;
+  asm("{\n"
+      ".reg .b16 lo, hi, one;\n"
+      "mov.b32 {lo, hi}, %1;\n"
+      "mov.b16 one, 0x3C00;\n"
+      "fma.rm.f32.f16 %0, lo, one, %2;\n"
+      "}\n"
+      : "=r"(r)
+      : "r"(h2), "f"(addend));
+  return r;
+}
+
 // ---------------------------------------------------------------------------
 // misc
 // ---------------------------------------------------------------------------
