@@ -74,6 +74,11 @@ struct PipeCfg {
   static constexpr int NRS = NSB == 4 ? 8 : 4;                     // row-sum slots: step j's is read at step j+1, when P V j+1 may be out
   static constexpr int P_PER_COL = BYTE_PV ? 4 : 2;                // P_TMEM: elements of P in a TMEM column
   static constexpr int NPB = P_TMEM ? NSB : NGRP;                  // P buffers
+  // Where the accumulator is 256 channels wide, the way round P V -> rescaling -> next P V is the longest one: P V takes the channels
+  // in two halves, and one is rescaled while P V of the other runs (2 x 16 x 4096 at d=256 432 -> 397 us, causal 267 -> 245).
+  // (In two halves of the keys, so that P V of 128-column steps can begin before all of P is there: half-int8 443 -> 441 us, causal
+  // 504 -> 547.)
+  static constexpr int NOH = !FULL && D == 256 ? 2 : 1;
   static constexpr int NPBAR = P_TMEM ? 0 : NGRP;                  // ... and their barriers, where they are in shared memory
   // Who carries the row sum l = l*alpha + rowsum(P)?  Where a KV step is as wide as the head (G >= D) the accumulator
   // warps do, next to the accumulator row: the softmax groups then meet once per step (running max) instead of
@@ -116,7 +121,7 @@ struct PipeCfg {
   static constexpr int MAGIC_BYTES = 4096;
   static constexpr int OFF_TILE = OFF_MAGIC + MAGIC_BYTES;         // [4] TileInfo: the work-item ring
   static constexpr int OFF_BAR = OFF_TILE + 4 * (int)sizeof(TileInfo);
-  static constexpr int NUM_BARS = 14 + NPBAR + 2 * NSK + 2 * NSV + 12 + NSB;
+  static constexpr int NUM_BARS = 14 + NPBAR + 2 * NSK + 2 * NSV + 12 + NSB + (NOH - 1);
   static constexpr int OFF_MISC = OFF_BAR + NUM_BARS * 8;
   static constexpr int SMEM_BYTES = OFF_MISC + 32 + 1024;
   // S buffer b at COL_S + b*G; then O_j (full-int8: the accumulator itself lives in registers) or the fp32
@@ -140,14 +145,16 @@ struct PipeCfg {
   static constexpr uint32_t SBO_P = 8 * G;
   // V rows: boxes of at most 128 bytes of channels
   static constexpr int V_ROWB = D * (BYTE_PV ? 1 : 2) < 128 ? D * (BYTE_PV ? 1 : 2) : 128;
+  static constexpr int PV_K = BYTE_PV ? 32 : 16, PV_STEPS = G / PV_K;     // keys of one P V MMA, and how many it takes
   static constexpr int V_BOXES = D * (BYTE_PV ? 1 : 2) / V_ROWB;
   static constexpr int V_BOXCH = D / V_BOXES;                      // channels of one box
   static constexpr uint64_t SWZ_V = (V_ROWB == 128) ? kSwz128 : (V_ROWB == 64) ? kSwz64 : kSwz32;
   static constexpr uint32_t SBO_V = 8 * V_ROWB;
   static constexpr uint32_t IDESC_QK = make_idesc(2, 1, 1, 0, 0, kBM, G);
   // (kind::f8f6f4: A / B format 1 = e5m2, D format 1 = f32)
-  static constexpr uint32_t IDESC_PV = FULL ? make_idesc(2, 1, 1, 0, 1, kBM, D)
-                                       : F8V ? make_idesc(1, 1, 1, 0, 1, kBM, D) : make_idesc(1, 0, 0, 0, 1, kBM, D);
+  static constexpr int PV_N = D / NOH;                              // channels of one P V MMA
+  static constexpr uint32_t IDESC_PV = FULL ? make_idesc(2, 1, 1, 0, 1, kBM, PV_N)
+                                       : F8V ? make_idesc(1, 1, 1, 0, 1, kBM, PV_N) : make_idesc(1, 0, 0, 0, 1, kBM, PV_N);
   // fp16 x fp16 -> fp32, K = 16: writes the fp32 constant 1.5*2^23 into a whole accumulator tile
   static constexpr uint32_t IDESC_ARM_S = make_idesc(1, 0, 0, 0, 0, kBM, G);
   static constexpr uint32_t IDESC_ARM_O = make_idesc(1, 0, 0, 0, 0, kBM, D);
@@ -179,7 +186,7 @@ intfa_fwd_pipe_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
   constexpr int NGRP = C::NGRP;
   constexpr int B_QFULL = 0;      // TMA: Q tile landed
   constexpr int B_QEMPTY = 1;     // commit: last Q K^T of the work item done
-  constexpr int B_OFULL = 2;      // [NO] commit: O_j = P V in TMEM buffer (step mod NO)
+  constexpr int B_OFULL = 2;      // [NO] commit: O_j = P V in TMEM buffer (step mod NO) ([NOH]: P V of a half of the channels)
   constexpr int B_FIN = 4;        // [2] softmax (4 warps of one group): final (m, l) of the work item published; one
                                   //     barrier per slot, so that a short next work item cannot complete it twice
                                   //     before a slow accumulator warp has waited for the first completion
@@ -203,6 +210,7 @@ intfa_fwd_pipe_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
   constexpr int B_SFULL = B_AFULL + 4;   // [NSB] commit: S = Q K^T in TMEM buffer b; scale loader: the step's K scales in
                                          //     shared memory (the arrival of the warp that wrote them is what lets the
                                          //     softmax warps see them)
+  constexpr int B_OHI = B_SFULL + NSB;   // NOH == 2: accumulator warps (4): the upper half of the row is at step j's running max
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + C::OFF_MISC);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + C::OFF_MISC + 4);
   TileInfo* tile_slot = reinterpret_cast<TileInfo*>(smem + C::OFF_TILE);
@@ -219,7 +227,8 @@ intfa_fwd_pipe_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
       mbar_init(BAR(B_FINFREE + b), 4);
       mbar_init(BAR(B_FIN + b), 4);
     }
-    for (int b = 0; b < NO; ++b) mbar_init(BAR(B_OFULL + b), 1);
+    for (int b = 0; b < (NO > C::NOH ? NO : C::NOH); ++b) mbar_init(BAR(B_OFULL + b), 1);
+    if (C::NOH > 1) mbar_init(BAR(B_OHI), 4);
     for (int s = 0; s < NSK; ++s) {
       mbar_init(BAR(B_QKRDY + s), 1 + SFREE_ARRIVALS);
       mbar_init(BAR(B_KEMPTY + s), 1);
@@ -481,6 +490,15 @@ intfa_fwd_pipe_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
       bool ok = true;
       const uint64_t descP0 = make_smem_desc(sP, 16, C::SBO_P, C::SWZ_P);
       const uint64_t descV0 = make_smem_desc(sV, C::V_BOXES > 1 ? G * C::V_ROWB : 16, C::SBO_V, C::SWZ_V);
+      // P_TMEM: the MMAs of a step (8 TMEM columns of P each) into the accumulator columns from d on; fp16 or e5m2 P and V (MN-major)
+      auto pv_tmem = [&](uint32_t d, uint32_t b, uint64_t vd, uint32_t keep) {
+#pragma unroll
+        for (int kk = 0; kk < C::PV_STEPS; ++kk) {
+          const uint64_t vdk = vd + (uint64_t)(kk * ((C::PV_K * C::V_ROWB) >> 4));
+          if constexpr (F8V) umma_f8_ts(d, tS + b * G + kk * 8, vdk, C::IDESC_PV, kk > 0 ? 1u : keep);
+          else umma_f16_ts(d, tS + b * G + kk * 8, vdk, C::IDESC_PV, kk > 0 ? 1u : keep);
+        }
+      };
 #pragma unroll 1
       while (ok) {
         const TileInfo t = next_tile(tseq);
@@ -493,29 +511,33 @@ intfa_fwd_pipe_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
           tc_fence_after();
           const uint64_t ad0 = descP0 + (uint64_t)(b * (C::P_BYTES >> 4));
           const uint64_t vd0 = descV0 + (uint64_t)(s * (C::V_BYTES >> 4));
+          if constexpr (C::NOH > 1) {
+            // the lower half of the channels
+            if (elect_one()) {
+              pv_tmem(tA, b, vd0, (j > 0 || p.state_in) ? 1u : 0u);
+              umma_commit(BAR(B_OFULL));
+            }
+            __syncwarp();
+            ok = mbar_wait_warp(BAR(B_OHI), kv_it & 1, abort_flag, p.status, code_hi | PW_PVRDY);
+            if (!ok) break;
+            tc_fence_after();
+          }
           if (elect_one()) {
             if constexpr (FULL) {
               const uint32_t tOj = tO + kv_it % NO * D;
               umma_f16(tOj, descArm, descArm, C::IDESC_ARM_O, 0);
 #pragma unroll
               for (int kk = 0; kk < G / 32; ++kk) umma_i8(tOj, ad0 + 2 * kk, vd0 + kk * ((32 * C::V_ROWB) >> 4), C::IDESC_PV, 1);
-            } else if constexpr (F8V) {
-              // e5m2 P x e5m2 V (both one byte, laid out like the int8 tiles), fp32 accumulate straight into the accumulator
-              const uint32_t keep = (j > 0 || p.state_in) ? 1u : 0u;
-#pragma unroll
-              for (int kk = 0; kk < G / 32; ++kk) {
-                if constexpr (C::P_TMEM) umma_f8_ts(tA, tS + b * G + kk * 8, vd0 + kk * ((32 * C::V_ROWB) >> 4), C::IDESC_PV, kk > 0 ? 1u : keep);
-                else umma_f8(tA, ad0 + 2 * kk, vd0 + kk * ((32 * C::V_ROWB) >> 4), C::IDESC_PV, kk > 0 ? 1u : keep);
-              }
+            } else if constexpr (C::P_TMEM) {
+              // straight into the fp32 accumulator; the first P V of a fresh work item overwrites it
+              pv_tmem(tA + (C::NOH - 1) * C::PV_N, b, vd0 + (C::NOH - 1) * (C::V_BOXES / 2 * G * C::V_ROWB >> 4), (j > 0 || p.state_in) ? 1u : 0u);
             } else {
-              // fp16 P (TMEM) x fp16 V (MN-major), fp32 accumulate straight
-              // into the accumulator; the first P V of a fresh work item overwrites it
+              // e5m2 P (shared memory) x e5m2 V: both one byte, laid out like the int8 tiles
               const uint32_t keep = (j > 0 || p.state_in) ? 1u : 0u;
 #pragma unroll
-              for (int kk = 0; kk < G / 16; ++kk)
-                umma_f16_ts(tA, tS + b * G + kk * 8, vd0 + (uint64_t)(kk * ((16 * C::V_ROWB) >> 4)), C::IDESC_PV, kk > 0 ? 1u : keep);
+              for (int kk = 0; kk < G / 32; ++kk) umma_f8(tA, ad0 + 2 * kk, vd0 + kk * ((32 * C::V_ROWB) >> 4), C::IDESC_PV, kk > 0 ? 1u : keep);
             }
-            umma_commit(BAR(B_OFULL + kv_it % NO));
+            umma_commit(BAR(B_OFULL + (C::NOH > 1 ? 1 : kv_it % NO)));
             umma_commit(BAR(B_VEMPTY + s));
             umma_commit(C::P_TMEM ? BAR(B_QKRDY + (kv_it + NSB) % NSK) : BAR(B_PFREE + b));
           }
