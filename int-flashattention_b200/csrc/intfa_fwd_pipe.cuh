@@ -48,9 +48,11 @@ struct PipeCfg {
   // the S buffer's later return than they gain: fp8 V 301 -> 322 us, full-int8 383 -> 388, 64-column steps 714 -> 737.
   static constexpr bool P_TMEM = !BYTE_PV || (F8V && G == 64);
   // Softmax groups of 128 threads.  Three (with 96 registers a thread, 16-column buffers) hide the hand-overs better than two
-  // (152 registers, 32 columns) where P is one byte and a step is 128 wide, and for full-int8 at head dim 64: batch 2, 32/8
-  // heads, 3072 tokens, full-int8 causal 267 -> 240 us, fp8 V causal 116 -> 105 us.  Head dim 256 loses: 216 -> 237 us.
-  static constexpr int NGRP = (!BYTE_PV && G == 128) || (BYTE_PV && G == 128 && D == 128 && DQ == 128) || (FULL && G == 64 && D == 64) ? 3 : 2;
+  // (152 registers, 32 columns) nearly everywhere (two -> three: full-int8 4 x 32 x 8192 4578 -> 4164 us, 2 x 32 x 4096 with 64-column
+  // steps 802 -> 759, at d=64 634 -> 602 and 565 -> 527 with 128-column steps, 2 x 32 x 2048 causal at d=32 145 -> 134; half-int8
+  // 487 -> 450, at d=64 460 -> 405; fp8 V 496 -> 448).  Half-int8 with 64-column steps does not gain (d=256 407 -> 407), full-int8 at
+  // head dim 256 has no room for a third P buffer beside its K tiles.
+  static constexpr int NGRP = (!BYTE_PV && G == 128) || (F8V && G == 128 && D == 128) || (FULL && DQ <= 128) ? 3 : 2;
   static constexpr int THREADS = 256 + 128 * NGRP;
   // Registers: the CTA is launched with LAUNCH_REGS per thread and setmaxnreg only moves registers around
   // INSIDE that allocation -- an increase beyond it would block for ever, hence the static_assert below.
