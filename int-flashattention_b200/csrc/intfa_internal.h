@@ -48,20 +48,28 @@ size_t decode_workspace_bytes(const IntfaFwdParams* a);
 // (programmatic stream serialisation): its setup and the launch itself overlap the other's tail.  Each begins with
 // pdl_wait(), which returns when everything before it on the stream is done and visible, and only then may let the next one
 // begin (pdl_launch()): what a kernel reads ahead of its own wait is therefore older than the kernel before it.
+// `cluster`: CTAs of a cluster (the x dimension of the grid is a multiple of it).
 template <typename K, typename... A>
-inline int launch_kernel(const char* what, K kernel, dim3 grid, int threads, size_t smem, cudaStream_t stream, const A&... args) {
+inline int launch_clusters(const char* what, K kernel, dim3 grid, int cluster, int threads, size_t smem, cudaStream_t stream, const A&... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = dim3(threads);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
-  cudaLaunchAttribute attr = {};
-  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr.val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = &attr;
-  cfg.numAttrs = 1;
+  cudaLaunchAttribute attr[2] = {};
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = (unsigned)cluster;
+  attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = cluster > 1 ? 2 : 1;
   const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, args...);
   return e == cudaSuccess ? INTFA_OK : set_error(INTFA_ERR_CUDA, "%s launch: %s", what, cudaGetErrorString(e));
+}
+template <typename K, typename... A>
+inline int launch_kernel(const char* what, K kernel, dim3 grid, int threads, size_t smem, cudaStream_t stream, const A&... args) {
+  return launch_clusters(what, kernel, grid, 1, threads, smem, stream, args...);
 }
 
 int fwd_dispatch(const IntfaFwdParams* a, cudaStream_t stream);

@@ -12,9 +12,9 @@
 //
 // Each row of D fp16 is read by D/8 lanes with one 128-bit load per lane; the row/column
 // maxima are reduced with warp shuffles.  Per-token: one pass.  V (per-channel or
-// per-(batch,head)): a column-absmax pass, then the quantising pass.  The fused entry (quant_qkv) runs the Q rows,
-// the K rows and the V column-absmax pass as ONE launch (partial maxima per chunk, plain stores) and the V
-// quantising pass as a second.  The stand-alone V entries: partial maxima as well (intfa_quant_v_partial, which the Python
+// per-(batch,head)): one pass where a cluster of CTAs holds a slab in registers (v_slab), else a column-absmax pass, then the
+// quantising pass.  The fused entry (quant_qkv) runs small calls as ONE launch; larger ones take the Q and the K rows first and V
+// second, where V has two passes the column-absmax one with the first launch (partial maxima per chunk, plain stores).  The stand-alone V entries: partial maxima as well (intfa_quant_v_partial, which the Python
 // operators call), or atomicMax into a small array (intfa_quant_v, intfa_v_colmax, intfa_quant_v_static).
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
@@ -249,6 +249,113 @@ __global__ void __launch_bounds__(256) v_colmax_kernel(const __half* __restrict_
   colmax_chunk<D, ATOMIC>(x, sB, sH, sN, colmax, H, N, rows_per_cta, blockIdx.x, blockIdx.y, gridDim.y);
 }
 
+// V of one (batch, head) in one pass: the CTAs of a cluster take its rows in equal chunks, keep them in registers (U loads a
+// thread), exchange their channels' maxima through distributed shared memory and quantise what they hold.  V is read once,
+// there are no partial maxima in memory, and one launch does it.  Bound by memory; `early` (V is older than the kernel before
+// this one on the stream): loads before pdl_wait.
+template <int D, int U>
+__device__ __forceinline__ void v_slab(const __half* __restrict__ x, long long sB, long long sH, long long sN, int8_t* __restrict__ x8,
+                                       float* __restrict__ scale, int per_channel, int H, int N, int rows_per_cta, int bh, int early) {
+  constexpr int LPR = D / 8;
+  constexpr int RPC = 256 / LPR;         // rows that the CTA loads at a time
+  __shared__ float red[8][D];
+  __shared__ float s_max[D];             // the chunk's maxima, read by the other CTAs of the cluster
+  __shared__ float s_scale[D];
+  __shared__ float s_all[8];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int sub = threadIdx.x % LPR;
+  const int b = bh / H, h = bh - b * H;
+  const uint32_t rank = cluster_rank(), ncta = cluster_size();
+  const int r0 = (int)rank * rows_per_cta + threadIdx.x / LPR;
+  const int r_end = min(N, ((int)rank + 1) * rows_per_cta);
+  const __half* base = x + b * sB + h * sH + sub * 8;
+  const uint64_t once = l2_policy_evict_first();
+  if (!early) {
+    pdl_wait();
+    pdl_launch();
+  }
+  uint4 v[U];
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    const int r = r0 + u * RPC;
+    v[u] = r < r_end ? ld_hint(base + r * sN, once) : make_uint4(0, 0, 0, 0);
+  }
+  if (early) {
+    pdl_wait();
+    pdl_launch();
+  }
+  __half2 m[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) m[i] = __float2half2_rn(0.f);
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    const __half2* hv = reinterpret_cast<const __half2*>(&v[u]);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) m[i] = __hmax2(m[i], __habs2(hv[i]));
+  }
+#pragma unroll
+  for (int o = LPR; o < 32; o <<= 1)
+#pragma unroll
+    for (int i = 0; i < 4; ++i) m[i] = __hmax2(m[i], shfl_xor_h2(m[i], o));
+  if (lane < LPR) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      red[warp][sub * 8 + 2 * i] = __low2float(m[i]);
+      red[warp][sub * 8 + 2 * i + 1] = __high2float(m[i]);
+    }
+  }
+  __syncthreads();
+  const int ch = threadIdx.x;
+  if (ch < D) {
+    float a = 0.f;
+#pragma unroll
+    for (int w = 0; w < 8; ++w) a = fmaxf(a, red[w][ch]);
+    s_max[ch] = a;
+  }
+  cluster_arrive();
+  cluster_wait();
+  float a = 0.f;
+  if (ch < D)
+    for (uint32_t c = 0; c < ncta; ++c) a = fmaxf(a, ld_peer(s_max + ch, c));
+  cluster_arrive();                      // (the CTA must not end before its peers have read its maxima: waited for below)
+  if (!per_channel) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) a = fmaxf(a, __shfl_xor_sync(0xffffffffu, a, o));
+    if (lane == 0) s_all[warp] = a;
+    __syncthreads();
+#pragma unroll
+    for (int w = 0; w < 8; ++w) a = fmaxf(a, s_all[w]);
+  }
+  if (ch < D) {
+    const float s = scale_from_amax(a);
+    s_scale[ch] = safe_rcp(s);
+    if (rank == 0) {
+      if (per_channel) scale[(long long)bh * D + ch] = s;
+      else if (ch == 0) scale[bh] = s;
+    }
+  }
+  __syncthreads();
+  uint64_t k[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) k[i] = f2_pack(s_scale[sub * 8 + 2 * i], s_scale[sub * 8 + 2 * i + 1]);
+  int8_t* o = x8 + (long long)bh * N * D + sub * 8;
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    const int r = r0 + u * RPC;
+    if (r < r_end) st_hint(o + (long long)r * D, quant8(v[u], k), once);
+  }
+  cluster_wait();
+}
+// CTAs of a cluster at most (16 hold longer slabs, but wait for one another longer: 128 slabs of 2048 x 128 24.9 -> 27.9 us, 256 of
+// 2048 x 64 22.4 -> 37.4)
+constexpr int kSlabCluster = 8;
+template <int D, int U>
+__global__ void __launch_bounds__(256, U == 16 ? 3 : U == 8 ? 4 : 6) v_slab_kernel(const __half* __restrict__ x, long long sB, long long sH, long long sN,
+                                                     int8_t* __restrict__ x8, float* __restrict__ scale, int per_channel, int H, int N,
+                                                     int rows_per_cta, int early) {
+  v_slab<D, U>(x, sB, sH, sN, x8, scale, per_channel, H, N, rows_per_cta, blockIdx.x / cluster_size(), early);
+}
+
 // The first launch of the fused prologue: one grid over three jobs -- CTAs [0, gq) quantise the rows of Q,
 // [gq, gq+gk) those of K (both per token, contiguous tensors), the rest take one (chunk, batch*head) piece of V each and
 // store its column absmax as a partial result.  Nothing is shared between the jobs, so no ordering is needed.
@@ -257,6 +364,24 @@ struct QkvJob {
   const __half* k; int8_t* k8; float* ks; long long k_rows; int gk;
   const __half* v; long long vB, vH, vN; unsigned int* partial; int Hkv, Nk, rows_per_cta, chunks, BHkv;
 };
+// Small calls: all of it in one launch.  CTAs [0, gv) are the clusters of v_slab, then as above; only where every CTA is resident at
+// once, because v_slab's registers leave room for fewer of the others than their loads need to fill the memory.
+struct SlabJob {
+  int8_t* v8; float* vs; int per_channel, gv;
+};
+template <int D, int U>
+__global__ void __launch_bounds__(256) quant_qkv_slab_kernel(const QkvJob j, const SlabJob s) {
+  const int cta = (int)blockIdx.x - s.gv;
+  if (cta < 0) {
+    v_slab<D, U>(j.v, j.vB, j.vH, j.vN, s.v8, s.vs, s.per_channel, j.Hkv, j.Nk, j.rows_per_cta, blockIdx.x / cluster_size(), 0);
+    return;
+  }
+  pdl_wait();
+  pdl_launch();
+  if (cta < j.gq) pertoken_rows<D, true>(j.q, 0, 0, 0, j.q8, j.qs, 1, 1, j.q_rows, cta, j.gq);
+  else if (cta < j.gq + j.gk) pertoken_rows<D, true>(j.k, 0, 0, 0, j.k8, j.ks, 1, 1, j.k_rows, cta - j.gq, j.gk);
+}
+
 template <int D>
 __global__ void __launch_bounds__(256) quant_qkv_kernel(const QkvJob j) {
   const int cta = blockIdx.x;
@@ -406,6 +531,39 @@ static int v_grid(int BH, int N, int sms, int* rows_per_cta) {
   return chunks;
 }
 
+// V in one pass (v_slab): where the registers of a cluster hold a (batch, head), that is up to 262144/D rows.  rows_per_cta: equal
+// chunks over as many CTAs as have 4 loads a thread to make; U of them rounded up to what is compiled.  Two passes before -> now,
+// quantise V alone: 4 heads of 512 x 64 11.9 -> 7.9 us, 128 x 1024 x 64 10.6 -> 9.1, 256 x 2048 x 64 30.2 -> 22.4, 256 x 4096 x 64
+// 58.9 -> 49.3, 2048 x 64 x 128 20.9 -> 10.1; 128 x 2048 x 128 with nothing in L2 28 -> 25, out of L2 23.6 -> 24.9.
+struct Slab {
+  int cluster = 0, rows_per_cta = 0, U = 0;
+};
+static Slab slab_plan(int N, int D) {
+  Slab s;
+  const int rpc = 256 / (D / 8);                        // rows of one load
+  if (N > kSlabCluster * 16 * rpc) return s;
+  s.cluster = (N + 4 * rpc - 1) / (4 * rpc);
+  if (s.cluster > kSlabCluster) s.cluster = kSlabCluster;
+  s.rows_per_cta = (N + s.cluster - 1) / s.cluster;
+  const int loads = (s.rows_per_cta + rpc - 1) / rpc;
+  s.U = loads <= 4 ? 4 : loads <= 8 ? 8 : 16;
+  return s;
+}
+#define INTFA_U_SWITCH(U, CALL)                       \
+  switch (U) {                                        \
+    case 4: { constexpr int UU = 4; CALL; } break;    \
+    case 8: { constexpr int UU = 8; CALL; } break;    \
+    default: { constexpr int UU = 16; CALL; } break;  \
+  }
+static int v_slab_launch(const Slab& sl, const void* v, const int64_t* st, void* v8, float* scale, int mode, int B, int H, int N, int D,
+                         bool early, cudaStream_t stream) {
+  const int pc = mode == INTFA_VSCALE_PER_CHANNEL;
+  int rc = INTFA_OK;
+  INTFA_D_SWITCH(D, INTFA_U_SWITCH(sl.U, (rc = launch_clusters("v_slab", v_slab_kernel<DD, UU>, dim3(sl.cluster * B * H), sl.cluster, 256, 0, stream,
+                 (const __half*)v, (long long)st[0], (long long)st[1], (long long)st[2], (int8_t*)v8, scale, pc, H, N, sl.rows_per_cta, early ? 1 : 0))))
+  return rc;
+}
+
 int v_colmax(const void* v, const int64_t* st, void* colmax, int B, int H, int N, int D, cudaStream_t stream) {
   const int sms = sm_count_cached();
   if (sms <= 0) return set_error(INTFA_ERR_CUDA, "cannot query SM count");
@@ -466,6 +624,21 @@ int quant_qkv(const void* q, const void* k, const void* v, const int64_t* v_st, 
   j.chunks = 0; j.rows_per_cta = 0; j.vB = j.vH = j.vN = 0;
   int gv = 0;
   if (v) {
+    const Slab sl = slab_plan(Nk, D);
+    if (sl.cluster > 0) {
+      int rc = INTFA_OK;
+      const int slabs = sl.cluster * B * Hkv;
+      if (slabs + j.gq + j.gk <= 2 * sms) {
+        j.vB = v_st[0]; j.vH = v_st[1]; j.vN = v_st[2];
+        j.rows_per_cta = sl.rows_per_cta;
+        const SlabJob s = {(int8_t*)v8, vs, mode == INTFA_VSCALE_PER_CHANNEL, slabs};
+        const int grid = (slabs + j.gq + j.gk + sl.cluster - 1) / sl.cluster * sl.cluster;
+        INTFA_D_SWITCH(D, INTFA_U_SWITCH(sl.U, (rc = launch_clusters("quant_qkv", quant_qkv_slab_kernel<DD, UU>, dim3(grid), sl.cluster, 256, 0, stream, j, s))))
+        return rc;
+      }
+      INTFA_D_SWITCH(D, (rc = launch_kernel("quant_qkv", quant_qkv_kernel<DD>, dim3(j.gq + j.gk), 256, 0, stream, j)))
+      return rc ? rc : v_slab_launch(sl, v, v_st, v8, vs, mode, B, Hkv, Nk, D, true, stream);
+    }
     j.vB = v_st[0]; j.vH = v_st[1]; j.vN = v_st[2];
     j.chunks = v_grid(B * Hkv, Nk, sms, &j.rows_per_cta);
     gv = j.chunks * B * Hkv;
@@ -481,6 +654,8 @@ int quant_v_partial(const void* v, const int64_t* st, void* v8, float* scale, in
                     cudaStream_t stream) {
   const int sms = sm_count_cached();
   if (sms <= 0) return set_error(INTFA_ERR_CUDA, "cannot query SM count");
+  const Slab sl = slab_plan(N, D);
+  if (sl.cluster > 0) return v_slab_launch(sl, v, st, v8, scale, mode, B, H, N, D, false, stream);
   int rows_per_cta;
   const int chunks = v_grid(B * H, N, sms, &rows_per_cta);
   dim3 grid(chunks, B * H);
