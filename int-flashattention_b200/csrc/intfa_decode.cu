@@ -17,13 +17,16 @@
 // the next kernel's lanes want it) and the maximum of each 64 keys; `pv_full_kernel` takes the prefix maximum at its
 // first group, and from there on does what the one-pass kernel does: m' = max(m, groupmax*c), p = exp2(s*c - m'), P8, O_j
 // (with s*c - m' as one fma on masked groups too, where that kernel rounds s*c first).  The final maximum is known too, so that every partial result is scaled to it at once
-// (acc += exp2(m_j - m_final) * O_j) and the splits add up without weights.
+// (acc += exp2(m_j - m_final) * O_j) and the splits add up without weights.  Where the splits of a K/V head fit a cluster of CTAs one
+// kernel does both passes and the sum (`fused_full_kernel`).
 // half-int8: P is fp16, whose rounding is relative: every warp keeps a running maximum of its own and the partial results
 // are combined with their weights (`pv_half_kernel`: scores and P V in one pass over K and V).
 #include <cuda_fp16.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
+
+#include <atomic>
 
 #include "intfa_internal.h"
 #include "intfa_ptx.cuh"
@@ -33,6 +36,7 @@ namespace intfa {
 namespace {
 
 constexpr int kThreads = 128, kWarps = 4;
+constexpr int kMaxCluster = 8;            // CTAs of a cluster that every GPU grants
 constexpr int kMaxLocalUnits = 128;       // 64-key units per CTA of pv_full_kernel (their maxima sit in shared memory)
 constexpr float kMagicF = 12582912.0f;    // 1.5*2^23: added to an int32 below 2^22 as a bit pattern, it reads as fp32 1.5*2^23 + value
 constexpr int kMagicI = 0x4B400000;
@@ -262,28 +266,24 @@ __device__ __forceinline__ void cta_out(const DParams& p, const Unit& u, int spl
   }
 }
 
-// ---------------------------------------------------------------------------------------------------------------
-// full-int8, second pass: P from the kept scores, O = P V.  One warp takes 64 keys at a time (32 in flight ahead of the
-// arithmetic).  Bound by reading V.
-// ---------------------------------------------------------------------------------------------------------------
+// The work of one CTA in the second pass, on `nun` units of 64 keys from group g0 on (upg units a group): mg holds the running maximum
+// (scaled) at the group of each, ends[1] the final maximum; score(key tile of 8, row tile) is what this lane wants of the scores.
+// One warp takes 64 keys at a time, 32 in flight ahead of the arithmetic.
 template <int D, int NT>
-__global__ void __launch_bounds__(kThreads, NT == 1 ? 3 : 2) pv_full_kernel(const DParams p) {
-  constexpr int RT = 8 * NT, VB = D / 8, MT = D / 16;       // VB: bytes (channels) of a key that a lane holds; MT: 16-channel tiles
-  constexpr int W = VB / 4;                                 // ... in words
-  __shared__ __align__(16) float red[kWarps * RT * (D + 4)];
-  __shared__ __align__(16) float mg[kMaxLocalUnits * RT];   // running maximum (scaled) at the group of each 64-key unit of this CTA
-  __shared__ __align__(16) float ends[2][RT];               // prefix before the first group; final maximum
-  __shared__ float ml[RT][2];
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
-  const int units = gridDim.x / p.splits;
-  const Unit u = unit_of(p, blockIdx.x % units);
-  const int split = blockIdx.x / units;
-  const int g0 = split * p.per_split, g1 = min(p.groups, g0 + p.per_split);
-  const int8_t* vb = static_cast<const int8_t*>(p.v) + u.b * p.vB + u.hk * p.vH + g * VB;
-
-  // this lane's 8 keys of a 32-key step: 2t, 2t+1 of each of the four 8-key tiles
+struct PvFull {
+  static constexpr int RT = 8 * NT, VB = D / 8, MT = D / 16;       // VB: bytes (channels) of a key that a lane holds; MT: 16-channel tiles
+  static constexpr int W = VB / 4;                                 // ... in words
+  const DParams& p;
+  const int8_t* vb;
+  const int lane, warp, g, t, g0, upg, nun;
   uint32_t vn[8][W];
-  auto load_v = [&](int key0) {
+  float acc[NT][MT][4], lsum[NT];
+  __device__ __forceinline__ PvFull(const DParams& p, const Unit& u, int g0, int upg, int nun)
+      : p(p), lane(threadIdx.x & 31), warp(threadIdx.x >> 5), g(lane >> 2), t(lane & 3), g0(g0), upg(upg), nun(nun) {
+    vb = static_cast<const int8_t*>(p.v) + u.b * p.vB + u.hk * p.vH + g * VB;
+  }
+  // this lane's 8 keys of a 32-key step: 2t, 2t+1 of each of the four 8-key tiles
+  __device__ __forceinline__ void load_v(int key0) {
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
       const int key = min(key0 + (i >> 1) * 8 + 2 * t + (i & 1), p.nvis - 1);
@@ -296,10 +296,145 @@ __global__ void __launch_bounds__(kThreads, NT == 1 ? 3 : 2) pv_full_kernel(cons
         vn[i][0] = x.x; vn[i][1] = x.y;
       }
     }
-  };
-  // (V is older than the first pass)
+  }
+  __device__ __forceinline__ void load_first() {
+    if (warp < nun) load_v((g0 * upg + warp) * 64);
+  }
+  template <typename Score>
+  __device__ __forceinline__ void run(const float* mg, const float (*ends)[RT], Score score) {
+    float m_fin[NT][2], m_fin_g[NT];
+#pragma unroll
+    for (int n = 0; n < NT; ++n) {
+      lsum[n] = 0.f;
+      m_fin[n][0] = ends[1][n * 8 + 2 * t];
+      m_fin[n][1] = ends[1][n * 8 + 2 * t + 1];
+      m_fin_g[n] = ends[1][n * 8 + g];
+#pragma unroll
+      for (int i = 0; i < MT; ++i) acc[n][i][0] = acc[n][i][1] = acc[n][i][2] = acc[n][i][3] = 0.f;
+    }
+#pragma unroll 1
+    for (int un = warp; un < nun; un += kWarps) {
+      float nm[NT], w_g[NT], rs[NT];
+      int o[NT][MT][4];
+#pragma unroll
+      for (int n = 0; n < NT; ++n) {
+        const float m = mg[un * RT + n * 8 + g];
+        nm[n] = -m;
+        w_g[n] = ex2_approx(m - m_fin_g[n]);
+        rs[n] = 0.f;
+#pragma unroll
+        for (int i = 0; i < MT; ++i) o[n][i][0] = o[n][i][1] = o[n][i][2] = o[n][i][3] = kMagicI;
+      }
+#pragma unroll
+      for (int half = 0; half < 2; ++half) {
+        const int key0 = (g0 * upg + un) * 64 + half * 32;
+        uint32_t vc[8][W];
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+#pragma unroll
+          for (int j = 0; j < W; ++j) vc[i][j] = vn[i][j];
+        float2 s[NT][4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+          for (int n = 0; n < NT; ++n) s[n][i] = score(key0 / 8 + i, n);
+        if (half == 0) load_v(key0 + 32);
+        else if (un + kWarps < nun) load_v(key0 - 32 + kWarps * 64);
+        // P8 of this lane's keys: trunc(fp16(fp16(fp16(p)*127) + 0.5)), as in the 128-row kernel
+        uint32_t b[NT][2];
+#pragma unroll
+        for (int n = 0; n < NT; ++n)
+#pragma unroll
+          for (int q = 0; q < 2; ++q) {
+            const float2 x = s[n][2 * q], y = s[n][2 * q + 1];
+            const float p0 = ex2_approx(fmaf(x.x, p.c, nm[n])), p1 = ex2_approx(fmaf(x.y, p.c, nm[n]));
+            const float p2 = ex2_approx(fmaf(y.x, p.c, nm[n])), p3 = ex2_approx(fmaf(y.y, p.c, nm[n]));
+            rs[n] += (p0 + p1) + (p2 + p3);
+            const __half2 h01 = __floats2half2_rn(p0, p1), h23 = __floats2half2_rn(p2, p3);
+            const uint32_t z01 = h2_fma(*reinterpret_cast<const uint32_t*>(&h01), 0x57F057F0u, 0x38003800u);
+            const uint32_t z23 = h2_fma(*reinterpret_cast<const uint32_t*>(&h23), 0x57F057F0u, 0x38003800u);
+            uint32_t u0, u1, u2, u3;
+            h2_floor_add(z01, kMagicF, u0, u1);
+            h2_floor_add(z23, kMagicF, u2, u3);
+            b[n][q] = __byte_perm(__byte_perm(u0, u1, 0x0040), __byte_perm(u2, u3, 0x0040), 0x5410);
+          }
+        // O^T (channels x rows): the 4 keys of a quad transposed, so that a word holds one channel's 4 keys
+#pragma unroll
+        for (int j = 0; j < W; ++j) {
+          uint32_t chn[4][2];
+#pragma unroll
+          for (int q = 0; q < 2; ++q) {
+            const uint32_t x0 = vc[4 * q][j], x1 = vc[4 * q + 1][j], x2 = vc[4 * q + 2][j], x3 = vc[4 * q + 3][j];
+            const uint32_t a = __byte_perm(x0, x1, 0x5140), c = __byte_perm(x0, x1, 0x7362);
+            const uint32_t d = __byte_perm(x2, x3, 0x5140), e = __byte_perm(x2, x3, 0x7362);
+            chn[0][q] = __byte_perm(a, d, 0x5410);
+            chn[1][q] = __byte_perm(a, d, 0x7632);
+            chn[2][q] = __byte_perm(c, e, 0x5410);
+            chn[3][q] = __byte_perm(c, e, 0x7632);
+          }
+#pragma unroll
+          for (int n = 0; n < NT; ++n) {
+            mma_s8(o[n][2 * j], chn[0][0], chn[1][0], chn[0][1], chn[1][1], b[n][0], b[n][1]);
+            mma_s8(o[n][2 * j + 1], chn[2][0], chn[3][0], chn[2][1], chn[3][1], b[n][0], b[n][1]);
+          }
+        }
+      }
+#pragma unroll
+      for (int n = 0; n < NT; ++n) {
+        lsum[n] = fmaf(w_g[n], rs[n], lsum[n]);
+        const float w0 = ex2_approx(mg[un * RT + n * 8 + 2 * t] - m_fin[n][0]), w1 = ex2_approx(mg[un * RT + n * 8 + 2 * t + 1] - m_fin[n][1]);
+#pragma unroll
+        for (int i = 0; i < MT; ++i) {
+          acc[n][i][0] = fmaf(unmagic(o[n][i][0]), w0, acc[n][i][0]);
+          acc[n][i][1] = fmaf(unmagic(o[n][i][1]), w1, acc[n][i][1]);
+          acc[n][i][2] = fmaf(unmagic(o[n][i][2]), w0, acc[n][i][2]);
+          acc[n][i][3] = fmaf(unmagic(o[n][i][3]), w1, acc[n][i][3]);
+        }
+      }
+    }
+  }
+  // the warps' results into red; the sum of the CTA's l on top of what is in ml (written before a barrier)
+  __device__ __forceinline__ void results(float* red, float (*ml)[2]) {
+#pragma unroll
+    for (int n = 0; n < NT; ++n) {
+      // tile i of the lane: channel g*VB + 2i (entries 0, 1) and + 1 (2, 3) of rows 2t (0, 2) and 2t+1 (1, 3)
+#pragma unroll
+      for (int i = 0; i < MT; ++i) {
+        float* d = red + (warp * RT + n * 8 + 2 * t) * (D + 4) + g * VB + 2 * i;
+        *reinterpret_cast<float2*>(d) = make_float2(acc[n][i][0], acc[n][i][2]);
+        *reinterpret_cast<float2*>(d + D + 4) = make_float2(acc[n][i][1], acc[n][i][3]);
+      }
+      float l = lsum[n];
+      l += __shfl_xor_sync(0xffffffffu, l, 1);
+      l += __shfl_xor_sync(0xffffffffu, l, 2);
+      // (one warp after the other, so that the sum has one order)
+      for (int w = 0; w < kWarps; ++w) {
+        if (w == warp && t == 0) ml[n * 8 + g][1] += l;
+        __syncthreads();
+      }
+    }
+  }
+};
+
+// ---------------------------------------------------------------------------------------------------------------
+// full-int8, second pass: P from the kept scores, O = P V.  Bound by reading V.
+// ---------------------------------------------------------------------------------------------------------------
+template <int D, int NT>
+__global__ void __launch_bounds__(kThreads, NT == 1 ? 3 : 2) pv_full_kernel(const DParams p) {
+  constexpr int RT = 8 * NT;
+  __shared__ __align__(16) float red[kWarps * RT * (D + 4)];
+  __shared__ __align__(16) float mg[kMaxLocalUnits * RT];   // running maximum (scaled) at the group of each 64-key unit of this CTA
+  __shared__ __align__(16) float ends[2][RT];               // prefix before the first group; final maximum
+  __shared__ float ml[RT][2];
+  const int tid = threadIdx.x;
+  const int units = gridDim.x / p.splits;
+  const Unit u = unit_of(p, blockIdx.x % units);
+  const int split = blockIdx.x / units;
+  const int g0 = split * p.per_split, g1 = min(p.groups, g0 + p.per_split);
   const int upg = p.G / 64, nun = (g1 - g0) * upg;          // 64-key units of this CTA
-  if (warp < nun) load_v((g0 * upg + warp) * 64);
+  PvFull<D, NT> pv(p, u, g0, upg, nun);
+  // (V is older than the first pass)
+  pv.load_first();
   pdl_wait();
   pdl_launch();
 
@@ -345,123 +480,169 @@ __global__ void __launch_bounds__(kThreads, NT == 1 ? 3 : 2) pv_full_kernel(cons
     __syncthreads();
   }
 
-  const float2* sc = reinterpret_cast<const float2*>(p.scores) + ((long long)u.id * p.groups * (p.G / 8) * NT) * 32 + lane;
-  float acc[NT][MT][4], lsum[NT];
-  float m_fin[NT][2], m_fin_g[NT];
-#pragma unroll
-  for (int n = 0; n < NT; ++n) {
-    lsum[n] = 0.f;
-    m_fin[n][0] = ends[1][n * 8 + 2 * t];
-    m_fin[n][1] = ends[1][n * 8 + 2 * t + 1];
-    m_fin_g[n] = ends[1][n * 8 + g];
-#pragma unroll
-    for (int i = 0; i < MT; ++i) acc[n][i][0] = acc[n][i][1] = acc[n][i][2] = acc[n][i][3] = 0.f;
-  }
-#pragma unroll 1
-  for (int un = warp; un < nun; un += kWarps) {
-    float nm[NT], w_g[NT], rs[NT];
-    int o[NT][MT][4];
-#pragma unroll
-    for (int n = 0; n < NT; ++n) {
-      const float m = mg[un * RT + n * 8 + g];
-      nm[n] = -m;
-      w_g[n] = ex2_approx(m - m_fin_g[n]);
-      rs[n] = 0.f;
-#pragma unroll
-      for (int i = 0; i < MT; ++i) o[n][i][0] = o[n][i][1] = o[n][i][2] = o[n][i][3] = kMagicI;
-    }
-#pragma unroll
-    for (int half = 0; half < 2; ++half) {
-      const int key0 = (g0 * upg + un) * 64 + half * 32;
-      uint32_t vc[8][W];
-#pragma unroll
-      for (int i = 0; i < 8; ++i)
-#pragma unroll
-        for (int j = 0; j < W; ++j) vc[i][j] = vn[i][j];
-      float2 s[NT][4];
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int n = 0; n < NT; ++n) s[n][i] = sc[((key0 / 8 + i) * NT + n) * 32];
-      if (half == 0) load_v(key0 + 32);
-      else if (un + kWarps < nun) load_v(key0 - 32 + kWarps * 64);
-      // P8 of this lane's keys: trunc(fp16(fp16(fp16(p)*127) + 0.5)), as in the 128-row kernel
-      uint32_t b[NT][2];
-#pragma unroll
-      for (int n = 0; n < NT; ++n)
-#pragma unroll
-        for (int q = 0; q < 2; ++q) {
-          const float2 x = s[n][2 * q], y = s[n][2 * q + 1];
-          const float p0 = ex2_approx(fmaf(x.x, p.c, nm[n])), p1 = ex2_approx(fmaf(x.y, p.c, nm[n]));
-          const float p2 = ex2_approx(fmaf(y.x, p.c, nm[n])), p3 = ex2_approx(fmaf(y.y, p.c, nm[n]));
-          rs[n] += (p0 + p1) + (p2 + p3);
-          const __half2 h01 = __floats2half2_rn(p0, p1), h23 = __floats2half2_rn(p2, p3);
-          const uint32_t z01 = h2_fma(*reinterpret_cast<const uint32_t*>(&h01), 0x57F057F0u, 0x38003800u);
-          const uint32_t z23 = h2_fma(*reinterpret_cast<const uint32_t*>(&h23), 0x57F057F0u, 0x38003800u);
-          uint32_t u0, u1, u2, u3;
-          h2_floor_add(z01, kMagicF, u0, u1);
-          h2_floor_add(z23, kMagicF, u2, u3);
-          b[n][q] = __byte_perm(__byte_perm(u0, u1, 0x0040), __byte_perm(u2, u3, 0x0040), 0x5410);
-        }
-      // O^T (channels x rows): the 4 keys of a quad transposed, so that a word holds one channel's 4 keys
-#pragma unroll
-      for (int j = 0; j < W; ++j) {
-        uint32_t chn[4][2];
-#pragma unroll
-        for (int q = 0; q < 2; ++q) {
-          const uint32_t x0 = vc[4 * q][j], x1 = vc[4 * q + 1][j], x2 = vc[4 * q + 2][j], x3 = vc[4 * q + 3][j];
-          const uint32_t a = __byte_perm(x0, x1, 0x5140), c = __byte_perm(x0, x1, 0x7362);
-          const uint32_t d = __byte_perm(x2, x3, 0x5140), e = __byte_perm(x2, x3, 0x7362);
-          chn[0][q] = __byte_perm(a, d, 0x5410);
-          chn[1][q] = __byte_perm(a, d, 0x7632);
-          chn[2][q] = __byte_perm(c, e, 0x5410);
-          chn[3][q] = __byte_perm(c, e, 0x7632);
-        }
-#pragma unroll
-        for (int n = 0; n < NT; ++n) {
-          mma_s8(o[n][2 * j], chn[0][0], chn[1][0], chn[0][1], chn[1][1], b[n][0], b[n][1]);
-          mma_s8(o[n][2 * j + 1], chn[2][0], chn[3][0], chn[2][1], chn[3][1], b[n][0], b[n][1]);
-        }
-      }
-    }
-#pragma unroll
-    for (int n = 0; n < NT; ++n) {
-      lsum[n] = fmaf(w_g[n], rs[n], lsum[n]);
-      const float w0 = ex2_approx(mg[un * RT + n * 8 + 2 * t] - m_fin[n][0]), w1 = ex2_approx(mg[un * RT + n * 8 + 2 * t + 1] - m_fin[n][1]);
-#pragma unroll
-      for (int i = 0; i < MT; ++i) {
-        acc[n][i][0] = fmaf(unmagic(o[n][i][0]), w0, acc[n][i][0]);
-        acc[n][i][1] = fmaf(unmagic(o[n][i][1]), w1, acc[n][i][1]);
-        acc[n][i][2] = fmaf(unmagic(o[n][i][2]), w0, acc[n][i][2]);
-        acc[n][i][3] = fmaf(unmagic(o[n][i][3]), w1, acc[n][i][3]);
-      }
-    }
-  }
-  // ---- the warps' results
+  const float2* sc = reinterpret_cast<const float2*>(p.scores) + ((long long)u.id * p.groups * (p.G / 8) * NT) * 32 + (tid & 31);
+  pv.run(mg, ends, [&](int kt, int n) { return sc[(kt * NT + n) * 32]; });
   if (tid < RT) {
     ml[tid][0] = ends[1][tid];
     ml[tid][1] = 0.f;
   }
   __syncthreads();
+  pv.results(red, ml);
+  cta_out<true, D, NT>(p, u, split, red, ml);
+}
+
+// ---------------------------------------------------------------------------------------------------------------
+// full-int8, both passes in one kernel: a unit's splits are a cluster.  Each CTA computes the scores of its keys and keeps them in
+// shared memory; the CTAs exchange their maxima, which gives each the running maximum before its first key and the final one, and then
+// their results, of which every CTA adds up and writes some rows -- both through distributed shared memory.  The scores make no way
+// through L2 (a quarter of the bytes of K at 4 rows a head), there is no scratch, and one launch instead of three.  Bound by reading K
+// and V, 12 warps an SM (make_plan says what it gives and where).
+// ---------------------------------------------------------------------------------------------------------------
+template <int D, int NT>
+struct FusedCfg {
+  static constexpr int RT = 8 * NT;
+  // shared memory of one CTA for scores, so that three CTAs (16 rows: two) fit an SM, as the launch bounds have it
+  static constexpr int MAX_SCORES = NT == 1 ? 66 << 10 : 100 << 10;
+  static constexpr int RED_BYTES = kWarps * RT * (D + 4) * 4;
+  static int score_bytes(int keys) { return keys * NT * 32; }
+};
+template <int D, int NT>
+__global__ void __launch_bounds__(kThreads, NT == 1 ? 3 : 2) fused_full_kernel(const DParams p) {
+  constexpr int RT = 8 * NT, CH = D / 64;
+  extern __shared__ __align__(16) uint8_t dyn[];
+  __shared__ __align__(16) float mg[kMaxLocalUnits * RT];
+  __shared__ __align__(16) float ends[2][RT];
+  __shared__ float cmax[RT];                                // this CTA's maximum (scaled), for its peers
+  __shared__ float ml[RT][2];
+  float2* sc = reinterpret_cast<float2*>(dyn);              // [key tile of 8][NT][32 lanes]; afterwards the results
+  float* red = reinterpret_cast<float*>(dyn);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
+  const uint32_t rank = cluster_rank();
+  const Unit u = unit_of(p, blockIdx.x / p.splits);
+  const int g0 = (int)rank * p.per_split, g1 = min(p.groups, g0 + p.per_split);
+  const int upg = p.G / 64, nun = (g1 - g0) * upg;
+  pdl_wait();
+  pdl_launch();
+  {
+    QRows<D, NT> q;
+    q.load(p, u, g, t);
+    const int8_t* kb = p.k + u.b * p.kB + u.hk * p.kH + t * 16;
+    const long long ksb = u.b * p.ksB + u.hk * p.ksH;
+    const int kf16 = p.scale_f16 & INTFA_SCALE_F16_K;
+    // 64 keys in two halves, one loaded while the other is computed
+    struct Half {
+      uint4 kw[4][CH];
+      float k0[4], k1[4];
+    } a, b;
+    auto load_k = [&](int kt, Half& x) {
 #pragma unroll
-  for (int n = 0; n < NT; ++n) {
-    // tile i of the lane: channel g*VB + 2i (entries 0, 1) and + 1 (2, 3) of rows 2t (0, 2) and 2t+1 (1, 3)
+      for (int i = 0; i < 4; ++i) {
+        const int8_t* row = kb + (long long)min((kt + i) * 8 + g, p.nvis - 1) * p.kN;
 #pragma unroll
-    for (int i = 0; i < MT; ++i) {
-      float* d = red + (warp * RT + n * 8 + 2 * t) * (D + 4) + g * VB + 2 * i;
-      *reinterpret_cast<float2*>(d) = make_float2(acc[n][i][0], acc[n][i][2]);
-      *reinterpret_cast<float2*>(d + D + 4) = make_float2(acc[n][i][1], acc[n][i][3]);
-    }
-    float l = lsum[n];
-    l += __shfl_xor_sync(0xffffffffu, l, 1);
-    l += __shfl_xor_sync(0xffffffffu, l, 2);
-    // (one warp after the other, so that the sum has one order)
-    for (int w = 0; w < kWarps; ++w) {
-      if (w == warp && t == 0) ml[n * 8 + g][1] += l;
-      __syncthreads();
+        for (int c = 0; c < CH; ++c) x.kw[i][c] = ld16(row + c * 64);
+        const int key = (kt + i) * 8 + 2 * t;
+        x.k0[i] = scale_at(p.ks, ksb + min(key, p.nvis - 1), kf16);
+        x.k1[i] = scale_at(p.ks, ksb + min(key + 1, p.nvis - 1), kf16);
+      }
+    };
+    const int kt0 = g0 * upg * 8;
+    float mx[NT];
+    auto scores = [&](int kt, const Half& x) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        int d[4];
+        qk_tile<D, NT>(q, x.kw[i], d);
+        const int key = (kt0 + kt + i) * 8 + 2 * t;
+#pragma unroll
+        for (int hr = 0; hr < NT; ++hr) {
+          float2 s;
+          s.x = key <= q.last[hr] ? unmagic(d[2 * hr]) * q.s[hr] * x.k0[i] : -INFINITY;
+          s.y = key + 1 <= q.last[hr] ? unmagic(d[2 * hr + 1]) * q.s[hr] * x.k1[i] : -INFINITY;
+          mx[hr] = max3(mx[hr], s.x, s.y);
+          sc[((kt + i) * NT + hr) * 32 + lane] = s;
+        }
+      }
+    };
+    if (warp < nun) load_k(kt0 + warp * 8, a);
+#pragma unroll 1
+    for (int un = warp; un < nun; un += kWarps) {
+#pragma unroll
+      for (int i = 0; i < NT; ++i) mx[i] = -INFINITY;
+      load_k(kt0 + un * 8 + 4, b);
+      scores(un * 8, a);
+      if (un + kWarps < nun) load_k(kt0 + (un + kWarps) * 8, a);
+      scores(un * 8 + 4, b);
+#pragma unroll
+      for (int hr = 0; hr < NT; ++hr) {
+        mx[hr] = fmaxf(mx[hr], __shfl_xor_sync(0xffffffffu, mx[hr], 1));
+        mx[hr] = fmaxf(mx[hr], __shfl_xor_sync(0xffffffffu, mx[hr], 2));
+        if (t == 0) mg[un * RT + g + 8 * hr] = mx[hr];
+      }
     }
   }
-  cta_out<true, D, NT>(p, u, split, red, ml);
+  PvFull<D, NT> pv(p, u, g0, upg, nun);
+  pv.load_first();
+  __syncthreads();
+  if (tid < RT) {
+    float m = -INFINITY;
+    for (int i = 0; i < nun; i += upg) {
+      float x = mg[i * RT + tid];
+      if (upg == 2) x = fmaxf(x, mg[(i + 1) * RT + tid]);
+      m = fmaxf(m, x * p.c);
+      mg[i * RT + tid] = m;
+      if (upg == 2) mg[(i + 1) * RT + tid] = m;
+    }
+    cmax[tid] = m;
+  }
+  cluster_arrive();
+  cluster_wait();
+  if (tid < RT) {
+    float pre = -INFINITY, all = -INFINITY;
+    for (uint32_t c = 0; c < (uint32_t)p.splits; ++c) {
+      const float x = ld_peer(&cmax[tid], c);
+      all = fmaxf(all, x);
+      if (c < rank) pre = fmaxf(pre, x);
+    }
+    ends[0][tid] = pre;
+    ends[1][tid] = all;
+    ml[tid][0] = all;
+    ml[tid][1] = 0.f;
+  }
+  __syncthreads();
+  for (int i = tid; i < nun * RT; i += kThreads) mg[i] = fmaxf(mg[i], ends[0][i % RT]);
+  __syncthreads();
+  const int kt0 = g0 * upg * 8;
+  pv.run(mg, ends, [&](int kt, int n) { return sc[((kt - kt0) * NT + n) * 32 + lane]; });
+  __syncthreads();                                          // (the scores are done with)
+  pv.results(red, ml);
+#pragma unroll
+  for (int e = tid; e < RT * D / 4; e += kThreads) {
+    float4* x = reinterpret_cast<float4*>(red + e / (D / 4) * (D + 4) + e % (D / 4) * 4);
+    float4 a = x[0];
+#pragma unroll
+    for (int w = 1; w < kWarps; ++w) {
+      const float4 y = x[w * RT * (D + 4) / 4];
+      a.x += y.x; a.y += y.y; a.z += y.z; a.w += y.w;
+    }
+    x[0] = a;
+  }
+  cluster_arrive();
+  cluster_wait();
+  for (int e = tid; e < RT * D / 4; e += kThreads) {
+    const int r = e / (D / 4), ch = e % (D / 4) * 4, row = u.tile * RT + r;
+    if (r % p.splits != (int)rank || row >= p.R) continue;
+    float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
+    float l = 0.f;
+    for (uint32_t c = 0; c < (uint32_t)p.splits; ++c) {
+      const float4 y = ld_peer4(red + r * (D + 4) + ch, c);
+      a.x += y.x; a.y += y.y; a.z += y.z; a.w += y.w;
+      l += ld_peer(&ml[r][1], c);
+    }
+    finish_row4<true>(p, u, row, ch, a, l);
+    if (ch == 0) store_lse(p, u, row, ml[r][0], l);
+  }
+  cluster_arrive();                                         // (no CTA ends while a peer reads from it)
+  cluster_wait();
 }
 
 // ---------------------------------------------------------------------------------------------------------------
@@ -753,7 +934,7 @@ __global__ void __launch_bounds__(kCombineThreads) combine_many_kernel(const DPa
 // host side
 // ---------------------------------------------------------------------------------------------------------------
 struct Plan {
-  bool use = false, full = false;
+  bool use = false, full = false, fused = false;           // fused: one kernel, the splits of a unit are a cluster
   int NT = 1, tiles = 1, units = 0, slice = 0, nvis = 0, groups = 0, splits = 1, per_split = 1, score_splits = 1;
   size_t off_gmax = 0, off_part = 0, off_ml = 0, bytes = 0;
 };
@@ -860,12 +1041,41 @@ Plan make_plan(const IntfaFwdParams* a, int sms) {
   if (pl.score_splits > score_cap) pl.score_splits = score_cap;
   if ((long long)pl.slice * pl.splits > 0x7fffffffLL || (long long)pl.slice * pl.score_splits > 0x7fffffffLL) return pl;
   if (!faster_than_tiles(a, pl, wave, sms)) return pl;
+  // One kernel (fused_full_kernel) where the splits of a unit make a cluster whose CTAs hold their scores, if need be more of them than
+  // fill one wave.  No scratch to speak of, so nothing is cut into slices.  Only where the CTAs fit one wave or fill several well
+  // (three kernels -> one, 8 K/V heads of 128 channels, one row of 32 heads: 16 x 4097 keys 34.8 -> 31.7 us, 8 x 2048 16.6 -> 15.3, 1 x
+  // 4096 12.1 -> 9.9, 64 x 4097 136 -> 115; 512 CTAs on 444 places 46 -> 50, clusters of 5 in 4.3 waves 220 -> 267), and with tiles of
+  // 16 rows, which leave 8 warps an SM to read with, where a CTA has the fewest keys (2 x 2048 keys, 8 rows a head 15.0 -> 14.0; 1 500
+  // keys a CTA 34.8 -> 37.2).
+  if (pl.full) {
+    const int max_keys = (pl.NT == 1 ? FusedCfg<128, 1>::MAX_SCORES : FusedCfg<128, 2>::MAX_SCORES) / (pl.NT * 32);
+    int n = wave / (int)units < 1 ? 1 : wave / (int)units;
+    per = (items + n - 1) / n;
+    if (per < per_min) per = per_min;
+    if (per > max_keys / a->G) per = max_keys / a->G;
+    n = (items + per - 1) / per;
+    per = (items + n - 1) / n;
+    const long long ctas = units * n, waves_up = (ctas + wave - 1) / wave;
+    const bool fits = waves_up == 1 || (n <= 3 && ctas * 5 >= waves_up * wave * 4);
+    if (n <= kMaxCluster && (pl.NT == 1 ? fits : waves_up == 1 && per <= per_min)) {
+      pl.fused = true;
+      pl.per_split = per;
+      pl.splits = (items + per - 1) / per;
+      pl.slice = pl.units;
+    }
+  }
   size_t used = 0;
   auto take = [&](size_t bytes) {
     const size_t r = used;
     used += (bytes + 255) / 256 * 256;
     return r;
   };
+  if (pl.fused) {
+    take(1);                    // (none is used; but a call that brings no scratch at all runs on 128-row tiles, as ever)
+    pl.bytes = used;
+    pl.use = true;
+    return pl;
+  }
   if (pl.full) {
     take(pl.slice * per_unit_scores);                                      // scores, at 0
     pl.off_gmax = take(pl.slice * per_unit_max);
@@ -879,6 +1089,21 @@ Plan make_plan(const IntfaFwdParams* a, int sms) {
   return pl;
 }
 
+template <int D, int NT>
+int run_fused(const Plan& pl, const DParams& p, cudaStream_t stream) {
+  using F = FusedCfg<D, NT>;
+  static std::atomic<bool> attr_done[64];
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return set_error(INTFA_ERR_CUDA, "cannot query the current device");
+  if (!attr_done[dev].load(std::memory_order_acquire)) {
+    const cudaError_t e = cudaFuncSetAttribute(fused_full_kernel<D, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, F::MAX_SCORES);
+    if (e != cudaSuccess) return set_error(INTFA_ERR_CUDA, "cudaFuncSetAttribute: %s", cudaGetErrorString(e));
+    attr_done[dev].store(true, std::memory_order_release);
+  }
+  int smem = F::score_bytes(pl.per_split * p.G);
+  if (smem < F::RED_BYTES) smem = F::RED_BYTES;
+  return launch_clusters("decode", fused_full_kernel<D, NT>, pl.units * pl.splits, pl.splits, kThreads, smem, stream, p);
+}
 template <int D, int NT>
 int run_slice(const Plan& pl, int units, const DParams& p, cudaStream_t stream) {
   int rc;
@@ -900,6 +1125,10 @@ int run_slice(const Plan& pl, int units, const DParams& p, cudaStream_t stream) 
 // (Slices share scratch: each kernel waits for the one before it on the stream before it writes any.)
 template <int D, int NT>
 int run(const Plan& pl, DParams p, cudaStream_t stream) {
+  if (pl.fused) {
+    p.unit0 = 0;
+    return run_fused<D, NT>(pl, p, stream);
+  }
   for (p.unit0 = 0; p.unit0 < pl.units; p.unit0 += pl.slice)
     if (const int rc = run_slice<D, NT>(pl, pl.units - p.unit0 < pl.slice ? pl.units - p.unit0 : pl.slice, p, stream)) return rc;
   return INTFA_OK;
