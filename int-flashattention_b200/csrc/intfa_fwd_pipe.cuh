@@ -96,12 +96,18 @@ struct PipeCfg {
   // code costs the steps that need no mask more (instruction cache) than it gives (2 x 16 x 4096 at d=32: 573 -> 631).
   __host__ __device__ static constexpr bool band_fast(bool ragged) { return G == 128 || D == 256 || (G == 32 && ragged); }
   // instructions of never-executed filler between the softmax passes (see intfa_fwd_pipe_softmax.inc), the best of a sweep in
-  // steps of 1 KB for each kind of instantiation (`ragged`: masks partial tiles; `steady`: see the kernel).  Between the best
-  // and the worst of a sweep lie 1 to 2 % non-causal, 5 to 15 % causal.
+  // steps of 1 KB for each kind of instantiation (`ragged`: masks partial tiles; `steady`: see the kernel).  With three groups of
+  // 128-column steps the sweep changes 1 to 3 % (steady 4157 to 4189 us but for 4361 at 256; causal 315 to 338); with 64-column steps and
+  // at head dim 256 it changes up to 20 % (half-int8 causal at d=128 406 to 520 us, at d=256 245 to 287).
   __host__ __device__ static constexpr int code_filler_of(bool ragged, bool steady) {
-    if (P_TMEM) return G == 128 ? (ragged ? 0 : 192) : D == 256 ? (ragged ? 384 : 0) : D == 128 ? (ragged ? 256 : 128) : ragged ? 128 : 256;
-    return NGRP == 3 ? (!FULL ? 192 : (ragged && G == 128) ? 64 : steady ? 128 : 256)
-         : ragged ? (G == 32 ? 128 : FULL && G == 128 && D <= 64 ? 384 : 256) : G == 128 ? (!FULL ? 320 : DQ == 256 ? 448 : 64) : D == 32 ? 256 : 320;
+    if (P_TMEM) {
+      if (G == 128) return ragged || D == 128 ? 64 : 192;
+      return D == 256 ? (ragged ? 384 : 0) : !ragged ? 384 : D == 128 ? 256 : 128;
+    }
+    if (F8V) return 192;
+    if (DQ == 256) return ragged ? 384 : 0;
+    if (ragged) return G == 32 ? 384 : G == 128 ? 256 : D == 128 ? 0 : 128;
+    return G < 128 ? 256 : steady ? 128 : 64;
   }
   static constexpr bool MORE_SOFTMAX_REGS = !FULL || G == 128;
   static constexpr int SOFTMAX_REGS = NGRP == 3 ? (FULL ? 96 : 112) : MORE_SOFTMAX_REGS ? 152 : 136;
