@@ -163,9 +163,9 @@ int intfa_quant_v(const void* v, const int64_t v_stride[3],
                   void* workspace, size_t workspace_bytes, void* stream);
 
 /*
- * intfa_quant_v in two launches and nothing to clear: the first takes the column absmax of v chunk by chunk into
- * `workspace` (intfa_quant_v_partial_workspace_bytes() bytes, contents irrelevant), the second quantises.  Bit-identical
- * to intfa_quant_v, which needs less scratch but clears it with a memset.
+ * intfa_quant_v with nothing to clear: in one launch where a cluster of CTAs holds a (batch, head) of v, else in two, the first of
+ * which takes the column absmax of v chunk by chunk into `workspace` (intfa_quant_v_partial_workspace_bytes() bytes, contents
+ * irrelevant).  Bit-identical to intfa_quant_v, which needs less scratch but clears it with a memset.
  */
 size_t intfa_quant_v_partial_workspace_bytes(int32_t B, int32_t H, int32_t N, int32_t D);
 int intfa_quant_v_partial(const void* v, const int64_t v_stride[3],
@@ -187,10 +187,9 @@ int intfa_v_quant_from_colmax(const void* v, const int64_t v_stride[3], const vo
                               int32_t B, int32_t H, int32_t N, int32_t D, void* stream);
 
 /*
- * The whole quantisation prologue of one attention call in TWO launches and no memset: the first quantises the rows
- * of q and of k per token (as intfa_quant_pertoken) and, in the same grid, takes the column absmax of v chunk by
- * chunk into `workspace` (partial maxima, plain stores -- nothing to clear); the second quantises v (as
- * intfa_quant_v).  Results are bit-identical to the separate entry points.
+ * The whole quantisation prologue of one attention call in one or two launches and no memset: the rows of q and of k per
+ * token (as intfa_quant_pertoken), v as intfa_quant_v_partial does; its absmax pass, where it has one, runs in the grid of q
+ * and k.  Results are bit-identical to the separate entry points.
  * Replaces: quant_pertoken(q), quant_pertoken(k), quant_pertensor(v) as benchmark.py:158-160 calls them in a row.
  * q [B,H,Nq,D] and k [B,H_kv,Nk,D]: fp16, CONTIGUOUS; v [B,H_kv,Nk,D]: fp16 with element strides for (B,H,N), or
  * NULL (half-int8: V stays fp16) -- then v8, v_scale, workspace are not used.  `workspace`: device scratch of
