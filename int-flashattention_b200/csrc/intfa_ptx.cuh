@@ -57,34 +57,38 @@ __device__ __forceinline__ uint32_t mbar_try_wait(uint32_t bar, uint32_t parity)
 
 // (The slow path is small: there is one copy of it at every wait, and the instruction cache has to hold the loops of all
 // warp roles at once.)
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag, int* status, int code) {
-  if (mbar_try_wait(bar, parity)) return true;
+// Made by a whole converged warp, with one verdict for all its lanes: the votes are inside the loop, so that its exits are uniform
+// for the compiler.
+__device__ __forceinline__ bool mbar_wait2_warp(uint32_t bar0, uint32_t parity0, int code0, uint32_t bar1, uint32_t parity1, int code1,
+                                                volatile int* abort_flag, int* status) {
+  // (two barriers at once: where both phases are complete already, the two looks cost one latency)
+  auto look = [&]() {
+    const uint32_t a = mbar_try_wait(bar0, parity0), b = mbar_try_wait(bar1, parity1);
+    return a & b;
+  };
+  if (__all_sync(0xffffffffu, look())) return true;
   const uint32_t t0 = (uint32_t)clock();
 #pragma unroll 1
-  while (!mbar_try_wait(bar, parity)) {
+  while (!__all_sync(0xffffffffu, look())) {
+    if ((uint32_t)clock() - t0 > (uint32_t)abort_flag[1]) {
+      *abort_flag = 1;
+      if (status) atomicCAS(status, 0, mbar_try_wait(bar0, parity0) ? code1 : code0);
+    }
+    if (__any_sync(0xffffffffu, *abort_flag)) return false;
+  }
+  return true;
+}
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile int* abort_flag, int* status, int code) {
+  if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+  const uint32_t t0 = (uint32_t)clock();
+#pragma unroll 1
+  while (!__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) {
     if ((uint32_t)clock() - t0 > (uint32_t)abort_flag[1]) {
       *abort_flag = 1;
       if (status) atomicCAS(status, 0, code);
     }
-    if (*abort_flag) return false;
+    if (__any_sync(0xffffffffu, *abort_flag)) return false;
   }
-  return true;
-}
-
-// The same wait made by a whole converged warp, with one verdict for all its lanes.
-__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile int* abort_flag,
-                                               int* status, int code) {
-  return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, status, code));
-}
-
-// Two barriers at once: where both phases are complete already, the two looks cost one latency.
-__device__ __forceinline__ bool mbar_wait2_warp(uint32_t bar0, uint32_t parity0, int code0, uint32_t bar1, uint32_t parity1, int code1,
-                                                volatile int* abort_flag, int* status) {
-  const uint32_t a = mbar_try_wait(bar0, parity0), b = mbar_try_wait(bar1, parity1);
-  if (__all_sync(0xffffffffu, a & b)) return true;
-#pragma unroll 1
-  for (int w = 0; w < 2; ++w)
-    if (!mbar_wait_warp(w ? bar1 : bar0, w ? parity1 : parity0, abort_flag, status, w ? code1 : code0)) return false;
   return true;
 }
 
