@@ -97,6 +97,11 @@ __device__ __forceinline__ TileInfo decode_tile(const KParams& p, int tile, int 
 // KV tile visited at step j of a work item with n steps: ascending, or last tile first
 __device__ __forceinline__ int kv_tile_of_step(const KParams& p, int j, int n) { return p.kv_desc ? n - 1 - j : j; }
 
+// How full-int8 rounds P: trunc(fp16(fp16(fp16(p)*127) + 0.5)) as the Triton ops, or fp32 p*127 to nearest even as the CUDA path.
+// P_TRITON_WRAP: the former where p may exceed 1.  The running max is that of s times sm_scale, as in the reference, so with sm_scale
+// below zero it is not that of s*sm_scale, and the bytes of P wrap, each by itself.
+enum PRound { P_TRITON, P_RNE, P_TRITON_WRAP };
+
 template <bool B>
 struct Const {
   static constexpr bool value = B;
@@ -182,7 +187,7 @@ static constexpr CUtensorMapSwizzle swizzle_of_row_bytes(int bytes) {
 
 // One CTA per SM.  The tensor maps describe the tensors with their own head dim (a->D); the boxes are as wide as the
 // kernel's tiles, so at head dim 16 the upper half of every 32-wide box lies outside the tensor and arrives as zeros.
-template <int D, int G, bool FULL, bool PRNE, bool RAGGED, int DQ = D, bool F8V = false, bool STEADY = false>
+template <int D, int G, bool FULL, int PROUND, bool RAGGED, int DQ = D, bool F8V = false, bool STEADY = false>
 static int launch_pipe(const IntfaFwdParams* a, const KParams& kp, cudaStream_t stream) {
   using C = PipeCfg<D, G, FULL, DQ, F8V>;
   static_assert(C::SMEM_BYTES <= 227 * 1024, "shared memory");
@@ -193,7 +198,7 @@ static int launch_pipe(const IntfaFwdParams* a, const KParams& kp, cudaStream_t 
   if ((rc = make_tmap(&tmQ, a->q, 1, a->q_stride, a->B, a->H, a->Nq, hd, C::QK_ROWB, kBM, swzQK))) return rc;
   if ((rc = make_tmap(&tmK, a->k, 1, a->k_stride, a->B, kv_heads(a), a->Nk, hd, C::QK_ROWB, G, swzQK))) return rc;
   if ((rc = make_tmap(&tmV, a->v, C::BYTE_PV ? 1 : 2, a->v_stride, a->B, kv_heads(a), a->Nk, hd, C::V_BOXCH, G, swzV))) return rc;
-  auto kern = intfa_fwd_pipe_kernel<D, G, FULL, PRNE, RAGGED, DQ, F8V, STEADY>;
+  auto kern = intfa_fwd_pipe_kernel<D, G, FULL, PROUND, RAGGED, DQ, F8V, STEADY>;
   static std::atomic<bool> attr_done[64];     // per instantiation and device (the attribute is per device)
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return set_error(INTFA_ERR_CUDA, "cannot query the current device");
@@ -240,26 +245,27 @@ int fwd_dispatch(const IntfaFwdParams* a, cudaStream_t stream) {
   kp.num_tiles = (int)((long long)a->B * a->H * kp.MB);   // fits: intfa_fwd() has checked it
   const bool full = a->variant == INTFA_VARIANT_FULL;
   const bool f8v = a->variant == INTFA_VARIANT_HALF_FP8;
-  const bool rne = full && a->p_round == 1;
+  const bool rne = full && a->p_round == 1, wrap = full && !rne && kp.c < 0.f;
   const int D = a->D, G = a->G;
   // Sequence lengths that are not multiples of the tile sizes run the instantiation that masks the last tiles
   // (so do calls with one v_scale row per KV tile: the code for them is compiled into that instantiation only)
   const bool ragged = (a->Nq % kBM) != 0 || (a->Nk % a->G) != 0 || a->vs_stride_blk != 0;
   // HD: head dim of the call; DD, DQ: the kernel's tile width and Q/K width for it; HALF: half-int8 built for this G
-  // (full-int8, head dim 128, non-causal: an instantiation whose service warps poll less, see the kernel)
-  if (D == 128 && G == 128 && full && !rne && !ragged && !kp.causal) return launch_pipe<128, 128, true, false, false, 128, false, true>(a, kp, stream);
+  // (full-int8, head dim 128, non-causal: an instantiation that takes the running max over earlier, see the kernel)
+  if (D == 128 && G == 128 && full && !rne && !wrap && !ragged && !kp.causal) return launch_pipe<128, 128, true, P_TRITON, false, 128, false, true>(a, kp, stream);
 #define INTFA_CASE(HD, DD, GG, DQ, HALF)                                                                 \
   if (D == HD && G == GG) {                                                                              \
-    if (full && ragged) return rne ? launch_pipe<DD, GG, true, true, true, DQ>(a, kp, stream)            \
-                                   : launch_pipe<DD, GG, true, false, true, DQ>(a, kp, stream);          \
-    if (full) return rne ? launch_pipe<DD, GG, true, true, false, DQ>(a, kp, stream)                     \
-                         : launch_pipe<DD, GG, true, false, false, DQ>(a, kp, stream);                   \
+    if (wrap) return launch_pipe<DD, GG, true, P_TRITON_WRAP, true, DQ>(a, kp, stream);                  \
+    if (full && ragged) return rne ? launch_pipe<DD, GG, true, P_RNE, true, DQ>(a, kp, stream)           \
+                                   : launch_pipe<DD, GG, true, P_TRITON, true, DQ>(a, kp, stream);       \
+    if (full) return rne ? launch_pipe<DD, GG, true, P_RNE, false, DQ>(a, kp, stream)                    \
+                         : launch_pipe<DD, GG, true, P_TRITON, false, DQ>(a, kp, stream);                \
     if constexpr (HALF) {                                                                                \
       constexpr int DH = DQ;       /* (half-int8 takes all channels in one pass) */                      \
-      if (f8v) return ragged ? launch_pipe<DH, GG, false, false, true, DH, true>(a, kp, stream)          \
-                             : launch_pipe<DH, GG, false, false, false, DH, true>(a, kp, stream);        \
-      return ragged ? launch_pipe<DH, GG, false, false, true, DH>(a, kp, stream)                         \
-                    : launch_pipe<DH, GG, false, false, false, DH>(a, kp, stream);                       \
+      if (f8v) return ragged ? launch_pipe<DH, GG, false, P_TRITON, true, DH, true>(a, kp, stream)       \
+                             : launch_pipe<DH, GG, false, P_TRITON, false, DH, true>(a, kp, stream);     \
+      return ragged ? launch_pipe<DH, GG, false, P_TRITON, true, DH>(a, kp, stream)                      \
+                    : launch_pipe<DH, GG, false, P_TRITON, false, DH>(a, kp, stream);                    \
     }                                                                                                    \
   }
   INTFA_CASE(128, 128, 128, 128, true)

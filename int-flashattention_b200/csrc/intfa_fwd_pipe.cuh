@@ -173,8 +173,9 @@ enum PipeWait { PW_TILE = 32, PW_QE, PW_KE, PW_VE, PW_QF, PW_QKRDY, PW_PVRDY, PW
 
 // RAGGED: Nq / Nk are not multiples of 128 / G -- the last query tile and the last KV step are partial.  A separate
 // instantiation, so that the code of the common case stays as small as it was (instruction cache).
+// PROUND: how full-int8 rounds P (see PRound).
 // STEADY: non-causal full-int8 with three groups, whose groups take the running max over before pass A (see the softmax warps).
-template <int D, int G, bool FULL, bool PRNE, bool RAGGED, int DQ = D, bool F8V = false, bool STEADY = false>
+template <int D, int G, bool FULL, int PROUND, bool RAGGED, int DQ = D, bool F8V = false, bool STEADY = false>
 __global__ void __launch_bounds__((PipeCfg<D, G, FULL, DQ, F8V>::THREADS), 1)
 intfa_fwd_pipe_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                       const __grid_constant__ CUtensorMap tmV, const KParams p) {

@@ -1,0 +1,39 @@
+"""GPU: sm_scale below zero.  The running maximum is that of the scores times sm_scale, as in the reference
+(flash_atten_full_int8.py:45), so P can exceed 1; the bytes that full-int8 makes of it wrap, each by itself."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+CASES = [
+    # D, G, Nq, Nk, causal (the last rows of the sequence), kv_order
+    (16, 32, 130, 200, False, "ascending"),
+    (32, 32, 200, 300, True, "ascending"),
+    (32, 64, 128, 256, False, "descending"),
+    (32, 128, 128, 384, True, "ascending"),
+    (64, 64, 256, 256, False, "ascending"),
+    (64, 128, 100, 300, False, "descending"),
+    (64, 64, 3, 500, False, "ascending"),                     # few rows
+    (128, 64, 100, 256, True, "ascending"),
+    (128, 128, 256, 384, False, "ascending"),
+    (128, 128, 128, 384, True, "ascending"),
+    (256, 64, 128, 300, False, "ascending"),
+    (256, 128, 128, 384, True, "ascending"),
+]
+
+
+@pytest.mark.parametrize("D,G,Nq,Nk,causal,kv_order", CASES)
+def test_bytes_of_p_wrap_one_by_one(D, G, Nq, Nk, causal, kv_order, pkg, oracle):
+    g = torch.Generator().manual_seed(Nk + D)
+    q, k, v = (torch.randn(1, 2, n, D, generator=g).half() for n in (Nq, Nk, Nk))
+    (q8, qs), (k8, ks), (v8, vs) = oracle.quant_pertoken(q), oracle.quant_pertoken(k), oracle.quant_perchannel(v)
+    sm, off = -0.28 * D ** -0.5, (Nk - Nq if causal else 0)
+    ref = oracle.attention_full_int8(q8, k8, v8, qs, ks, vs, causal, sm, G=G, kv_order=kv_order, q_offset=off)
+    out = pkg.attention_full_int8(*(t.cuda() for t in (q8, k8, v8, qs.float(), ks.float(), vs.float())), causal, sm, G=G,
+                                  kv_order=kv_order, q_offset=off).cpu()
+    pkg.check_status()
+    # P stays below 16 here.  One fp16 rounding where the oracle has two makes 7e-5 of the result, the output's rounding 3e-4; a last
+    # bit of exp2 that takes one P in a hundred thousand across the end of the bytes, by 256, up to 1e-2.  A carry from one byte into
+    # the next, planted in the oracle, makes 5.9e-2 to 1.5e-1 in these cases.
+    err = ((out.float() - ref.float()).norm() / ref.float().norm()).item()
+    assert err < 1.5e-2, err
