@@ -349,8 +349,9 @@ __device__ __forceinline__ void v_slab(const __half* __restrict__ x, long long s
 // CTAs of a cluster at most (16 hold longer slabs, but wait for one another longer: 128 slabs of 2048 x 128 24.9 -> 27.9 us, 256 of
 // 2048 x 64 22.4 -> 37.4)
 constexpr int kSlabCluster = 8;
+__host__ __device__ constexpr int slab_ctas_per_sm(int U) { return U == 16 ? 3 : U == 4 ? 6 : 4; }
 template <int D, int U>
-__global__ void __launch_bounds__(256, U == 16 ? 3 : U == 8 ? 4 : 6) v_slab_kernel(const __half* __restrict__ x, long long sB, long long sH, long long sN,
+__global__ void __launch_bounds__(256, slab_ctas_per_sm(U)) v_slab_kernel(const __half* __restrict__ x, long long sB, long long sH, long long sN,
                                                      int8_t* __restrict__ x8, float* __restrict__ scale, int per_channel, int H, int N,
                                                      int rows_per_cta, int early) {
   v_slab<D, U>(x, sB, sH, sN, x8, scale, per_channel, H, N, rows_per_cta, blockIdx.x / cluster_size(), early);
@@ -532,27 +533,45 @@ static int v_grid(int BH, int N, int sms, int* rows_per_cta) {
 }
 
 // V in one pass (v_slab): where the registers of a cluster hold a (batch, head), that is up to 262144/D rows.  rows_per_cta: equal
-// chunks over as many CTAs as have 4 loads a thread to make; U of them rounded up to what is compiled.  Two passes before -> now,
-// quantise V alone: 4 heads of 512 x 64 11.9 -> 7.9 us, 128 x 1024 x 64 10.6 -> 9.1, 256 x 2048 x 64 30.2 -> 22.4, 256 x 4096 x 64
-// 58.9 -> 49.3, 2048 x 64 x 128 20.9 -> 10.1; 128 x 2048 x 128 with nothing in L2 28 -> 25, out of L2 23.6 -> 24.9.
+// chunks over as many CTAs as have 4 loads a thread to make; U of them rounded up to what is compiled.  (A CTA takes registers for U
+// loads: rounded up to 16, 9 and 10 of them left three CTAs an SM where 10 leave four, 128 heads of 1152 x 128 18.9 -> 14.4 us, 222 of
+// 2049 x 64 29.5 -> 22.8.)  Two passes before -> now, quantise V alone: 4 heads of 512 x 64 11.9 -> 7.9 us, 128 x 1024 x 64 10.6 -> 9.1,
+// 256 x 2048 x 64 30.2 -> 22.4, 256 x 4096 x 64 58.9 -> 49.3, 2048 x 64 x 128 20.9 -> 10.1.
+// Two passes stay where they are the faster ones.  Their second one reads V out of L2, so that is where there are several waves of
+// clusters, which wait for one another within themselves (256 channels, `in_qkv` even at the best fill: there Q and K fill up the first
+// pass), and more so where a part of the loads is padding; and single heads of the narrowest rows, for which 8 CTAs are few.  One pass:
+//   512 heads of 256 x 256 29.8 -> 30.4 us; 222 of 513 x 128 15.7 -> 16.6, 512 of 1025 x 64 37.9 -> 38.9 (29.7 -> 38.9
+//   with V in L2), 300 of 257 x 256 20.0 -> 23.6; 1 of 16384 x 16 4.3 -> 5.0
+//   in_qkv: 512 x 256 x 256 55.4 -> 61.2; 512 x 512 x 128 56.1 -> 58.3; 300 x 768 x 128 49.6 -> 51.0; 300 x 1025 x 64 34.8 -> 37.9
+// One side is left where the two differ: V alone, several waves, 50 MB and more.  Out of L2 one pass is faster (128 x 2048 x 128 28 ->
+// 25 us, 512 x 512 x 128 29.8 -> 27.3), with V in L2 slower (23.6 -> 24.9, 23.3 -> 26.3); the call cannot know, and after Q and K of the
+// same size V is in L2 no more.
 struct Slab {
   int cluster = 0, rows_per_cta = 0, U = 0;
 };
-static Slab slab_plan(int N, int D) {
+static Slab slab_plan(int N, int D, long long heads, int sms, bool in_qkv) {
   Slab s;
   const int rpc = 256 / (D / 8);                        // rows of one load
   if (N > kSlabCluster * 16 * rpc) return s;
-  s.cluster = (N + 4 * rpc - 1) / (4 * rpc);
-  if (s.cluster > kSlabCluster) s.cluster = kSlabCluster;
-  s.rows_per_cta = (N + s.cluster - 1) / s.cluster;
+  int cluster = (N + 4 * rpc - 1) / (4 * rpc);
+  if (cluster > kSlabCluster) cluster = kSlabCluster;
+  s.rows_per_cta = (N + cluster - 1) / cluster;
   const int loads = (s.rows_per_cta + rpc - 1) / rpc;
-  s.U = loads <= 4 ? 4 : loads <= 8 ? 8 : 16;
+  s.U = loads <= 4 ? 4 : loads <= 8 ? 8 : loads <= 10 ? 10 : 16;
+  const double waves = (double)heads * cluster / ((double)sms * slab_ctas_per_sm(s.U));
+  const bool padded = loads == 5;
+  const bool two = in_qkv ? (D == 256 && waves > 1.75) || (D == 128 && ((s.U == 4 && waves > 1.6) || (s.U == 8 && loads < 8 && waves > 3.5))) ||
+                                (padded && waves > 2.5)
+                          : (D == 256 && s.U == 4 && cluster > 4 && waves > 2.8) || (padded && waves > (D >= 128 ? 2.5 : 3.5)) ||
+                                (D <= 32 && loads > 13 && heads <= 4);
+  if (!two) s.cluster = cluster;
   return s;
 }
 #define INTFA_U_SWITCH(U, CALL)                       \
   switch (U) {                                        \
     case 4: { constexpr int UU = 4; CALL; } break;    \
     case 8: { constexpr int UU = 8; CALL; } break;    \
+    case 10: { constexpr int UU = 10; CALL; } break;  \
     default: { constexpr int UU = 16; CALL; } break;  \
   }
 static int v_slab_launch(const Slab& sl, const void* v, const int64_t* st, void* v8, float* scale, int mode, int B, int H, int N, int D,
@@ -624,7 +643,7 @@ int quant_qkv(const void* q, const void* k, const void* v, const int64_t* v_st, 
   j.chunks = 0; j.rows_per_cta = 0; j.vB = j.vH = j.vN = 0;
   int gv = 0;
   if (v) {
-    const Slab sl = slab_plan(Nk, D);
+    const Slab sl = slab_plan(Nk, D, (long long)B * Hkv, sms, true);
     if (sl.cluster > 0) {
       int rc = INTFA_OK;
       const int slabs = sl.cluster * B * Hkv;
@@ -654,7 +673,7 @@ int quant_v_partial(const void* v, const int64_t* st, void* v8, float* scale, in
                     cudaStream_t stream) {
   const int sms = sm_count_cached();
   if (sms <= 0) return set_error(INTFA_ERR_CUDA, "cannot query SM count");
-  const Slab sl = slab_plan(N, D);
+  const Slab sl = slab_plan(N, D, (long long)B * H, sms, false);
   if (sl.cluster > 0) return v_slab_launch(sl, v, st, v8, scale, mode, B, H, N, D, false, stream);
   int rows_per_cta;
   const int chunks = v_grid(B * H, N, sms, &rows_per_cta);
