@@ -420,7 +420,9 @@ struct PvFull {
 // full-int8, second pass: P from the kept scores, O = P V.  Bound by reading V.
 // ---------------------------------------------------------------------------------------------------------------
 template <int D, int NT>
-__global__ void __launch_bounds__(kThreads, NT == 1 ? 3 : 2) pv_full_kernel(const DParams p) {
+constexpr int pv_full_ctas() { return NT == 1 ? (D == 64 ? 4 : 3) : 2; }   // of an SM
+template <int D, int NT>
+__global__ void __launch_bounds__(kThreads, (pv_full_ctas<D, NT>())) pv_full_kernel(const DParams p) {
   constexpr int RT = 8 * NT;
   __shared__ __align__(16) float red[kWarps * RT * (D + 4)];
   __shared__ __align__(16) float mg[kMaxLocalUnits * RT];   // running maximum (scaled) at the group of each 64-key unit of this CTA
@@ -1004,9 +1006,11 @@ Plan make_plan(const IntfaFwdParams* a, int sms) {
   if (units > (1 << 22)) return pl;
   pl.units = pl.slice = (int)units;
   pl.groups = (pl.nvis + a->G - 1) / a->G;
-  // Splits: one wave of resident CTAs, as the kernels' launch bounds have it (two CTAs an SM or four for full-int8 at 8 rows:
-  // 35 -> 44 us at batch 16, 4097 keys; three for half-int8 at 128 channels: 26.5 -> 30 us at 32768 keys)
-  const int wave = sms * (pl.NT == 1 && (pl.full || a->D == 64) ? 3 : 2);
+  // Splits: one wave of resident CTAs, as the kernels' launch bounds have it (full-int8 at 8 rows and 128 channels: two CTAs an SM or
+  // four 35 -> 44 us at batch 16, 4097 keys; at 64 channels four, planned for three 264 heads of 6000 keys 65.8, for four 50.0; half-int8
+  // at 128 channels: three 26.5 -> 30 us at 32768 keys)
+  const int wave = sms * (pl.full ? (pl.NT == 2 ? pv_full_ctas<64, 2>() : a->D == 64 ? pv_full_ctas<64, 1>() : pv_full_ctas<128, 1>())
+                                  : pl.NT == 1 && a->D == 64 ? 3 : 2);
   const int key_units = (pl.nvis + 63) / 64;
   size_t per_unit_scores = 0, per_unit_max = 0;
   if (pl.full) {
@@ -1049,6 +1053,7 @@ Plan make_plan(const IntfaFwdParams* a, int sms) {
   // keys a CTA 34.8 -> 37.2).
   if (pl.full) {
     const int max_keys = (pl.NT == 1 ? FusedCfg<128, 1>::MAX_SCORES : FusedCfg<128, 2>::MAX_SCORES) / (pl.NT * 32);
+    const int wave = sms * (pl.NT == 1 ? 3 : 2);
     int n = wave / (int)units < 1 ? 1 : wave / (int)units;
     per = (items + n - 1) / n;
     if (per < per_min) per = per_min;
