@@ -85,6 +85,10 @@ template <bool B>
 struct Const {
   static constexpr bool value = B;
 };
+template <int N>
+struct Int {
+  static constexpr int value = N;
+};
 // one (batch, K/V head, row tile)
 struct Unit {
   int id, b, hk, tile;                    // id: counted from the launch's first, as scratch is
@@ -503,10 +507,18 @@ __global__ void __launch_bounds__(kThreads, (pv_full_ctas<D, NT>())) pv_full_ker
 template <int D, int NT>
 struct FusedCfg {
   static constexpr int RT = 8 * NT;
-  // shared memory of one CTA for scores, so that three CTAs (16 rows: two) fit an SM, as the launch bounds have it
-  static constexpr int MAX_SCORES = NT == 1 ? 66 << 10 : 100 << 10;
+  // Scores of a CTA in bytes.  The CTAs of an SM must not need more than 196 KB of its shared memory: the next larger setting, 228 KB,
+  // leaves 28 KB of L1, through which the loads in flight go (12 K/V heads of 128 channels, 8118 keys: 1984 keys a CTA 59 us, three
+  // kernels 42; every call takes half as long again with that setting).  Three CTAs an SM, 60 KB each beside their static 4 KB.
+  static constexpr int MAX_SCORES = NT == 1 ? 60 << 10 : 100 << 10;
   static constexpr int RED_BYTES = kWarps * RT * (D + 4) * 4;
-  static int score_bytes(int keys) { return keys * NT * 32; }
+  // Dynamic shared memory of a CTA.  At 64 channels the registers leave room for four an SM: where those would need the 228 KB
+  // setting the size is rounded up to one of which three fit (320 heads of 1367 keys 28.3 -> 20.2 us, 400 of 4097 73 -> 61).
+  static int smem_bytes(int keys) {
+    const int b = keys * NT * 32;
+    if (D == 64 && NT == 1 && b > (43 << 10) && b < (52 << 10)) return 52 << 10;
+    return b < RED_BYTES ? RED_BYTES : b;
+  }
 };
 template <int D, int NT>
 __global__ void __launch_bounds__(kThreads, NT == 1 ? 3 : 2) fused_full_kernel(const DParams p) {
@@ -981,6 +993,90 @@ bool faster_than_tiles(const IntfaFwdParams* a, const Plan& pl, int wave, int sm
   return here < t.fill + t.step * (rounds > 1 ? rounds * mean : steps) + t.next * (rounds - 1);
 }
 
+// Clusters of n CTAs of fused_full_kernel that the current device holds at once; 0: none, or it cannot be asked.  Not SMs * CTAs an SM / n:
+// a cluster stays within a group of SMs, which n need not divide (three CTAs an SM, n = 3 to 8: 426, 416, 410, 426, 392, 384 CTAs of
+// 444).  Asked once per device, kernel and n, for CTAs of up to 40 KB and for the largest.
+template <int D, int NT>
+int fused_places_of(int n, int smem) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(n);
+  cfg.blockDim = dim3(kThreads);
+  cfg.dynamicSmemBytes = smem;
+  cudaLaunchAttribute attr = {};
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = (unsigned)n;
+  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  int clusters = 0;
+  if (cudaFuncSetAttribute(fused_full_kernel<D, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, FusedCfg<D, NT>::MAX_SCORES) != cudaSuccess ||
+      cudaOccupancyMaxActiveClusters(&clusters, fused_full_kernel<D, NT>, &cfg) != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
+  return clusters;
+}
+int fused_places(int D, int NT, int n, int keys) {
+  static std::atomic<int> cache[64][2][2][kMaxCluster + 1][2];           // number + 1; 0: not asked yet
+  constexpr int kSmall = 40 << 10;
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
+  const int large = keys * NT * 32 > kSmall;
+  std::atomic<int>& c = cache[dev][D == 128][NT - 1][n][large];
+  int v = c.load(std::memory_order_relaxed);
+  if (v == 0) {
+    auto ask = [&](auto d, auto nt) {
+      using F = FusedCfg<decltype(d)::value, decltype(nt)::value>;
+      return fused_places_of<decltype(d)::value, decltype(nt)::value>(n, large ? F::MAX_SCORES : kSmall);
+    };
+    v = 1 + (D == 128 ? (NT == 2 ? ask(Int<128>(), Int<2>()) : ask(Int<128>(), Int<1>()))
+                      : (NT == 2 ? ask(Int<64>(), Int<2>()) : ask(Int<64>(), Int<1>())));
+    c.store(v, std::memory_order_relaxed);
+  }
+  return v - 1;
+}
+
+// Is fused_full_kernel with clusters of n CTAs and `keys` keys a CTA faster than the three kernels of `pl`?  `wave`: the CTAs it is
+// laid out for, `wave3`: the resident ones of pv_full_kernel; `fewest`: no CTA has more keys than a split is given at least.  Fitted to
+// 1 893 calls timed on both, inputs in and out of L2 (1 to 16 rows a head, 6 to 15 164 keys, 1 to 4 448 units).  Of these it takes 1 174:
+// 8 % faster at the median, 5 of them slower by more than 4 %.  Of the others most would be slower, by up to 83 %; 55 would be faster by
+// more than 5 %, chiefly some with 16 rows.
+bool fused_is_faster(int D, const Plan& pl, int n, int keys, int wave, int wave3, bool fewest) {
+  const int places = fused_places(D, pl.NT, n, keys);
+  if (places <= 0) return false;
+  const long long ctas = (long long)pl.units * n;
+  auto full = [](long long have, long long of, int percent) { return have * 100 >= of * percent; };
+  if (pl.units <= places) {              // one wave
+    // 128 channels, more than 256 keys a CTA: a warp has more than one unit in each pass, which few CTAs do not make up for (two units
+    // of 443 keys 6.7 -> 7.1 us; 16 rows, 8 units of 501 keys 9.7 -> 10.5)
+    const bool chain = D == 128 && keys > 256;
+    // 16 rows, 8 warps an SM to read with: where a CTA has the fewest keys (2 x 2048 keys, 8 rows a head 15.0 -> 14.0; 1 500 keys a
+    // CTA 34.8 -> 37.2)
+    if (pl.NT == 2) return fewest && !(chain && (ctas < 24 || (n <= 2 && ctas <= 60)));
+    // Many keys in fewer CTAs than there is room for do not keep the memory busy, while the scores' kernel fills the chip with any
+    // number of units: 64 channels, 112 units of 3260 keys 18.8 -> 20.1, 108 of 2960 17.4 -> 15.2, 224 of 1490 17.2 -> 19.6; 128
+    // channels, 244 of 1610 28.0 -> 32.8, 429 of 1720 40.4 -> 37.1
+    if (D == 64) return n == 1 ? keys <= 1408 || full(ctas, wave, 60) : keys <= 768 || keys >= 1408 || full(ctas, wave, n == 2 ? 80 : 91);
+    if (chain && (n > 1 ? pl.units == 1 : pl.units < 36)) return false;
+    if (n == 1) return full(ctas, wave, 85) || keys <= 512 || (keys <= 1280 && full(ctas, wave, 55));
+    return keys <= 1536;                 // (more leave less L1: 132 units of 4809 keys 35.7 -> 36.8)
+  }
+  if (pl.NT == 2) return false;          // (248 units of 1636 keys 36.0 -> 43.2)
+  // Several waves: where the last one is nearly full, and the three kernels are not well off with one or two
+  const int slices = (pl.units + pl.slice - 1) / pl.slice;
+  const long long ctas3 = (long long)pl.slice * pl.splits, waves3 = (ctas3 + wave3 - 1) / wave3;
+  const long long waves = (pl.units + places - 1) / places, waves_up = (ctas + wave - 1) / wave;
+  if (n > 3) return false;                                               // (72 units of 9216 keys 24.5 -> 37.0)
+  if (n > 1 && slices == 1 && waves3 == 1 && full(ctas3, wave3, D == 64 ? 55 : 70)) return false;     // (144 units of 4980 keys 38.9 -> 58.1)
+  if (D == 64) {
+    if (n == 1 && keys <= 1280) return true;                             // (560 units of 701 keys 19.7 -> 14.3)
+    if (slices == 1 && waves3 == 2 && full(ctas3, 2 * wave3, 93)) return false;                       // (1 184 units of 1304 keys 48.2 -> 54.4)
+    return full(pl.units, waves * places, 83) || full(ctas, waves_up * wave, 83);
+  }
+  if (keys <= 64 && waves > 2) return false;                             // (one warp of four works: 2 499 units of 61 keys 33.5 -> 35.6)
+  return full(pl.units, waves * places, waves > 3 ? 80 : 83);            // (512 units of 4097 keys 135 -> 115, 556 of 984 36.9 -> 38.5)
+}
+
 Plan make_plan(const IntfaFwdParams* a, int sms) {
   Plan pl;
   const int Hkv = a->H_kv > 0 ? a->H_kv : a->H;
@@ -1046,26 +1142,21 @@ Plan make_plan(const IntfaFwdParams* a, int sms) {
   if ((long long)pl.slice * pl.splits > 0x7fffffffLL || (long long)pl.slice * pl.score_splits > 0x7fffffffLL) return pl;
   if (!faster_than_tiles(a, pl, wave, sms)) return pl;
   // One kernel (fused_full_kernel) where the splits of a unit make a cluster whose CTAs hold their scores, if need be more of them than
-  // fill one wave.  No scratch to speak of, so nothing is cut into slices.  Only where the CTAs fit one wave or fill several well
-  // (three kernels -> one, 8 K/V heads of 128 channels, one row of 32 heads: 16 x 4097 keys 34.8 -> 31.7 us, 8 x 2048 16.6 -> 15.3, 1 x
-  // 4096 12.1 -> 9.9, 64 x 4097 136 -> 115; 512 CTAs on 444 places 46 -> 50, clusters of 5 in 4.3 waves 220 -> 267), and with tiles of
-  // 16 rows, which leave 8 warps an SM to read with, where a CTA has the fewest keys (2 x 2048 keys, 8 rows a head 15.0 -> 14.0; 1 500
-  // keys a CTA 34.8 -> 37.2).
+  // fill one wave.  No scratch to speak of, so nothing is cut into slices.
   if (pl.full) {
     const int max_keys = (pl.NT == 1 ? FusedCfg<128, 1>::MAX_SCORES : FusedCfg<128, 2>::MAX_SCORES) / (pl.NT * 32);
-    const int wave = sms * (pl.NT == 1 ? 3 : 2);
-    int n = wave / (int)units < 1 ? 1 : wave / (int)units;
+    const int fill = sms * (pl.NT == 1 ? 3 : 2);              // CTAs to share the work out to
+    int n = fill / (int)units < 1 ? 1 : fill / (int)units;
     per = (items + n - 1) / n;
     if (per < per_min) per = per_min;
     if (per > max_keys / a->G) per = max_keys / a->G;
     n = (items + per - 1) / per;
     per = (items + n - 1) / n;
-    const long long ctas = units * n, waves_up = (ctas + wave - 1) / wave;
-    const bool fits = waves_up == 1 || (n <= 3 && ctas * 5 >= waves_up * wave * 4);
-    if (n <= kMaxCluster && (pl.NT == 1 ? fits : waves_up == 1 && per <= per_min)) {
+    n = (items + per - 1) / per;
+    if (n <= kMaxCluster && fused_is_faster(a->D, pl, n, per * a->G, fill, wave, per <= per_min)) {
       pl.fused = true;
       pl.per_split = per;
-      pl.splits = (items + per - 1) / per;
+      pl.splits = n;
       pl.slice = pl.units;
     }
   }
@@ -1105,9 +1196,7 @@ int run_fused(const Plan& pl, const DParams& p, cudaStream_t stream) {
     if (e != cudaSuccess) return set_error(INTFA_ERR_CUDA, "cudaFuncSetAttribute: %s", cudaGetErrorString(e));
     attr_done[dev].store(true, std::memory_order_release);
   }
-  int smem = F::score_bytes(pl.per_split * p.G);
-  if (smem < F::RED_BYTES) smem = F::RED_BYTES;
-  return launch_clusters("decode", fused_full_kernel<D, NT>, pl.units * pl.splits, pl.splits, kThreads, smem, stream, p);
+  return launch_clusters("decode", fused_full_kernel<D, NT>, pl.units * pl.splits, pl.splits, kThreads, F::smem_bytes(pl.per_split * p.G), stream, p);
 }
 template <int D, int NT>
 int run_slice(const Plan& pl, int units, const DParams& p, cudaStream_t stream) {
