@@ -98,14 +98,15 @@ struct PipeCfg {
   // instructions of never-executed filler between the softmax passes (see intfa_fwd_pipe_softmax.inc), the best of a sweep in
   // steps of 1 KB for each kind of instantiation (`ragged`: masks partial tiles; `steady`: see the kernel).  With three groups of
   // 128-column steps the sweep changes 1 to 3 % (steady 4157 to 4189 us but for 4361 at 256; causal 315 to 338); with 64-column steps and
-  // at head dim 256 it changes up to 20 % (half-int8 causal at d=128 406 to 520 us, at d=256 245 to 287).
+  // at head dim 256 it changes up to 20 % (half-int8 causal at d=128 406 to 520 us, at d=256 245 to 287; full-int8 there, 64-column
+  // steps of ragged lengths, 16 heads of 4001 498 to 549 us, causal 330 to 382).
   __host__ __device__ static constexpr int code_filler_of(bool ragged, bool steady) {
     if (P_TMEM) {
       if (G == 128) return ragged || D == 128 ? 64 : 192;
       return D == 256 ? (ragged ? 384 : 0) : !ragged ? 384 : D == 128 ? 256 : 128;
     }
     if (F8V) return 192;
-    if (DQ == 256) return ragged ? 384 : 0;
+    if (DQ == 256) return ragged ? (G == 64 ? 208 : 384) : 0;
     if (ragged) return G == 32 ? 384 : G == 128 ? 256 : D == 128 ? 0 : 128;
     return G < 128 ? 256 : steady ? 128 : 64;
   }

@@ -12,7 +12,7 @@ CASES = [
     (32, 64, 128, 256, False, "descending"),
     (32, 128, 128, 384, True, "ascending"),
     (64, 64, 256, 256, False, "ascending"),
-    (64, 128, 100, 300, False, "descending"),
+    (64, 128, 100, 384, False, "descending"),
     (64, 64, 3, 500, False, "ascending"),                     # few rows
     (128, 64, 100, 256, True, "ascending"),
     (128, 128, 256, 384, False, "ascending"),
