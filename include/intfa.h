@@ -108,9 +108,9 @@ typedef struct IntfaFwdParams {
                                    path's layout (csrc/flash_fwd_kernel_full_qi8.h:156-160,348,399,
                                    csrc/mask.h:313-340); this is the element stride of the tile axis. */
   /* Test hooks for the bounded device-side waits (both 0 in normal use).  debug_wait_limit_kcycles: give up a wait
-     after this many thousand SM cycles instead of about a second.  debug_skip_k_load = n > 0: the producer leaves
-     out the K tile of the n-th KV step the CTA runs, so the wait for it runs out, the CTA drains and `status`
-     receives the wait's code -- the path a lost transfer would take. */
+     after this many thousand SM cycles instead of about a second (2^21 of them, which larger numbers count as).
+     debug_skip_k_load = n > 0: the producer leaves out the K tile of the n-th KV step the CTA runs, so the wait for it
+     runs out, the CTA drains and `status` receives the wait's code -- the path a lost transfer would take. */
   int32_t debug_wait_limit_kcycles; int32_t debug_skip_k_load;
   int32_t scale_f16;            /* bit set: that scale tensor is fp16 (as benchmark.py makes them), else fp32.
                                    INTFA_SCALE_F16_Q / _K / _V; the kernel widens in place
@@ -129,8 +129,9 @@ typedef struct IntfaFwdParams {
  */
 int intfa_fwd(const IntfaFwdParams* p, void* stream);
 
-/* Scratch that intfa_fwd() makes use of for these arguments (pointers are not looked at); 0: none.  At most 256 MiB, or
-   72 bytes a key where a single K/V head has so many that it needs more. */
+/* Scratch that intfa_fwd() asks for with these arguments on the current device (pointers are not looked at); 0: none.  256 bytes where
+   it uses none but takes a call without any for one of the unsplit way.  At most 256 MiB, or 72 bytes a key where a single
+   K/V head has so many that it needs more. */
 size_t intfa_fwd_workspace_bytes(const IntfaFwdParams* p);
 
 /*

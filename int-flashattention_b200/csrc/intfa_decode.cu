@@ -18,7 +18,7 @@
 // first group, and from there on does what the one-pass kernel does: m' = max(m, groupmax*c), p = exp2(s*c - m'), P8, O_j
 // (with s*c - m' as one fma on masked groups too, where that kernel rounds s*c first).  The final maximum is known too, so that every partial result is scaled to it at once
 // (acc += exp2(m_j - m_final) * O_j) and the splits add up without weights.  Where the splits of a K/V head fit a cluster of CTAs one
-// kernel does both passes and the sum (`fused_full_kernel`).
+// kernel may do both passes and the sum (`fused_full_kernel`; `fused_is_faster` says where).
 // half-int8: P is fp16, whose rounding is relative: every warp keeps a running maximum of its own and the partial results
 // are combined with their weights (`pv_half_kernel`: scores and P V in one pass over K and V).
 #include <cuda_fp16.h>
@@ -502,7 +502,7 @@ __global__ void __launch_bounds__(kThreads, (pv_full_ctas<D, NT>())) pv_full_ker
 // shared memory; the CTAs exchange their maxima, which gives each the running maximum before its first key and the final one, and then
 // their results, of which every CTA adds up and writes some rows -- both through distributed shared memory.  The scores make no way
 // through L2 (a quarter of the bytes of K at 4 rows a head), there is no scratch, and one launch instead of three.  Bound by reading K
-// and V, 12 warps an SM (make_plan says what it gives and where).
+// and V, 12 warps an SM (fused_is_faster says what it gives and where).
 // ---------------------------------------------------------------------------------------------------------------
 template <int D, int NT>
 struct FusedCfg {
@@ -959,13 +959,15 @@ struct Plan {
 constexpr size_t kMaxScratch = (size_t)256 << 20;
 
 // Which path?  Times in microseconds, fitted to 3 781 calls that were timed on both (1 to 256 rows a head, 50 to 16384 keys, 1 to
-// 512 heads in all; B200):
+// 512 heads in all; B200).  The kernels timed were earlier ones of both paths: the 128-row kernel has become 4 to 32 % faster since,
+// full-int8 here up to 30 % where one kernel does for three, which the model does not know: near the line the slower
+// path may be taken.
 //   here       `fixed` and `combine` for the launches; `unit` per 64 keys of a row tile and SM (times `one_half` for tiles of 8
 //              rows); `wave` for each further wave of CTAs
 //   128 rows   `fill`, then `step` per KV step of G keys and `next` for each further work item of an SM.  The work items of
 //              these calls are of one length, so an SM has a whole number of them.
-// Typical error 5 to 15 %.  Over those calls the choice costs 0.3 % against the better path each time, and 48 of them more
-// than 10 %.  (One step time for any G and head dim, and no term for waves, before: 0.5 %, 72 of 1 610 calls more than 10 %, up
+// Typical error 5 to 15 %.  Over those calls, on those kernels, the choice cost 0.3 % against the better path each time, and 48 of them
+// more than 10 %.  (One step time for any G and head dim, and no term for waves, before: 0.5 %, 72 of 1 610 calls more than 10 %, up
 // to twice the time for half-int8 with 64-column steps.)
 struct FewTimes {
   double fixed, combine, unit, one_half, wave;

@@ -87,9 +87,6 @@ struct PipeCfg {
   // twice.  Where the head is wider than the step (head_dim 128 at G = 64) the accumulator warps are the busier
   // side and the softmax groups keep l, handing it over like the running max (measured: 582 against 474 TOPS).
   static constexpr bool L_IN_ACC = G >= D;
-  // setmaxnreg split between the softmax and the accumulator warps.  The accumulator row of 128 channels fits either
-  // way; with 128-column KV steps, and for half-int8 (no accumulator row in registers), the softmax passes gain more
-  // from 16 further registers than the update loses (measured +2..3 %); full-int8 at G = 64 is the other way round.
   // A vectorised pass A for the causal diagonal band and the last, partial step (otherwise those take the general, scalar
   // path): compiled in for 128-column KV steps, where it measured +2..5 % on causal workloads, and for 32-column steps of
   // ragged lengths (batch 8, 32 heads, 1000 tokens causal at d=32: 273 -> 212 us, 64 x 32 x 250: 327 -> 224).  Elsewhere its
@@ -97,9 +94,10 @@ struct PipeCfg {
   __host__ __device__ static constexpr bool band_fast(bool ragged) { return G == 128 || D == 256 || (G == 32 && ragged); }
   // instructions of never-executed filler between the softmax passes (see intfa_fwd_pipe_softmax.inc), the best of a sweep in
   // steps of 1 KB for each kind of instantiation (`ragged`: masks partial tiles; `steady`: see the kernel).  With three groups of
-  // 128-column steps the sweep changes 1 to 3 % (steady 4157 to 4189 us but for 4361 at 256; causal 315 to 338); with 64-column steps and
-  // at head dim 256 it changes up to 20 % (half-int8 causal at d=128 406 to 520 us, at d=256 245 to 287; full-int8 there, 64-column
-  // steps of ragged lengths, 16 heads of 4001 498 to 549 us, causal 330 to 382).
+  // 128-column steps the sweep changed 1 to 3 % (steady 4157 to 4189 us but for 4361 at 256; causal 315 to 338); with 64-column steps and
+  // at head dim 256 up to 20 % (half-int8 causal at d=128 406 to 520 us, at d=256 245 to 287).  These sweeps are older than the
+  // votes inside the wait loops; of the kernels as they are only full-int8 at head dim 256, 64-column steps of ragged lengths, has been
+  // swept (16 heads of 4001 498 to 549 us, causal 330 to 382).
   __host__ __device__ static constexpr int code_filler_of(bool ragged, bool steady) {
     if (P_TMEM) {
       if (G == 128) return ragged || D == 128 ? 64 : 192;
@@ -110,6 +108,10 @@ struct PipeCfg {
     if (ragged) return G == 32 ? 384 : G == 128 ? 256 : D == 128 ? 0 : 128;
     return G < 128 ? 256 : steady ? 128 : 64;
   }
+  // setmaxnreg split between the softmax and the accumulator warps, two groups.  The accumulator row of 128 channels fits either
+  // way; with 128-column KV steps, and for half-int8 (no accumulator row in registers), the softmax passes gain more
+  // from 16 further registers than the update loses (measured +2..3 %); full-int8 at head dim 256 with 64-column steps is the other
+  // way round.
   static constexpr bool MORE_SOFTMAX_REGS = !FULL || G == 128;
   static constexpr int SOFTMAX_REGS = NGRP == 3 ? (FULL ? 96 : 112) : MORE_SOFTMAX_REGS ? 152 : 136;
   static constexpr int CORR_REGS = NGRP == 3 ? (FULL ? 152 : 96) : MORE_SOFTMAX_REGS ? 168 : 184;
@@ -136,7 +138,7 @@ struct PipeCfg {
   // S buffer b at COL_S + b*G; then O_j (full-int8: the accumulator itself lives in registers) or the fp32
   // accumulator the second MMA adds into (half-int8)
   static constexpr int COL_S = 0, COL_O = NSB * G, COL_ACC = NSB * G;
-  // full-int8: two O_j buffers where TMEM has the room (64-column steps), so that P V of the next step does not wait for
+  // full-int8: two O_j buffers where TMEM has the room (head dim 256, 64-column steps), so that P V of the next step does not wait for
   // the accumulator warps.  (Not with three groups: alpha and the row sums of a step would be overwritten too early.)
   static constexpr int NO = FULL && NGRP == 2 && NSB * G + 2 * D <= 512 ? 2 : 1;
   static_assert(NSB * G + NO * D <= 512, "TMEM columns");

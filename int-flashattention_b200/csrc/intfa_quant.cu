@@ -613,7 +613,7 @@ int v_quant_from_colmax(const void* v, const int64_t* st, const void* colmax, vo
 }
 
 // ---------------------------------------------------------------------------------------------
-// fused prologue: Q, K (per token) and V (per channel / per batch-head) in TWO launches, no memset
+// fused prologue: Q, K (per token) and V (per channel / per batch-head) in one or two launches, no memset
 // ---------------------------------------------------------------------------------------------
 size_t quant_qkv_workspace_bytes(int B, int Hkv, int Nk, int D) {
   const int sms = sm_count_cached();

@@ -101,8 +101,8 @@ def quant_pertoken(X):
 
 def quant_qkv(q, k, v=None, v_mode="per_channel"):
     """The quantisation prologue of one attention call in one or two launches (one when v is None): per-token q and k
-    (benchmark.py:96-100) and, in the same grid, the column absmax of v; then the v quantisation (benchmark.py:102-107
-    or its per-channel form).  Bit-identical to quant_pertoken / quant_perchannel / quant_pertensor called one by one.
+    (benchmark.py:96-100), and v (benchmark.py:102-107 or its per-channel form) with them, or after them where the call is
+    larger; where v takes two passes the first, its column absmax, is in the grid of q and k.  Bit-identical to quant_pertoken / quant_perchannel / quant_pertensor called one by one.
     Returns (q8, q_scale, k8, k_scale) and, with v, (v8, v_scale) appended."""
     return (_native_mod or _native()).quant_qkv(q, k, v, _lib.VSCALE_PER_CHANNEL if v_mode == "per_channel" else _lib.VSCALE_PER_TENSOR)
 
