@@ -1076,7 +1076,8 @@ bool fused_is_faster(int D, const Plan& pl, int n, int keys, int wave, int wave3
     return full(pl.units, waves * places, 83) || full(ctas, waves_up * wave, 83);
   }
   if (keys <= 64 && waves > 2) return false;                             // (one warp of four works: 2 499 units of 61 keys 33.5 -> 35.6)
-  return full(pl.units, waves * places, waves > 3 ? 80 : 83);            // (512 units of 4097 keys 135 -> 115, 556 of 984 36.9 -> 38.5)
+  // (512 units of 4097 keys 135 -> 115, 1 104 of 1711 108 -> 102, 556 of 984 36.9 -> 38.5)
+  return full(pl.units, waves * places, waves > 2 ? 80 : 83);
 }
 
 Plan make_plan(const IntfaFwdParams* a, int sms) {
